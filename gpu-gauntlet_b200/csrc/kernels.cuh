@@ -2,7 +2,7 @@
 //
 //   ke_kernel          element stiffness, FP64 (and an FP32 copy), per element
 //   binv_kernel        3x3 block diagonal, constrained rule, FP64 inversion
-//   task_ke_kernel     the per-task 3 x 3npe blocks the PCG kernels read
+//   row_fill_kernel    the assembled row blocks the PCG kernels read (rows.cuh)
 //   applyk_*_kernel    y = K x colour by colour (test hook, reference layout;
 //                      also the FP64 K x of the set-up and correction steps)
 //   power_start_kernel, binv_apply_kernel
@@ -34,6 +34,7 @@
 #include <cstdint>
 
 #include "element.cuh"
+#include "rows.cuh"
 
 namespace pg {
 
@@ -57,39 +58,53 @@ struct PcgResult {
 // Byte offsets of the shared-memory arrays of one block (computed on the
 // host from the plan's maxima; T is the inner vector type).
 struct SmemLayout {
-    int r, u, p, s, w, B, yt, kt;  // T
+    int r, u, p, s, w, B, yt, kt;  // T (yt: the load-case kernel's row products)
+    int t;                         // T: D^-1 r on every local node (Chebyshev smoother)
     int x, xl, ytd, red, scal, sp;  // double
     int qw, cs, cv;                 // double, per coarse row of the part: A_c^-1 P^T w,
                                     // A_c^-1 P^T s and c = A_c^-1 P^T r (two copies of cs, cv)
     int ctl;                        // int[4]: decision broadcast
-    int clk;                        // long long[8]: phase timers
+    int dec;                        // Decision
+    int clk;                        // long long[9]: phase timers
     int nb, ainv;                   // T: per-node basis data, A_c^-1 rows
     int nslot;                      // int
-    int gid, tptr;                 // int
-    int tnode;                     // uint16
+    int gid;                       // int
+    int gq, go;                    // int: the row groups' q-step offsets, staged offsets
+    int rcol;                      // uint16: columns of the row blocks
     int cm;                        // uint8
+    int kq;                        // q-steps of row blocks the kt area holds
     int total;
 };
 
-// Copies of every block's partial sums in the exchange buffer: each block
-// reads one copy, which spreads the pollers of a slot line over kRep lines.
+// Copies of every block's partial sums in the exchange buffer: block g reads
+// copy g mod the number of copies.  More copies mean fewer readers polling
+// one line, but more stores; each block writes lines of its own (128 bytes a
+// copy: with several blocks' values in one line every store meets the
+// others' pollers).  Measured on the 60k-DOF plate (148 blocks, us per
+// iteration): block Jacobi (the dot products only) 3.79 / 3.55 / 3.41 / 3.50 /
+// 3.84 / 4.83 with 1 / 2 / 4 / 8 / 16 / 32 copies; mixed two-level Chebyshev,
+// whose blocks also read 444 coarse values, 8.23 / 7.53 / 7.08 / 6.70 / 7.10 /
+// 9.30.  Lines shared by 8 blocks: 3.84 and 7.74 (8 copies); coarse values in
+// lines apart from the dot products': 6.88.
 constexpr int kRep = 8;
+__host__ __device__ constexpr int dot_copies(bool coarse) { return coarse ? kRep : 4; }
 
 struct PcgArgs {
-    int G, NT, Nn;
-    int npe;                     // 3 (DKT) or 4 (Q4): the batch kernel's dispatch
+    int G, Nn;
     const int* node_off;
     const int* nown;
     const int* nodes;
-    const int* task_off;
-    const int* tp_off;
-    const int* tptr;
-    const uint16_t* task_nodes;  // [NT][npe] -> staged [npe][part tasks]
-    const double* kt64;          // [3*nd][NT] task blocks, FP64
-    const float* kt32;           // [3*nd][NT] task blocks, FP32
+    // row blocks (see row_matvec): group offsets of each part, q-step
+    // offsets of each group, columns and blocks of each q-step
+    const int* grp_off;          // [G+1]
+    const int* grp_q;            // [groups+1]
+    const uint16_t* rcol;        // [q-steps][30]
+    const double* rk64;          // [q-steps][9][30]
+    const float* rk32;
     const double* binv64;        // [Nn][9]
     const float* binv32;         // [Nn][9]
     const uint8_t* cons;         // [3Nn]
+    const uint8_t* shared;       // [Nn] 1: a ghost of some part
     const float* F;              // [3Nn]
     double* x;                   // [3Nn]
     unsigned long long* llv;     // [2][3Nn][2] tagged w / r values of the owners
@@ -104,7 +119,6 @@ struct PcgArgs {
     // older tags from earlier launches of the plan, which never match
     unsigned tag0;
     unsigned long long timeout_ns;
-    int ke_smem;                 // Ke blocks in shared memory: 0 none, 1 owned tasks, 2 all
     int timing;
     int test_stall;  // test hook: block 0 waits once for a tag nobody writes
     // two-level preconditioner (coarse = 1): u = M_bj r + P A_c^-1 P^T r
@@ -481,9 +495,8 @@ __device__ __forceinline__ double warp_reduce_scatter(double (&v)[KM]) {
 }
 
 // Block-wide totals of the first K (<= KM) of the KM values v, published
-// as this block's partial sums: copy r < kRep goes to slots
-// pb[r][g][2k, 2k+1].  Every block reads the copy g % kRep, so each slot
-// line has about G / kRep readers instead of G.  After the warps' own
+// as this block's partial sums: copy r < kRep goes to words
+// pb[r][g][2k, 2k + 1].  After the warps' own
 // reduce-scatter, lane l of warp 0 adds value k = l mod KM over warps
 // l / KM, l / KM + 32 / KM, ... and the 32 / KM lanes of one value finish
 // with an xor butterfly: IEEE addition is commutative, so every one of them
@@ -508,9 +521,9 @@ __device__ void block_publish(double (&v)[KM], double* red, unsigned long long* 
         for (int r = w0; r < kRep; r += SH) Tag<double>::put(pb + ((size_t)r * G + g) * 16 + 2 * k, tk, f);
 }
 
-// One exchange round, all threads of the block: waits for the K tagged
-// FP64 partial sums of every block (slots of 16 words; staged to
-// sp[G * K]) and for the tagged values of this block's ghost DOFs in vector
+// One exchange round outside the main loop's path (the coarse start, residual
+// replacements, the final residual), all threads of the block: waits for the
+// K tagged FP64 partial sums of every block (staged to sp[G * K]) and for the tagged values of this block's ghost DOFs in vector
 // buffer vb (written to dst[3 * no .. 3 * nloc)).  Items 0 .. ng - 1 are
 // the ghosts, which their owners publish before their partial sums, then
 // the partials.  Each thread takes items tid, tid + nt, tid + 2 nt, ...
@@ -521,8 +534,8 @@ __device__ void block_publish(double (&v)[KM], double* red, unsigned long long* 
 // The block that publishes last finds every other item already there; with
 // S slots per thread it reads them in ceil(items / (S nt)) round trips.
 // Returns false if a wait gave up.
-template <typename T, int S>
-__device__ bool exchange_round_s(const unsigned long long* __restrict__ pb, int G, int K,
+template <typename T, int S = 3>
+__device__ bool exchange_round(const unsigned long long* __restrict__ pb, int G, int K,
                                const unsigned long long* __restrict__ vb, T* dst, int no, int nloc,
                                const int* __restrict__ gid, int g, unsigned f, double* sp,
                                Waiter& wt) {
@@ -586,28 +599,6 @@ __device__ bool exchange_round_s(const unsigned long long* __restrict__ pb, int 
     return true;
 }
 
-// exchange_round_s with two slots per thread while the round's items fit
-// in two per thread (block Jacobi: 3 partials per block), else, when XS
-// allows, three (the two-level preconditioner's 6 partials per block and
-// the ghosts make about 2.5 items per thread on the 60k-DOF plate, and the
-// block that publishes last then reads them in one round trip, not two).
-// Measured on that plate, in A/B runs on one B200: with XS = 3 the mixed-
-// precision two-level solves run 0.9% (Chebyshev) and 1.8% faster, and the
-// mixed block-Jacobi solves, whose rounds keep two slots, 0.9-1.8% slower
-// (the larger kernel); in the FP64 kernels the third slot's code made block
-// Jacobi 2.4% slower, and in the batch kernel it costs spills, so those
-// keep XS = 2.
-template <typename T, int XS = 3>
-__device__ __forceinline__ bool exchange_round(const unsigned long long* __restrict__ pb, int G, int K,
-                                               const unsigned long long* __restrict__ vb, T* dst, int no,
-                                               int nloc, const int* __restrict__ gid, int g, unsigned f,
-                                               double* sp, Waiter& wt) {
-    const int n = 3 * (nloc - no) + G * K;
-    if constexpr (XS >= 3)
-        if (n > 2 * (int)blockDim.x) return exchange_round_s<T, 3>(pb, G, K, vb, dst, no, nloc, gid, g, f, sp, wt);
-    return exchange_round_s<T, 2>(pb, G, K, vb, dst, no, nloc, gid, g, f, sp, wt);
-}
-
 // Warp 0: adds the first K of each block's `stride` staged partials
 // (sp[G][stride]) in block order (the same bits in every block) into out[K].
 template <int K>
@@ -627,68 +618,6 @@ __device__ __forceinline__ void sum_partials(const double* __restrict__ sp, int 
     if (lane == 0)
 #pragma unroll
         for (int k = 0; k < K; k++) out[k] = v[k];
-}
-
-// ---------------------------------------------------------------------------
-// task matvec: the owned rows of K u, one (element, owned node) per thread
-// ---------------------------------------------------------------------------
-
-// Task block layout: entry (row r of the node, column c of the rotated
-// element) of task t sits at kt[(r * ND + c) * stride + t], so consecutive
-// threads read consecutive words.  Task node ids sit at tn[j * ts + t];
-// results go to yt[r * ys + t].  Tasks t >= ksplit read their blocks from
-// kt2 (stride2) instead of kt (stride): the ring-1 tasks of a 2-ring plan
-// when only the owned tasks' blocks are staged in shared memory.
-template <int NPE, typename T, typename KT>
-__device__ __forceinline__ void task_matvec(const T* __restrict__ u, T* __restrict__ yt, int ys,
-                                            int count, const uint16_t* __restrict__ tn, int ts,
-                                            const KT* __restrict__ kt, size_t stride,
-                                            int ksplit = 1 << 30,
-                                            const KT* __restrict__ kt2 = nullptr,
-                                            size_t stride2 = 0) {
-    constexpr int ND = 3 * NPE;
-    // FP64 blocks split the last partial pass into task rows; FP32 blocks do
-    // not (measured on the 60k-DOF plate: the split saves 2% in FP64 and
-    // costs 6% in mixed precision, whose whole-task pass is cheaper)
-    constexpr bool split = sizeof(T) == 8;
-    const int nt = blockDim.x, full = (!split || count <= nt) ? count : count - count % nt;
-    // whole tasks while every thread has one
-    for (int t = threadIdx.x; t < full; t += nt) {
-        const KT* kb = t < ksplit ? kt + t : kt2 + t;
-        const size_t ks = t < ksplit ? stride : stride2;
-        T a0 = T(0), a1 = T(0), a2 = T(0);
-#pragma unroll
-        for (int j = 0; j < NPE; j++) {
-            const int b = 3 * (int)tn[j * ts + t];
-#pragma unroll
-            for (int d = 0; d < 3; d++) {
-                const T v = u[b + d];
-                const int c = 3 * j + d;
-                a0 += (T)kb[(size_t)(0 * ND + c) * ks] * v;
-                a1 += (T)kb[(size_t)(1 * ND + c) * ks] * v;
-                a2 += (T)kb[(size_t)(2 * ND + c) * ks] * v;
-            }
-        }
-        yt[t] = a0;
-        yt[ys + t] = a1;
-        yt[2 * ys + t] = a2;
-    }
-    // the remaining rem < nt tasks one row per thread (3 rem rows), so the
-    // last pass costs about a third of a task instead of a whole one (FP64)
-    const int rem = count - full;
-    for (int q = threadIdx.x; q < 3 * rem; q += nt) {
-        const int t = full + q % rem, r = q / rem;
-        const KT* kb = t < ksplit ? kt + t : kt2 + t;
-        const size_t ks = t < ksplit ? stride : stride2;
-        T acc = T(0);
-#pragma unroll
-        for (int j = 0; j < NPE; j++) {
-            const int b = 3 * (int)tn[j * ts + t];
-#pragma unroll
-            for (int d = 0; d < 3; d++) acc += (T)kb[(size_t)(r * ND + 3 * j + d) * ks] * u[b + d];
-        }
-        yt[r * ys + t] = acc;
-    }
 }
 
 // Bending moments at each element's centroid (postprocess.ts:59-264):
@@ -768,82 +697,47 @@ __global__ void node_moments_kernel(int Nn, const int* __restrict__ inc_ptr,
     M[2 * (size_t)Nn + n] = c > 0 ? sxy / c : 0.0;
 }
 
-// Task blocks of every task from the element matrices (setup, per solve):
-// the owned node's 3 rows, columns rotated to start at the owned node.
-template <int NPE>
-__global__ void task_ke_kernel(int NT, const int* __restrict__ task_elem,
-                               const uint8_t* __restrict__ task_pos,
-                               const double* __restrict__ ke64, double* __restrict__ kt64,
-                               float* __restrict__ kt32) {
-    constexpr int ND = 3 * NPE, KK = ND * ND;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= NT) return;
-    const int e = task_elem[t], k = task_pos[t];
-    const double* K = ke64 + (size_t)e * KK;
-    for (int r = 0; r < 3; r++)
-        for (int j = 0; j < NPE; j++)
-            for (int d = 0; d < 3; d++) {
-                const double v = K[(3 * k + r) * ND + 3 * ((k + j) % NPE) + d];
-                const size_t o = (size_t)(r * ND + 3 * j + d) * NT + t;
-                kt64[o] = v;
-                if (kt32) kt32[o] = (float)v;
-            }
-}
-
 // ---------------------------------------------------------------------------
 // persistent PCG
 // ---------------------------------------------------------------------------
 
 enum { STOP_CONVERGED = 0, STOP_MAX_ITER = 1, STOP_BREAKDOWN = 2, STOP_ZERO_RHS = 3, STOP_STAGNATED = 4 };
-enum { ACT_UPDATE = 0, ACT_STOP = 1, ACT_RU = 2, ACT_NONFINITE = 3 };
+enum { ACT_UPDATE = 0, ACT_STOP = 1, ACT_RU = 2, ACT_NONFINITE = 3, ACT_TIMEOUT = 4 };
 enum { ST_OK = 0, ST_TIMEOUT = 4, ST_NONFINITE = 5 };
 
-// Threads per block: at most kMaxThreads (the launch bound of the 96-register
-// build); up to kLeanThreads a build with 128 registers per thread runs
-// instead (no spills); the batch and load-case kernels always run
-// kBatchThreads / kMultiThreads.
+// Threads per block: up to kLeanThreads the build with one row group a warp
+// in registers (128 registers a thread) runs, the automatic choice; above, up
+// to kMaxThreads, one with none (96 registers).  The batch and load-case
+// kernels always run kBatchThreads / kMultiThreads.
 constexpr int kMaxThreads = 576;
 constexpr int kLeanThreads = 512;
+constexpr int kResident = 1;
 constexpr int kBatchThreads = 512;
 constexpr int kMultiThreads = 512;  // the load-case kernel (128 registers)
 
 // Per-phase SM cycles of thread 0 of block 0, when timing is requested:
-// 0 K.u, 1 gather + dots + publish w, 2 block reduction and publishing the
-// partials, 3 the Chebyshev smoother's K t, 4 exchange wait, 5 the barrier
-// after the decision, 6 thread 0's decision, 7 vector updates (and the
-// residual replacement rounds of the mixed mode).
+// 0 K.u, dots and publishing w, 1 unused (0), 2 block reduction and
+// publishing the partials, 3 the Chebyshev smoother's K t, 4 exchange wait
+// and sum of the partials, 5 the barrier after the decision, 6 warp 0's
+// decision, 7 vector updates (and the residual replacement rounds of the
+// mixed mode).
 struct PhaseClock {
     bool on;
-    long long last;
-    long long* t;  // 8 accumulators in shared memory
+    long long* t;  // 8 accumulators and the last time stamp, in shared memory
     __device__ __forceinline__ void start(bool enable, long long* acc) {
         on = enable;
         t = acc;
-        if (on)
-            for (int k = 0; k < 8; k++) t[k] = 0;
-        last = on ? clock64() : 0;
+        if (!on) return;
+        for (int k = 0; k < 8; k++) t[k] = 0;
+        t[8] = clock64();
     }
     __device__ __forceinline__ void lap(int k) {
         if (!on) return;
         const long long now = clock64();
-        t[k] += now - last;
-        last = now;
+        t[k] += now - t[8];
+        t[8] = now;
     }
 };
-
-// Owned-node gather of task results: w_n = sum of the node's task rows.
-template <typename T>
-__device__ __forceinline__ void gather3(const T* __restrict__ yt, int ntask, int ta, int tb,
-                                        T& w0, T& w1, T& w2) {
-    w0 = T(0);
-    w1 = T(0);
-    w2 = T(0);
-    for (int t = ta; t < tb; t++) {
-        w0 += yt[t];
-        w1 += yt[ntask + t];
-        w2 += yt[2 * ntask + t];
-    }
-}
 
 __device__ __forceinline__ void block_jacobi3(const float* Bn, const float* rv, float* u) {
     u[0] = Bn[0] * rv[0] + Bn[1] * rv[1] + Bn[2] * rv[2];
@@ -854,23 +748,6 @@ __device__ __forceinline__ void block_jacobi3(const double* Bn, const double* rv
     u[0] = Bn[0] * rv[0] + Bn[1] * rv[1] + Bn[2] * rv[2];
     u[1] = Bn[3] * rv[0] + Bn[4] * rv[1] + Bn[5] * rv[2];
     u[2] = Bn[6] * rv[0] + Bn[7] * rv[1] + Bn[8] * rv[2];
-}
-
-// Polynomial smoother at one node: with t = D^-1 r in un and the node's
-// task results K t in yt[ta, tb), un = ca t - cb D_n^-1 (K t); constrained
-// rows of K are the identity.
-template <typename T>
-__device__ __forceinline__ void smooth_node(T* un, const T* __restrict__ yt, int ys, int ta, int tb,
-                                            const T* Bn, const unsigned char* cn, T ca, T cb) {
-    T k3[3];
-    gather3(yt, ys, ta, tb, k3[0], k3[1], k3[2]);
-#pragma unroll
-    for (int d = 0; d < 3; d++)
-        if (cn[d]) k3[d] = un[d];
-    T v[3];
-    block_jacobi3(Bn, k3, v);
-#pragma unroll
-    for (int d = 0; d < 3; d++) un[d] = ca * un[d] - cb * v[d];
 }
 
 // Restriction of a nodal 3-vector to the node's aggregate modes (P^T v):
@@ -928,6 +805,229 @@ __device__ __forceinline__ void coarse_apply(const T* __restrict__ Ai, int G, in
     }
 }
 
+// ---------------------------------------------------------------------------
+// the main loop's exchange: three warps the dot products, the others the ghosts
+// ---------------------------------------------------------------------------
+
+// One warp: the total of partial sum k over all blocks, added in a fixed
+// order (lane l blocks l, l + 32, ..., then an xor butterfly, so every lane
+// of every block holds the same bits).  Up to five blocks a lane are polled
+// at once, straight into registers.  False if a wait gave up.
+__device__ __forceinline__ bool poll_total(const unsigned long long* __restrict__ pb, int G, int g, int copies, int k,
+                                           unsigned f, double& out, Waiter& wt) {
+    constexpr int NB = 5;
+    const int lane = threadIdx.x & 31;
+    pb += (size_t)(g % copies) * G * 16 + 2 * k + 16 * lane;
+    double acc = 0.0;
+    bool ok = true;
+    wt.spins = 0;
+    for (int base = lane; base < G && ok; base += 32 * NB, pb += 512 * NB) {
+        unsigned long long lo[NB], hi[NB];
+        for (;;) {
+            bool got = true;
+#pragma unroll
+            for (int i = 0; i < NB; i++) {
+                lo[i] = hi[i] = (unsigned long long)f << 32;  // past the last block: 0
+                if (base + 32 * i < G) ld_relaxed2(pb + 512 * i, lo[i], hi[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < NB; i++) got = got && (unsigned)(lo[i] >> 32) == f && (unsigned)(hi[i] >> 32) == f;
+            if (got) break;
+            if (!wt.keep_going()) {
+                ok = false;
+                break;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < NB; i++)
+            acc += __longlong_as_double((long long)((hi[i] << 32) | (lo[i] & 0xffffffffull)));
+    }
+    __syncwarp();
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    out = acc;
+    return __all_sync(0xffffffffu, ok);
+}
+
+// Block-wide totals of the K values v of every thread, published as this
+// block's partial sums: all threads store their values (red[k][thread]),
+// and after one barrier warp k adds value k of all threads (lane l threads
+// l, l + 32, ..., then an xor butterfly) and its first kRep lanes write one
+// copy each.  Returns false in the warps that have no value.  All threads
+// call it; `red` must not be written again before a later barrier.  Fewer
+// warps than values: warp k takes values k, k + nw, ...
+template <int K>
+__device__ __forceinline__ void sum_publish(const double (&v)[K], double* red, unsigned long long* pb, int G, int g,
+                                            unsigned f) {
+    constexpr int copies = dot_copies(K > 3);
+    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
+#pragma unroll
+    for (int k = 0; k < K; k++) red[k * nt + tid] = v[k];
+    __syncthreads();
+    for (int k = warp; k < K; k += nw) {
+        const double* q = red + k * nt + lane;
+        double t = 0.0;
+        if (nw == 16) {  // the automatic block size: all loads at once, a tree of additions
+            double s[16];
+#pragma unroll
+            for (int i = 0; i < 16; i++) s[i] = q[32 * i];
+#pragma unroll
+            for (int h = 8; h > 0; h >>= 1)
+#pragma unroll
+                for (int i = 0; i < h; i++) s[i] += s[i + h];
+            t = s[0];
+        } else {
+            for (int w = 0; w < nw; w++) t += q[32 * w];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane < copies) Tag<double>::put(pb + ((size_t)lane * G + g) * 16 + 2 * k, t, f);
+    }
+}
+
+// This thread's share (items t, t + stride, ...) of the round's other
+// values: the 3 (nloc - no) ghost DOFs of vector buffer vb into dst, then
+// (KC = 3) partial sums 3..5 of every block into sp[3 b + m].  S items in
+// flight; a slot takes its next item as soon as its item has arrived.
+template <typename T, int S>
+__device__ bool poll_ghosts(const unsigned long long* __restrict__ pb, int G, int KC,
+                            const unsigned long long* __restrict__ vb, T* dst, int no, int nloc,
+                            const int* __restrict__ gid, int g, unsigned f, double* sp, int t, int stride,
+                            Waiter& wt) {
+    constexpr int TW = Tag<T>::W;
+    const int ng = 3 * (nloc - no), n = ng + KC * G;
+    pb += (size_t)(g % kRep) * G * 16 + 6;
+    auto addr = [&](int i) -> const unsigned long long* {
+        if (i < ng) {
+            const int k = 3 * no + i;
+            return vb + (size_t)(3 * gid[k / 3] + k % 3) * TW;
+        }
+        return pb + (size_t)((i - ng) / 3) * 16 + 2 * ((i - ng) % 3);
+    };
+    int it[S];
+    const unsigned long long* pp[S];
+#pragma unroll
+    for (int s = 0; s < S; s++) {
+        it[s] = t + s * stride;
+        pp[s] = it[s] < n ? addr(it[s]) : nullptr;
+    }
+    int next = t + S * stride;
+    wt.spins = 0;
+    for (;;) {
+        unsigned long long lo[S], hi[S];
+        bool any = false;
+#pragma unroll
+        for (int s = 0; s < S; s++) {
+            lo[s] = hi[s] = 0;
+            if (it[s] >= n) continue;
+            any = true;
+            if (it[s] >= ng || TW == 2) {
+                ld_relaxed2(pp[s], lo[s], hi[s]);
+            } else {
+                lo[s] = ld_relaxed(pp[s]);
+                hi[s] = lo[s];
+            }
+        }
+        if (!any) break;
+        bool moved = false;
+#pragma unroll
+        for (int s = 0; s < S; s++) {
+            if (it[s] >= n) continue;
+            if ((unsigned)(lo[s] >> 32) != f || (unsigned)(hi[s] >> 32) != f) continue;
+            const int i = it[s];
+            if (i >= ng) {
+                sp[i - ng] = __longlong_as_double((long long)((hi[s] << 32) | (lo[s] & 0xffffffffull)));
+            } else if constexpr (TW == 2) {
+                dst[3 * no + i] = (T)__longlong_as_double((long long)((hi[s] << 32) | (lo[s] & 0xffffffffull)));
+            } else {
+                dst[3 * no + i] = (T)__uint_as_float((unsigned)lo[s]);
+            }
+            it[s] = next;
+            next += stride;
+            pp[s] = it[s] < n ? addr(it[s]) : nullptr;
+            moved = true;
+        }
+        if (!moved && !wt.keep_going()) return false;
+    }
+    return true;
+}
+
+// One group's rows in registers: the first kRegSteps q-steps.
+template <typename T>
+struct RegRows {
+    T k[9 * kRegSteps];
+    int c[kRegSteps];  // 3 x local column
+};
+
+// Where the rows outside the registers are.
+template <typename T>
+struct RowMem {
+    const int* gq;        // shared: [groups + 1] q-steps before each group of the part
+    const int* go;        // shared: [groups] staged q-step of the group's first one, or -1
+    const uint16_t* col;  // shared: [q-steps][30]
+    const T* ks;          // shared: staged q-steps
+    const T* kg;          // global: the part's q-steps
+};
+
+// s += q-steps [done, w) of group grp times v (lanes < 30).
+template <typename T>
+__device__ __forceinline__ void rows_rest(const RowMem<T>& A, const T* __restrict__ v, int grp, int done, T (&s)[3]) {
+    const int lane = threadIdx.x & 31;
+    const int q0 = A.gq[grp], w = A.gq[grp + 1] - q0;
+    if (done >= w || lane >= kRowLanes) return;
+    const int g0 = A.go[grp];
+    const uint16_t* cq = A.col + (q0 + done) * kRowLanes + lane;
+    if (g0 >= 0)
+        row_steps<T, T>(v, cq, A.ks + g0 * 9 * kRowLanes + lane, w - done, s);
+    else
+        row_steps<T, T>(v, cq, A.kg + (size_t)(q0 + done) * 9 * kRowLanes + lane, w - done, s);
+}
+
+// Component of K v of this lane's DOF in a group whose rows are in registers.
+template <typename T>
+__device__ __forceinline__ T rows_reg(const RegRows<T>& R, const RowMem<T>& A, const T* __restrict__ v, int grp,
+                                      bool more) {
+    T s[3] = {T(0), T(0), T(0)};
+#pragma unroll
+    for (int q = 0; q < kRegSteps; q++) {
+        const T v0 = v[R.c[q]], v1 = v[R.c[q] + 1], v2 = v[R.c[q] + 2];
+#pragma unroll
+        for (int r = 0; r < 3; r++)
+            s[r] = fma(R.k[9 * q + 3 * r + 2], v2, fma(R.k[9 * q + 3 * r + 1], v1, fma(R.k[9 * q + 3 * r], v0, s[r])));
+    }
+    if (more) rows_rest(A, v, grp, kRegSteps, s);
+    return row_join(s);
+}
+
+// ... in any other group.
+template <typename T>
+__device__ __forceinline__ T rows_mem(const RowMem<T>& A, const T* __restrict__ v, int grp) {
+    T s[3] = {T(0), T(0), T(0)};
+    rows_rest(A, v, grp, 0, s);
+    return row_join(s);
+}
+
+// Decision state, in shared memory and touched by warp 0 alone: registers of
+// every warp are worth more than its loads.  Reciprocals of the previous
+// gamma and alpha (0 before the first update, so beta = 0 and p.Ap = delta
+// there) and squared thresholds keep divisions and square roots off the path
+// to the barrier.
+struct Decision {
+    double inv_gamma, inv_alpha;
+    double thr_check;         // rho at or below it needs the full tests
+    double thr_abs, thr_rel, thr_ru, bnorm, best_trn, final_res, true_rel;
+    int xupd, xupd_ref, nru;  // updates, at the last replacement, replacements
+    int stall;                // replacements since the FP64 residual last halved
+    int stop, first;
+};
+
+// State of one DOF (this lane's in one group of 10 nodes).
+template <typename T>
+struct Dof {
+    T r, s, u, w;
+    T b[3];  // row of the node's 3x3 inverse, cyclically from the diagonal
+};
+
 // The whole PCG solve.  T = double: plain FP64.  T = float (MIXED): inner
 // iterations in FP32 with FP64 dot products, FP64 solution x, and FP64
 // true-residual replacement r = F - K x ("reliable update") whenever the
@@ -935,42 +1035,66 @@ __device__ __forceinline__ void coarse_apply(const T* __restrict__ Ai, int G, in
 // updates, or when it meets the tolerance (convergence is then decided on
 // the true residual).
 //
+// Lanes and registers.  Every vector step works on groups of 10 local nodes
+// (owned nodes first), one warp a group, lane 3 i + d on component d of the
+// group's node i (lanes 30 and 31 idle).  Group j nw + w belongs to warp w.
+// Its first NG groups (1, or 0 in the build for more threads) are resident:
+// rows, vectors and block inverse in registers for the whole solve, and only
+// u (or t), which the neighbours' rows read, in shared memory.  Further
+// groups keep their state in shared memory.  The lanes of a row's product
+// hold w of their own DOF, so dot products, the published w, the update and
+// the block-Jacobi product follow in registers and shuffles.
+// An iteration is bound by latency: a warp issues an instruction about every
+// 7 cycles, so what counts is the number of instructions of one warp from
+// barrier to barrier.  Hence one group a warp, three barriers an iteration,
+// the sums over the block's threads and over the blocks one warp a value,
+// and x updated behind the publication, while the block waits anyway.
+// Measured (us per iteration, before: element tasks in shared memory, 16
+// warps, five barriers): 60k-DOF Q4 plate on 148 blocks FP64 block Jacobi 5.13 ->
+// 3.32, FP64 two-level 6.94 -> 5.82, mixed two-level Chebyshev 7.96 -> 6.68;
+// 3,267-DOF plate on 9 blocks 4.18 -> 3.0; 121k-DOF DKT plate 9.38 -> 6.2.
+// Two groups a warp in 8 warps (255 registers) was slower (5.7 on the 60k-DOF
+// plate): one warp's instructions then make up most of the iteration.
+//
 // Exchange rounds: round e (e = 1, 2, ...) carries every block's partial
 // sums and the owners' values of one vector (w, or the replaced r), in
 // buffers [e & 1]; x rounds (for the FP64 residual) use their own tags.
 // A block overwrites buffer [e & 1] only after it has seen every block's
 // round e - 1 partials, and every block reads round e - 2 before it
 // publishes round e - 1, so no reader can still need the old values.
-template <int NPE, typename T, bool MIXED, int XS = (MIXED ? 3 : 2)>
+template <typename T, bool MIXED, int NG, bool COARSE, bool CHEB>
 __device__ __forceinline__ void pcg_body(const PcgArgs& a, const int g, unsigned char* sm) {
-    constexpr int ND = 3 * NPE, TW = Tag<T>::W;
+    constexpr int TW = Tag<T>::W;
+    constexpr int NR = NG > 0 ? NG : 1;  // array bound
     const SmemLayout& L = a.L;
     const int tid = threadIdx.x, nt = blockDim.x;
+    const int lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
     const int n0 = a.node_off[g], nloc = a.node_off[g + 1] - n0, no = a.nown[g];
-    // tasks [0, nta) of the part; the owned nodes' are [0, ntm) (all of them
-    // unless the plan has a 2-ring halo: then ring-1 nodes' tasks follow)
-    const int t0 = a.task_off[g], nta = a.task_off[g + 1] - t0;
-    const int nn1 = a.n1[g], ntm = a.tptr[a.tp_off[g] + no];
-    const bool cheb = a.smoother == 1;
+    const int nn1 = a.n1[g];
+    const int gb = a.grp_off[g], ng1 = a.grp_off[g + 1] - gb;  // groups of rows (n1 of them)
+    const int ngo = (no + kRowGroup - 1) / kRowGroup, ngl = (nloc + kRowGroup - 1) / kRowGroup;
+    // this lane's node within a group and its DOF component
+    const int li = lane / 3, ld = lane % 3;
+    const bool lact = lane < kRowLanes;
     const T ca = (T)a.cheb_a, cbc = (T)a.cheb_b;
     const size_t N3 = 3 * (size_t)a.Nn;
+    const int res0 = NG * nw * kRowGroup;  // nodes below res0 are resident
 
-    T* r = (T*)(sm + L.r);
+    // u, w, t hold every local node; r, s, B and cm the state of the nodes that
+    // are not resident (index from the first of them)
     T* u = (T*)(sm + L.u);
-    T* p = (T*)(sm + L.p);
-    T* s = (T*)(sm + L.s);
     T* w = (T*)(sm + L.w);
-    T* B = (T*)(sm + L.B);
-    T* yt = (T*)(sm + L.yt);
-    T* kts = (T*)(sm + L.kt);
+    T* t = (T*)(sm + L.t);  // Chebyshev smoother: D^-1 r
+    T* r = (T*)(sm + L.r) - 3 * res0;
+    T* p = (T*)(sm + L.p);  // p and x: the owned nodes
+    T* s = (T*)(sm + L.s) - 3 * res0;
+    T* B = (T*)(sm + L.B) - 9 * res0;
     double* x = (double*)(sm + L.x);
+    unsigned char* cm = (unsigned char*)(sm + L.cm) - 3 * res0;
     double* red = (double*)(sm + L.red);
     double* scal = (double*)(sm + L.scal);
     double* sp = (double*)(sm + L.sp);
     int* gid = (int*)(sm + L.gid);
-    int* tptr = (int*)(sm + L.tptr);
-    uint16_t* tn = (uint16_t*)(sm + L.tnode);
-    unsigned char* cm = (unsigned char*)(sm + L.cm);
     // coarse state per row of this part: c = A_c^-1 P^T r and cs = A_c^-1 P^T s
     // in two copies (copy cb is current; an update writes copy cb ^ 1, so
     // nodes can read the current copy while the new one is written), and
@@ -978,39 +1102,42 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& a, const int g, unsigned
     double* qw = (double*)(sm + L.qw);
     double* csb = (double*)(sm + L.cs);
     double* cvb = (double*)(sm + L.cv);
-    int* ctl = (int*)(sm + L.ctl);  // [0] action, [1] final residual needed
+    int* ctl = (int*)(sm + L.ctl);  // [0] action, [1] final residual needed, [2] a wait gave up
     T* nb = (T*)(sm + L.nb);
     int* nslot = (int*)(sm + L.nslot);
-    const int rows = a.coarse ? 3 * (a.cagg_off[g + 1] - a.cagg_off[g]) : 0;
-    const T* aig = a.coarse ? (MIXED ? (const T*)a.ainv32 : (const T*)a.ainv64) + (size_t)a.ainv_off[g] * a.C
+    const int rows = COARSE ? 3 * (a.cagg_off[g + 1] - a.cagg_off[g]) : 0;
+    const T* aig = COARSE ? (MIXED ? (const T*)a.ainv32 : (const T*)a.ainv64) + (size_t)a.ainv_off[g] * a.C
                             : nullptr;
     T* ais = (T*)(sm + L.ainv);
     const T* Ai = a.ainv_smem ? (const T*)ais : aig;
-    const int KP = a.coarse ? 6 : 3;  // partial sums per block in a main round
-    // FP64 views for the true residual: own arrays in MIXED mode (ytd may
-    // share the dead yt / w / u space),
-    // the (then dead) p / yt arrays in FP64 mode
-    double* xl = MIXED ? (double*)(sm + L.xl) : (double*)p;
-    double* ytd = MIXED ? (double*)(sm + L.ytd) : (double*)yt;
-    const T* ktg = MIXED ? (const T*)a.kt32 : (const T*)a.kt64;
+    // FP64 x on every local node for the true residual, in the space of w
+    // (and u): neither is live then
+    double* xl = (double*)(sm + L.xl);
     const T* Bg = MIXED ? (const T*)a.binv32 : (const T*)a.binv64;
 
     // ---- load the part ----
+    int* gq = (int*)(sm + L.gq);
+    int* go = (int*)(sm + L.go);
+    uint16_t* rcol = (uint16_t*)(sm + L.rcol);
+    T* kts = (T*)(sm + L.kt);
+    const int qb = a.grp_q[gb];
+    const T* kg = (MIXED ? (const T*)a.rk32 : (const T*)a.rk64) + (size_t)qb * 9 * kRowLanes;
+    for (int i = tid; i <= ng1; i += nt) gq[i] = a.grp_q[gb + i] - qb;
     for (int i = tid; i < nloc; i += nt) gid[i] = a.nodes[n0 + i];
-    for (int i = tid; i <= nn1; i += nt) tptr[i] = a.tptr[a.tp_off[g] + i];
-    for (int i = tid; i < NPE * nta; i += nt) {
-        const int t = i % nta, j = i / nta;
-        tn[i] = a.task_nodes[(size_t)(t0 + t) * NPE + j];
-    }
-    // Ke blocks staged in shared memory: none, the owned tasks' (ke_smem 1)
-    // or every task's (2)
-    const int nk = a.ke_smem == 2 ? nta : ntm;
-    if (a.ke_smem)
-        for (int i = tid; i < 3 * ND * nk; i += nt) {
-            const int t = i % nk, q = i / nk;
-            kts[i] = ktg[(size_t)q * a.NT + t0 + t];
+    __syncthreads();
+    if (tid == 0) {
+        // the q-steps not in registers go to shared memory while they fit
+        int used = 0;
+        for (int k = 0; k < ng1; k++) {
+            const int need = max(0, gq[k + 1] - gq[k] - (k < NG * nw ? kRegSteps : 0));
+            const bool fits = used + need <= L.kq;
+            go[k] = fits ? used : -1;
+            if (fits) used += need;
         }
-    if (a.coarse) {
+        ctl[2] = 0;
+    }
+    for (int i = tid; i < gq[ng1] * kRowLanes; i += nt) rcol[i] = a.rcol[(size_t)qb * kRowLanes + i];
+    if (COARSE) {
         for (int i = tid; i < nloc; i += nt) {
             nslot[i] = a.node_slot[n0 + i];
 #pragma unroll
@@ -1021,38 +1148,183 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& a, const int g, unsigned
             for (int i = tid; i < rows * a.C; i += nt) ais[i] = aig[i];
     }
     __syncthreads();
-    for (int n = tid; n < nloc; n += nt) {
-        const int G3 = 3 * gid[n];
-        T rv[3];
+    const RowMem<T> A{gq, go, rcol, kts, kg};
+    RegRows<T> R[NR];
+    unsigned more = 0;  // bit j: resident group j has q-steps beyond the registers'
+    if constexpr (NG > 0) {
 #pragma unroll
-        for (int d = 0; d < 3; d++) {
-            const unsigned char c = a.cons[G3 + d];
-            cm[3 * n + d] = c;
-            rv[d] = c ? T(0) : (T)a.F[G3 + d];
-            r[3 * n + d] = rv[d];
-            p[3 * n + d] = T(0);
-            s[3 * n + d] = T(0);
-            if (n < no) x[3 * n + d] = 0.0;
+        for (int j = 0; j < NG; j++) {
+            const int grp = warp + j * nw;
+            const int w0 = grp < ng1 ? gq[grp + 1] - gq[grp] : 0;
+            if (w0 > kRegSteps) more |= 1u << j;
+#pragma unroll
+            for (int q = 0; q < kRegSteps; q++) {
+                const bool has = q < w0 && lact;
+                const size_t o = has ? (size_t)(gq[grp] + q) : 0;
+                R[j].c[q] = has ? 3 * (int)rcol[o * kRowLanes + lane] : 0;
+#pragma unroll
+                for (int k = 0; k < 9; k++) R[j].k[9 * q + k] = has ? kg[(o * 9 + k) * kRowLanes + lane] : T(0);
+            }
         }
-        T* Bn = B + 9 * n;
+    }
+    for (int k = warp; k < ng1; k += nw) {
+        if (go[k] < 0) continue;
+        const int skip = k < NG * nw ? kRegSteps : 0, need = gq[k + 1] - gq[k] - skip;
+        const T* src = kg + (size_t)(gq[k] + skip) * 9 * kRowLanes;
+        T* dst = kts + go[k] * 9 * kRowLanes;
+        for (int i = lane; i < need * 9 * kRowLanes; i += 32) dst[i] = src[i];
+    }
+    Dof<T> D[NR];
+    unsigned cbits = 0;  // bit j: this lane's DOF of resident group j is constrained
+    unsigned sbits = 0;  // bit j: ... is on a node that other parts hold as a ghost
+    // this DOF's row of P: its node's three coarse values enter it with m0, m1,
+    // m2 (0 on constrained DOFs), and it enters their restriction likewise
+    struct Prow {
+        double m1, m2;
+        bool m0;  // 1 or 0
+        int q;    // 3 x the node's aggregate slot
+    };
+    auto prow = [&](int n, bool live, bool c) -> Prow {
+        Prow o{0.0, 0.0, false, 0};
+        if (!live) return o;
+        o.q = 3 * nslot[n];
+        if (c) return o;
+        const T* bs = nb + 3 * n;  // dx, dy, 1/h
+        if (ld == 0) {
+            o.m0 = true;
+            o.m1 = (double)bs[1];
+            o.m2 = (double)bs[0];
+        } else if (ld == 1) {
+            o.m1 = (double)bs[2];
+        } else {
+            o.m2 = -(double)bs[2];
+        }
+        return o;
+    };
+    Prow Pr[NR];
+    // start of one DOF: r = F, everything else 0
+    auto load_dof = [&](int n, bool live, Dof<T>& o) -> bool {
+        o = Dof<T>{};
+        if (!live) return false;
+        const int G3 = 3 * gid[n] + ld;
+        const bool c = a.cons[G3] != 0;
+        o.r = c ? T(0) : (T)a.F[G3];
 #pragma unroll
-        for (int q = 0; q < 9; q++) Bn[q] = Bg[(size_t)gid[n] * 9 + q];
-        block_jacobi3(Bn, rv, u + 3 * n);
+        for (int q = 0; q < 3; q++) o.b[q] = Bg[(size_t)gid[n] * 9 + 3 * ld + (ld + q) % 3];
+        return c;
+    };
+    // a group outside the registers: this lane's DOF to and from shared memory
+    auto get_dof = [&](int n, bool live, Dof<T>& o) -> bool {
+        o = Dof<T>{};
+        if (!live) return false;
+        const int k = 3 * n + ld;
+        o.r = r[k];
+        o.s = s[k];
+        o.u = n < nn1 || !CHEB ? u[k] : T(0);
+        o.w = w[k];
+#pragma unroll
+        for (int q = 0; q < 3; q++) o.b[q] = B[3 * k + q];
+        return (cm[k] & 1) != 0;
+    };
+    if constexpr (NG > 0) {
+#pragma unroll
+        for (int j = 0; j < NG; j++) {
+            const int n = (warp + j * nw) * kRowGroup + li;
+            const bool c = load_dof(n, lact && n < nloc, D[j]);
+            if (c) cbits |= 1u << j;
+            if (lact && n < no && a.shared[gid[n]]) sbits |= 1u << j;
+            Pr[j] = Prow{0.0, 0.0, false, 0};
+            if (COARSE) Pr[j] = prow(n, lact && n < nloc, c);
+            const T z = jacobi_lane(D[j].b, D[j].r);
+            if (lact && n < nloc) (CHEB ? t : u)[3 * n + ld] = z;
+            D[j].u = z;
+            if (lact && n < no) {
+                p[3 * n + ld] = T(0);
+                x[3 * n + ld] = 0.0;
+            }
+        }
+    }
+    for (int grp = warp + NG * nw; grp < ngl; grp += nw) {
+        const int n = grp * kRowGroup + li, k = 3 * n + ld;
+        const bool live = lact && n < nloc;
+        Dof<T> o;
+        const bool c = load_dof(n, live, o);
+        const T z = jacobi_lane(o.b, o.r);
+        if (live) {
+            cm[k] = (c ? 1 : 0) | (n < no && a.shared[gid[n]] ? 2 : 0);
+            r[k] = o.r;
+            s[k] = T(0);
+            if (n < no) {
+                p[k] = T(0);
+                x[k] = 0.0;
+            }
+#pragma unroll
+            for (int q = 0; q < 3; q++) B[3 * k + q] = o.b[q];
+            (CHEB ? t : u)[k] = z;
+        }
     }
     __syncthreads();
 
-    const T* kt = a.ke_smem ? kts : ktg + t0;
-    const size_t kstride = a.ke_smem ? (size_t)nk : (size_t)a.NT;
-    // the smoother's K t also runs ring-1 tasks, whose blocks may stay in global memory
-    const int ksplit = a.ke_smem == 1 ? ntm : (1 << 30);
-    if (cheb) {
-        // u0 = a t - b D^-1 K t, t = D^-1 r0 (u holds t on every local node)
-        task_matvec<NPE, T, T>(u, yt, nta, nta, tn, nta, kt, kstride, ksplit, ktg + t0, (size_t)a.NT);
-        __syncthreads();
-        for (int n = tid; n < nn1; n += nt)
-            smooth_node(u + 3 * n, yt, nta, tptr[n], tptr[n + 1], B + 9 * n, cm + 3 * n, ca, cbc);
-        __syncthreads();
-    }
+    // runs f(n, dof, constrained, row of P, component of K v) over this warp's
+    // groups below `groups`; resident ones straight from registers
+    auto each_row = [&](const T* v, int groups, auto&& f) {
+        if constexpr (NG > 0) {
+#pragma unroll
+            for (int j = 0; j < NG; j++) {
+                const int grp = warp + j * nw, n = grp * kRowGroup + li;
+                if (grp < groups) f(n, D[j], ((cbits >> j) & 1u) != 0, Pr[j], rows_reg(R[j], A, v, grp, (more >> j) & 1u));
+            }
+        }
+        for (int grp = warp + NG * nw; grp < groups; grp += nw) {
+            const int n = grp * kRowGroup + li;
+            const bool live = lact && n < nloc;
+            Dof<T> o;
+            const bool c = get_dof(n, live, o);
+            Prow pr{0.0, 0.0, false, 0};
+            if (COARSE) pr = prow(n, live, c);
+            f(n, o, c, pr, rows_mem(A, v, grp));
+        }
+    };
+    // (P c) at this lane's DOF, lane 3 i + m of a node holding value m of its
+    // aggregate; all lanes of the warp call it
+    auto prolong = [&](const Prow& pr, double cv) -> T {
+        const int b = lane - ld;
+        const double c0 = __shfl_sync(0xffffffffu, cv, b);
+        const double c1 = __shfl_sync(0xffffffffu, cv, b + 1), c2 = __shfl_sync(0xffffffffu, cv, b + 2);
+        return (T)fma(pr.m2, c2, fma(pr.m1, c1, pr.m0 ? c0 : 0.0));
+    };
+    // P^T v of this lane's DOF value added to acc[0..2]
+    auto restrict_dof = [&](const Prow& pr, double v, double* acc) {
+        acc[0] += pr.m0 ? v : 0.0;
+        acc[1] = fma(pr.m1, v, acc[1]);
+        acc[2] = fma(pr.m2, v, acc[2]);
+    };
+    // u = a t - b D^-1 K t (+ P c with c from cf(row of P)): the Chebyshev
+    // smoother on every row, t on every local node
+    auto smooth = [&](auto&& cf) {
+        each_row(t, ng1, [&](int n, Dof<T>& o, bool c, const Prow& pr, T kt) {
+            const bool live = lact && n < nn1;
+            const T tk = live ? t[3 * n + ld] : T(0);
+            T z = ca * tk - cbc * jacobi_lane(o.b, c ? tk : kt);
+            if (COARSE) z += prolong(pr, cf(pr));
+            if (live) u[3 * n + ld] = z;
+            o.u = z;
+        });
+    };
+    // (K x) in FP64 at this lane's DOF of group grp, x = xl, rows from memory
+    auto true_row = [&](int grp) -> double {
+        if constexpr (MIXED) {
+            double sd[3] = {0.0, 0.0, 0.0};
+            const int q0 = gq[grp];
+            if (lact)
+                row_steps<double, double>(xl, rcol + q0 * kRowLanes + lane,
+                                          a.rk64 + (size_t)(qb + q0) * 9 * kRowLanes + lane, gq[grp + 1] - q0, sd);
+            return row_join(sd);
+        } else {
+            return rows_mem(A, (const T*)xl, grp);
+        }
+    };
+
     PhaseClock clk;
     clk.start(a.timing && g == 0 && tid == 0, (long long*)(sm + L.clk));
     Waiter wt;
@@ -1060,244 +1332,357 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& a, const int g, unsigned
     unsigned e = a.tag0 + 1, xe = a.tag0 + 1;  // round tags
     int status = ST_OK;
 
-    // ---- two-level: u0 = M_bj r0 + P A_c^-1 P^T r0 (one exchange round) ----
-    if (a.coarse) {
+    // ---- two-level: c0 = A_c^-1 P^T r0 (one exchange round), u0 = S r0 + P c0 ----
+    if (COARSE) {
         double v0[4] = {0.0, 0.0, 0.0, 0.0};
-        for (int n = tid; n < no; n += nt) restrict3(r + 3 * n, cm + 3 * n, nb + 3 * n, v0);
+        if constexpr (NG > 0) {
+#pragma unroll
+            for (int j = 0; j < NG; j++) {
+                const int n = (warp + j * nw) * kRowGroup + li;
+                if (lact && n < no) restrict_dof(Pr[j], (double)D[j].r, v0);
+            }
+        }
+        for (int grp = warp + NG * nw; grp < ngo; grp += nw) {
+            const int n = grp * kRowGroup + li;
+            if (lact && n < no) restrict_dof(prow(n, true, (cm[3 * n + ld] & 1) != 0), (double)r[3 * n + ld], v0);
+        }
         unsigned long long* pb0 = a.llp + (size_t)(e & 1) * kRep * a.G * 16;
         block_publish<4>(v0, red, pb0, a.G, g, 3, e);
-        const bool ok = exchange_round<T, XS>(pb0, a.G, 3, nullptr, w, no, no, gid, g, e, sp, wt);
-        if (__syncthreads_or(!ok)) {
-            status = ST_TIMEOUT;
-        } else {
-            coarse_apply<T>(Ai, a.G, rows, sp, 3, 0, cvb, 0);
-            __syncthreads();
-            for (int n = tid; n < nloc; n += nt) prolong3(cvb + 3 * nslot[n], cm + 3 * n, nb + 3 * n, u + 3 * n);
-            __syncthreads();
-        }
+        const bool ok = exchange_round<T>(pb0, a.G, 3, nullptr, w, no, no, gid, g, e, sp, wt);
+        if (__syncthreads_or(!ok)) status = ST_TIMEOUT;
+        else coarse_apply<T>(Ai, a.G, rows, sp, 3, 0, cvb, 0);
+        __syncthreads();
         e++;
     }
+    if (CHEB) {
+        smooth([&](const Prow& pr) { return cvb[pr.q + ld]; });
+        __syncthreads();
+    } else if (COARSE) {
+        if constexpr (NG > 0) {
+#pragma unroll
+            for (int j = 0; j < NG; j++) {
+                const int n = (warp + j * nw) * kRowGroup + li;
+                const bool live = lact && n < nloc;
+                D[j].u += prolong(Pr[j], cvb[Pr[j].q + ld]);
+                if (live) u[3 * n + ld] = D[j].u;
+            }
+        }
+        for (int grp = warp + NG * nw; grp < ngl; grp += nw) {
+            const int n = grp * kRowGroup + li;
+            const bool live = lact && n < nloc;
+            const Prow pr = prow(n, live, live && (cm[3 * n + ld] & 1));
+            const T pc = prolong(pr, cvb[pr.q + ld]);
+            if (live) u[3 * n + ld] += pc;
+        }
+        __syncthreads();
+    }
 
-    // decision state (thread 0): reciprocals of the previous gamma and
-    // alpha, and squared thresholds, so the step to the barrier has one
-    // division and no square root
-    double inv_gamma = 1.0, inv_alpha = 1.0, bnorm = 0.0, rn_ref = 0.0;
-    const double thr_abs = a.tol * a.tol;
-    double thr_rel = 0.0, thr_ru = 0.0;
+    Decision* dec = (Decision*)(sm + L.dec);
+    if (tid == 0) {
+        *dec = Decision{};
+        dec->thr_abs = a.stop_rule == 0 ? a.tol * a.tol : 0.0;
+        dec->thr_check = dec->best_trn = INFINITY;
+        dec->true_rel = -1.0;
+        dec->stop = -1;
+        dec->first = 1;
+    }
     int cb = 0;  // current copy of the coarse state
-    double best_trn = INFINITY;  // mixed: smallest FP64 residual seen at a replacement
-    int stall = 0;               // replacements since it last halved
-    int it = 0, stop = -1, xupd = 0, xupd_ref = 0, nru = 0;
-    double final_res = 0.0, true_rel = -1.0;
-    bool first = true;
+    int it = 0;
+
+    // x += alpha p of the last update, for the resident groups: due
+    // (pending) until flush()
+    double alpha = 0.0;
+    bool pending = false;
+    auto flush = [&]() {
+        if (!pending) return;
+        pending = false;
+        if constexpr (NG > 0) {
+#pragma unroll
+            for (int j = 0; j < NG; j++) {
+                const int n = (warp + j * nw) * kRowGroup + li, k = 3 * n + ld;
+                if (lact && n < no) x[k] = fma(alpha, (double)p[k], x[k]);
+            }
+        }
+    };
+    // x of every local node into xl: owned ones published and copied, ghosts
+    // polled; true when no wait gave up (all threads call it)
+    auto share_x = [&]() -> bool {
+        flush();
+        __syncthreads();  // x by its other layout of threads
+        for (int k = tid; k < 3 * no; k += nt) {
+            Tag<double>::put(a.llx + (size_t)(3 * gid[k / 3] + k % 3) * 2, x[k], xe);
+            xl[k] = x[k];
+        }
+        bool ok = true;
+        for (int k = 3 * no + tid; k < 3 * nloc && ok; k += nt) {
+            double xv = 0.0;
+            ok = poll<double>(a.llx + (size_t)(3 * gid[k / 3] + k % 3) * 2, xe, xv, wt);
+            xl[k] = xv;
+        }
+        xe++;
+        return !__syncthreads_or(!ok);
+    };
+    // f(n, constrained, row of P, (K x)_k) over this warp's owned groups; with
+    // `set` its result becomes r of the lanes' owned DOFs
+    auto each_true = [&](bool set, auto&& f) {
+        if constexpr (NG > 0) {
+#pragma unroll
+            for (int j = 0; j < NG; j++) {
+                const int grp = warp + j * nw, n = grp * kRowGroup + li;
+                if (grp < ngo) {
+                    double kx;
+                    if constexpr (MIXED) kx = true_row(grp);
+                    else kx = rows_reg(R[j], A, (const T*)xl, grp, (more >> j) & 1u);
+                    const T v = f(n, ((cbits >> j) & 1u) != 0, Pr[j], kx);
+                    if (set && lact && n < no) D[j].r = v;
+                }
+            }
+        }
+        for (int grp = warp + NG * nw; grp < ngo; grp += nw) {
+            const int n = grp * kRowGroup + li;
+            const bool own = lact && n < no, c = own && (cm[3 * n + ld] & 1);
+            Prow pr{0.0, 0.0, false, 0};
+            if (COARSE) pr = prow(n, own, c);
+            const T v = f(n, c, pr, true_row(grp));
+            if (set && own) r[3 * n + ld] = v;
+        }
+    };
 
     for (; status == ST_OK; it++) {
         const bool tr = it == a.trace_it && tid == 0;
         if (tr) a.trace[4 * g] = gtimer();
-        // ---- w = A u on owned rows ----
-        task_matvec<NPE, T, T>(u, yt, nta, ntm, tn, nta, kt, kstride);
-        __syncthreads();
-        clk.lap(0);
-        // ---- gather, BC rows, dot products, publish w ----
-        double v[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        // ---- w = A u on owned rows, BC rows, dot products, publish w ----
+        double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
         unsigned long long* vb = a.llv + (size_t)(e & 1) * N3 * 2;
         unsigned long long* pb = a.llp + (size_t)(e & 1) * kRep * a.G * 16;
-        for (int k = tid; k < 3 * no; k += nt) {
-            const int n = k / 3, d = k - 3 * n;
-            const int tb = tptr[n + 1];
-            T wk = T(0);
-            for (int t = tptr[n]; t < tb; t++) wk += yt[d * nta + t];
-            const bool c = cm[k] != 0;
-            const T uk = u[k], rk = r[k];
-            if (c) wk = uk;
-            w[k] = wk;
-            v[0] += (double)rk * (double)uk;
-            v[1] += (double)wk * (double)uk;
-            v[2] += (double)rk * (double)rk;
-            Tag<T>::put(vb + (size_t)(3 * gid[n] + d) * TW, wk, e);
-            if (a.coarse && !c) {
-                const T* bs = nb + 3 * n;  // dx, dy, 1/h
-                const double wd = (double)wk;
-                if (d == 0) {
-                    v[3] += wd;
-                    v[4] += (double)bs[1] * wd;
-                    v[5] += (double)bs[0] * wd;
-                } else if (d == 1) {
-                    v[4] += (double)bs[2] * wd;
-                } else {
-                    v[5] -= (double)bs[2] * wd;
-                }
+        each_row(u, ngo, [&](int n, Dof<T>& o, bool c, const Prow& pr, T wk) {
+            if (lact && n < no) {
+                if (c) wk = o.u;
+                o.w = wk;
+                if (n >= res0) w[3 * n + ld] = wk;
+                // only nodes that another part reads
+                if (NG > 0 && n < res0 ? (sbits & 1u) != 0 : (cm[3 * n + ld] & 2) != 0)
+                    Tag<T>::put(vb + (size_t)(3 * gid[n] + ld) * TW, wk, e);
+                v[0] += (double)o.r * (double)o.u;
+                v[1] += (double)wk * (double)o.u;
+                v[2] += (double)o.r * (double)o.r;
+                if (COARSE) restrict_dof(pr, (double)wk, v + 3);
             }
-        }
-        clk.lap(1);
-        if (a.coarse) {
-            block_publish<8>(v, red, pb, a.G, g, 6, e);
+        });
+        clk.lap(0);
+        if (COARSE) {
+            sum_publish<6>(v, red, pb, a.G, g, e);
         } else {
-            double v4[4] = {v[0], v[1], v[2], 0.0};
-            block_publish<4>(v4, red, pb, a.G, g, 3, e);
+            const double v3[3] = {v[0], v[1], v[2]};
+            sum_publish<3>(v3, red, pb, a.G, g, e);
         }
         if (tr) a.trace[4 * g + 1] = gtimer();
         clk.lap(2);
-        // ---- exchange: every block's partials and this block's ghost w ----
-        {
-            bool ok = exchange_round<T, XS>(pb, a.G, KP, vb, w, no, nloc, gid, g, e, sp, wt);
+        flush();
+        // ---- exchange and decision: warps 0 .. 2 the three dot products, the
+        //      others the ghosts' w and the coarse partials; then warp 0 decides
+        //      while the rest apply A_c^-1 to this round's P^T w ----
+        const int wd = nw > 3 ? 3 : 0;  // first of the other warps (0: too few, every warp takes its share)
+        if (warp >= wd) {
+            const int st = nt - 32 * wd, t0 = tid - 32 * wd;
+            const int items = 3 * (nloc - no) + (COARSE ? 3 * a.G : 0);
+            const bool ok = items <= 2 * st
+                ? poll_ghosts<T, 2>(pb, a.G, COARSE ? 3 : 0, vb, w, no, nloc, gid, g, e, sp, t0, st, wt)
+                : poll_ghosts<T, 4>(pb, a.G, COARSE ? 3 : 0, vb, w, no, nloc, gid, g, e, sp, t0, st, wt);
+            if (!ok) ctl[2] = 1;
+        }
+        double inv_g = 0.0, inv_a = 0.0, check = 0.0;
+        int nupd = 0, nref = 0;
+        if (warp < 3) {
+            if (warp == 0) {  // the decision's state, loaded while the block waits
+                inv_g = dec->inv_gamma;
+                inv_a = dec->inv_alpha;
+                check = dec->thr_check;
+                nupd = dec->xupd;
+                nref = dec->xupd_ref;
+            }
+            double d = 0.0;
+            bool ok = true;
+            for (int k = warp; k < 3; k += min(nw, 3)) {
+                ok = poll_total(pb, a.G, g, dot_copies(COARSE), k, e, d, wt) && ok;
+                if (lane == 0) scal[k] = d;
+            }
             if (a.test_stall && it == 0 && tid == 0) {
                 double never;  // a tag no block writes: the wait must run out
                 ok = ok && poll<double>(a.llp + (size_t)kRep * a.G * 32, 0xffffffffu, never, wt);
             }
-            if (__syncthreads_or(!ok)) { status = ST_TIMEOUT; break; }
-            sum_partials<3>(sp, a.G, KP, scal);
+            if (!ok) ctl[2] = 1;
+            asm volatile("bar.sync 2, %0;" ::"r"(32 * min(nw, 3)) : "memory");
         }
-        e++;
+        if (COARSE && (warp > 0 || nw == 1)) {
+            asm volatile("bar.sync 1, %0;" ::"r"(nw == 1 ? 32 : nt - 32) : "memory");
+            coarse_apply<T>(Ai, a.G, rows, sp, 3, 0, qw, nw == 1 ? 0 : 1);
+        }
         clk.lap(4);
-        // ---- decisions: thread 0 decides (warp 0 just summed the partials),
-        //      the block follows after one barrier ----
-        __syncwarp();
-        if (tid == 0) {
+        if (warp == 0) {
+            const bool ok = ctl[2] == 0;  // the others' waits are checked behind the barrier
             const double gamma = scal[0], delta = scal[1], rho = scal[2];
+            const double beta = gamma * inv_g;
+            const double pap = fma(-beta * gamma, inv_a, delta);
+            const double al = gamma * recip(pap);
             int act = ACT_UPDATE;
-            if (!isfinite(gamma) || !isfinite(delta) || !isfinite(rho)) {
-                if (g == 0) {
-                    a.res->nonfinite_it = it;
-                    a.res->nonfinite_vals[0] = gamma;
-                    a.res->nonfinite_vals[1] = delta;
-                    a.res->nonfinite_vals[2] = rho;
-                }
-                act = ACT_NONFINITE;
-            } else if (first && rho < 1e-60) {
-                bnorm = sqrt(rho);
-                stop = STOP_ZERO_RHS; final_res = 0.0; true_rel = 0.0; act = ACT_STOP;
-            } else {
-                // ||r|| < tol  <=>  rho < tol^2, and so on for the other tests
-                if (first) {
-                    bnorm = sqrt(rho);
-                    rn_ref = bnorm;
-                    thr_rel = a.tol * bnorm * (a.tol * bnorm);
-                    thr_ru = a.reliable_delta * rn_ref * (a.reliable_delta * rn_ref);
-                } else {
-                    const bool conv = (a.stop_rule == 0 && rho < thr_abs) || rho < thr_rel;
-                    if (MIXED && (conv || rho <= thr_ru || xupd - xupd_ref >= a.reliable_interval))
-                        act = ACT_RU;
-                    else if (!MIXED && conv) {
-                        stop = STOP_CONVERGED; final_res = sqrt(rho); act = ACT_STOP;
-                    }
-                }
-                if (act == ACT_UPDATE && xupd >= a.maxit) {
-                    stop = STOP_MAX_ITER; final_res = sqrt(rho); act = ACT_STOP;
-                }
-                if (act == ACT_UPDATE) {
-                    const double beta = first ? 0.0 : gamma * inv_gamma;
-                    const double pap = first ? delta : delta - beta * gamma * inv_alpha;
-                    if (fabs(pap) < 1e-30) {
-                        stop = STOP_BREAKDOWN; xupd++; final_res = sqrt(rho); act = ACT_STOP;
+            // the common case in one test: finite sums, no stop, no
+            // replacement due, no breakdown
+            const double sum = fabs(gamma) + fabs(delta) + rho;
+            if (!(sum < 1e300 && rho > check && fabs(pap) >= 1e-30 && nupd < a.maxit && ok) ||
+                (MIXED && nupd - nref >= a.reliable_interval)) {
+                if (lane == 0) {
+                    int stop = -1;
+                    if (!ok) {
+                        act = ACT_TIMEOUT;
+                    } else if (!isfinite(gamma) || !isfinite(delta) || !isfinite(rho)) {
+                        if (g == 0) {
+                            a.res->nonfinite_it = it;
+                            a.res->nonfinite_vals[0] = gamma;
+                            a.res->nonfinite_vals[1] = delta;
+                            a.res->nonfinite_vals[2] = rho;
+                        }
+                        act = ACT_NONFINITE;
+                    } else if (dec->first && rho < 1e-60) {
+                        dec->bnorm = sqrt(rho);
+                        dec->true_rel = 0.0;
+                        stop = STOP_ZERO_RHS;
                     } else {
-                        // two independent reciprocals; only alpha gates the barrier
-                        const double alpha = gamma * recip(pap);
-                        inv_gamma = recip(gamma);
-                        inv_alpha = pap * inv_gamma;
-                        first = false;
-                        xupd++;
-                        scal[3] = alpha;
-                        scal[4] = beta;
+                        // ||r|| < tol  <=>  rho < tol^2, and so on for the other tests
+                        if (dec->first) {
+                            const double bn = sqrt(rho);
+                            dec->bnorm = bn;
+                            dec->thr_rel = a.tol * bn * (a.tol * bn);
+                            dec->thr_ru = a.reliable_delta * bn * (a.reliable_delta * bn);
+                            dec->thr_check = fmax(fmax(dec->thr_abs, dec->thr_rel), MIXED ? dec->thr_ru : 0.0);
+                        } else {
+                            const bool conv = rho < dec->thr_abs || rho < dec->thr_rel;
+                            if (MIXED && (conv || rho <= dec->thr_ru || dec->xupd - dec->xupd_ref >= a.reliable_interval))
+                                act = ACT_RU;
+                            else if (!MIXED && conv)
+                                stop = STOP_CONVERGED;
+                        }
+                        if (act == ACT_UPDATE && stop < 0 && dec->xupd >= a.maxit) stop = STOP_MAX_ITER;
+                        if (act == ACT_UPDATE && stop < 0 && fabs(pap) < 1e-30) {
+                            stop = STOP_BREAKDOWN;
+                            dec->xupd++;
+                        }
                     }
+                    if (stop >= 0) {
+                        act = ACT_STOP;
+                        dec->stop = stop;
+                        dec->final_res = stop == STOP_ZERO_RHS ? 0.0 : sqrt(rho);
+                    }
+                    ctl[1] = act == ACT_STOP && dec->true_rel < 0.0;
                 }
             }
-            ctl[0] = act;
-            ctl[1] = (act == ACT_STOP && true_rel < 0.0) ? 1 : 0;
+            if (lane == 0) {
+                scal[3] = al;
+                scal[4] = beta;
+                ctl[0] = act;
+            }
             clk.lap(6);
+            __syncthreads();
+            if (lane == 0 && act == ACT_UPDATE) {
+                // off the barrier's path: the reciprocals of the next decision
+                dec->first = 0;
+                dec->xupd = nupd + 1;
+                const double ig = recip(gamma);
+                dec->inv_gamma = ig;
+                dec->inv_alpha = pap * ig;
+            }
+        } else {
+            __syncthreads();
         }
-        // meanwhile warps 1.. apply A_c^-1 to this round's P^T w
-        if (a.coarse) coarse_apply<T>(Ai, a.G, rows, sp, 6, 3, qw, 1);
-        __syncthreads();
-        const int act = ctl[0];
+        e++;
+        const int act = ctl[2] ? ACT_TIMEOUT : ctl[0];
         if (tr) a.trace[4 * g + 2] = gtimer();
+        if (act == ACT_TIMEOUT) { status = ST_TIMEOUT; break; }
         if (act == ACT_NONFINITE) { status = ST_NONFINITE; break; }
         if (act == ACT_STOP) break;
         clk.lap(5);
 
         if (MIXED && act == ACT_RU) {
             // ---- reliable update: r = F - K x in FP64 ----
-            for (int n = tid; n < no; n += nt)
-#pragma unroll
-                for (int d = 0; d < 3; d++)
-                    Tag<double>::put(a.llx + (size_t)(3 * gid[n] + d) * 2, x[3 * n + d], xe);
-            bool ok = true;
-            for (int k = tid; k < 3 * nloc && ok; k += nt) {
-                if (k < 3 * no) { xl[k] = x[k]; continue; }
-                double xv;
-                ok = poll<double>(a.llx + (size_t)(3 * gid[k / 3] + k % 3) * 2, xe, xv, wt);
-                xl[k] = xv;
-            }
-            if (__syncthreads_or(!ok)) { status = ST_TIMEOUT; break; }
-            xe++;
-            task_matvec<NPE, double, double>(xl, ytd, ntm, ntm, tn, nta, a.kt64 + t0, (size_t)a.NT);
-            __syncthreads();
+            if (!share_x()) { status = ST_TIMEOUT; break; }
             double vt[4] = {0.0, 0.0, 0.0, 0.0};
-            const int KR = a.coarse ? 4 : 1;
+            const int KR = COARSE ? 4 : 1;
             unsigned long long* rb = a.llv + (size_t)(e & 1) * N3 * 2;
-            unsigned long long* qb = a.llp + (size_t)(e & 1) * kRep * a.G * 16;
-            for (int n = tid; n < no; n += nt) {
-                double kx[3], rtv[3];
-                gather3(ytd, ntm, tptr[n], tptr[n + 1], kx[0], kx[1], kx[2]);
-                const int G3 = 3 * gid[n];
-#pragma unroll
-                for (int d = 0; d < 3; d++) {
-                    const int k = 3 * n + d;
-                    const double rt = cm[k] ? -xl[k] : (double)a.F[G3 + d] - kx[d];
-                    vt[0] += rt * rt;
-                    rtv[d] = rt;
-                    r[k] = (T)rt;
-                    Tag<T>::put(rb + (size_t)(G3 + d) * TW, (T)rt, e);
-                }
-                if (a.coarse) restrict3(rtv, cm + 3 * n, nb + 3 * n, vt + 1);
-            }
-            block_publish<4>(vt, red, qb, a.G, g, KR, e);
-            ok = exchange_round<T, XS>(qb, a.G, KR, rb, r, no, nloc, gid, g, e, sp, wt);
+            unsigned long long* qbuf = a.llp + (size_t)(e & 1) * kRep * a.G * 16;
+            each_true(true, [&](int n, bool c, const Prow& pr, double kx) -> T {
+                if (!lact || n >= no) return T(0);
+                const int G3 = 3 * gid[n] + ld;
+                const double rt = c ? -xl[3 * n + ld] : (double)a.F[G3] - kx;
+                vt[0] += rt * rt;
+                Tag<T>::put(rb + (size_t)G3 * TW, (T)rt, e);
+                if (COARSE) restrict_dof(pr, rt, vt + 1);
+                return (T)rt;
+            });
+            block_publish<4>(vt, red, qbuf, a.G, g, KR, e);
+            // the ghosts' r arrive in w (xl, in the same space, is dead now)
+            const bool ok = exchange_round<T>(qbuf, a.G, KR, rb, w, no, nloc, gid, g, e, sp, wt);
             if (__syncthreads_or(!ok)) { status = ST_TIMEOUT; break; }
             sum_partials<1>(sp, a.G, KR, scal);
             // c = A_c^-1 P^T r from the true residual (cs is unchanged)
-            if (a.coarse) coarse_apply<T>(Ai, a.G, rows, sp, 4, 1, cvb + cb * rows, 0);
+            if (COARSE) coarse_apply<T>(Ai, a.G, rows, sp, 4, 1, cvb + cb * rows, 0);
             __syncthreads();
             e++;
-            for (int n = tid; n < nloc; n += nt) {
-                block_jacobi3(B + 9 * n, r + 3 * n, u + 3 * n);
-                if (a.coarse && !cheb)
-                    prolong3(cvb + cb * rows + 3 * nslot[n], cm + 3 * n, nb + 3 * n, u + 3 * n);
+            auto coarse_c = [&](const Prow& pr) { return cvb[cb * rows + pr.q + ld]; };
+            auto restart = [&](int n, Dof<T>& o, const Prow& pr) {
+                const bool live = lact && n < nloc;
+                if (live && n >= no) o.r = w[3 * n + ld];
+                T z = jacobi_lane(o.b, o.r);
+                if (COARSE && !CHEB) z += prolong(pr, coarse_c(pr));
+                if (live) (CHEB ? t : u)[3 * n + ld] = z;
+                o.u = z;
+            };
+            if constexpr (NG > 0) {
+#pragma unroll
+                for (int j = 0; j < NG; j++) restart((warp + j * nw) * kRowGroup + li, D[j], Pr[j]);
             }
-            if (cheb) {
+            for (int grp = warp + NG * nw; grp < ngl; grp += nw) {
+                const int n = grp * kRowGroup + li;
+                Dof<T> o;
+                const bool live = lact && n < nloc, c = get_dof(n, live, o);
+                Prow pr{0.0, 0.0, false, 0};
+                if (COARSE && !CHEB) pr = prow(n, live, c);
+                restart(n, o, pr);
+                if (live) r[3 * n + ld] = o.r;
+            }
+            if (CHEB) {
                 __syncthreads();
-                task_matvec<NPE, T, T>(u, yt, nta, nta, tn, nta, kt, kstride, ksplit, ktg + t0, (size_t)a.NT);
-                __syncthreads();
-                for (int n = tid; n < nn1; n += nt) {
-                    smooth_node(u + 3 * n, yt, nta, tptr[n], tptr[n + 1], B + 9 * n, cm + 3 * n, ca, cbc);
-                    if (a.coarse)
-                        prolong3(cvb + cb * rows + 3 * nslot[n], cm + 3 * n, nb + 3 * n, u + 3 * n);
-                }
+                smooth(coarse_c);
             }
             if (tid == 0) {
                 const double trn = sqrt(scal[0]);
-                int act2 = ACT_UPDATE;
-                nru++;
-                rn_ref = trn;
-                thr_ru = a.reliable_delta * rn_ref * (a.reliable_delta * rn_ref);
-                xupd_ref = xupd;
+                int stop = -1;
+                ctl[0] = ACT_UPDATE;
+                ctl[1] = 0;
+                dec->nru++;
+                dec->thr_ru = a.reliable_delta * trn * (a.reliable_delta * trn);
+                dec->thr_check = fmax(fmax(dec->thr_abs, dec->thr_rel), dec->thr_ru);
+                dec->xupd_ref = dec->xupd;
                 if (!isfinite(trn)) {
-                    act2 = ACT_NONFINITE;
-                } else if ((a.stop_rule == 0 && trn < a.tol) || trn / bnorm < a.tol) {
-                    stop = STOP_CONVERGED; final_res = trn; true_rel = trn / bnorm; act2 = ACT_STOP;
-                } else if (xupd >= a.maxit) {
-                    stop = STOP_MAX_ITER; final_res = trn; true_rel = trn / bnorm; act2 = ACT_STOP;
-                } else if (trn < 0.5 * best_trn) {
-                    best_trn = trn;
-                    stall = 0;
-                } else if (++stall >= 3) {
+                    ctl[0] = ACT_NONFINITE;
+                } else if ((a.stop_rule == 0 && trn < a.tol) || trn / dec->bnorm < a.tol) {
+                    stop = STOP_CONVERGED;
+                } else if (dec->xupd >= a.maxit) {
+                    stop = STOP_MAX_ITER;
+                } else if (trn < 0.5 * dec->best_trn) {
+                    dec->best_trn = trn;
+                    dec->stall = 0;
+                } else if (++dec->stall >= 3) {
                     // three replacements in a row without halving the FP64
                     // residual: the FP32 inner iterations no longer reduce
                     // the error (condition number near 1 / FP32 epsilon)
-                    stop = STOP_STAGNATED; final_res = trn; true_rel = trn / bnorm; act2 = ACT_STOP;
+                    stop = STOP_STAGNATED;
                 }
-                ctl[0] = act2;
-                ctl[1] = 0;
+                if (stop >= 0) {
+                    ctl[0] = ACT_STOP;
+                    dec->stop = stop;
+                    dec->final_res = trn;
+                    dec->true_rel = trn / dec->bnorm;
+                }
             }
             __syncthreads();
             if (ctl[0] == ACT_NONFINITE) { status = ST_NONFINITE; break; }
@@ -1312,173 +1697,110 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& a, const int g, unsigned
         //      P^T r_new = P^T r - alpha P^T s give cs = qw + beta cs and
         //      c_new = c - alpha cs, so u = M_bj r_new + P c_new needs no
         //      coarse solve after the decision ----
-        const double alpha = scal[3], beta = scal[4];
+        alpha = scal[3];
+        const double beta = scal[4];
         const T bt = (T)beta, at = (T)alpha;
-        if (cheb) {
-            // s, r on every local node, p and x on owned nodes, t = D^-1 r
-            // into u; then K t on owned and ring-1 rows and
-            // u = a t - b D^-1 K t (+ P c_new, c by the recurrences below)
-            const double* cso = csb + cb * rows;
-            const double* cvo = cvb + cb * rows;
-            if (a.coarse && tid < rows) {
-                const double c1 = __fma_rn(beta, cso[tid], qw[tid]);
-                csb[(cb ^ 1) * rows + tid] = c1;
-                cvb[(cb ^ 1) * rows + tid] = __fma_rn(-alpha, c1, cvo[tid]);
-            }
-            for (int n = tid; n < nloc; n += nt) {
-                T rv[3];
+        const double* cso = csb + cb * rows;
+        const double* cvo = cvb + cb * rows;
+        for (int q = tid; q < rows; q += nt) {
+            const double c1 = __fma_rn(beta, cso[q], qw[q]);
+            csb[(cb ^ 1) * rows + q] = c1;
+            cvb[(cb ^ 1) * rows + q] = __fma_rn(-alpha, c1, cvo[q]);
+        }
+        // c_new of this lane's node, value m = lane % 3 (by the recurrences)
+        auto c_new = [&](const Prow& pr) -> double {
+            const int q = pr.q + ld;
+            return __fma_rn(-alpha, __fma_rn(beta, cso[q], qw[q]), cvo[q]);
+        };
+        // s, r on every local node; D^-1 r (+ P c_new) into u, or with the
+        // Chebyshev smoother t = D^-1 r
+        auto update = [&](int n, Dof<T>& o, const Prow& pr) {
+            o.s = fma(bt, o.s, o.w);
+            o.r = fma(-at, o.s, o.r);
+            T z = jacobi_lane(o.b, o.r);
+            if (COARSE && !CHEB) z += prolong(pr, c_new(pr));
+            if (lact && n < nloc) (CHEB ? t : u)[3 * n + ld] = z;
+            o.u = z;
+        };
+        if constexpr (NG > 0) {
 #pragma unroll
-                for (int d = 0; d < 3; d++) {
-                    const int k = 3 * n + d;
-                    const T sk = w[k] + bt * s[k];
-                    s[k] = sk;
-                    if (n < no) {
-                        const T pk = u[k] + bt * p[k];
-                        p[k] = pk;
-                        x[k] += alpha * (double)pk;
-                    }
-                    rv[d] = r[k] - at * sk;
-                    r[k] = rv[d];
-                }
-                block_jacobi3(B + 9 * n, rv, u + 3 * n);
+            for (int j = 0; j < NG; j++) {
+                const int n = (warp + j * nw) * kRowGroup + li;
+                if (lact && n >= no && n < nloc) D[j].w = w[3 * n + ld];  // a ghost's w
+                if (lact && n < no) p[3 * n + ld] = fma(bt, p[3 * n + ld], D[j].u);
+                update(n, D[j], Pr[j]);
             }
-            __syncthreads();
-            clk.lap(7);
-            task_matvec<NPE, T, T>(u, yt, nta, nta, tn, nta, kt, kstride, ksplit, ktg + t0, (size_t)a.NT);
+            pending = true;
+        }
+        for (int grp = warp + NG * nw; grp < ngl; grp += nw) {
+            const int n = grp * kRowGroup + li, k = 3 * n + ld;
+            const bool live = lact && n < nloc;
+            Dof<T> o;
+            const bool c = get_dof(n, live, o);
+            if (live && n < no) {
+                const T pk = fma(bt, p[k], o.u);
+                p[k] = pk;
+                x[k] = fma(alpha, (double)pk, x[k]);
+            }
+            Prow pr{0.0, 0.0, false, 0};
+            if (COARSE && !CHEB) pr = prow(n, live, c);
+            update(n, o, pr);
+            if (live) {
+                s[k] = o.s;
+                r[k] = o.r;
+            }
+        }
+        __syncthreads();
+        clk.lap(7);
+        if (CHEB) {
+            smooth(c_new);
             __syncthreads();
             clk.lap(3);
-            for (int n = tid; n < nn1; n += nt) {
-                smooth_node(u + 3 * n, yt, nta, tptr[n], tptr[n + 1], B + 9 * n, cm + 3 * n, ca, cbc);
-                if (a.coarse) {
-                    const int sl = 3 * nslot[n];
-                    double c3[3];
-#pragma unroll
-                    for (int m = 0; m < 3; m++)
-                        c3[m] = __fma_rn(-alpha, __fma_rn(beta, cso[sl + m], qw[sl + m]), cvo[sl + m]);
-                    prolong3(c3, cm + 3 * n, nb + 3 * n, u + 3 * n);
-                }
-            }
-            if (a.coarse) cb ^= 1;
-            __syncthreads();
-            clk.lap(7);
-            if (tr) a.trace[4 * g + 3] = gtimer();
-        } else if (a.coarse) {
-            const double* cso = csb + cb * rows;
-            const double* cvo = cvb + cb * rows;
-            if (tid < rows) {
-                const double c1 = __fma_rn(beta, cso[tid], qw[tid]);
-                csb[(cb ^ 1) * rows + tid] = c1;
-                cvb[(cb ^ 1) * rows + tid] = __fma_rn(-alpha, c1, cvo[tid]);
-            }
-            for (int n = tid; n < nloc; n += nt) {
-                T rv[3];
-#pragma unroll
-                for (int d = 0; d < 3; d++) {
-                    const int k = 3 * n + d;
-                    const T pk = u[k] + bt * p[k];
-                    const T sk = w[k] + bt * s[k];
-                    p[k] = pk;
-                    s[k] = sk;
-                    if (n < no) x[k] += alpha * (double)pk;
-                    rv[d] = r[k] - at * sk;
-                    r[k] = rv[d];
-                }
-                block_jacobi3(B + 9 * n, rv, u + 3 * n);
-                const int sl = 3 * nslot[n];
-                double c3[3];
-#pragma unroll
-                for (int m = 0; m < 3; m++)
-                    c3[m] = __fma_rn(-alpha, __fma_rn(beta, cso[sl + m], qw[sl + m]), cvo[sl + m]);
-                prolong3(c3, cm + 3 * n, nb + 3 * n, u + 3 * n);
-            }
-            cb ^= 1;
-            __syncthreads();
-            clk.lap(7);
-            if (tr) a.trace[4 * g + 3] = gtimer();
-        } else {
-            // p, s, x, r updates and u = M_bj r on owned and ghost nodes
-            for (int n = tid; n < nloc; n += nt) {
-                T rv[3];
-#pragma unroll
-                for (int d = 0; d < 3; d++) {
-                    const int k = 3 * n + d;
-                    const T pk = u[k] + bt * p[k];
-                    const T sk = w[k] + bt * s[k];
-                    p[k] = pk;
-                    s[k] = sk;
-                    if (n < no) x[k] += alpha * (double)pk;
-                    rv[d] = r[k] - at * sk;
-                    r[k] = rv[d];
-                }
-                block_jacobi3(B + 9 * n, rv, u + 3 * n);
-            }
-            __syncthreads();
-            clk.lap(7);
-            if (tr) a.trace[4 * g + 3] = gtimer();
         }
+        if (COARSE) cb ^= 1;
+        if (tr) a.trace[4 * g + 3] = gtimer();
     }
 
     // ---- write x; FP64 true residual ||F - K x|| unless already known ----
-    for (int n = tid; n < no; n += nt)
-#pragma unroll
-        for (int d = 0; d < 3; d++) a.x[3 * gid[n] + d] = x[3 * n + d];
+    flush();
+    __syncthreads();
+    for (int k = tid; k < 3 * no; k += nt) a.x[3 * gid[k / 3] + k % 3] = x[k];
     if (status == ST_OK && ctl[1]) {
-        for (int n = tid; n < no; n += nt)
-#pragma unroll
-            for (int d = 0; d < 3; d++)
-                Tag<double>::put(a.llx + (size_t)(3 * gid[n] + d) * 2, x[3 * n + d], xe);
-        bool ok = true;
-        for (int k = tid; k < 3 * nloc && ok; k += nt) {
-            if (k < 3 * no) { xl[k] = x[k]; continue; }
-            double xv;
-            ok = poll<double>(a.llx + (size_t)(3 * gid[k / 3] + k % 3) * 2, xe, xv, wt);
-            xl[k] = xv;
-        }
-        if (__syncthreads_or(!ok)) {
+        if (!share_x()) {
             status = ST_TIMEOUT;
         } else {
-            if (MIXED || !a.ke_smem)
-                task_matvec<NPE, double, double>(xl, ytd, ntm, ntm, tn, nta, a.kt64 + t0, (size_t)a.NT);
-            else
-                task_matvec<NPE, double, double>(xl, ytd, ntm, ntm, tn, nta, (const double*)kts, kstride);
-            __syncthreads();
             double v[2] = {0.0, 0.0};
-            for (int n = tid; n < no; n += nt) {
-                double kx[3];
-                gather3(ytd, ntm, tptr[n], tptr[n + 1], kx[0], kx[1], kx[2]);
-                const int G3 = 3 * gid[n];
-#pragma unroll
-                for (int d = 0; d < 3; d++) {
-                    const int k = 3 * n + d;
-                    const double f = cm[k] ? 0.0 : (double)a.F[G3 + d];
-                    const double rt = cm[k] ? -xl[k] : f - kx[d];
-                    v[0] += rt * rt;
-                    v[1] += f * f;
-                }
-            }
+            each_true(false, [&](int n, bool c, const Prow&, double kx) -> T {
+                if (!lact || n >= no) return T(0);
+                const double f = c ? 0.0 : (double)a.F[3 * gid[n] + ld];
+                const double rt = c ? -xl[3 * n + ld] : f - kx;
+                v[0] += rt * rt;
+                v[1] += f * f;
+                return T(0);
+            });
             unsigned long long* pb = a.llp + (size_t)(e & 1) * kRep * a.G * 16;
             block_publish<2>(v, red, pb, a.G, g, 2, e);
             if (g == 0) {
-                ok = exchange_round<T, XS>(pb, a.G, 2, nullptr, w, no, no, gid, g, e, sp, wt);
+                const bool ok = exchange_round<T>(pb, a.G, 2, nullptr, w, no, no, gid, g, e, sp, wt);
                 if (__syncthreads_or(!ok)) {
                     status = ST_TIMEOUT;
                 } else {
                     sum_partials<2>(sp, a.G, 2, scal);
                     __syncthreads();
-                    if (tid == 0) true_rel = scal[1] > 0 ? sqrt(scal[0] / scal[1]) : 0.0;
+                    if (tid == 0) dec->true_rel = scal[1] > 0 ? sqrt(scal[0] / scal[1]) : 0.0;
                 }
             }
         }
     }
     if (g == 0 && tid == 0) {
         a.res->status = status;
-        a.res->iterations = xupd;
-        a.res->converged = (stop == STOP_CONVERGED || stop == STOP_ZERO_RHS) ? 1 : 0;
-        a.res->stop_reason = stop < 0 ? STOP_MAX_ITER : stop;
-        a.res->final_residual = final_res;
-        a.res->true_rel_residual = true_rel < 0.0 ? 0.0 : true_rel;
-        a.res->b_norm = bnorm;
-        a.res->reliable_updates = nru;
+        a.res->iterations = dec->xupd;
+        a.res->converged = (dec->stop == STOP_CONVERGED || dec->stop == STOP_ZERO_RHS) ? 1 : 0;
+        a.res->stop_reason = dec->stop < 0 ? STOP_MAX_ITER : dec->stop;
+        a.res->final_residual = dec->final_res;
+        a.res->true_rel_residual = dec->true_rel < 0.0 ? 0.0 : dec->true_rel;
+        a.res->b_norm = dec->bnorm;
+        a.res->reliable_updates = dec->nru;
         a.res->reductions = (int)(e - 1 - a.tag0);
         a.res->last_tag = e > xe ? e : xe;
         for (int k = 0; k < 8; k++) a.res->phase_cycles[k] = clk.on ? clk.t[k] : 0;
@@ -1486,14 +1808,15 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& a, const int g, unsigned
 }
 
 // One plate on the whole grid: part g = block g; MAXT: the launch bound.
-template <int NPE, typename T, bool MIXED, int MAXT>
+// COARSE / CHEB: the two-level preconditioner and the Chebyshev smoother, as
+// template arguments: what a method does not use takes no registers.
+template <typename T, bool MIXED, int MAXT, bool COARSE, bool CHEB>
 __global__ void __launch_bounds__(MAXT, 1) pcg_kernel(const __grid_constant__ PcgArgs a) {
     extern __shared__ __align__(16) unsigned char sm[];
-    pcg_body<NPE, T, MIXED>(a, blockIdx.x, sm);
+    pcg_body<T, MIXED, MAXT <= kLeanThreads ? kResident : 0, COARSE, CHEB>(a, blockIdx.x, sm);
 }
 
-// Many independent plates of one element type (NPE) in one launch.  The
-// grid is cut into teams of consecutive blocks; teams of one size form a
+// Many independent plates in one launch.  The grid is cut into teams of consecutive blocks; teams of one size form a
 // class with one queue of plates (largest estimated work first).  A free
 // team takes its class's next plate: team block 0 claims a queue position
 // with an atomic counter and logs it in the team's claim slot k (tag
@@ -1517,7 +1840,7 @@ struct BatchArgs {
     unsigned long long timeout_ns;  // limit of one wait for a claim
 };
 
-template <int NPE, typename T, bool MIXED>
+template <typename T, bool MIXED, bool COARSE, bool CHEB>
 __global__ void __launch_bounds__(kBatchThreads, 1) pcg_batch_kernel(const __grid_constant__ BatchArgs b) {
     extern __shared__ __align__(16) unsigned char sm[];
     volatile int* s_plate = (volatile int*)sm;  // between plates the shared memory is free
@@ -1554,10 +1877,20 @@ __global__ void __launch_bounds__(kBatchThreads, 1) pcg_batch_kernel(const __gri
         const int pi = *s_plate;
         __syncthreads();  // read by all before the plate's data overwrite it
         if (pi < 0) break;
-        const PcgArgs& a = b.plates[pi];
+        // the plate's arguments, read all through the solve
+        PcgArgs& a = *(PcgArgs*)sm;  // (the layouts leave the space)
+        for (int i = threadIdx.x; i < (int)(sizeof(PcgArgs) / 4); i += blockDim.x)
+            ((int*)&a)[i] = ((const int*)(b.plates + pi))[i];
+        __syncthreads();
         if (g == 0 && threadIdx.x == 0) b.times[2 * pi] = gtimer();
         // a plate with fewer parts than the team has blocks leaves the rest idle
-        if (g < a.G) pcg_body<NPE, T, MIXED, 2>(a, g, sm);
+        if (g < a.G) {
+            // with the smoother a plate on a 1-ring halo runs block Jacobi
+            if (CHEB && a.smoother)
+                pcg_body<T, MIXED, kResident, COARSE, CHEB>(a, g, sm);
+            else
+                pcg_body<T, MIXED, kResident, COARSE, false>(a, g, sm);
+        }
         __syncthreads();  // shared memory is reloaded for the next plate
         if (g == 0 && threadIdx.x == 0) b.times[2 * pi + 1] = gtimer();
     }

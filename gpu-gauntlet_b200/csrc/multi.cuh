@@ -1,9 +1,10 @@
 // Load cases of one plate solved together: NR right-hand sides of the same
 // operator advance in lockstep through one persistent launch.
 //
-// Every per-DOF vector of the single solve (r, u, p, s, w, x and the task
-// results) holds NR values per DOF, case-interleaved ([dof][case]), so the
-// element matvec reads each Ke coefficient once for NR vectors and the
+// Every per-DOF vector of the single solve (r, u, p, s, w, x and the row
+// products) holds NR values per DOF, case-interleaved ([dof][case]), so the
+// product reads each row block once for NR vectors (rows.cuh; a warp's first
+// group of rows from registers) and the
 // coarse correction applies each A_c^-1 row to NR restrictions.  One
 // exchange round per iteration carries every case's partial sums and ghost
 // values, so the grid-wide wait -- the dominant cost of a single 60k-DOF
@@ -38,51 +39,99 @@ struct alignas(sizeof(T) * NR <= 16 ? sizeof(T) * NR : 16) CaseVec {
     T v[NR];
 };
 
-// Task matvec for NR case-interleaved vectors: yt[(r * ys + t) * NR + k] =
-// row r of task t's block times case k of u.  Whole tasks, one per thread.
-template <int NPE, typename T, typename KT, int NR>
-__device__ __forceinline__ void task_matvec_multi(const T* __restrict__ u, T* __restrict__ yt, int ys,
-                                                  int count, const uint16_t* __restrict__ tn, int ts,
-                                                  const KT* __restrict__ kt, size_t stride,
-                                                  int ksplit = 1 << 30,
-                                                  const KT* __restrict__ kt2 = nullptr,
-                                                  size_t stride2 = 0) {
-    constexpr int ND = 3 * NPE;
+// s[r][k] += the blocks of q-steps [0, steps) at b (lane offset included) times
+// case k of u at the columns c.
+template <typename T, typename KT, int NR>
+__device__ __forceinline__ void row_steps_multi(const T* __restrict__ u, const uint16_t* __restrict__ c,
+                                                const KT* __restrict__ k, int steps, T (&s)[3][NR]) {
     using V = CaseVec<T, NR>;
-    for (int t = threadIdx.x; t < count; t += blockDim.x) {
-        const KT* kb = t < ksplit ? kt + t : kt2 + t;
-        const size_t ks = t < ksplit ? stride : stride2;
-        T a0[NR], a1[NR], a2[NR];
+#pragma unroll 1
+    for (int q = 0; q < steps; q++) {
+        const V* v = reinterpret_cast<const V*>(u) + 3 * (int)c[q * kRowLanes];
+        const V v0 = v[0], v1 = v[1], v2 = v[2];
+        const KT* b = k + q * 9 * kRowLanes;
 #pragma unroll
-        for (int k = 0; k < NR; k++) a0[k] = a1[k] = a2[k] = T(0);
+        for (int r = 0; r < 3; r++) {
+            const T k0 = (T)b[3 * r * kRowLanes], k1 = (T)b[(3 * r + 1) * kRowLanes], k2 = (T)b[(3 * r + 2) * kRowLanes];
 #pragma unroll
-        for (int j = 0; j < NPE; j++) {
-            const int b = 3 * (int)tn[j * ts + t];
+            for (int i = 0; i < NR; i++) s[r][i] = fma(k2, v2.v[i], fma(k1, v1.v[i], fma(k0, v0.v[i], s[r][i])));
+        }
+    }
+}
+
+// Writes the rows' products of one group to y ([3 rows][case]): lane 3 i + d
+// gets component d of row i of every case (rows.cuh).
+template <typename T, int NR>
+__device__ __forceinline__ void join_store(const T (&s)[3][NR], T* __restrict__ y, int grp, int nrows) {
+    const int lane = threadIdx.x & 31, n = grp * kRowGroup + lane / 3;
+    CaseVec<T, NR> o;
 #pragma unroll
-            for (int d = 0; d < 3; d++) {
-                const int c = 3 * j + d;
-                const T k0 = (T)kb[(size_t)(0 * ND + c) * ks];
-                const T k1 = (T)kb[(size_t)(1 * ND + c) * ks];
-                const T k2 = (T)kb[(size_t)(2 * ND + c) * ks];
-                const V uv = *reinterpret_cast<const V*>(u + (size_t)(b + d) * NR);
+    for (int i = 0; i < NR; i++) {
+        const T si[3] = {s[0][i], s[1][i], s[2][i]};
+        o.v[i] = row_join(si);
+    }
+    if (lane < kRowLanes && n < nrows) reinterpret_cast<CaseVec<T, NR>*>(y)[3 * n + lane % 3] = o;
+}
+
+// y = K u on the part's first nrows rows for NR case-interleaved vectors, one
+// warp a group of rows; each block entry is read once for all cases, a warp's
+// first group from registers.
+template <typename T, int NR>
+__device__ __forceinline__ void rows_multi(const RegRows<T>& R, const RowMem<T>& A, const T* __restrict__ u,
+                                           T* __restrict__ y, int nrows) {
+    using V = CaseVec<T, NR>;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int grp = warp; grp * kRowGroup < nrows; grp += nw) {
+        T s[3][NR];
 #pragma unroll
-                for (int k = 0; k < NR; k++) {
-                    a0[k] += k0 * uv.v[k];
-                    a1[k] += k1 * uv.v[k];
-                    a2[k] += k2 * uv.v[k];
-                }
+        for (int r = 0; r < 3; r++)
+#pragma unroll
+            for (int i = 0; i < NR; i++) s[r][i] = T(0);
+        const int q0 = A.gq[grp], w = A.gq[grp + 1] - q0;
+        int done = 0;
+        if (grp == warp) {
+            done = kRegSteps;
+#pragma unroll
+            for (int q = 0; q < kRegSteps; q++) {
+                const V* v = reinterpret_cast<const V*>(u) + R.c[q];
+                const V v0 = v[0], v1 = v[1], v2 = v[2];
+#pragma unroll
+                for (int r = 0; r < 3; r++)
+#pragma unroll
+                    for (int i = 0; i < NR; i++)
+                        s[r][i] = fma(R.k[9 * q + 3 * r + 2], v2.v[i],
+                                      fma(R.k[9 * q + 3 * r + 1], v1.v[i], fma(R.k[9 * q + 3 * r], v0.v[i], s[r][i])));
             }
         }
-        V o0, o1, o2;
-#pragma unroll
-        for (int k = 0; k < NR; k++) {
-            o0.v[k] = a0[k];
-            o1.v[k] = a1[k];
-            o2.v[k] = a2[k];
+        if (done < w && lane < kRowLanes) {
+            const int g0 = A.go[grp];
+            const uint16_t* cq = A.col + (q0 + done) * kRowLanes + lane;
+            if (g0 >= 0)
+                row_steps_multi<T, T, NR>(u, cq, A.ks + g0 * 9 * kRowLanes + lane, w - done, s);
+            else
+                row_steps_multi<T, T, NR>(u, cq, A.kg + (size_t)(q0 + done) * 9 * kRowLanes + lane, w - done, s);
         }
-        *reinterpret_cast<V*>(yt + ((size_t)0 * ys + t) * NR) = o0;
-        *reinterpret_cast<V*>(yt + ((size_t)1 * ys + t) * NR) = o1;
-        *reinterpret_cast<V*>(yt + ((size_t)2 * ys + t) * NR) = o2;
+        join_store<T, NR>(s, y, grp, nrows);
+    }
+}
+
+// The same in FP64 from global memory (the true residuals of mixed solves).
+template <int NR>
+__device__ __forceinline__ void rows_multi64(const int* __restrict__ gq, const uint16_t* __restrict__ col,
+                                             const double* __restrict__ kg, const double* __restrict__ u,
+                                             double* __restrict__ y, int nrows) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int grp = warp; grp * kRowGroup < nrows; grp += nw) {
+        double s[3][NR];
+#pragma unroll
+        for (int r = 0; r < 3; r++)
+#pragma unroll
+            for (int i = 0; i < NR; i++) s[r][i] = 0.0;
+        const int q0 = gq[grp];
+        if (lane < kRowLanes)
+            row_steps_multi<double, double, NR>(u, col + q0 * kRowLanes + lane, kg + (size_t)q0 * 9 * kRowLanes + lane,
+                                                gq[grp + 1] - q0, s);
+        join_store<double, NR>(s, y, grp, nrows);
     }
 }
 
@@ -233,15 +282,16 @@ struct CaseState {
     bool first, done, asked;
 };
 
-template <int NPE, typename T, bool MIXED, int NR>
+template <typename T, bool MIXED, int NR>
 __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, unsigned char* sm) {
-    constexpr int ND = 3 * NPE, TW = Tag<T>::W, SW = multi_slot_words<NR>();
+    constexpr int TW = Tag<T>::W, SW = multi_slot_words<NR>();
     const SmemLayout& L = a.L;
     const int tid = threadIdx.x, nt = blockDim.x, kc = tid % NR;
     const int lane = tid & 31;
     const int n0 = a.node_off[g], nloc = a.node_off[g + 1] - n0, no = a.nown[g];
-    const int t0 = a.task_off[g], nta = a.task_off[g + 1] - t0;
-    const int nn1 = a.n1[g], ntm = a.tptr[a.tp_off[g] + no];
+    const int nn1 = a.n1[g];
+    const int gb = a.grp_off[g], ng1 = a.grp_off[g + 1] - gb, qb = a.grp_q[gb];
+    const int warp = tid >> 5, nw = nt >> 5;
     const bool cheb = a.smoother == 1;
     const T ca = (T)a.cheb_a, cbc = (T)a.cheb_b;
     const size_t N3 = 3 * (size_t)a.Nn;
@@ -252,15 +302,16 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
     T* s = (T*)(sm + L.s);
     T* w = (T*)(sm + L.w);
     T* B = (T*)(sm + L.B);
-    T* yt = (T*)(sm + L.yt);
+    T* yt = (T*)(sm + L.yt);  // row products, [3 rows][case]
     T* kts = (T*)(sm + L.kt);
     double* x = (double*)(sm + L.x);
     double* red = (double*)(sm + L.red);
     double* scal = (double*)(sm + L.scal);  // [0, 3NR) dots, [3NR, 4NR) alpha, [4NR, 5NR) beta
     double* sp = (double*)(sm + L.sp);
     int* gid = (int*)(sm + L.gid);
-    int* tptr = (int*)(sm + L.tptr);
-    uint16_t* tn = (uint16_t*)(sm + L.tnode);
+    int* gq = (int*)(sm + L.gq);
+    int* go = (int*)(sm + L.go);
+    uint16_t* rcol = (uint16_t*)(sm + L.rcol);
     unsigned char* cm = (unsigned char*)(sm + L.cm);
     double* qw = (double*)(sm + L.qw);
     double* csb = (double*)(sm + L.cs);
@@ -279,22 +330,25 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
     // share the yt / w / u space), the (then dead) p / yt arrays in FP64
     double* xl = MIXED ? (double*)(sm + L.xl) : (double*)p;
     double* ytd = MIXED ? (double*)(sm + L.ytd) : (double*)yt;
-    const T* ktg = MIXED ? (const T*)a.kt32 : (const T*)a.kt64;
+    const T* kg = (MIXED ? (const T*)a.rk32 : (const T*)a.rk64) + (size_t)qb * 9 * kRowLanes;
+    const double* kg64 = a.rk64 + (size_t)qb * 9 * kRowLanes;
     const T* Bg = MIXED ? (const T*)a.binv32 : (const T*)a.binv64;
 
     // ---- load the part ----
     for (int i = tid; i < nloc; i += nt) gid[i] = a.nodes[n0 + i];
-    for (int i = tid; i <= nn1; i += nt) tptr[i] = a.tptr[a.tp_off[g] + i];
-    for (int i = tid; i < NPE * nta; i += nt) {
-        const int t = i % nta, j = i / nta;
-        tn[i] = a.task_nodes[(size_t)(t0 + t) * NPE + j];
-    }
-    const int nk = a.ke_smem == 2 ? nta : ntm;
-    if (a.ke_smem)
-        for (int i = tid; i < 3 * ND * nk; i += nt) {
-            const int t = i % nk, q = i / nk;
-            kts[i] = ktg[(size_t)q * a.NT + t0 + t];
+    for (int i = tid; i <= ng1; i += nt) gq[i] = a.grp_q[gb + i] - qb;
+    __syncthreads();
+    if (tid == 0) {
+        // the q-steps not in registers go to shared memory while they fit
+        int used = 0;
+        for (int k = 0; k < ng1; k++) {
+            const int need = max(0, gq[k + 1] - gq[k] - (k < nw ? kRegSteps : 0));
+            const bool fits = used + need <= L.kq;
+            go[k] = fits ? used : -1;
+            if (fits) used += need;
         }
+    }
+    for (int i = tid; i < gq[ng1] * kRowLanes; i += nt) rcol[i] = a.rcol[(size_t)qb * kRowLanes + i];
     if (a.coarse) {
         for (int i = tid; i < nloc; i += nt) {
             nslot[i] = a.node_slot[n0 + i];
@@ -306,6 +360,26 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
             for (int i = tid; i < rows * a.C; i += nt) ais[i] = aig[i];
     }
     __syncthreads();
+    const RowMem<T> A{gq, go, rcol, kts, kg};
+    RegRows<T> R;
+    {
+        const int w0 = warp < ng1 ? gq[warp + 1] - gq[warp] : 0;
+#pragma unroll
+        for (int q = 0; q < kRegSteps; q++) {
+            const bool has = q < w0 && lane < kRowLanes;
+            const size_t o = has ? (size_t)(gq[warp] + q) : 0;
+            R.c[q] = has ? 3 * (int)rcol[o * kRowLanes + lane] : 0;
+#pragma unroll
+            for (int k = 0; k < 9; k++) R.k[9 * q + k] = has ? kg[(o * 9 + k) * kRowLanes + lane] : T(0);
+        }
+    }
+    for (int k = warp; k < ng1; k += nw) {
+        if (go[k] < 0) continue;
+        const int skip = k < nw ? kRegSteps : 0, need = gq[k + 1] - gq[k] - skip;
+        const T* src = kg + (size_t)(gq[k] + skip) * 9 * kRowLanes;
+        T* dst = kts + go[k] * 9 * kRowLanes;
+        for (int i = lane; i < need * 9 * kRowLanes; i += 32) dst[i] = src[i];
+    }
     for (int n = tid; n < nloc; n += nt) {
         const int G3 = 3 * gid[n];
 #pragma unroll
@@ -332,15 +406,11 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
     }
     __syncthreads();
 
-    const T* kt = a.ke_smem ? kts : ktg + t0;
-    const size_t kstride = a.ke_smem ? (size_t)nk : (size_t)a.NT;
-    const int ksplit = a.ke_smem == 1 ? ntm : (1 << 30);
     // u = ca t - cb D^-1 (K t) at node n of case kc (t in u, K t in yt)
     auto smooth = [&](int n) {
-        T k3[3] = {T(0), T(0), T(0)}, tv[3], v3[3];
-        for (int t = tptr[n]; t < tptr[n + 1]; t++)
+        T k3[3], tv[3], v3[3];
 #pragma unroll
-            for (int d = 0; d < 3; d++) k3[d] += yt[((size_t)d * nta + t) * NR + kc];
+        for (int d = 0; d < 3; d++) k3[d] = yt[(3 * n + d) * NR + kc];
 #pragma unroll
         for (int d = 0; d < 3; d++) {
             tv[d] = u[(3 * n + d) * NR + kc];
@@ -360,7 +430,7 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
         for (int d = 0; d < 3; d++) u[(3 * n + d) * NR + kc] = uv[d];
     };
     if (cheb) {
-        task_matvec_multi<NPE, T, T, NR>(u, yt, nta, nta, tn, nta, kt, kstride, ksplit, ktg + t0, (size_t)a.NT);
+        rows_multi<T, NR>(R, A, u, yt, nn1);
         __syncthreads();
         for (int q = tid; q < nn1 * NR; q += nt) smooth(q / NR);
         __syncthreads();
@@ -413,18 +483,16 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
 
     for (int it = 0; status == ST_OK; it++) {
         // ---- w = A u on owned rows, every case ----
-        task_matvec_multi<NPE, T, T, NR>(u, yt, nta, ntm, tn, nta, kt, kstride);
+        rows_multi<T, NR>(R, A, u, yt, no);
         __syncthreads();
         clk.lap(0);
-        // ---- gather, BC rows, dot products, publish w ----
+        // ---- BC rows, dot products, publish w ----
         double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
         unsigned long long* vb = a.llv + (size_t)(e & 1) * N3 * NR * 2;
         unsigned long long* pb = a.llp + (size_t)(e & 1) * kRep * a.G * SW;
         for (int q = tid; q < 3 * no * NR; q += nt) {
             const int k3 = q / NR, n = k3 / 3, d = k3 - 3 * n;
-            const int tb = tptr[n + 1];
-            T wk = T(0);
-            for (int t = tptr[n]; t < tb; t++) wk += yt[((size_t)d * nta + t) * NR + kc];
+            T wk = yt[q];
             const bool c = cm[k3] != 0;
             const T uk = u[q], rk = r[q];
             if (c) wk = uk;
@@ -562,17 +630,16 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
             }
             if (__syncthreads_or(!ok)) { status = ST_TIMEOUT; break; }
             xe++;
-            task_matvec_multi<NPE, double, double, NR>(xl, ytd, ntm, ntm, tn, nta, a.kt64 + t0, (size_t)a.NT);
+            rows_multi64<NR>(gq, rcol, kg64, xl, ytd, no);
             __syncthreads();
             double vt[4] = {0.0, 0.0, 0.0, 0.0};
             unsigned long long* rb = a.llv + (size_t)(e & 1) * N3 * NR * 2;
             unsigned long long* qb = a.llp + (size_t)(e & 1) * kRep * a.G * SW;
             for (int q = tid; q < no * NR; q += nt) {
                 const int n = q / NR, G3 = 3 * gid[n];
-                double kx[3] = {0.0, 0.0, 0.0}, rtv[3];
-                for (int t = tptr[n]; t < tptr[n + 1]; t++)
+                double kx[3], rtv[3];
 #pragma unroll
-                    for (int d = 0; d < 3; d++) kx[d] += ytd[((size_t)d * ntm + t) * NR + kc];
+                for (int d = 0; d < 3; d++) kx[d] = ytd[(3 * n + d) * NR + kc];
 #pragma unroll
                 for (int d = 0; d < 3; d++) {
                     const int i = (3 * n + d) * NR + kc;
@@ -599,7 +666,7 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
                 coarse_apply_multi<T, NR>(Ai, a.G, rows, sp, KR * NR, NR, cvb + cb * RN, 0, (unsigned)ctl[2]);
             __syncthreads();
             e++;
-            // u from r for every case: the FP64 task results may have used u's
+            // u from r for every case: the FP64 products may have used u's
             // space, and for a case that kept r and c this gives u's old bits
             for (int q = tid; q < nloc * NR; q += nt) {
                 const int n = q / NR;
@@ -618,8 +685,7 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
             }
             if (cheb) {
                 __syncthreads();
-                task_matvec_multi<NPE, T, T, NR>(u, yt, nta, nta, tn, nta, kt, kstride, ksplit, ktg + t0,
-                                                 (size_t)a.NT);
+                rows_multi<T, NR>(R, A, u, yt, nn1);
                 __syncthreads();
                 for (int q = tid; q < nn1 * NR; q += nt) {
                     const int n = q / NR;
@@ -722,7 +788,7 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
         __syncthreads();
         clk.lap(7);
         if (cheb) {
-            task_matvec_multi<NPE, T, T, NR>(u, yt, nta, nta, tn, nta, kt, kstride, ksplit, ktg + t0, (size_t)a.NT);
+            rows_multi<T, NR>(R, A, u, yt, nn1);
             __syncthreads();
             clk.lap(3);
             for (int q = tid; q < nn1 * NR; q += nt) {
@@ -766,18 +832,17 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
         if (__syncthreads_or(!ok)) {
             status = ST_TIMEOUT;
         } else {
-            if (MIXED || !a.ke_smem)
-                task_matvec_multi<NPE, double, double, NR>(xl, ytd, ntm, ntm, tn, nta, a.kt64 + t0, (size_t)a.NT);
+            if constexpr (MIXED)
+                rows_multi64<NR>(gq, rcol, kg64, xl, ytd, no);
             else
-                task_matvec_multi<NPE, double, double, NR>(xl, ytd, ntm, ntm, tn, nta, (const double*)kts, kstride);
+                rows_multi<T, NR>(R, A, xl, ytd, no);
             __syncthreads();
             double v2[2] = {0.0, 0.0};
             for (int q = tid; q < no * NR; q += nt) {
                 const int n = q / NR, G3 = 3 * gid[n];
-                double kx[3] = {0.0, 0.0, 0.0};
-                for (int t = tptr[n]; t < tptr[n + 1]; t++)
+                double kx[3];
 #pragma unroll
-                    for (int d = 0; d < 3; d++) kx[d] += ytd[((size_t)d * ntm + t) * NR + kc];
+                for (int d = 0; d < 3; d++) kx[d] = ytd[(3 * n + d) * NR + kc];
 #pragma unroll
                 for (int d = 0; d < 3; d++) {
                     const int i = (3 * n + d) * NR + kc;
@@ -821,10 +886,10 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
 // NR load cases of one plate on the whole grid: part g = block g.  a.F and
 // a.x hold NR vectors of 3 Nn back to back, a.res NR result records, and the
 // exchange buffers are sized for NR cases.
-template <int NPE, typename T, bool MIXED, int NR>
+template <typename T, bool MIXED, int NR>
 __global__ void __launch_bounds__(kMultiThreads, 1) pcg_multi_kernel(const __grid_constant__ PcgArgs a) {
     extern __shared__ __align__(16) unsigned char sm[];
-    pcg_multi_body<NPE, T, MIXED, NR>(a, blockIdx.x, sm);
+    pcg_multi_body<T, MIXED, NR>(a, blockIdx.x, sm);
 }
 
 }  // namespace pg

@@ -202,7 +202,7 @@ void strip_partition(const float* xy, int Nn, int G, std::vector<int>& part_of) 
     }
 }
 
-std::string build_partition(const pg_problem& p, int G, int rings, HostPlan& plan) {
+std::string build_partition(const pg_problem& p, int G, int rings, HostPlan& plan, bool with_tasks) {
     const int Nn = plan.Nn, npe = plan.npe;
     if (G < 1) G = 1;
     if (G > std::max(Nn, 1)) G = std::max(Nn, 1);
@@ -224,21 +224,23 @@ std::string build_partition(const pg_problem& p, int G, int rings, HostPlan& pla
     plan.task_nodes.clear();
     plan.tptr.clear();
     plan.n1.assign(G, 0);
-    plan.max_nloc = plan.max_nown = plan.max_ntask = plan.max_ntask_own = plan.max_n1 = 0;
+    plan.max_nloc = plan.max_nown = plan.max_ntask = plan.max_n1 = 0;
 
     // Each part's lists are built independently (host threads over parts,
     // each with its own node -> local-index map), then concatenated in part
     // order.
     struct PartOut {
         std::vector<int> nodes, tptr, task_elem;
+        std::vector<int> steps;  // q-steps of each group of 10 rows
         std::vector<uint8_t> task_pos;
         std::vector<uint16_t> task_nodes;
-        int nown = 0, n1 = 0, nloc = 0, ntask_own = 0;
+        int nown = 0, n1 = 0, nloc = 0, ntask = 0;
         bool too_large = false;
     };
     std::vector<PartOut> out(G);
     const bool two = rings == 2;
-    auto build_part = [&](int g, std::vector<int>& local, std::vector<int>& ghosts, std::vector<int>& ring2) {
+    auto build_part = [&](int g, std::vector<int>& local, std::vector<int>& ghosts, std::vector<int>& ring2,
+                          std::vector<int>& stamp, int& row_id) {
         // fills `dst` (sorted) with the nodes of elements around `from` not yet numbered
         auto next_ring = [&](const std::vector<int>& from, std::vector<int>& dst) {
             dst.clear();
@@ -272,35 +274,36 @@ std::string build_partition(const pg_problem& p, int G, int rings, HostPlan& pla
             o.nodes.insert(o.nodes.end(), ghosts.begin(), ghosts.end());
             o.nodes.insert(o.nodes.end(), ring2.begin(), ring2.end());
             const int ntn = o.n1;
-            size_t ntask = 0;
-            for (int i = 0; i < ntn; i++) {
-                const int n = i < (int)own.size() ? own[i] : ghosts[i - own.size()];
-                ntask += (size_t)(plan.inc_ptr[n + 1] - plan.inc_ptr[n]);
-            }
-            o.tptr.resize(ntn + 1);
-            o.task_elem.resize(ntask);
-            o.task_pos.resize(ntask);
-            o.task_nodes.resize(ntask * npe);
-            int* te = o.task_elem.data();
-            uint8_t* tpos = o.task_pos.data();
-            uint16_t* tnod = o.task_nodes.data();
-            int t = 0;
-            for (int i = 0; i < ntn; i++) {
-                const int n = i < (int)own.size() ? own[i] : ghosts[i - own.size()];
-                if (i == (int)own.size()) o.ntask_own = t;
-                o.tptr[i] = t;
-                for (int q = plan.inc_ptr[n]; q < plan.inc_ptr[n + 1]; q++, t++) {
-                    const int e = plan.inc_idx[q] / 4, k = plan.inc_idx[q] % 4;
-                    te[t] = e;
-                    tpos[t] = (uint8_t)k;
-                    const uint32_t* en = p.elements + (size_t)e * npe;
-                    uint16_t* dst = tnod + (size_t)t * npe;
-                    for (int j = 0, kj = k; j < npe; j++, kj = kj + 1 == npe ? 0 : kj + 1)
-                        dst[j] = (uint16_t)local[en[kj]];
+            for (int i = 0; i < ntn; i++) o.ntask += plan.inc_ptr[o.nodes[i] + 1] - plan.inc_ptr[o.nodes[i]];
+            if (with_tasks) {
+                for (int i = 0; i < ntn; i++) {
+                    const int n = o.nodes[i];
+                    o.tptr.push_back((int)o.task_elem.size());
+                    for (int q = plan.inc_ptr[n]; q < plan.inc_ptr[n + 1]; q++) {
+                        const int e = plan.inc_idx[q] / 4, k = plan.inc_idx[q] % 4;
+                        o.task_elem.push_back(e);
+                        o.task_pos.push_back((uint8_t)k);
+                        for (int j = 0; j < npe; j++)
+                            o.task_nodes.push_back((uint16_t)local[p.elements[(size_t)e * npe + (k + j) % npe]]);
+                    }
                 }
+                o.tptr.push_back((int)o.task_elem.size());
             }
-            if (ntn == (int)own.size()) o.ntask_own = t;
-            o.tptr[ntn] = t;
+            // slots of each row: the distinct nodes of its elements
+            o.steps.assign((ntn + 9) / 10, 0);
+            for (int i = 0; i < ntn; i++, row_id++) {
+                const int n = o.nodes[i];
+                int slots = 0;
+                for (int q = plan.inc_ptr[n]; q < plan.inc_ptr[n + 1]; q++) {
+                    const uint32_t* en = p.elements + (size_t)(plan.inc_idx[q] / 4) * npe;
+                    for (int k = 0; k < npe; k++)
+                        if (stamp[en[k]] != row_id) {
+                            stamp[en[k]] = row_id;
+                            slots++;
+                        }
+                }
+                o.steps[i / 10] = std::max(o.steps[i / 10], (slots + 2) / 3);
+            }
         }
         for (int n : own) local[n] = -1;
         for (int n : ghosts) local[n] = -1;
@@ -313,8 +316,9 @@ std::string build_partition(const pg_problem& p, int G, int rings, HostPlan& pla
         // an exception must not leave a worker thread (std::terminate):
         // recorded here, raised again on the calling thread
         try {
-            std::vector<int> local(Nn, -1), ghosts, ring2;
-            for (int g; !failed && (g = next.fetch_add(1)) < G;) build_part(g, local, ghosts, ring2);
+            std::vector<int> local(Nn, -1), ghosts, ring2, stamp(Nn, -1);
+            int row_id = 0;
+            for (int g; !failed && (g = next.fetch_add(1)) < G;) build_part(g, local, ghosts, ring2, stamp, row_id);
         } catch (...) {
             failed = true;
         }
@@ -353,10 +357,15 @@ std::string build_partition(const pg_problem& p, int G, int rings, HostPlan& pla
         plan.max_nloc = std::max(plan.max_nloc, o.nloc);
         plan.max_nown = std::max(plan.max_nown, o.nown);
         plan.max_n1 = std::max(plan.max_n1, o.n1);
-        plan.max_ntask = std::max(plan.max_ntask, (int)o.task_elem.size());
-        plan.max_ntask_own = std::max(plan.max_ntask_own, o.ntask_own);
+        plan.max_ntask = std::max(plan.max_ntask, o.ntask);
     }
     plan.tp_off[G] = (int)plan.tptr.size();
+    plan.grp_off.assign(1, 0);
+    plan.grp_q.assign(1, 0);
+    for (int g = 0; g < G; g++) {
+        for (int w : out[g].steps) plan.grp_q.push_back(plan.grp_q.back() + w);
+        plan.grp_off.push_back((int)plan.grp_q.size() - 1);
+    }
     return "";
 }
 

@@ -28,7 +28,8 @@ struct HostPlan {
     int Nn = 0, Ne = 0, npe = 4, colors = 0, G = 0, rings = 1;
     // per part: [node_off[g], node_off[g+1]) local nodes (owned first), nown[g] owned
     std::vector<int> node_off, nown, nodes;
-    // per part: [task_off[g], task_off[g+1]) tasks (global task numbering)
+    // The incidences of the parts' rows ("tasks"), filled on request for the
+    // plan inspection; per part [task_off[g], task_off[g+1])
     std::vector<int> task_off;
     std::vector<int> task_elem;           // element of each task
     std::vector<uint8_t> task_pos;        // position of the owned node in the element
@@ -38,13 +39,17 @@ struct HostPlan {
     // rings = 2, else nown[g]); n1[g]+1 task offsets (relative to the part)
     // at tp_off[g]; the owned nodes' tasks are the first tptr[nown] of them
     std::vector<int> tptr, tp_off, n1;
+    // row blocks (rows.cuh): the n1[g] rows of part g in groups of 10 rows,
+    // groups [grp_off[g], grp_off[g + 1]); group k holds q-steps
+    // [grp_q[k], grp_q[k + 1]), a third of its widest row's slots rounded up
+    std::vector<int> grp_off, grp_q;
     // node -> (element*4 + position) incidence, for block-diagonal assembly
     std::vector<int> inc_ptr, inc_idx;
     // the colouring actually used (the caller's, or a greedy one when the
     // caller's colouring had node-sharing elements of one colour)
     std::vector<uint32_t> color_offsets, elements_by_color;
     bool recolored = false;
-    int max_nloc = 0, max_nown = 0, max_ntask = 0, max_ntask_own = 0, max_n1 = 0;
+    int max_nloc = 0, max_nown = 0, max_ntask = 0, max_n1 = 0;
 
     // Two-level coarse space: one aggregate per part (its owned nodes), 3
     // modes each (the plate's rigid-body motions: w = 1; w = y, thx = 1;
@@ -75,7 +80,9 @@ std::string build_structure(const pg_problem& p, HostPlan& plan);
 void strip_partition(const float* xy, int Nn, int G, std::vector<int>& part_of);
 // Partitions into G parts (G <= node_count) and fills the part arrays, with
 // a ghost halo of `rings` (1 or 2) element layers.
-std::string build_partition(const pg_problem& p, int G, int rings, HostPlan& plan);
+// with_tasks also fills the task lists (task_* and tptr; the solver multiplies
+// with row blocks and does not read them).
+std::string build_partition(const pg_problem& p, int G, int rings, HostPlan& plan, bool with_tasks = false);
 
 // Coarse space of the two-level preconditioner from the element matrices
 // ke64 ([Ne][(3 npe)^2], FP64): per-node basis data, per-part aggregate

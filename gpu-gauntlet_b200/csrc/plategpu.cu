@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <chrono>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -114,7 +115,7 @@ struct Plan {
     pg_problem prob_view{};
     double E = 0, nu = 0, t = 0;
     bool has_elem_t = false;
-    DevBuf<int> node_off, nown, nodes, task_off, tp_off, tptr, task_elem, inc_ptr, inc_idx, n1;
+    DevBuf<int> node_off, nown, nodes, inc_ptr, inc_idx, n1;
     double lambda_max = 0;  // of D^-1 K, for the polynomial smoother (0 = not estimated)
     bool setup_done = false;  // element matrices, block inverses and task blocks queued
     // exchange buffers: tags up to tag0 may sit in them (valid when ll_ready)
@@ -123,13 +124,15 @@ struct Plan {
     // last launch shape that passed the residency check
     const void* ok_fn = nullptr;
     int ok_threads = 0, ok_smem = 0;
-    DevBuf<uint16_t> task_nodes;
-    DevBuf<uint8_t> task_pos;
+    DevBuf<uint16_t> rcol;
+    DevBuf<int> grp_off, grp_q;
+    DevBuf<double> rk64;
+    DevBuf<float> rk32;
     DevBuf<float> mesh_nodes, elem_t, F;
     DevBuf<uint32_t> mesh_elements, cob_off, cob_list;
-    DevBuf<uint8_t> cons;
-    DevBuf<double> ke64, kt64, binv64, x;
-    DevBuf<float> ke32, kt32, binv32;
+    DevBuf<uint8_t> cons, shared;
+    DevBuf<double> ke64, binv64, x;
+    DevBuf<float> ke32, binv32;
     DevBuf<unsigned long long> llv, llx, llp;
     DevBuf<int> cagg_off, node_slot, ainv_off;
     DevBuf<double> node_basis, ainv64;
@@ -242,66 +245,95 @@ int auto_ctas(const pg_ctx* c, int Nn) {
     return std::max(1, std::min(G, c->sms));
 }
 
-// ke_mode: Ke task blocks in shared memory for 0 = no task, 1 = the owned
-// nodes' tasks, 2 = every task (ring-1 tasks too, with a 2-ring halo).
-pg::SmemLayout make_layout(const pg::HostPlan& hp, bool mixed, int ke_mode, bool coarse,
-                           bool ainv_smem) {
-    const size_t T = mixed ? 4 : 8, nd = 3 * hp.npe;
-    const size_t nloc = hp.max_nloc, nown = hp.max_nown, ntask = hp.max_ntask;
-    const size_t ntask_own = hp.max_ntask_own, n1 = std::max(hp.max_n1, hp.max_nown);
+// Row groups of a block that stay in registers in a launch of `threads`.
+int resident_groups(int threads) { return threads <= pg::kLeanThreads ? pg::kResident * (threads / 32) : 0; }
+
+// Row groups and q-steps of the parts with the most of each.
+void largest_rows(const pg::HostPlan& hp, int* groups, int* steps) {
+    *groups = *steps = 0;
+    for (int g = 0; g < hp.G; g++) {
+        *groups = std::max(*groups, hp.grp_off[g + 1] - hp.grp_off[g]);
+        *steps = std::max(*steps, hp.grp_q[hp.grp_off[g + 1]] - hp.grp_q[hp.grp_off[g]]);
+    }
+}
+
+// Shared memory of one block of the one-plate and batch kernels: the part's
+// vectors (u, w and t of every local node, the rest of the nodes that are not
+// resident), its row columns and kq staged q-steps of row blocks.
+pg::SmemLayout make_layout(const pg::HostPlan& hp, int threads, bool mixed, bool cheb, bool coarse, bool ainv_smem,
+                           int kq) {
+    const size_t T = mixed ? 4 : 8, res = (size_t)pg::kRowGroup * resident_groups(threads);
+    const size_t nloc = hp.max_nloc;
+    const size_t xloc = nloc - std::min<size_t>(nloc, res);                            // not resident
+    int groups = 0, steps = 0;
+    largest_rows(hp, &groups, &steps);
     size_t off = 0;
     auto take = [&](size_t bytes) {
-        const int o = (int)off;
+        const size_t o = off;
         off = (off + bytes + 15) & ~(size_t)15;
-        return o;
+        return (int)std::min<size_t>(o, INT_MAX);
     };
     pg::SmemLayout L{};
-    L.x = take(3 * nown * 8);
-    L.xl = take(mixed ? 3 * nloc * 8 : 0);
-    L.red = take(32 * 8 * 8);  // [warps][8]
+    take(sizeof(pg::PcgArgs));  // the batch kernel's copy of its plate's arguments
+    L.x = take(3 * (size_t)hp.max_nown * 8);
+    L.red = take((size_t)(coarse ? 6 : 3) * threads * 8);  // [values][threads]
     L.scal = take(8 * 8);
-    L.sp = take((size_t)6 * hp.G * 8);
+    L.sp = take((size_t)4 * hp.G * 8);
     L.qw = take(coarse ? (size_t)3 * hp.max_kagg * 8 : 0);
     L.cs = take(coarse ? (size_t)2 * 3 * hp.max_kagg * 8 : 0);
     L.cv = take(coarse ? (size_t)2 * 3 * hp.max_kagg * 8 : 0);
     L.ctl = take(4 * 4);
-    L.clk = take(8 * 8);
-    L.r = take(3 * nloc * T);
-    L.p = take(3 * nloc * T);
-    L.s = take(3 * nloc * T);
-    L.B = take(9 * nloc * T);
-    // yt, w, u back to back: the mixed-precision FP64 residual's task
-    // results (ytd) reuse them when they fit, since none of the three is
-    // live during a residual replacement or the final residual
-    L.yt = take(3 * ntask * T);
+    L.dec = take(sizeof(pg::Decision));
+    L.clk = take(9 * 8);
+    L.r = take(3 * xloc * T);
+    L.p = take(3 * (size_t)hp.max_nown * T);
+    L.s = take(3 * xloc * T);
+    L.B = take(9 * xloc * T);
+    // w and u back to back: the FP64 x of the true residual (xl) takes w's
+    // place, and with FP32 vectors u's too; neither is live then
     L.w = take(3 * nloc * T);
+    L.xl = L.w;
     L.u = take(3 * nloc * T);
-    if (mixed)
-        L.ytd = 3 * ntask_own * 8 <= off - (size_t)L.yt ? L.yt : take(3 * ntask_own * 8);
-    L.kt = take(ke_mode == 2 ? 3 * nd * ntask * T : ke_mode == 1 ? 3 * nd * ntask_own * T : 0);
+    L.t = take(cheb ? 3 * nloc * T : 0);
+    L.kt = take((size_t)kq * 9 * pg::kRowLanes * T);
+    L.kq = kq;
     L.nb = take(coarse ? 3 * nloc * T : 0);
     L.ainv = take(coarse && ainv_smem ? (size_t)3 * hp.max_kagg * hp.C * T : 0);
     L.nslot = take(coarse ? nloc * 4 : 0);
     L.gid = take(nloc * 4);
-    L.tptr = take((n1 + 1) * 4);
-    L.tnode = take(hp.npe * ntask * 2);
-    L.cm = take(3 * nloc);
-    L.total = (int)off;
+    L.gq = take((size_t)(groups + 1) * 4);
+    L.go = take((size_t)groups * 4);
+    L.rcol = take((size_t)steps * pg::kRowLanes * 2);
+    L.cm = take(3 * xloc);
+    L.total = (int)std::min<size_t>(off, INT_MAX);
     return L;
+}
+
+// q-steps of row blocks that the largest part keeps outside its registers.
+int steps_outside(const pg::HostPlan& hp, int threads) {
+    int most = 0;
+    for (int g = 0; g < hp.G; g++) {
+        const int b = hp.grp_off[g], n = hp.grp_off[g + 1] - b;
+        int need = hp.grp_q[b + n] - hp.grp_q[b];
+        for (int k = 0; k < std::min(n, resident_groups(threads)); k++)
+            need -= std::min(pg::kRegSteps, hp.grp_q[b + k + 1] - hp.grp_q[b + k]);
+        most = std::max(most, need);
+    }
+    return most;
 }
 
 // Shared-memory layout of a launch of NR load cases: every per-DOF vector
 // and the task results hold NR values per entry; the partial sums 6 per case.
-pg::SmemLayout make_layout_multi(const pg::HostPlan& hp, bool mixed, int ke_mode, bool coarse,
-                                 bool ainv_smem, int NR) {
-    const size_t T = mixed ? 4 : 8, nd = 3 * hp.npe, R = NR;
-    const size_t nloc = hp.max_nloc, nown = hp.max_nown, ntask = hp.max_ntask;
-    const size_t ntask_own = hp.max_ntask_own, n1 = std::max(hp.max_n1, hp.max_nown);
+pg::SmemLayout make_layout_multi(const pg::HostPlan& hp, bool mixed, bool coarse, bool ainv_smem, int NR, int kq) {
+    const size_t T = mixed ? 4 : 8, R = NR;
+    const size_t nloc = hp.max_nloc, nown = hp.max_nown, n1 = std::max(hp.max_n1, hp.max_nown);
+    int groups = 0, steps = 0;
+    largest_rows(hp, &groups, &steps);
     size_t off = 0;
     auto take = [&](size_t bytes) {
-        const int o = (int)off;
+        const size_t o = off;
         off = (off + bytes + 15) & ~(size_t)15;
-        return o;
+        return (int)std::min<size_t>(o, INT_MAX);
     };
     pg::SmemLayout L{};
     L.x = take(3 * nown * 8 * R);
@@ -313,27 +345,28 @@ pg::SmemLayout make_layout_multi(const pg::HostPlan& hp, bool mixed, int ke_mode
     L.cs = take(coarse ? 2 * 3 * (size_t)hp.max_kagg * 8 * R : 0);
     L.cv = take(coarse ? 2 * 3 * (size_t)hp.max_kagg * 8 * R : 0);
     L.ctl = take(4 * 4);
-    L.clk = take(8 * 8);
+    L.clk = take(9 * 8);
     L.r = take(3 * nloc * T * R);
     L.p = take(3 * nloc * T * R);
     L.s = take(3 * nloc * T * R);
     L.B = take(9 * nloc * T);
-    // yt, w, u back to back: the FP64 residual's task results (ytd) reuse
-    // them when they fit (u is rebuilt from r after every replacement)
-    L.yt = take(3 * ntask * T * R);
+    // yt, w, u back to back: the FP64 residual's products (ytd, 24 nown NR
+    // bytes) take their place (u is rebuilt from r after every replacement)
+    L.yt = take(3 * n1 * T * R);
     L.w = take(3 * nloc * T * R);
     L.u = take(3 * nloc * T * R);
-    if (mixed)
-        L.ytd = 3 * ntask_own * 8 * R <= off - (size_t)L.yt ? L.yt : take(3 * ntask_own * 8 * R);
-    L.kt = take(ke_mode == 2 ? 3 * nd * ntask * T : ke_mode == 1 ? 3 * nd * ntask_own * T : 0);
+    L.ytd = L.yt;
+    L.kt = take((size_t)kq * 9 * pg::kRowLanes * T);
+    L.kq = kq;
     L.nb = take(coarse ? 3 * nloc * T : 0);
     L.ainv = take(coarse && ainv_smem ? (size_t)3 * hp.max_kagg * hp.C * T : 0);
     L.nslot = take(coarse ? nloc * 4 : 0);
     L.gid = take(nloc * 4);
-    L.tptr = take((n1 + 1) * 4);
-    L.tnode = take(hp.npe * ntask * 2);
+    L.gq = take((size_t)(groups + 1) * 4);
+    L.go = take((size_t)groups * 4);
+    L.rcol = take((size_t)steps * pg::kRowLanes * 2);
     L.cm = take(3 * nloc);
-    L.total = (int)off;
+    L.total = (int)std::min<size_t>(off, INT_MAX);
     return L;
 }
 
@@ -368,20 +401,15 @@ std::unique_ptr<Plan> build_plan(pg_ctx* c, const pg_problem& p, int G, int ring
     cudaStream_t st = c->stream;
     const size_t Nn = p.node_count, Ne = p.element_count, npe = p.nodes_per_element;
     const size_t kk = 9 * npe * npe;
-    const size_t NT = hp.task_elem.size();
     // every device array of the plan in one allocation
     Arena ar;
     auto carve = [&](auto& buf, size_t count, const void* host) { ar.add(buf, count, host); };
     carve(pl->node_off, hp.node_off.size(), hp.node_off.data());
     carve(pl->nown, hp.nown.size(), hp.nown.data());
     carve(pl->nodes, hp.nodes.size(), hp.nodes.data());
-    carve(pl->task_off, hp.task_off.size(), hp.task_off.data());
-    carve(pl->tp_off, hp.tp_off.size(), hp.tp_off.data());
-    carve(pl->tptr, hp.tptr.size(), hp.tptr.data());
     carve(pl->n1, hp.n1.size(), hp.n1.data());
-    carve(pl->task_elem, hp.task_elem.size(), hp.task_elem.data());
-    carve(pl->task_pos, hp.task_pos.size(), hp.task_pos.data());
-    carve(pl->task_nodes, hp.task_nodes.size(), hp.task_nodes.data());
+    carve(pl->grp_off, hp.grp_off.size(), hp.grp_off.data());
+    carve(pl->grp_q, hp.grp_q.size(), hp.grp_q.data());
     carve(pl->inc_ptr, hp.inc_ptr.size(), hp.inc_ptr.data());
     carve(pl->inc_idx, hp.inc_idx.size(), hp.inc_idx.data());
     carve(pl->mesh_nodes, 2 * Nn, p.nodes);
@@ -389,13 +417,16 @@ std::unique_ptr<Plan> build_plan(pg_ctx* c, const pg_problem& p, int G, int ring
     carve(pl->cob_off, hp.color_offsets.size(), hp.color_offsets.data());
     carve(pl->cob_list, hp.elements_by_color.size(), hp.elements_by_color.data());
     carve(pl->cons, 3 * Nn, p.constrained);
+    carve(pl->shared, std::max<size_t>(1, Nn), nullptr);
     pl->has_elem_t = p.elem_t != nullptr;
     if (p.elem_t) carve(pl->elem_t, Ne, p.elem_t);
     carve(pl->F, 3 * Nn, nullptr);
     carve(pl->ke64, std::max<size_t>(1, Ne * kk), nullptr);
     carve(pl->ke32, std::max<size_t>(1, Ne * kk), nullptr);
-    carve(pl->kt64, std::max<size_t>(1, NT * 9 * npe), nullptr);
-    carve(pl->kt32, std::max<size_t>(1, NT * 9 * npe), nullptr);
+    const size_t steps = std::max<size_t>(1, hp.grp_q.back());
+    carve(pl->rcol, steps * pg::kRowLanes, nullptr);
+    carve(pl->rk64, steps * 9 * pg::kRowLanes, nullptr);
+    carve(pl->rk32, steps * 9 * pg::kRowLanes, nullptr);
     carve(pl->binv64, 9 * Nn, nullptr);
     carve(pl->binv32, 9 * Nn, nullptr);
     carve(pl->x, 3 * Nn, nullptr);
@@ -471,14 +502,21 @@ void run_setup(pg_ctx* c, Plan* pl) {
             Nn, hp.npe, pl->inc_ptr.p, pl->inc_idx.p, pl->ke64.p, pl->cons.p, pl->binv64.p,
             pl->binv32.p);
     CK(cudaGetLastError());
-    const int NT = (int)hp.task_elem.size();
-    if (NT > 0 && hp.npe == 4)
-        pg::task_ke_kernel<4><<<(NT + 127) / 128, 128, 0, c->stream>>>(
-            NT, pl->task_elem.p, pl->task_pos.p, pl->ke64.p, pl->kt64.p, pl->kt32.p);
-    else if (NT > 0)
-        pg::task_ke_kernel<3><<<(NT + 127) / 128, 128, 0, c->stream>>>(
-            NT, pl->task_elem.p, pl->task_pos.p, pl->ke64.p, pl->kt64.p, pl->kt32.p);
-    CK(cudaGetLastError());
+    if (Nn > 0) {
+        CK(cudaMemsetAsync(pl->shared.p, 0, Nn, c->stream));
+        pg::mark_ghosts_kernel<<<hp.G, 128, 0, c->stream>>>(pl->node_off.p, pl->nown.p, pl->nodes.p, pl->shared.p);
+        CK(cudaGetLastError());
+    }
+    if (hp.grp_q.back() > 0) {
+        int groups = 0;
+        for (int g = 0; g < hp.G; g++) groups = std::max(groups, hp.grp_off[g + 1] - hp.grp_off[g]);
+        const dim3 grid(hp.G, std::min(64, (groups * pg::kRowLanes + 239) / 240));
+        auto fill = hp.npe == 4 ? pg::row_fill_kernel<4> : pg::row_fill_kernel<3>;
+        fill<<<grid, 240, 0, c->stream>>>(pl->node_off.p, pl->nown.p, pl->n1.p, pl->nodes.p, pl->grp_off.p,
+                                          pl->grp_q.p, pl->inc_ptr.p, pl->inc_idx.p, pl->mesh_elements.p,
+                                          pl->ke64.p, pl->rcol.p, pl->rk64.p, pl->rk32.p);
+        CK(cudaGetLastError());
+    }
 }
 
 // y = K x on the device (colour by colour, then the identity rows of the
@@ -794,28 +832,31 @@ void prepare_many(pg_ctx* c, const std::vector<Plan*>& pls, const pg_options& o)
     }
 }
 
-// Shared-memory layout of a launch: keep in shared memory what fits, in this
-// order of preference: every task's Ke blocks (only differs from the owned
-// tasks' with a 2-ring halo) and the A_c^-1 rows; the owned tasks' blocks
-// and A_c^-1; then the larger of the owned tasks' blocks and A_c^-1; then
-// neither (read from L2).
-pg::SmemLayout choose_layout(pg_ctx* c, const pg::HostPlan& hp, const pg_options& o, int* ke_mode,
-                             bool* ainv_smem) {
+// Threads of a one-plate launch: the caller's, or the resident build's.
+int solve_threads(const pg_options& o) { return o.threads ? o.threads : pg::kLeanThreads; }
+
+// Shared-memory layout of a launch of `threads` threads a block: the row
+// blocks that the registers do not hold and the A_c^-1 rows are read once
+// per iteration each, so as many of their bytes as fit stay in shared memory
+// (the A_c^-1 rows as a whole, the row blocks group by group); the rest is
+// read from L2.
+pg::SmemLayout choose_layout(pg_ctx* c, const pg::HostPlan& hp, const pg_options& o, int threads, bool* ainv_smem) {
     const bool mixed = o.precision == PG_PREC_MIXED, coarse = o.preconditioner == PG_PRECOND_TWO_LEVEL;
-    const int full = hp.rings == 2 ? 2 : 1;
-    const bool ke_first = 3 * 3 * hp.npe * (size_t)hp.max_ntask_own >= (size_t)3 * hp.max_kagg * hp.C;
-    const int cand[6][2] = {{full, 1}, {1, 1}, {ke_first ? full : 0, ke_first ? 0 : 1},
-                            {ke_first ? 1 : 0, ke_first ? 0 : 1}, {0, 1}, {0, 0}};
-    pg::SmemLayout L{};
-    for (auto& cd : cand) {
-        *ke_mode = cd[0];
-        *ainv_smem = coarse && cd[1];
-        L = make_layout(hp, mixed, *ke_mode, coarse, *ainv_smem);
-        if (L.total <= c->max_smem) break;
-    }
-    if (L.total > c->max_smem)
-        throw Fail{PG_EUNSUPPORTED, "partition too large for shared memory: use more ctas"};
-    return L;
+    const bool cheb = o.smoother == PG_SMOOTHER_CHEBYSHEV;
+    const int need = steps_outside(hp, threads);
+    const size_t step = 9 * pg::kRowLanes * (mixed ? 4 : 8);
+    auto staged = [&](bool ainv, size_t* bytes) {  // q-steps that fit beside the rest, or -1
+        const pg::SmemLayout L = make_layout(hp, threads, mixed, cheb, coarse, ainv, 0);
+        if (L.total > c->max_smem) return -1;
+        const int q = (int)std::min<size_t>(need, (size_t)(c->max_smem - L.total) / step);
+        *bytes = q * step + (ainv ? (size_t)3 * hp.max_kagg * hp.C * (mixed ? 4 : 8) : 0);
+        return q;
+    };
+    size_t b0 = 0, b1 = 0;
+    const int q0 = staged(false, &b0), q1 = coarse ? staged(true, &b1) : -1;
+    if (q0 < 0) throw Fail{PG_EUNSUPPORTED, "partition too large for shared memory: use more ctas"};
+    *ainv_smem = q1 >= 0 && b1 >= b0;
+    return make_layout(hp, threads, mixed, cheb, coarse, *ainv_smem, *ainv_smem ? q1 : q0);
 }
 
 // Clears what a launch of pl needs cleared: its result record, and its
@@ -833,28 +874,26 @@ void reset_for_launch(pg_ctx* c, Plan* pl, pg::PcgResult* res) {
     CK(cudaMemsetAsync(res, 0, sizeof(pg::PcgResult), c->stream));
 }
 
-pg::PcgArgs fill_args(Plan* pl, const pg_options& o, const pg::SmemLayout& L, int ke_mode,
-                      bool ainv_smem, int* abort_flag, pg::PcgResult* res) {
+pg::PcgArgs fill_args(Plan* pl, const pg_options& o, const pg::SmemLayout& L, bool ainv_smem, int* abort_flag,
+                      pg::PcgResult* res) {
     const pg::HostPlan& hp = pl->hp;
     const bool coarse = o.preconditioner == PG_PRECOND_TWO_LEVEL;
     const bool cheb = o.smoother == PG_SMOOTHER_CHEBYSHEV;
     pg::PcgArgs a{};
     a.G = pl->G;
-    a.NT = (int)hp.task_elem.size();
     a.Nn = hp.Nn;
-    a.npe = hp.npe;
     a.node_off = pl->node_off.p;
     a.nown = pl->nown.p;
     a.nodes = pl->nodes.p;
-    a.task_off = pl->task_off.p;
-    a.tp_off = pl->tp_off.p;
-    a.tptr = pl->tptr.p;
-    a.task_nodes = pl->task_nodes.p;
-    a.kt64 = pl->kt64.p;
-    a.kt32 = pl->kt32.p;
+    a.grp_off = pl->grp_off.p;
+    a.grp_q = pl->grp_q.p;
+    a.rcol = pl->rcol.p;
+    a.rk64 = pl->rk64.p;
+    a.rk32 = pl->rk32.p;
     a.binv64 = pl->binv64.p;
     a.binv32 = pl->binv32.p;
     a.cons = pl->cons.p;
+    a.shared = pl->shared.p;
     a.F = pl->F.p;
     a.x = pl->x.p;
     a.llv = pl->llv.p;
@@ -867,7 +906,6 @@ pg::PcgArgs fill_args(Plan* pl, const pg_options& o, const pg::SmemLayout& L, in
     a.maxit = o.max_iterations;
     a.stop_rule = o.stop_rule;
     a.timeout_ns = (unsigned long long)(o.wait_timeout_ms * 1e6);
-    a.ke_smem = ke_mode;
     a.timing = o.phase_timing ? 1 : 0;
     a.test_stall = o.test_stall ? 1 : 0;
     a.coarse = coarse ? 1 : 0;
@@ -938,6 +976,32 @@ void opt_in_smem(pg_ctx* c, const void* fn) {
     }
 }
 
+template <typename T, bool MIXED, int MAXT>
+const void* solve_kernel_of(bool coarse, bool cheb) {
+    if (coarse)
+        return cheb ? (const void*)pg::pcg_kernel<T, MIXED, MAXT, true, true>
+                    : (const void*)pg::pcg_kernel<T, MIXED, MAXT, true, false>;
+    return cheb ? (const void*)pg::pcg_kernel<T, MIXED, MAXT, false, true>
+                : (const void*)pg::pcg_kernel<T, MIXED, MAXT, false, false>;
+}
+
+const void* solve_kernel(const pg_options& o, bool lean) {
+    const bool coarse = o.preconditioner == PG_PRECOND_TWO_LEVEL, cheb = o.smoother == PG_SMOOTHER_CHEBYSHEV;
+    constexpr int LT = pg::kLeanThreads, MT = pg::kMaxThreads;
+    if (o.precision == PG_PREC_MIXED)
+        return lean ? solve_kernel_of<float, true, LT>(coarse, cheb) : solve_kernel_of<float, true, MT>(coarse, cheb);
+    return lean ? solve_kernel_of<double, false, LT>(coarse, cheb) : solve_kernel_of<double, false, MT>(coarse, cheb);
+}
+
+template <typename T, bool MIXED>
+const void* batch_kernel_of(bool coarse, bool cheb) {
+    if (coarse)
+        return cheb ? (const void*)pg::pcg_batch_kernel<T, MIXED, true, true>
+                    : (const void*)pg::pcg_batch_kernel<T, MIXED, true, false>;
+    return cheb ? (const void*)pg::pcg_batch_kernel<T, MIXED, false, true>
+                : (const void*)pg::pcg_batch_kernel<T, MIXED, false, false>;
+}
+
 // Queues set-up (first solve of the plan) and the persistent PCG launch on
 // the context stream, then waits for the result record (one readback).
 // x_dst (optional) receives the solution by a copy of `kind` queued right
@@ -945,42 +1009,22 @@ void opt_in_smem(pg_ctx* c, const void* fn) {
 void run_solve(pg_ctx* c, Plan* pl, const pg_options& o, pg_info* info, void* x_dst = nullptr,
                cudaMemcpyKind kind = cudaMemcpyDeviceToDevice) {
     const pg::HostPlan& hp = pl->hp;
-    const bool mixed = o.precision == PG_PREC_MIXED;
-    int threads = o.threads;
-    if (!threads) {
-        // one thread per task of the largest part, within the launch bound:
-        // up to 512 threads the kernel has 128 registers (576: 96), which
-        // measured faster for FP32 inner iterations and for FP64 block
-        // Jacobi; FP64 with the Chebyshev smoother keeps 576 threads (its
-        // split task passes: fewer of them)
-        const bool wide = !mixed && o.smoother == PG_SMOOTHER_CHEBYSHEV;
-        threads = std::min(wide ? pg::kMaxThreads : pg::kLeanThreads, std::max(128, (hp.max_ntask + 31) / 32 * 32));
-    }
+    const int threads = solve_threads(o);
     const bool lean = threads <= pg::kLeanThreads;
     prepare_plan_data(c, pl, o, info);
-    int ke_mode = 0;
     bool ainv_smem = false;
-    const pg::SmemLayout L = choose_layout(c, hp, o, &ke_mode, &ainv_smem);
+    const pg::SmemLayout L = choose_layout(c, hp, o, threads, &ainv_smem);
 
     CK(cudaEventRecord(c->ev[0], c->stream));
     run_setup(c, pl);
     CK(cudaEventRecord(c->ev[1], c->stream));
     reset_for_launch(c, pl, pl->res.p);
     CK(cudaMemsetAsync(pl->abort_flag.p, 0, sizeof(int), c->stream));
-    pg::PcgArgs a = fill_args(pl, o, L, ke_mode, ainv_smem, pl->abort_flag.p, pl->res.p);
+    pg::PcgArgs a = fill_args(pl, o, L, ainv_smem, pl->abort_flag.p, pl->res.p);
     if (a.trace_it > 0)
         CK(cudaMemsetAsync(pl->trace.p, 0, pl->trace.n * sizeof(unsigned long long), c->stream));
 
-    const void* fn;
-    constexpr int LT = pg::kLeanThreads, MT = pg::kMaxThreads;
-    if (hp.npe == 4)
-        fn = mixed ? (lean ? (const void*)pg::pcg_kernel<4, float, true, LT> : (const void*)pg::pcg_kernel<4, float, true, MT>)
-                   : (lean ? (const void*)pg::pcg_kernel<4, double, false, LT>
-                           : (const void*)pg::pcg_kernel<4, double, false, MT>);
-    else
-        fn = mixed ? (lean ? (const void*)pg::pcg_kernel<3, float, true, LT> : (const void*)pg::pcg_kernel<3, float, true, MT>)
-                   : (lean ? (const void*)pg::pcg_kernel<3, double, false, LT>
-                           : (const void*)pg::pcg_kernel<3, double, false, MT>);
+    const void* fn = solve_kernel(o, lean);
     opt_in_smem(c, fn);
     if (pl->ok_fn != fn || pl->ok_threads != threads || pl->ok_smem != L.total) {
         int nb = 0;
@@ -1117,7 +1161,8 @@ pgi::OperatorView operator_view(Plan* pl) {
 // Whether the smallest layout of the persistent kernel (element blocks and
 // coarse rows in L2) fits one block's shared memory for this plan's parts.
 bool persistent_fits(const pg_ctx* c, const Plan* pl, const pg_options& o) {
-    const pg::SmemLayout L = make_layout(pl->hp, o.precision == PG_PREC_MIXED, 0, false, false);
+    const pg::SmemLayout L = make_layout(pl->hp, solve_threads(o), o.precision == PG_PREC_MIXED, o.smoother == PG_SMOOTHER_CHEBYSHEV,
+                                          o.preconditioner == PG_PRECOND_TWO_LEVEL, false, 0);
     return L.total <= c->max_smem;
 }
 
@@ -1162,36 +1207,30 @@ void solve_with_fallback(pg_ctx* c, Plan* pl, const pg_options& o, pg_info* info
     fp64_correction(c, pl, o, fi, x_dst, kind);
 }
 
-// Layout of an NR-case launch: the first of the single solve's preferences
-// that fits; false when none does (the plate's parts are then solved with
-// fewer cases per launch).
-bool choose_layout_multi(pg_ctx* c, const pg::HostPlan& hp, const pg_options& o, int NR, int* ke_mode,
+// Layout of an NR-case launch, row blocks and A_c^-1 rows in shared memory as
+// in choose_layout (*all: every row block is on chip); false when none fits
+// (the plate's parts are then solved with fewer cases per launch).
+bool choose_layout_multi(pg_ctx* c, const pg::HostPlan& hp, const pg_options& o, int NR, bool* all,
                          bool* ainv_smem, pg::SmemLayout* out) {
     const bool mixed = o.precision == PG_PREC_MIXED, coarse = o.preconditioner == PG_PRECOND_TWO_LEVEL;
-    const int full = hp.rings == 2 ? 2 : 1;
-    const bool ke_first = 3 * 3 * hp.npe * (size_t)hp.max_ntask_own >= (size_t)3 * hp.max_kagg * hp.C;
-    const int cand[6][2] = {{full, 1}, {1, 1}, {ke_first ? full : 0, ke_first ? 0 : 1},
-                            {ke_first ? 1 : 0, ke_first ? 0 : 1}, {0, 1}, {0, 0}};
-    for (auto& cd : cand) {
-        *ke_mode = cd[0];
-        *ainv_smem = coarse && cd[1];
-        *out = make_layout_multi(hp, mixed, *ke_mode, coarse, *ainv_smem, NR);
-        if (out->total <= c->max_smem) return true;
+    const int need = steps_outside(hp, pg::kMultiThreads);
+    const size_t step = 9 * pg::kRowLanes * (mixed ? 4 : 8);
+    for (int ainv = coarse ? 1 : 0; ainv >= 0; ainv--) {
+        const pg::SmemLayout L = make_layout_multi(hp, mixed, coarse, ainv != 0, NR, 0);
+        if (L.total > c->max_smem) continue;
+        const int q = (int)std::min<size_t>(need, (size_t)(c->max_smem - L.total) / step);
+        *ainv_smem = ainv != 0;
+        *all = q == need && (ainv || !coarse);
+        *out = make_layout_multi(hp, mixed, coarse, ainv != 0, NR, q);
+        return true;
     }
     return false;
 }
 
-const void* multi_kernel(int npe, bool mixed, int NR) {
-    if (npe == 4) {
-        if (NR == 2) return mixed ? (const void*)pg::pcg_multi_kernel<4, float, true, 2>
-                                  : (const void*)pg::pcg_multi_kernel<4, double, false, 2>;
-        return mixed ? (const void*)pg::pcg_multi_kernel<4, float, true, 4>
-                     : (const void*)pg::pcg_multi_kernel<4, double, false, 4>;
-    }
-    if (NR == 2) return mixed ? (const void*)pg::pcg_multi_kernel<3, float, true, 2>
-                              : (const void*)pg::pcg_multi_kernel<3, double, false, 2>;
-    return mixed ? (const void*)pg::pcg_multi_kernel<3, float, true, 4>
-                 : (const void*)pg::pcg_multi_kernel<3, double, false, 4>;
+const void* multi_kernel(bool mixed, int NR) {
+    if (NR == 2)
+        return mixed ? (const void*)pg::pcg_multi_kernel<float, true, 2> : (const void*)pg::pcg_multi_kernel<double, false, 2>;
+    return mixed ? (const void*)pg::pcg_multi_kernel<float, true, 4> : (const void*)pg::pcg_multi_kernel<double, false, 4>;
 }
 
 // count <= NR load cases of plan pl in one launch of the NR-case kernel
@@ -1204,10 +1243,9 @@ void run_solve_multi(pg_ctx* c, Plan* pl, const pg_options& o, int NR, int count
     const bool mixed = o.precision == PG_PREC_MIXED;
     const size_t n = 3 * (size_t)hp.Nn;
     prepare_plan_data(c, pl, o);
-    int ke_mode = 0;
-    bool ainv_smem = false;
+    bool all = false, ainv_smem = false;
     pg::SmemLayout L{};
-    if (!choose_layout_multi(c, hp, o, NR, &ke_mode, &ainv_smem, &L))
+    if (!choose_layout_multi(c, hp, o, NR, &all, &ainv_smem, &L))
         throw Fail{PG_EUNSUPPORTED, "load-case partition too large for shared memory"};
     cudaStream_t st = c->stream;
     if (pl->m_nr != NR) {
@@ -1240,7 +1278,7 @@ void run_solve_multi(pg_ctx* c, Plan* pl, const pg_options& o, int NR, int count
     pl->m_ready = false;
     CK(cudaMemsetAsync(pl->mres.p, 0, NR * sizeof(pg::PcgResult), st));
     CK(cudaMemsetAsync(pl->abort_flag.p, 0, sizeof(int), st));
-    pg::PcgArgs a = fill_args(pl, o, L, ke_mode, ainv_smem, pl->abort_flag.p, pl->mres.p);
+    pg::PcgArgs a = fill_args(pl, o, L, ainv_smem, pl->abort_flag.p, pl->mres.p);
     a.F = pl->mF.p;
     a.x = pl->mx.p;
     a.llv = pl->mllv.p;
@@ -1248,7 +1286,7 @@ void run_solve_multi(pg_ctx* c, Plan* pl, const pg_options& o, int NR, int count
     a.llp = pl->mllp.p;
     a.tag0 = pl->m_tag0;
     a.trace_it = -1;
-    const void* fn = multi_kernel(hp.npe, mixed, NR);
+    const void* fn = multi_kernel(mixed, NR);
     opt_in_smem(c, fn);
     if (pl->m_ok_fn != fn || pl->m_ok_smem != L.total) {
         int nb = 0;
@@ -1374,6 +1412,19 @@ pg_options plate_options(const pg_options& o, const Plan* pl) {
     return oi;
 }
 
+// Whether a batch plate on a 2-ring halo keeps the Chebyshev smoother: its
+// vectors (24 words a local node), 3 words and npe column ids per element
+// incidence of its rows, and x must fit shared memory.  A larger part would
+// read most of its row blocks from L2 twice an iteration (K u and K t).
+bool smoother_halo_fits(const pg_ctx* c, const pg::HostPlan& hp, const pg_options& o) {
+    const size_t T = o.precision == PG_PREC_MIXED ? 4 : 8;
+    const size_t nloc = hp.max_nloc, inc = hp.max_ntask;
+    size_t b = 24 * nloc * T + 3 * inc * T + 2 * hp.npe * inc + 24 * (size_t)hp.max_nown + 7 * nloc +
+               4 * (size_t)hp.max_n1 + 48 * (size_t)hp.G + 2560;
+    if (T == 4) b += 24 * nloc;
+    return b <= (size_t)c->max_smem;
+}
+
 std::unique_ptr<pg_batch> build_batch(pg_ctx* c, const pg_problem* probs, int count,
                                       const pg_options& o) {
     auto b = std::make_unique<pg_batch>();
@@ -1410,10 +1461,11 @@ std::unique_ptr<pg_batch> build_batch(pg_ctx* c, const pg_problem* probs, int co
         for (int i = 0; i < count; i++) {
             const int G = b->sched.plate_size[i];
             b->plans.push_back(build_plan(c, probs[i], G, rings[i]));
-            int ke_mode = 0;
             bool ainv = false;
             try {
-                choose_layout(c, b->plans.back()->hp, plate_options(o, b->plans.back().get()), &ke_mode, &ainv);
+                const pg::HostPlan& hp = b->plans.back()->hp;
+                choose_layout(c, hp, plate_options(o, b->plans.back().get()), pg::kBatchThreads, &ainv);
+                if (rings[i] == 2 && !smoother_halo_fits(c, hp, o)) throw Fail{PG_EUNSUPPORTED, "halo"};
             } catch (const Fail&) {
                 fits = false;
                 if (rings[i] == 2 && G == c->sms) {
@@ -1513,11 +1565,10 @@ void run_batch(pg_batch* b, const pg_options& o, const float* const* F, double* 
     for (int i = 0; i < count; i++) {
         Plan* pl = b->plans[i].get();
         const pg_options oi = plate_options(o, pl);
-        int ke_mode = 0;
         bool ainv = false;
-        const pg::SmemLayout L = choose_layout(c, pl->hp, oi, &ke_mode, &ainv);
+        const pg::SmemLayout L = choose_layout(c, pl->hp, oi, pg::kBatchThreads, &ainv);
         reset_for_launch(c, pl, b->res.p + i);
-        pg::PcgArgs ai = fill_args(pl, oi, L, ke_mode, ainv, b->abort_flag.p, b->res.p + i);
+        pg::PcgArgs ai = fill_args(pl, oi, L, ainv, b->abort_flag.p, b->res.p + i);
         ai.timing = 0;
         ai.test_stall = 0;
         ai.trace_it = -1;
@@ -1531,25 +1582,18 @@ void run_batch(pg_batch* b, const pg_options& o, const float* const* F, double* 
     CK(cudaMemsetAsync(b->times.p, 0, b->times.n * sizeof(unsigned long long), st));
     const unsigned long long claim_timeout_ns = (unsigned long long)(o.wait_timeout_ms * 1e6);
     const bool mixed = o.precision == PG_PREC_MIXED;
-    auto kernel_of = [&](int kind) {
-        if (kind == 4)
-            return mixed ? (const void*)pg::pcg_batch_kernel<4, float, true>
-                         : (const void*)pg::pcg_batch_kernel<4, double, false>;
-        return mixed ? (const void*)pg::pcg_batch_kernel<3, float, true>
-                     : (const void*)pg::pcg_batch_kernel<3, double, false>;
-    };
+    const bool coarse = o.preconditioner == PG_PRECOND_TWO_LEVEL, cheb = o.smoother == PG_SMOOTHER_CHEBYSHEV;
+    const void* const fn = mixed ? batch_kernel_of<float, true>(coarse, cheb) : batch_kernel_of<double, false>(coarse, cheb);
+    const int prec_key = (mixed ? 1 : 2) + (coarse ? 4 : 0) + (cheb ? 8 : 0);
     int grid_max = 0;
     for (auto& ph : b->phases) grid_max = std::max(grid_max, ph->grid);
-    if (b->ok_precision != (mixed ? 1 : 2) || b->ok_smem != smem) {
-        for (int kind : {3, 4}) {
-            const void* fk = kernel_of(kind);
-            opt_in_smem(c, fk);
-            int nb = 0;
-            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fk, pg::kBatchThreads, smem));
-            if (nb < 1 || nb * c->sms < grid_max)
-                throw Fail{PG_EUNSUPPORTED, "batch grid does not fit on the device"};
-        }
-        b->ok_precision = mixed ? 1 : 2;  // residency checked for this precision and size
+    if (b->ok_precision != prec_key || b->ok_smem != smem) {
+        opt_in_smem(c, fn);
+        int nb = 0;
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, pg::kBatchThreads, smem));
+        if (nb < 1 || nb * c->sms < grid_max)
+            throw Fail{PG_EUNSUPPORTED, "batch grid does not fit on the device"};
+        b->ok_precision = prec_key;  // residency checked for this kernel and size
         b->ok_smem = smem;
     }
     // one persistent launch per phase, back to back (each after zeroing its
@@ -1557,7 +1601,6 @@ void run_batch(pg_batch* b, const pg_options& o, const float* const* F, double* 
     // precision / shared-memory size / time limit) into a CUDA graph
     auto launch_phases = [&](cudaStream_t s) -> cudaError_t {
         for (auto& ph : b->phases) {
-            const void* fn = kernel_of(ph->kind);
             cudaError_t e = cudaMemsetAsync(ph->class_next.p, 0, ph->class_next.n * sizeof(int), s);
             if (e == cudaSuccess)
                 e = cudaMemsetAsync(ph->claims.p, 0, ph->claims.n * sizeof(unsigned long long), s);
@@ -1575,7 +1618,6 @@ void run_batch(pg_batch* b, const pg_options& o, const float* const* F, double* 
         }
         return cudaSuccess;
     };
-    const int prec_key = mixed ? 1 : 2;
     if (!b->graph_failed && (!b->graph || b->graph_precision != prec_key || b->graph_smem != smem ||
                              b->graph_timeout_ns != claim_timeout_ns)) {
         if (b->graph) {
@@ -1945,25 +1987,27 @@ int pg_solve_load_cases(pg_ctx* c, const pg_problem* p, int count, const float* 
         bool cached = false;
         Plan* pl = get_plan(c, *p, G, halo_rings(o), &cached);
         prepare_plan_data(c, pl, o);
-        // group width: automatic = the widest whose layout keeps the Ke
-        // blocks in shared memory, else the widest that fits.  Ke blocks read
-        // from L2 by every block twice per iteration cost more than a wider
-        // group saves (60k-DOF plate, mixed two-level Chebyshev: four cases
-        // per launch with Ke in L2 1.64 ms per case, two with Ke in shared
-        // memory 1.35, one 1.71)
-        auto fits = [&](int NR, int* km = nullptr) {
-            int m = 0;
-            bool ai = false;
+        // group width: automatic = with the two-level preconditioner two cases,
+        // else the widest of 4 and 2 whose layout keeps the row blocks on
+        // chip, else the widest that fits.  A case adds 3 partial sums per block
+        // to what every block reads each round (block Jacobi) or 6 (two-level),
+        // and four cases' 3,552 values cost more than they share: 60k-DOF
+        // plate, ms per case with 1 / 2 / 4 cases a launch: FP64 block Jacobi
+        // 5.17 / 4.20 / 3.86, FP64 two-level 1.95 / 1.66 / 2.05, mixed two-level
+        // Chebyshev 1.37 / 1.26 / 1.58
+        auto fits = [&](int NR, bool* on_chip = nullptr) {
+            bool all = false, ai = false;
             pg::SmemLayout L{};
-            const bool ok = choose_layout_multi(c, pl->hp, o, NR, &m, &ai, &L);
-            if (km) *km = m;
+            const bool ok = choose_layout_multi(c, pl->hp, o, NR, &all, &ai, &L);
+            if (on_chip) *on_chip = ok && all;
             return ok;
         };
         int W = cases_per_launch;
         if (W == 0) {
-            int km4 = 0, km2 = 0;
-            const bool f4 = fits(4, &km4), f2 = fits(2, &km2);
-            W = (f4 && km4 > 0) ? 4 : (f2 && km2 > 0) ? 2 : f4 ? 4 : f2 ? 2 : 1;
+            bool all4 = false, all2 = false;
+            const bool f4 = fits(4, &all4), f2 = fits(2, &all2);
+            const bool two = o.preconditioner == PG_PRECOND_TWO_LEVEL && f2;
+            W = two ? 2 : all4 ? 4 : all2 ? 2 : f4 ? 4 : f2 ? 2 : 1;
         }
         else if (W > 1 && !fits(W)) throw Fail{PG_EUNSUPPORTED, "load-case partition too large for shared memory"};
         for (int k0 = 0; k0 < count;) {
@@ -2101,7 +2145,7 @@ int pg_plan_inspect_halo(const pg_problem* p, int ctas, int rings, int32_t* stat
         pg::HostPlan hp;
         e = pg::build_structure(*p, hp);
         if (rings != 1 && rings != 2) e = "rings must be 1 or 2";
-        if (e.empty()) e = pg::build_partition(*p, ctas > 0 ? ctas : 1, rings, hp);
+        if (e.empty()) e = pg::build_partition(*p, ctas > 0 ? ctas : 1, rings, hp, true);
         if (!e.empty()) { put(e); return PG_EINVAL; }
         const int Nn = hp.Nn, npe = hp.npe, C = hp.colors;
         int bad = 0;

@@ -1,0 +1,172 @@
+// The operator as assembled 3x3 node blocks ("row blocks"), the form the
+// persistent PCG kernels multiply with.
+//
+// Row n of a part holds one slot per node m that shares an element with n
+// (n itself included): the block K_nm = sum of the shared elements' 3x3
+// blocks, added in FP64 in element order and rounded once for FP32 solves.
+// Slots are sorted by global node id, so the parts that hold a row (its
+// owner, and with a 2-ring halo its neighbours) have the same slots in the
+// same order and compute the same bits.
+//
+// Rows are taken in groups of 10, one warp a group: lanes 3 i, 3 i + 1 and
+// 3 i + 2 share row i of the group and take its slots in turn (lane 3 i + d
+// slots d, d + 3, ...), each adding its slots' blocks to all three
+// components; two shuffles then give lane 3 i + d component d.  A group is
+// stored as q-steps (slots 3 q .. 3 q + 2 of its rows): 30 columns and
+// 9 x 30 block entries (row-major 3 r + c, then lane), so consecutive lanes
+// read consecutive words; rows with fewer slots are padded with zero blocks.
+//
+// Why: an assembled row of the Q4 grid has 9 blocks (648 B in FP64), its
+// four element tasks 4 x 36 entries (1,152 B) whose results had to be
+// written and gathered again behind a barrier.  K u was bound by the
+// shared-memory reads of those entries.  A warp's first group stays in
+// registers (3 q-steps: 27 entries a lane), so the parts of the
+// 60k-DOF plate read no coefficients at all; a lane reads u of a slot's node
+// once for three components (9 loads a lane where a thread per component
+// needs 27).
+#pragma once
+
+#include <cstdint>
+
+namespace pg {
+
+constexpr int kRowGroup = 10;   // rows per group (3 lanes each: 30 of a warp's 32)
+constexpr int kRowLanes = 30;
+constexpr int kRegSteps = 3;    // q-steps of a resident group kept in registers
+
+// Local index of global node m in a part: three runs of ascending node ids,
+// the owned nodes [0, no), ring 1 [no, n1) and the rest [n1, nloc) (one halo
+// ring: n1 = no).
+__device__ __forceinline__ int local_index(const int* __restrict__ nodes, int no, int n1, int nloc, int m) {
+    const int seg[4] = {0, no, n1, nloc};
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        int lo = seg[k], hi = seg[k + 1];
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (nodes[mid] < m) lo = mid + 1;
+            else hi = mid;
+        }
+        if (lo < seg[k + 1] && nodes[lo] == m) return lo;
+    }
+    return 0;
+}
+
+// Columns and blocks of every part's rows from the element matrices: one
+// thread per (row, slot residue), blockIdx.x the part, blockIdx.y a share of
+// its groups.
+template <int NPE>
+__global__ void row_fill_kernel(const int* __restrict__ node_off, const int* __restrict__ nown,
+                                const int* __restrict__ n1, const int* __restrict__ nodes,
+                                const int* __restrict__ grp_off, const int* __restrict__ grp_q,
+                                const int* __restrict__ inc_ptr, const int* __restrict__ inc_idx,
+                                const uint32_t* __restrict__ elements, const double* __restrict__ ke64,
+                                uint16_t* __restrict__ rcol, double* __restrict__ rk64,
+                                float* __restrict__ rk32) {
+    constexpr int ND = 3 * NPE;
+    const int g = blockIdx.x, n0 = node_off[g], nloc = node_off[g + 1] - n0, no = nown[g], nn1 = n1[g];
+    const int gb = grp_off[g], ng = grp_off[g + 1] - gb;
+    const int* pn = nodes + n0;
+    for (int t = blockIdx.y * blockDim.x + threadIdx.x; t < ng * kRowLanes; t += gridDim.y * blockDim.x) {
+        const int grp = t / kRowLanes, lane = t - grp * kRowLanes, i = grp * kRowGroup + lane / 3, d = lane % 3;
+        const int q0 = grp_q[gb + grp], q1 = grp_q[gb + grp + 1];
+        int q = q0;
+        if (i < nn1) {
+            const int n = pn[i], a = inc_ptr[n], b = inc_ptr[n + 1];
+            int prev = -1;
+            for (int j = 0;; j++) {
+                // the next node id of the row: the smallest above the last
+                int m = 0x7fffffff;
+                for (int k = a; k < b; k++) {
+                    const uint32_t* en = elements + (size_t)(inc_idx[k] >> 2) * NPE;
+#pragma unroll
+                    for (int p = 0; p < NPE; p++) {
+                        const int v = (int)en[p];
+                        if (v > prev && v < m) m = v;
+                    }
+                }
+                if (m == 0x7fffffff) break;
+                prev = m;
+                if (j % 3 != d) continue;
+                double blk[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+                for (int k = a; k < b; k++) {
+                    const int e = inc_idx[k] >> 2;
+                    const double* K = ke64 + (size_t)e * ND * ND + 3 * (inc_idx[k] & 3) * ND;
+#pragma unroll
+                    for (int p = 0; p < NPE; p++)
+                        if ((int)elements[(size_t)e * NPE + p] == m)
+#pragma unroll
+                            for (int r = 0; r < 9; r++) blk[r] += K[(r / 3) * ND + 3 * p + r % 3];
+                }
+                rcol[(size_t)q * kRowLanes + lane] = (uint16_t)local_index(pn, no, nn1, nloc, m);
+#pragma unroll
+                for (int r = 0; r < 9; r++) {
+                    const size_t o = ((size_t)q * 9 + r) * kRowLanes + lane;
+                    rk64[o] = blk[r];
+                    rk32[o] = (float)blk[r];
+                }
+                q++;
+            }
+        }
+        for (; q < q1; q++) {  // padding: a zero block on the row itself
+            rcol[(size_t)q * kRowLanes + lane] = (uint16_t)(i < nn1 ? i : 0);
+            for (int r = 0; r < 9; r++) {
+                const size_t o = ((size_t)q * 9 + r) * kRowLanes + lane;
+                rk64[o] = 0.0;
+                rk32[o] = 0.0f;
+            }
+        }
+    }
+}
+
+// shared[n] = 1 for every node that is a ghost of some part.
+__global__ void mark_ghosts_kernel(const int* __restrict__ node_off, const int* __restrict__ nown,
+                                   const int* __restrict__ nodes, uint8_t* __restrict__ shared) {
+    const int g = blockIdx.x;
+    for (int i = node_off[g] + nown[g] + threadIdx.x; i < node_off[g + 1]; i += blockDim.x) shared[nodes[i]] = 1;
+}
+
+// s += the blocks k[9 (q - qa) ..][lane] of q-steps [qa, qb) times u at the
+// columns c[q - qa][lane].
+template <typename T, typename KT>
+__device__ __forceinline__ void row_steps(const T* __restrict__ u, const uint16_t* __restrict__ c,
+                                          const KT* __restrict__ k, int steps, T (&s)[3]) {
+#pragma unroll 3
+    for (int q = 0; q < steps; q++) {
+        const T* v = u + 3 * (int)c[q * kRowLanes];
+        const T v0 = v[0], v1 = v[1], v2 = v[2];
+        const KT* b = k + q * 9 * kRowLanes;
+#pragma unroll
+        for (int r = 0; r < 3; r++)
+            s[r] = fma((T)b[(3 * r + 2) * kRowLanes], v2,
+                       fma((T)b[(3 * r + 1) * kRowLanes], v1, fma((T)b[3 * r * kRowLanes], v0, s[r])));
+    }
+}
+
+// Lane 3 i + d holds its share s of row i's three components: the sum of
+// component d over the row's three lanes, in an order that depends on d
+// alone.  Every lane of the warp calls it.
+template <typename T>
+__device__ __forceinline__ T row_join(const T (&s)[3]) {
+    const int lane = threadIdx.x & 31, d = lane % 3, b = lane - d;
+    // lane d sends component d + 1 to lane d + 1 and component d + 2 to lane d + 2
+    const T up = d == 0 ? s[1] : d == 1 ? s[2] : s[0];
+    const T dn = d == 0 ? s[2] : d == 1 ? s[0] : s[1];
+    const T own = d == 0 ? s[0] : d == 1 ? s[1] : s[2];
+    const T f1 = __shfl_sync(0xffffffffu, up, b + (d + 2) % 3);
+    const T f2 = __shfl_sync(0xffffffffu, dn, b + (d + 1) % 3);
+    return own + f1 + f2;
+}
+
+// Component d of D_n^-1 v for the node of lanes 3 i .. 3 i + 2, lane 3 i + d
+// holding v_d and row d of the node's 3x3 inverse from column d on, cyclically
+// (b[0] = B_dd, b[1] = B_d,d+1, b[2] = B_d,d+2).  All lanes of the warp call it.
+template <typename T>
+__device__ __forceinline__ T jacobi_lane(const T (&b)[3], T v) {
+    const int lane = threadIdx.x & 31, d = lane % 3, l0 = lane - d;
+    const T v1 = __shfl_sync(0xffffffffu, v, l0 + (d + 1) % 3);
+    const T v2 = __shfl_sync(0xffffffffu, v, l0 + (d + 2) % 3);
+    return b[0] * v + b[1] * v1 + b[2] * v2;
+}
+
+}  // namespace pg

@@ -171,11 +171,12 @@ typedef struct pg_info {
                                      then the correction's; the residuals refer to the final
                                      x and F; solve_ms covers both) */
     double phase_us[8];           /* with phase_timing, block 0's time (SM cycles at
-                                     the nominal clock) in: K.u; gather, dots and
-                                     publishing w; block reduction and publishing the
+                                     the nominal clock) in: K.u, dots and publishing w
+                                     (load cases: K.u); load cases: dots and publishing
+                                     w; block reduction and publishing the
                                      partials; the Chebyshev smoother's K t; the
                                      exchange wait; the barrier after the decision;
-                                     thread 0's decision; the other vector updates */
+                                     the decision; the other vector updates */
     double trace_ns[6];           /* with trace_iteration, over all blocks: spread of
                                      iteration starts; spread of partial publication;
                                      first start to last publication; last publication
