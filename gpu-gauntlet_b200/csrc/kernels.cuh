@@ -132,6 +132,7 @@ struct PcgArgs {
     const float* ainv32;        // [rows][C]
     int ainv_smem;
     int reliable_interval;
+    int stall_limit;            // replacements without halving the FP64 residual: stagnated
     double reliable_delta;
     // polynomial smoother (smoother = 1; needs a plan with a 2-ring halo):
     // u = a D^-1 r - b D^-1 K D^-1 r (the degree-2 Chebyshev step for
@@ -1671,8 +1672,8 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& a, const int g, unsigned
                 } else if (trn < 0.5 * dec->best_trn) {
                     dec->best_trn = trn;
                     dec->stall = 0;
-                } else if (++dec->stall >= 3) {
-                    // three replacements in a row without halving the FP64
+                } else if (++dec->stall >= a.stall_limit) {
+                    // that many replacements in a row without halving the FP64
                     // residual: the FP32 inner iterations no longer reduce
                     // the error (condition number near 1 / FP32 epsilon)
                     stop = STOP_STAGNATED;

@@ -926,6 +926,7 @@ pg::PcgArgs fill_args(Plan* pl, const pg_options& o, const pg::SmemLayout& L, bo
     // whose FP32 residual stalls along with the true one is still checked
     a.reliable_interval = o.reliable_interval > 0 ? o.reliable_interval : 200;
     a.reliable_delta = o.reliable_delta > 0 ? o.reliable_delta : 0.1;
+    a.stall_limit = 3;
     a.L = L;
     return a;
 }
@@ -1005,9 +1006,10 @@ const void* batch_kernel_of(bool coarse, bool cheb) {
 // Queues set-up (first solve of the plan) and the persistent PCG launch on
 // the context stream, then waits for the result record (one readback).
 // x_dst (optional) receives the solution by a copy of `kind` queued right
-// behind the kernel, so the call waits for the device once.
+// behind the kernel, so the call waits for the device once.  stall_limit:
+// residual replacements without halving that end a mixed solve.
 void run_solve(pg_ctx* c, Plan* pl, const pg_options& o, pg_info* info, void* x_dst = nullptr,
-               cudaMemcpyKind kind = cudaMemcpyDeviceToDevice) {
+               cudaMemcpyKind kind = cudaMemcpyDeviceToDevice, int stall_limit = 3) {
     const pg::HostPlan& hp = pl->hp;
     const int threads = solve_threads(o);
     const bool lean = threads <= pg::kLeanThreads;
@@ -1021,6 +1023,7 @@ void run_solve(pg_ctx* c, Plan* pl, const pg_options& o, pg_info* info, void* x_
     reset_for_launch(c, pl, pl->res.p);
     CK(cudaMemsetAsync(pl->abort_flag.p, 0, sizeof(int), c->stream));
     pg::PcgArgs a = fill_args(pl, o, L, ainv_smem, pl->abort_flag.p, pl->res.p);
+    a.stall_limit = stall_limit;
     if (a.trace_it > 0)
         CK(cudaMemsetAsync(pl->trace.p, 0, pl->trace.n * sizeof(unsigned long long), c->stream));
 
@@ -1100,6 +1103,9 @@ double correction_tolerance(const pg_options& o, double bnorm, double r0) {
     return r0 > 0 ? std::min(0.5, target / r0) : o.tolerance;
 }
 
+bool persistent_fits(const pg_ctx* c, const Plan* pl, const pg_options& o);
+void global_solve(pg_ctx* c, Plan* pl, const pg_options& o, pg_info* info, void* x_dst, cudaMemcpyKind kind);
+
 // After a mixed solve of pl stagnated (pl->x holds its x_m, pl->F the
 // load): solves K d = F - K x_m in FP64, its load the FP32-rounded residual
 // and its stop scaled to the residual x_m already reached, then x = x_m + d
@@ -1111,6 +1117,19 @@ void fp64_correction(pg_ctx* c, Plan* pl, const pg_options& o, pg_info* mi, void
     const int ni = (int)n;
     const double bnorm = mi->b_norm, r0 = mi->final_residual;
     cudaStream_t st = c->stream;
+    pg_options o64 = o;
+    o64.precision = PG_PREC_FP64;
+    o64.stop_rule = PG_STOP_RELATIVE;
+    o64.tolerance = correction_tolerance(o, bnorm, r0);
+    if (!persistent_fits(c, pl, o64)) {
+        // FP64 state does not fit shared memory: the whole solve again on the
+        // global-memory path
+        const double mixed_ms = mi->setup_ms + mi->solve_ms;
+        global_solve(c, pl, o, mi, x_dst, kind);
+        mi->fallback = 1;
+        mi->solve_ms += mixed_ms;
+        return;
+    }
     if (pl->xw.n != n) pl->xw.alloc(n);
     if (pl->kx.n != n) pl->kx.alloc(n);
     if (pl->rf.n != n) pl->rf.alloc(n);
@@ -1120,10 +1139,6 @@ void fp64_correction(pg_ctx* c, Plan* pl, const pg_options& o, pg_info* mi, void
     queue_apply_k(c, pl, pl->xw.p, pl->kx.p);
     pg::residual_f32_kernel<<<(ni + 255) / 256, 256, 0, st>>>(ni, pl->cons.p, pl->rf.p, pl->kx.p, pl->F.p);
     CK(cudaGetLastError());
-    pg_options o64 = o;
-    o64.precision = PG_PREC_FP64;
-    o64.stop_rule = PG_STOP_RELATIVE;
-    o64.tolerance = correction_tolerance(o, bnorm, r0);
     pg_info fi{};
     run_solve(c, pl, o64, &fi, nullptr, kind);
     pg::add_kernel<<<(ni + 255) / 256, 256, 0, st>>>(ni, pl->xw.p, pl->x.p);
@@ -1199,6 +1214,27 @@ void solve_with_fallback(pg_ctx* c, Plan* pl, const pg_options& o, pg_info* info
     pg_info local{};
     pg_info* fi = info ? info : &local;
     if (!persistent_fits(c, pl, o)) {
+        // FP64 state does not fit with one part per SM: the same method with
+        // FP32 vectors in the persistent kernel, where those fit (FP64 x, dot
+        // products and true-residual stop, as on the global-memory path that
+        // takes what is left: larger plates, the 2-ring halo, and solves that
+        // FP32 stalls).  The two-level solve replaces its residual as often as
+        // that path, every 50 updates: with 200 the FP32 residual of a plate this
+        // large drifts and the solve stalls, with 50 none did (plates of 380 to
+        // 420 elements a side, two seeds each).  Block Jacobi, whose residual stays
+        // flat for hundreds of updates, keeps 200; either gives up after 800
+        // updates without halving the true residual.  482k-DOF plate, 1e-8:
+        // two-level 144 -> 25 ms (1,230 iterations instead of 2,949 of two
+        // smoothing steps), block Jacobi 194 -> 58 ms
+        pg_options om = o;
+        om.precision = PG_PREC_MIXED;
+        const int ri = o.preconditioner == PG_PRECOND_TWO_LEVEL ? 50 : 200;
+        if (om.reliable_interval <= 0) om.reliable_interval = ri;
+        if (pl->G >= c->sms && o.precision == PG_PREC_FP64 && persistent_fits(c, pl, om)) {
+            run_solve(c, pl, om, fi, x_dst, kind, std::max(3, 800 / ri));
+            fi->global_path = 1;
+            if (fi->stop_reason != PG_STOP_STAGNATED) return;
+        }
         global_solve(c, pl, o, fi, x_dst, kind);
         return;
     }

@@ -184,11 +184,13 @@ typedef struct pg_info {
                                      of exchange completion; whole iteration */
     double smoother_lambda_max;   /* Chebyshev smoother: the lambda_max(D^-1 K) estimate used */
     int32_t global_path;          /* 1 when the plate's parts did not fit one block's shared
-                                     memory and the solve ran as flexible PCG over global
-                                     memory: FP32 vectors, FP64 x, dot products and true-
-                                     residual stop; block Jacobi, or damped block-Jacobi
-                                     smoothing steps when the two-level preconditioner or
-                                     the Chebyshev smoother was asked for */
+                                     memory and the solve ran with FP32 vectors, FP64 x, dot
+                                     products and true-residual stop: the method asked for in
+                                     the persistent kernel (threads > 0) when its FP32 layout
+                                     fits, else flexible PCG over global memory (threads 0):
+                                     block Jacobi, or damped block-Jacobi smoothing steps when
+                                     the two-level preconditioner or the Chebyshev smoother
+                                     was asked for */
     int32_t reserved;
     double plan_ms;               /* host wall time in this call of: building the partition
                                      plan (pg_solve; 0 when the plan was cached), */
