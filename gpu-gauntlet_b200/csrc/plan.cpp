@@ -369,22 +369,6 @@ std::string build_partition(const pg_problem& p, int G, int rings, HostPlan& pla
     return "";
 }
 
-// sum_{k in [k0, k1)} a[k] b[k] in four interleaved partial sums (the
-// dependent additions of a single running sum would bound the dense steps
-// of the coarse set-up by the adder's latency)
-static double dot4(const double* a, const double* b, int k0, int k1) {
-    double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
-    int k = k0;
-    for (; k + 4 <= k1; k += 4) {
-        s0 += a[k] * b[k];
-        s1 += a[k + 1] * b[k + 1];
-        s2 += a[k + 2] * b[k + 2];
-        s3 += a[k + 3] * b[k + 3];
-    }
-    for (; k < k1; k++) s0 += a[k] * b[k];
-    return (s0 + s1) + (s2 + s3);
-}
-
 std::string build_coarse_meta(const pg_problem& p, HostPlan& plan) {
     const int G = plan.G, Nn = plan.Nn;
     const int C = 3 * G;
@@ -422,7 +406,6 @@ std::string build_coarse_meta(const pg_problem& p, HostPlan& plan) {
     plan.cagg.clear();
     plan.ainv_off.assign(G + 1, 0);
     plan.ainv_src.clear();
-    plan.ainv.clear();
     plan.max_kagg = 0;
     std::vector<int> slot_of(G, -1);
     for (int g = 0; g < G; g++) {
@@ -453,102 +436,6 @@ std::string build_coarse_meta(const pg_problem& p, HostPlan& plan) {
         for (int a : list) slot_of[a] = -1;
     }
     plan.ainv_off[G] = (int)plan.ainv_src.size();
-    return "";
-}
-
-std::string build_coarse(const pg_problem& p, const std::vector<double>& ke64, HostPlan& plan) {
-    std::string e = build_coarse_meta(p, plan);
-    if (!e.empty()) return e;
-    const int Nn = plan.Nn, npe = plan.npe, nd = 3 * npe;
-    const int C = plan.C;
-    const std::vector<int>& owner = plan.coarse_owner;
-    const std::vector<double>& geom = plan.coarse_geom;
-    (void)Nn;
-    // basis of node n in mode m, DOF d (masked by constraints); Phi[d][m]
-    auto phi = [&](int n, double Phi[3][3]) {
-        const int a = owner[n];
-        const double ih = geom[3 * a + 2];
-        const double dx = (p.nodes[2 * n] - geom[3 * a]) * ih, dy = (p.nodes[2 * n + 1] - geom[3 * a + 1]) * ih;
-        const double v[3][3] = {{1.0, dy, dx}, {0.0, ih, 0.0}, {0.0, 0.0, -ih}};
-        for (int d = 0; d < 3; d++)
-            for (int m = 0; m < 3; m++) Phi[d][m] = p.constrained[3 * n + d] ? 0.0 : v[d][m];
-    };
-    // A_c = P^T K P, element by element
-    std::vector<double> Ac((size_t)C * C, 0.0);
-    const size_t kk = (size_t)nd * nd;
-    for (int e = 0; e < plan.Ne; e++) {
-        const double* K = ke64.data() + (size_t)e * kk;
-        double Ph[4][3][3];
-        int ag[4];
-        for (int i = 0; i < npe; i++) {
-            const int n = (int)p.elements[(size_t)e * npe + i];
-            phi(n, Ph[i]);
-            ag[i] = owner[n];
-        }
-        for (int i = 0; i < npe; i++)
-            for (int j = 0; j < npe; j++) {
-                double T[3][3];  // K_ij Phi_j
-                for (int d = 0; d < 3; d++)
-                    for (int m = 0; m < 3; m++) {
-                        double acc = 0;
-                        for (int f = 0; f < 3; f++) acc += K[(3 * i + d) * nd + 3 * j + f] * Ph[j][f][m];
-                        T[d][m] = acc;
-                    }
-                for (int mi = 0; mi < 3; mi++)
-                    for (int mj = 0; mj < 3; mj++) {
-                        double acc = 0;
-                        for (int d = 0; d < 3; d++) acc += Ph[i][d][mi] * T[d][mj];
-                        Ac[(size_t)(3 * ag[i] + mi) * C + 3 * ag[j] + mj] += acc;
-                    }
-            }
-    }
-    // Cholesky with dependent modes dropped, then the explicit inverse
-    std::vector<double> Lm((size_t)C * C, 0.0);
-    std::vector<char> keep(C, 1);
-    double dmax = 0;
-    for (int i = 0; i < C; i++) dmax = std::max(dmax, Ac[(size_t)i * C + i]);
-    plan.dropped_modes = 0;
-    for (int j = 0; j < C; j++) {
-        const double* lrow = Lm.data() + (size_t)j * C;
-        const double d = Ac[(size_t)j * C + j] - dot4(lrow, lrow, 0, j);
-        if (!(d > 1e-13 * dmax)) {
-            keep[j] = 0;
-            plan.dropped_modes++;
-            continue;
-        }
-        const double ljj = std::sqrt(d);
-        Lm[(size_t)j * C + j] = ljj;
-        for (int i = j + 1; i < C; i++) {
-            const double s = Ac[(size_t)i * C + j] - dot4(Lm.data() + (size_t)i * C, lrow, 0, j);
-            Lm[(size_t)i * C + j] = s / ljj;
-        }
-    }
-    // inverse of L (lower), dropped columns stay zero; kept transposed
-    // (Lt[j][k] = (L^-1)[k][j]) so that both loops below run along rows
-    std::vector<double> Lt((size_t)C * C, 0.0);
-    for (int j = 0; j < C; j++) {
-        if (!keep[j]) continue;
-        double* lj = Lt.data() + (size_t)j * C;
-        lj[j] = 1.0 / Lm[(size_t)j * C + j];
-        for (int i = j + 1; i < C; i++) {
-            if (!keep[i]) continue;
-            const double* li = Lm.data() + (size_t)i * C;
-            lj[i] = -dot4(li, lj, j, i) / li[i];
-        }
-    }
-    std::vector<double> Ainv((size_t)C * C, 0.0);  // L^-T L^-1
-    for (int i = 0; i < C; i++)
-        for (int j = 0; j <= i; j++) {
-            const double s = dot4(Lt.data() + (size_t)i * C, Lt.data() + (size_t)j * C, i, C);
-            Ainv[(size_t)i * C + j] = s;
-            Ainv[(size_t)j * C + i] = s;
-        }
-    // each part's rows of A_c^-1 (3 per aggregate of its list)
-    plan.ainv.resize(plan.ainv_src.size() * (size_t)C);
-    for (size_t r = 0; r < plan.ainv_src.size(); r++)
-        std::copy(Ainv.begin() + (size_t)plan.ainv_src[r] * C, Ainv.begin() + (size_t)(plan.ainv_src[r] + 1) * C,
-                  plan.ainv.begin() + r * C);
-    plan.coarse = true;
     return "";
 }
 

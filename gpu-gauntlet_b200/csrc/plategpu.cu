@@ -134,7 +134,7 @@ struct Plan {
     DevBuf<double> ke64, binv64, x;
     DevBuf<float> ke32, binv32;
     DevBuf<unsigned long long> llv, llx, llp;
-    DevBuf<int> cagg_off, node_slot, ainv_off;
+    DevBuf<int> cagg_off, node_slot, ainv_off, dropped;
     DevBuf<double> node_basis, ainv64;
     DevBuf<float> ainv32;
     DevBuf<int> abort_flag;
@@ -541,50 +541,41 @@ void queue_apply_k(pg_ctx* c, Plan* pl, const double* x, double* y) {
 // vector 1 + 0.5 sin(0.7 i) (0 on constrained DOFs): |z_iters| / |z_(iters-1)|
 // with z_(k+1) = D^-1 K z_k.  The iterates are left unnormalised; their
 // growth, at most about 9^iters for the plate operators, stays far inside
-// FP64's range.  queue_power_steps queues the steps (z_iters ends in pl->xw
-// for even iters, else pl->pw; z_(iters-1) in the other), lambda_from_power
-// reads them back once the stream has run them and sums the two norms on
-// the host, in order.
+// FP64's range.  queue_power_steps queues the steps and the two norms,
+// lambda_from_power reads the norms back once the stream has run them.
 void queue_power_steps(pg_ctx* c, Plan* pl, int iters) {
     const pg::HostPlan& hp = pl->hp;
     const size_t n = 3 * (size_t)hp.Nn;
     if (n == 0) return;
     run_setup(c, pl);
     if (pl->xw.n != n) pl->xw.alloc(n);
-    if (pl->kx.n != n) pl->kx.alloc(n);
     if (pl->pw.n != n) pl->pw.alloc(n);
     cudaStream_t st = c->stream;
     double* a = pl->xw.p;
     double* b = pl->pw.p;
     pg::power_start_kernel<<<((int)n + 255) / 256, 256, 0, st>>>((int)n, pl->cons.p, a);
     CK(cudaGetLastError());
+    int groups = 0, steps = 0;
+    largest_rows(hp, &groups, &steps);
+    const dim3 grid(hp.G, std::max(1, std::min(64, (groups + 7) / 8)));
     for (int it = 0; it < iters; it++) {
-        if (hp.npe == 4)
-            pg::power_step_kernel<4><<<(hp.Nn + 255) / 256, 256, 0, st>>>(
-                hp.Nn, pl->inc_ptr.p, pl->inc_idx.p, pl->mesh_elements.p, pl->ke64.p, pl->cons.p, pl->binv64.p, a, b);
-        else
-            pg::power_step_kernel<3><<<(hp.Nn + 255) / 256, 256, 0, st>>>(
-                hp.Nn, pl->inc_ptr.p, pl->inc_idx.p, pl->mesh_elements.p, pl->ke64.p, pl->cons.p, pl->binv64.p, a, b);
+        pg::power_step_kernel<<<grid, 256, 0, st>>>(pl->node_off.p, pl->nown.p, pl->nodes.p, pl->grp_off.p, pl->grp_q.p,
+                                                    pl->rcol.p, pl->rk64.p, pl->cons.p, pl->binv64.p, a, b);
         CK(cudaGetLastError());
         std::swap(a, b);
     }
+    // |z_iters|^2 and |z_(iters-1)|^2
+    if (pl->nrm.n != 2) pl->nrm.alloc(2);
+    pg::two_norms_kernel<<<1, 1024, 0, st>>>((int)n, a, b, pl->nrm.p);
+    CK(cudaGetLastError());
 }
 
 double lambda_from_power(pg_ctx* c, Plan* pl, int iters) {
-    const size_t n = 3 * (size_t)pl->hp.Nn;
-    if (n == 0 || iters < 1) return 1.0;
-    const double* last = iters % 2 == 0 ? pl->xw.p : pl->pw.p;
-    const double* prev = iters % 2 == 0 ? pl->pw.p : pl->xw.p;
-    std::vector<double> za(n), zb(n);
-    CK(cudaMemcpyAsync(za.data(), last, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpyAsync(zb.data(), prev, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    if (pl->hp.Nn == 0 || iters < 1) return 1.0;
+    double nn[2] = {0.0, 0.0};
+    CK(cudaMemcpyAsync(nn, pl->nrm.p, sizeof nn, cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    double na = 0.0, nb = 0.0;
-    for (size_t i = 0; i < n; i++) {
-        na += za[i] * za[i];
-        nb += zb[i] * zb[i];
-    }
-    const double lam = nb > 0 ? std::sqrt(na / nb) : 0.0;
+    const double lam = nn[1] > 0 ? std::sqrt(nn[0] / nn[1]) : 0.0;
     return std::isfinite(lam) && lam > 0 ? lam : (double)pl->hp.npe;
 }
 
@@ -622,17 +613,13 @@ void fill_options(const pg_options* in, pg_options* o) {
 // polynomial smoother, else 1.
 int halo_rings(const pg_options& o) { return o.smoother == PG_SMOOTHER_CHEBYSHEV ? 2 : 1; }
 
-// Coarse data of the two-level preconditioner, built once per plan.  One
-// plate: the aggregate lists and basis data on the host (build_coarse_meta),
-// A_c = P^T K P, its factorisation and inverse, and each part's A_c^-1 rows
-// on the device (coarse.cuh), from the element matrices already there.
-// Batches build the dense part on host threads (prepare_many, build_coarse).
-void upload_coarse(pg_ctx* c, Plan* pl);
-void carve_coarse(Arena& ar, Plan* pl, size_t n, const double* a64, const float* a32);
-
-void ensure_coarse(pg_ctx* c, Plan* pl) {
+// Coarse data of the two-level preconditioner, built once per plan: the
+// aggregate lists and basis data on the host (build_coarse_meta), A_c = P^T K P,
+// its inverse and each part's A_c^-1 rows on the device (coarse.cuh), from the
+// element matrices already there.  queue_coarse queues it on the context
+// stream, finish_coarse reads the count of dropped modes once it has run.
+void queue_coarse(pg_ctx* c, Plan* pl) {
     pg::HostPlan& hp = pl->hp;
-    if (hp.coarse) return;
     run_setup(c, pl);
     std::string e = pg::build_coarse_meta(pl->prob_view, hp);
     if (!e.empty()) throw Fail{PG_EINVAL, e};
@@ -640,32 +627,29 @@ void ensure_coarse(pg_ctx* c, Plan* pl) {
     const int C = hp.C;
     const size_t CC = (size_t)C * C;
     const int rows = (int)hp.ainv_src.size();
-    // the set-up's scratch arrays in one allocation, freed on return; A_c,
-    // L, Lt and A_c^-1 ([C][C] each, consecutive) in `mats`: the first three
-    // start zeroed, every entry of A_c^-1 is written by coarse_inverse_kernel
-    DevBuf<unsigned char> scratch;
-    DevBuf<int> owner, src, keep, dropped;
-    DevBuf<double> geom, mats;
-    {
-        Arena ar;
-        ar.add(owner, hp.coarse_owner.size(), hp.coarse_owner.data());
-        ar.add(geom, hp.coarse_geom.size(), hp.coarse_geom.data());
-        ar.add(src, hp.ainv_src.size(), hp.ainv_src.data());
-        ar.add(mats, 4 * CC, nullptr);
-        ar.add(keep, (size_t)C, nullptr);
-        ar.add(dropped, 1, nullptr);
-        ar.commit(scratch, st);
-    }
-    {
-        Arena ar;
-        carve_coarse(ar, pl, (size_t)rows * C, nullptr, nullptr);
-        ar.commit(pl->coarse_arena, st);
-    }
-    double* const Ac = mats.p;
-    double* const L = mats.p + CC;
-    double* const Lt = mats.p + 2 * CC;
-    double* const Ainv = mats.p + 3 * CC;
-    CK(cudaMemsetAsync(mats.p, 0, 3 * CC * sizeof(double), st));
+    const size_t n = (size_t)rows * C;
+    // the plan's arrays and the set-up's scratch (A_c and a second [C][C] to
+    // step into, the owners and geometry) in one allocation that the plan keeps
+    DevBuf<int> owner, src;
+    DevBuf<double> geom, mats, dmax;
+    Arena ar;
+    ar.add(pl->ainv64, n, nullptr);
+    ar.add(pl->ainv32, n, nullptr);
+    ar.add(pl->cagg_off, hp.cagg_off.size(), hp.cagg_off.data());
+    ar.add(pl->node_slot, hp.node_slot.size(), hp.node_slot.data());
+    ar.add(pl->node_basis, hp.node_basis.size(), hp.node_basis.data());
+    ar.add(pl->ainv_off, hp.ainv_off.size(), hp.ainv_off.data());
+    ar.add(pl->dropped, 1, nullptr);
+    ar.add(owner, hp.coarse_owner.size(), hp.coarse_owner.data());
+    ar.add(geom, hp.coarse_geom.size(), hp.coarse_geom.data());
+    ar.add(src, hp.ainv_src.size(), hp.ainv_src.data());
+    ar.add(mats, 2 * CC, nullptr);
+    ar.add(dmax, 1, nullptr);
+    ar.commit(pl->coarse_arena, st);
+    double* Ac = mats.p;
+    double* other = mats.p + CC;
+    CK(cudaMemsetAsync(Ac, 0, CC * sizeof(double), st));
+    CK(cudaMemsetAsync(pl->dropped.p, 0, sizeof(int), st));
     if (hp.Ne > 0) {
         if (hp.npe == 4)
             pg::coarse_assemble_kernel<4><<<(hp.Ne + 127) / 128, 128, 0, st>>>(
@@ -675,60 +659,34 @@ void ensure_coarse(pg_ctx* c, Plan* pl) {
                 hp.Ne, C, pl->mesh_nodes.p, pl->mesh_elements.p, pl->cons.p, owner.p, geom.p, pl->ke64.p, Ac);
         CK(cudaGetLastError());
     }
-    // the blocked factorisation when its panels fit in shared memory
-    // (1 KB left for the kernel's static shared memory)
-    const size_t smem_cap = (size_t)c->max_smem - 1024;
-    const bool blocked = pg::coarse_factor_blocked_smem(C) <= smem_cap;
-    const size_t fsm = blocked ? pg::coarse_factor_blocked_smem(C) : pg::coarse_factor_smem(C);
-    if (fsm > smem_cap) throw Fail{PG_EUNSUPPORTED, "coarse space too large for its factorisation"};
-    const void* ffn = blocked ? (const void*)pg::coarse_factor_kernel : (const void*)pg::coarse_factor_tiles_kernel;
-    if (fsm > 48 * 1024) CK(cudaFuncSetAttribute(ffn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsm));
-    {
-        const double* acp = Ac;
-        double *lp = L, *ltp = Lt;
-        int *kp = keep.p, *dp = dropped.p;
-        void* fargs[] = {(void*)&C, (void*)&acp, (void*)&lp, (void*)&ltp, (void*)&kp, (void*)&dp};
-        CK(cudaLaunchKernel(ffn, dim3(1), dim3(pg::kCoarseThreads), fargs, fsm, st));
+    pg::coarse_dmax_kernel<<<1, 512, 0, st>>>(C, Ac, dmax.p);
+    CK(cudaGetLastError());
+    const int nt = (C + pg::kCoarseTile - 1) / pg::kCoarseTile;
+    for (int k = 0; k < nt; k++) {
+        pg::coarse_step_kernel<<<dim3(nt, nt), pg::kCoarseThreads, 0, st>>>(C, k * pg::kCoarseTile, Ac, other, dmax.p,
+                                                                            pl->dropped.p);
+        CK(cudaGetLastError());
+        std::swap(Ac, other);
     }
-    CK(cudaGetLastError());
-    // A_c^-1 = L^-T L^-1: one block per 32 x 32 tile of the lower triangle
-    const int ntile = (C + 31) / 32;
-    pg::coarse_inverse_kernel<<<ntile * (ntile + 1) / 2, pg::kCoarseThreads, 0, st>>>(C, Lt, Ainv);
-    CK(cudaGetLastError());
     if (rows > 0) {
-        const long tot = (long)rows * C;
-        pg::coarse_rows_kernel<<<(int)std::min<long>((tot + 255) / 256, 4096), 256, 0, st>>>(
-            rows, C, src.p, Ainv, pl->ainv64.p, pl->ainv32.p);
+        pg::coarse_rows_kernel<<<(int)std::min<size_t>((n + 255) / 256, 4096), 256, 0, st>>>(
+            rows, C, src.p, Ac, pl->ainv64.p, pl->ainv32.p);
         CK(cudaGetLastError());
     }
+}
+
+void finish_coarse(pg_ctx* c, Plan* pl) {
     int nd = 0;
-    CK(cudaMemcpyAsync(&nd, dropped.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));  // nd; the scratch is freed on return
-    hp.dropped_modes = nd;
-    hp.coarse = true;
+    CK(cudaMemcpyAsync(&nd, pl->dropped.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));  // nd, and the uploads of queue_coarse have been read
+    pl->hp.dropped_modes = nd;
+    pl->hp.coarse = true;
 }
 
-// The plan's device copies of its aggregate lists and node basis data and
-// of its A_c^-1 rows (n entries in FP64 and FP32, copied from a64 / a32
-// when given, else left for coarse_rows_kernel).
-void carve_coarse(Arena& ar, Plan* pl, size_t n, const double* a64, const float* a32) {
-    const pg::HostPlan& hp = pl->hp;
-    ar.add(pl->ainv64, n, a64);
-    ar.add(pl->ainv32, n, a32);
-    ar.add(pl->cagg_off, hp.cagg_off.size(), hp.cagg_off.data());
-    ar.add(pl->node_slot, hp.node_slot.size(), hp.node_slot.data());
-    ar.add(pl->node_basis, hp.node_basis.size(), hp.node_basis.data());
-    ar.add(pl->ainv_off, hp.ainv_off.size(), hp.ainv_off.data());
-}
-
-// Device copies of a plan's coarse data built on the host (build_coarse).
-void upload_coarse(pg_ctx* c, Plan* pl) {
-    const pg::HostPlan& hp = pl->hp;
-    std::vector<float> a32(hp.ainv.begin(), hp.ainv.end());
-    Arena ar;
-    carve_coarse(ar, pl, hp.ainv.size(), hp.ainv.data(), a32.data());
-    ar.commit(pl->coarse_arena, c->stream);
-    CK(cudaStreamSynchronize(c->stream));  // a32 is read by the copy
+void ensure_coarse(pg_ctx* c, Plan* pl) {
+    if (pl->hp.coarse) return;
+    queue_coarse(c, pl);
+    finish_coarse(c, pl);
 }
 
 // Largest eigenvalue of D^-1 K for the polynomial smoother, estimated once
@@ -775,10 +733,8 @@ void prepare_plan_data(pg_ctx* c, Plan* pl, const pg_options& o, pg_info* info =
     }
 }
 
-// prepare_plan_data for many plans (a batch): the eigenvalue estimates run on
-// the device for all plates before one wait; for the coarse matrices the
-// element matrices come down in chunks of plates, the host work runs on
-// worker threads, and the results go back up.
+// prepare_plan_data for many plans (a batch): every plate's device work is
+// queued before the first wait.
 void prepare_many(pg_ctx* c, const std::vector<Plan*>& pls, const pg_options& o) {
     const bool coarse = o.preconditioner == PG_PRECOND_TWO_LEVEL;
     const bool cheb = o.smoother == PG_SMOOTHER_CHEBYSHEV;
@@ -791,45 +747,8 @@ void prepare_many(pg_ctx* c, const std::vector<Plan*>& pls, const pg_options& o)
     // eigenvalue estimates: every plate's power steps queued back to back
     for (Plan* pl : lam_todo) queue_power_steps(c, pl, 30);
     for (Plan* pl : lam_todo) pl->lambda_max = lambda_from_power(c, pl, 30);
-    const unsigned hw = std::max(1u, std::min(32u, std::thread::hardware_concurrency()));
-    for (size_t i = 0; i < todo.size();) {
-        size_t j = i, elems = 0;
-        while (j < todo.size() && (j == i || elems + (size_t)todo[j]->hp.Ne <= 1500000)) elems += todo[j++]->hp.Ne;
-        const size_t m = j - i;
-        std::vector<std::vector<double>> ke(m);
-        for (size_t k = 0; k < m; k++) {
-            Plan* pl = todo[i + k];
-            run_setup(c, pl);
-            const size_t kk = 9 * (size_t)pl->hp.npe * pl->hp.npe;
-            ke[k].resize(std::max<size_t>(1, (size_t)pl->hp.Ne * kk));
-            if (pl->hp.Ne > 0)
-                CK(cudaMemcpyAsync(ke[k].data(), pl->ke64.p, (size_t)pl->hp.Ne * kk * sizeof(double),
-                                   cudaMemcpyDeviceToHost, c->stream));
-        }
-        CK(cudaStreamSynchronize(c->stream));
-        std::vector<std::string> err(m);
-        std::atomic<size_t> next{0};
-        auto work = [&]() {
-            for (size_t k; (k = next.fetch_add(1)) < m;) {
-                Plan* pl = todo[i + k];
-                try {
-                    err[k] = pg::build_coarse(pl->prob_view, ke[k], pl->hp);
-                } catch (...) {
-                    err[k] = "host set-up of the batch failed";
-                }
-            }
-        };
-        std::vector<std::thread> th;
-        for (unsigned t = 1; t < std::min<size_t>(hw, m); t++) th.emplace_back(work);
-        work();
-        for (auto& t : th) t.join();
-        for (size_t k = 0; k < m; k++) {
-            if (!err[k].empty()) throw Fail{PG_EINVAL, err[k]};
-            Plan* pl = todo[i + k];
-            if (pl->hp.coarse && pl->ainv64.n == 0) upload_coarse(c, pl);
-        }
-        i = j;
-    }
+    for (Plan* pl : todo) queue_coarse(c, pl);
+    for (Plan* pl : todo) finish_coarse(c, pl);
 }
 
 // Threads of a one-plate launch: the caller's, or the resident build's.
