@@ -164,6 +164,15 @@ int pick_cot(int rows, int cin) {
     return 16;
 }
 
+// ... for a layer whose `tiles` pixel tiles leave the device idle (batch 1): the
+// widest whose blocks still number 148 or more, else 16.  The outputs'
+// sums do not depend on it.
+int pick_cot_small(int rows, int cin, int tiles) {
+    int c = pick_cot(rows, cin);
+    while (c > 16 && c % 32 == 0 && tiles * (rows / c) < 148) c /= 2;
+    return c;
+}
+
 // Launches kernel<<<grid, block, smem, st>>>(args...), with programmatic
 // stream serialisation when pdl is set (the kernel then starts while its
 // predecessor finishes and waits in pdl_wait before reading its results).
@@ -199,7 +208,8 @@ void conv_launch(const pgn::ConvArgs& a, int rows, cudaStream_t st, bool pdl) {
 // Dispatches the (input channels, output tile, epilogue) combinations the
 // network uses.
 void conv(int mode, int cin, int rows, const pgn::ConvArgs& a, cudaStream_t st, bool pdl = false) {
-    const int cot = pick_cot(rows, cin);
+    const int cot = mode == pgn::OUT_BF16_RELU && a.B == 1 ? pick_cot_small(rows, cin, ((a.W + 7) / 8) * ((a.H + 7) / 8))
+                                                          : pick_cot(rows, cin);
 #define PG_CONV(C, T, M)                                   \
     if (cin == C && cot == T && mode == M) {               \
         conv_launch<C, T, M>(a, rows, st, pdl);            \
@@ -209,6 +219,8 @@ void conv(int mode, int cin, int rows, const pgn::ConvArgs& a, cudaStream_t st, 
     PG_CONV(16, 16, OUT_BF16_RELU) PG_CONV(16, 32, OUT_BF16_RELU) PG_CONV(32, 32, OUT_BF16_RELU)
     PG_CONV(32, 64, OUT_BF16_RELU) PG_CONV(64, 64, OUT_BF16_RELU) PG_CONV(128, 32, OUT_BF16_RELU)
     PG_CONV(192, 32, OUT_BF16_RELU) PG_CONV(96, 32, OUT_BF16_RELU) PG_CONV(48, 16, OUT_BF16_RELU)
+    PG_CONV(32, 16, OUT_BF16_RELU) PG_CONV(64, 16, OUT_BF16_RELU) PG_CONV(64, 32, OUT_BF16_RELU)
+    PG_CONV(128, 16, OUT_BF16_RELU) PG_CONV(192, 16, OUT_BF16_RELU) PG_CONV(96, 16, OUT_BF16_RELU)
     PG_CONV(16, 16, OUT_F32)
     PG_CONV(16, 16, OUT_BF16_MASKED) PG_CONV(16, 48, OUT_BF16_MASKED) PG_CONV(32, 32, OUT_BF16_MASKED)
     PG_CONV(32, 48, OUT_BF16_MASKED) PG_CONV(64, 64, OUT_BF16_MASKED) PG_CONV(128, 32, OUT_BF16_MASKED)
@@ -314,12 +326,26 @@ Workspace* workspace(pg_net* n, int B, bool grads) {
     return w;
 }
 
+// Channels [from, ..) of a decoder input are read from the coarser level (up,
+// channel stride cs) instead of the concatenated buffer.
+pgn::ConvArgs upsampled(pgn::ConvArgs a, const bf16* up, int cs, int from) {
+    a.up = up;
+    a.up_cs = cs;
+    a.up_from = from;
+    return a;
+}
+
 // U-Net forward of ws->in ([B][H][W][16], channels 0..2 used) into ws->out.
+// Without gradient buffers the decoder's first convolutions upsample in their
+// own loads; with them the concatenated inputs are written, which the
+// weight gradients read.
 void net_forward(pg_net* n, Workspace* w, cudaStream_t st, const int* skip, bool pdl = false) {
     const int B = w->B;
     const int H0 = n->H, W0 = n->W, H1 = H0 / 2, W1 = W0 / 2, H2 = H1 / 2, W2 = W1 / 2, H3 = H2 / 2, W3 = W2 / 2;
     const pgn::LayerTable& T = n->T;
     auto wf = [&](int k) { return n->wf.p + T.l[k].off_f; };
+    const bool fuse = !w->grads;
+    auto dec = [&](pgn::ConvArgs a, const bf16* up, int cs, int from) { return fuse ? upsampled(a, up, cs, from) : a; };
     using namespace pgn;
     conv(OUT_BF16_RELU, 16, 16, cargs(B, H0, W0, w->in.p, 16, wf(E0A), 16, w->e0a.p, 16, 0, 16, skip), st, pdl);
     conv(OUT_BF16_RELU, 16, 16, pooled(cargs(B, H0, W0, w->e0a.p, 16, wf(E0B), 16, w->cat0.p, 48, 0, 16, skip), w->p1.p, 16), st, pdl);
@@ -329,14 +355,14 @@ void net_forward(pg_net* n, Workspace* w, cudaStream_t st, const int* skip, bool
     conv(OUT_BF16_RELU, 64, 64, pooled(cargs(B, H2, W2, w->e2a.p, 64, wf(E2B), 64, w->cat2.p, 192, 0, 64, skip), w->p3.p, 64), st, pdl);
     conv(OUT_BF16_RELU, 64, 128, cargs(B, H3, W3, w->p3.p, 64, wf(E3A), 128, w->e3a.p, 128, 0, 128, skip), st, pdl);
     conv(OUT_BF16_RELU, 128, 128, cargs(B, H3, W3, w->e3a.p, 128, wf(E3B), 128, w->e3.p, 128, 0, 128, skip), st, pdl);
-    launch(pdl, up2_kernel, dim3(ew_grid((long)B * H2 * W2 * 16)), dim3(256), 0, st, B, H2, W2, w->e3.p, 128, 128, w->cat2.p, 192, 64, skip);
-    conv(OUT_BF16_RELU, 192, 64, cargs(B, H2, W2, w->cat2.p, 192, wf(D2A), 64, w->d2a.p, 64, 0, 64, skip), st, pdl);
+    if (!fuse) launch(pdl, up2_kernel, dim3(ew_grid((long)B * H2 * W2 * 16)), dim3(256), 0, st, B, H2, W2, w->e3.p, 128, 128, w->cat2.p, 192, 64, skip);
+    conv(OUT_BF16_RELU, 192, 64, dec(cargs(B, H2, W2, w->cat2.p, 192, wf(D2A), 64, w->d2a.p, 64, 0, 64, skip), w->e3.p, 128, 64), st, pdl);
     conv(OUT_BF16_RELU, 64, 64, cargs(B, H2, W2, w->d2a.p, 64, wf(D2B), 64, w->d2.p, 64, 0, 64, skip), st, pdl);
-    launch(pdl, up2_kernel, dim3(ew_grid((long)B * H1 * W1 * 8)), dim3(256), 0, st, B, H1, W1, w->d2.p, 64, 64, w->cat1.p, 96, 32, skip);
-    conv(OUT_BF16_RELU, 96, 32, cargs(B, H1, W1, w->cat1.p, 96, wf(D1A), 32, w->d1a.p, 32, 0, 32, skip), st, pdl);
+    if (!fuse) launch(pdl, up2_kernel, dim3(ew_grid((long)B * H1 * W1 * 8)), dim3(256), 0, st, B, H1, W1, w->d2.p, 64, 64, w->cat1.p, 96, 32, skip);
+    conv(OUT_BF16_RELU, 96, 32, dec(cargs(B, H1, W1, w->cat1.p, 96, wf(D1A), 32, w->d1a.p, 32, 0, 32, skip), w->d2.p, 64, 32), st, pdl);
     conv(OUT_BF16_RELU, 32, 32, cargs(B, H1, W1, w->d1a.p, 32, wf(D1B), 32, w->d1.p, 32, 0, 32, skip), st, pdl);
-    launch(pdl, up2_kernel, dim3(ew_grid((long)B * H0 * W0 * 4)), dim3(256), 0, st, B, H0, W0, w->d1.p, 32, 32, w->cat0.p, 48, 16, skip);
-    conv(OUT_BF16_RELU, 48, 16, cargs(B, H0, W0, w->cat0.p, 48, wf(D0A), 16, w->d0a.p, 16, 0, 16, skip), st, pdl);
+    if (!fuse) launch(pdl, up2_kernel, dim3(ew_grid((long)B * H0 * W0 * 4)), dim3(256), 0, st, B, H0, W0, w->d1.p, 32, 32, w->cat0.p, 48, 16, skip);
+    conv(OUT_BF16_RELU, 48, 16, dec(cargs(B, H0, W0, w->cat0.p, 48, wf(D0A), 16, w->d0a.p, 16, 0, 16, skip), w->d1.p, 32, 16), st, pdl);
     conv(OUT_BF16_RELU, 16, 16, cargs(B, H0, W0, w->d0a.p, 16, wf(D0B), 16, w->d0.p, 16, 0, 16, skip), st, pdl);
     conv(OUT_F32, 16, 16, cargs(B, H0, W0, w->d0.p, 16, wf(OUTL), 16, w->out.p, 4, 0, 3, skip), st, pdl);
     LCK(cudaGetLastError());
@@ -1064,6 +1090,7 @@ __global__ void fp_init_kernel(FArgs a) {
 // U: x += alpha p, r -= alpha q with alpha = p.r / p.Kp of the last
 // direction (0 at the first iteration).
 __global__ void fp_update_kernel(FArgs a) {
+    pgn::pdl_trigger();
     pgn::pdl_wait();
     FState* st = a.st;
     const int it = st->it;
@@ -1120,6 +1147,7 @@ __global__ void fp_update_kernel(FArgs a) {
 // and |F - K x|^2 for the stop test.
 template <int NPE>
 __global__ void fp_true_res_kernel(FArgs a) {
+    pgn::pdl_trigger();
     pgn::pdl_wait();
     constexpr int ND = 3 * NPE;
     FState* st = a.st;
@@ -1172,6 +1200,7 @@ __global__ void fp_true_res_kernel(FArgs a) {
 // and the network input image (s_in r1).
 template <int NPE>
 __global__ void fp_prep_kernel(FArgs a) {
+    pgn::pdl_trigger();
     pgn::pdl_wait();
     FState* st = a.st;
     if (st->done) return;
@@ -1245,6 +1274,7 @@ __device__ __forceinline__ void write_sweep(const FArgs& a, int n, const float (
 // (when the correction gets smoothing sweeps): the first sweep's w.
 template <int NPE>
 __global__ void fp_net_kernel(FArgs a, float* __restrict__ w_next) {
+    pgn::pdl_trigger();
     pgn::pdl_wait();
     FState* st = a.st;
     if (st->done || st->skip_net) return;
@@ -1277,6 +1307,7 @@ __global__ void fp_net_kernel(FArgs a, float* __restrict__ w_next) {
 template <int NPE>
 __global__ void fp_sweep_kernel(FArgs a, const float* __restrict__ w_in, float* __restrict__ v_out,
                                 float* __restrict__ w_next) {
+    pgn::pdl_trigger();
     pgn::pdl_wait();
     FState* st = a.st;
     if (st->done || st->skip_net) return;
@@ -1308,6 +1339,7 @@ __global__ void fp_sweep_kernel(FArgs a, const float* __restrict__ w_in, float* 
 // Mode 2 (the smoothing steps without the network): z = t + omega D^-1 r1.
 // Mode 0: z = D^-1 r.
 __global__ void fp_prec_kernel(FArgs a) {
+    pgn::pdl_trigger();
     pgn::pdl_wait();
     FState* st = a.st;
     if (st->done) return;
@@ -1359,6 +1391,7 @@ __global__ void fp_prec_kernel(FArgs a) {
 // D: beta (Polak-Ribiere), p = z + beta p_old, q = K p.
 template <int NPE>
 __global__ void fp_dir_kernel(FArgs a) {
+    pgn::pdl_trigger();
     pgn::pdl_wait();
     FState* st = a.st;
     if (st->done) return;
@@ -1406,6 +1439,7 @@ __global__ void apply_op_kernel(Op op, const float* __restrict__ x, float* __res
 }
 
 __global__ void fp_tick_kernel(FArgs a, cudaGraphConditionalHandle h, int in_graph) {
+    pgn::pdl_trigger();
     pgn::pdl_wait();
     FState* st = a.st;
     st->gamma_prev = st->gamma_next;

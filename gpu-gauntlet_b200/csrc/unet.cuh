@@ -32,8 +32,13 @@ using bf162 = __nv_bfloat162;
 // Programmatic dependent launch: a kernel launched with programmatic stream
 // serialisation may start before its predecessor in the stream has
 // finished; it waits here, before reading anything the predecessor wrote
-// (a no-op for an ordinary launch).
+// (a no-op for an ordinary launch).  pdl_trigger lets the next kernel's blocks
+// start once every block of this one has called it: they then load what no
+// kernel writes (a convolution its weights) and wait, so the launch and those
+// loads are off the chain of kernels.  Every kernel of a chain calls
+// pdl_wait in every block, so a grid ends only after the one before it.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
@@ -83,6 +88,9 @@ struct ConvArgs {
     int B, H, W;
     const bf16* in;  // [B][H][W][in_cs], channels [0, CIN)
     int in_cs;
+    const bf16* up;  // non-NULL: channels [up_from, CIN) are the nearest 2x upsampling of
+    int up_cs;       //   [B][H/2][W/2][up_cs] (channel up_from + c from its channel c)
+    int up_from;
     const bf16* w;   // [9][w_rows][CIN]; this block uses rows co0 .. co0+COT-1
     int w_rows;
     void* out;       // channel co stored at [..][out_coff + co] when co < cout_real
@@ -102,17 +110,16 @@ __host__ __device__ constexpr int conv_smem_bytes(int cin, int cot) {
 
 // 3 x 3 convolution, zero padding, no bias.  A block computes an 8 x 8
 // pixel tile (four warps, each a 2-row x 8-column m16 tile) for COT output
-// channels.  The 10 x 10 input halo (CIN channels) and all nine taps'
-// COT x CIN weights are staged in shared memory by one cp.async group, so
-// the block pays one L2 round trip before its MMAs (streaming the taps one
-// by one left each small layer waiting nine times); COT is chosen so the
-// weights fit (conv_smem_bytes).
+// channels.  All nine taps' COT x CIN weights are staged in shared memory
+// before the block waits for the kernel before it, the 10 x 10 input halo (CIN
+// channels) behind that wait, so the block pays one L2 round trip before its
+// MMAs (streaming the taps one by one left each small layer waiting nine
+// times); COT is chosen so the weights fit (conv_smem_bytes).
 // Grid: (ceil(W/8), ceil(H/8) * B, w_rows / COT).
 template <int CIN, int COT, int MODE>
 __global__ void __launch_bounds__(kConvThreads) conv3x3_kernel(ConvArgs a) {
     static_assert(CIN % 16 == 0 && COT % 16 == 0, "channels in multiples of 16");
-    pdl_wait();
-    if (a.skip && *a.skip) return;
+    pdl_trigger();
     constexpr int SP = CIN + 8;  // padded pixel / weight-row stride in shared memory
     constexpr int C8 = CIN / 8;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -123,17 +130,27 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_kernel(ConvArgs a) {
     const int b = blockIdx.y / tiles_y;
     const int ty0 = (blockIdx.y - b * tiles_y) * 8, tx0 = blockIdx.x * 8;
     const int co0 = blockIdx.z * COT;
-    for (int q = tid; q < 100 * C8; q += kConvThreads) {
-        const int pix = q / C8, c8 = q - pix * C8;
-        const int gy = ty0 - 1 + pix / 10, gx = tx0 - 1 + pix % 10;
-        const bool ok = gy >= 0 && gy < a.H && gx >= 0 && gx < a.W;
-        const bf16* src = ok ? a.in + (((size_t)b * a.H + gy) * a.W + gx) * a.in_cs + c8 * 8 : a.in;
-        cp_async16(sIn + pix * SP + c8 * 8, src, ok);
-    }
     for (int q = tid; q < 9 * COT * C8; q += kConvThreads) {
         const int row = q / C8, c8 = q - row * C8;  // row = tap * COT + co
         const int tap = row / COT, co = row - tap * COT;
         cp_async16(sW + row * SP + c8 * 8, a.w + ((size_t)tap * a.w_rows + co0 + co) * CIN + c8 * 8, true);
+    }
+    pdl_wait();
+    if (a.skip && *a.skip) {
+        cp_async_wait<0>();
+        return;
+    }
+    for (int q = tid; q < 100 * C8; q += kConvThreads) {
+        const int pix = q / C8, c8 = q - pix * C8;
+        const int gy = ty0 - 1 + pix / 10, gx = tx0 - 1 + pix % 10;
+        const bool ok = gy >= 0 && gy < a.H && gx >= 0 && gx < a.W;
+        const bf16* src = a.in;
+        if (ok) {
+            src = a.in + (((size_t)b * a.H + gy) * a.W + gx) * a.in_cs + c8 * 8;
+            if (a.up && c8 * 8 >= a.up_from)
+                src = a.up + (((size_t)b * (a.H >> 1) + (gy >> 1)) * (a.W >> 1) + (gx >> 1)) * a.up_cs + c8 * 8 - a.up_from;
+        }
+        cp_async16(sIn + pix * SP + c8 * 8, src, ok);
     }
     cp_async_commit();
     float acc[COT / 8][4];
@@ -314,6 +331,7 @@ __global__ void __launch_bounds__((COT / 16) * (CIT / 16) * 32) wgrad_kernel(Wgr
 // out[b][y][x][coff + c] = in[b][y/2][x/2][c], c < C.
 __global__ void up2_kernel(int B, int H, int W, const bf16* __restrict__ in, int in_cs, int C,
                            bf16* __restrict__ out, int out_cs, int coff, const int* skip) {
+    pdl_trigger();
     pdl_wait();
     if (skip && *skip) return;
     const int C8 = C / 8;
