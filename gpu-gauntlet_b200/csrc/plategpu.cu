@@ -75,29 +75,65 @@ struct DevBuf {
     ~DevBuf() { release(); }
 };
 
+// Pinned host memory that grows.
+struct Pinned {
+    unsigned char* p = nullptr;
+    size_t n = 0;
+    unsigned char* get(size_t bytes) {
+        if (bytes > n) {
+            if (p) cudaFreeHost(p);
+            p = nullptr;
+            n = 0;
+            CK(cudaMallocHost(&p, bytes));
+            n = bytes;
+        }
+        return p;
+    }
+    ~Pinned() {
+        if (p) cudaFreeHost(p);
+    }
+};
+
 // Typed arrays carved out of one device allocation, each 256-byte aligned:
 // one cudaMalloc instead of one per array (each a driver call that maps
 // pages, which the first solve of a new mesh pays many times over).  add()
 // records an array (with the host data to copy into it, or none);
 // commit() allocates `store`, points the arrays into it and queues the
-// copies on `st`.
+// copies on `st`.  With `stage` the arrays with host data sit first and go up
+// in one copy from pinned memory, which the caller leaves alone until the
+// stream has run it (instead of a pageable copy each).
 struct Arena {
-    size_t total = 0;
-    std::vector<std::function<void(unsigned char*, cudaStream_t)>> bind;
+    struct Item {
+        std::function<void(unsigned char*)> bind;
+        const void* host;
+        size_t bytes, off;
+    };
+    std::vector<Item> items;
     template <typename B>
     void add(B& buf, size_t count, const void* host) {
         using T = typename B::value_type;
-        const size_t off = total;
-        total += (count * sizeof(T) + 255) & ~size_t(255);
         B* b = &buf;
-        bind.push_back([b, off, count, host](unsigned char* base, cudaStream_t st) {
-            b->view(reinterpret_cast<T*>(base + off), count);
-            if (host && count) CK(cudaMemcpyAsync(b->p, host, count * sizeof(T), cudaMemcpyHostToDevice, st));
-        });
+        items.push_back({[b, count](unsigned char* at) { b->view(reinterpret_cast<T*>(at), count); },
+                         count ? host : nullptr, count * sizeof(T), 0});
     }
-    void commit(DevBuf<unsigned char>& store, cudaStream_t st) {
+    void commit(DevBuf<unsigned char>& store, cudaStream_t st, Pinned* stage = nullptr) {
+        size_t total = 0, up = 0;
+        for (int pass = 0; pass < 2; pass++)
+            for (Item& i : items)
+                if ((i.host != nullptr) == (pass == 0)) {
+                    i.off = total;
+                    if (pass == 0) up = total + i.bytes;
+                    total += (i.bytes + 255) & ~size_t(255);
+                }
         store.alloc(total);
-        for (auto& f : bind) f(store.p, st);
+        unsigned char* s = stage && up ? stage->get(up) : nullptr;
+        for (Item& i : items) {
+            i.bind(store.p + i.off);
+            if (!i.host) continue;
+            if (s) std::memcpy(s + i.off, i.host, i.bytes);
+            else CK(cudaMemcpyAsync(store.p + i.off, i.host, i.bytes, cudaMemcpyHostToDevice, st));
+        }
+        if (s) CK(cudaMemcpyAsync(store.p, s, up, cudaMemcpyHostToDevice, st));
     }
 };
 
@@ -157,6 +193,7 @@ struct Plan {
     // FP64 correction after a stagnated mixed solve: the mixed x, K x and
     // the FP32 residual
     DevBuf<double> xw, kx, nrm, pw;
+    DevBuf<double4> em;  // element moments
     DevBuf<float> rf;
     // global-memory flexible PCG of a plate too large for the persistent
     // kernel's shared memory (created on first use)
@@ -222,6 +259,7 @@ struct pg_ctx {
     float* hF = nullptr;                     // pinned staging
     double* hx = nullptr;
     size_t hcap = 0;
+    Pinned stage;                            // a plan's host arrays on their way up
 };
 
 namespace {
@@ -436,8 +474,8 @@ std::unique_ptr<Plan> build_plan(pg_ctx* c, const pg_problem& p, int G, int ring
     carve(pl->abort_flag, 1, nullptr);
     carve(pl->trace, 4 * (size_t)pl->G, nullptr);
     carve(pl->res, 1, nullptr);
-    ar.commit(pl->arena, st);
-    // synchronous: uploads read the host plan arrays
+    ar.commit(pl->arena, st, &c->stage);
+    // synchronous: the upload reads the context's pinned staging
     CK(cudaStreamSynchronize(st));
     return pl;
 }
@@ -465,6 +503,9 @@ bool same_problem(const Plan& pl, const pg_problem& p) {
            (!p.elem_t || same(pl.h_elem_t.data(), p.elem_t, Ne * sizeof(float)));
 }
 
+// The cached plan of problem p (its header checked), or a new one.  A problem
+// equal to a plan's byte by byte was validated when the plan was made; one
+// that is not is validated here.
 Plan* get_plan(pg_ctx* c, const pg_problem& p, int G, int rings, bool* cached) {
     for (auto it = c->plans.begin(); it != c->plans.end(); ++it) {
         if ((*it)->G == G && (*it)->hp.rings == rings && same_problem(**it, p)) {
@@ -474,13 +515,15 @@ Plan* get_plan(pg_ctx* c, const pg_problem& p, int G, int rings, bool* cached) {
         }
     }
     *cached = false;
+    std::string e = pg::validate_problem(p, false);
+    if (!e.empty()) throw Fail{PG_EINVAL, e};
     auto pl = build_plan(c, p, G, rings);
     c->plans.push_front(std::move(pl));
     while (c->plans.size() > kMaxPlans) c->plans.pop_back();
     return c->plans.front().get();
 }
 
-// Element matrices, block-Jacobi inverses and task blocks: pure functions
+// Element matrices, block-Jacobi inverses and row blocks: pure functions
 // of the plan's own copies of the mesh, material and constraints, so they
 // are computed once per plan (queued on the context stream; pg_set_stream
 // drains the old stream before switching).
@@ -1336,6 +1379,13 @@ void check_problem(const pg_problem* p, bool need_rhs) {
     if (!e.empty()) throw Fail{PG_EINVAL, e};
 }
 
+// What get_plan does not check: counts, material and pointers.
+void check_header(const pg_problem* p, bool need_rhs) {
+    if (!p) throw Fail{PG_EINVAL, "problem is NULL"};
+    std::string e = pg::validate_header(*p, need_rhs);
+    if (!e.empty()) throw Fail{PG_EINVAL, e};
+}
+
 void zero_info(pg_info* info) {
     if (!info) return;
     std::memset(info, 0, sizeof(*info));
@@ -1390,8 +1440,7 @@ std::unique_ptr<pg_batch> build_batch(pg_ctx* c, const pg_problem* probs, int co
         check_problem(&probs[i], true);
         if (probs[i].node_count == 0) throw Fail{PG_EINVAL, "a plate of the batch has no nodes"};
         const size_t n = 3 * (size_t)probs[i].node_count;
-        for (size_t k = 0; k < n; k++)
-            if (!std::isfinite(probs[i].F[k])) throw Fail{PG_ENONFINITE, "F contains NaN or Inf"};
+        if (!pg::finite_f(probs[i].F, n)) throw Fail{PG_ENONFINITE, "F contains NaN or Inf"};
         nodes[i] = (int)probs[i].node_count;
     }
     // schedule, then check every plate's layout at its team size; lower the
@@ -1501,8 +1550,7 @@ void run_batch(pg_batch* b, const pg_options& o, const float* const* F, double* 
         for (int i = 0; i < count; i++) {
             if (!F[i]) continue;
             const size_t n = 3 * (size_t)b->plans[i]->hp.Nn;
-            for (size_t k = 0; k < n; k++)
-                if (!std::isfinite(F[i][k])) throw Fail{PG_ENONFINITE, "F contains NaN or Inf"};
+            if (!pg::finite_f(F[i], n)) throw Fail{PG_ENONFINITE, "F contains NaN or Inf"};
             b->hF[i].assign(F[i], F[i] + n);
             CK(cudaMemcpyAsync(b->plans[i]->F.p, b->hF[i].data(), n * sizeof(float), cudaMemcpyHostToDevice,
                                st));
@@ -1743,8 +1791,8 @@ void run_batch(pg_batch* b, const pg_options& o, const float* const* F, double* 
 void run_moments(pg_ctx* c, Plan* pl, const double* x_dev, double* M_dev) {
     const pg::HostPlan& hp = pl->hp;
     if (hp.Ne == 0 || hp.Nn == 0) return;
-    DevBuf<double4> em;
-    em.alloc(hp.Ne);
+    DevBuf<double4>& em = pl->em;  // kept: an allocation costs more than the kernels
+    if (em.n != (size_t)hp.Ne) em.alloc(hp.Ne);
     const double D = (pl->E * std::pow(pl->t, 3.0)) / (12.0 * (1.0 - std::pow(pl->nu, 2.0)));
     if (hp.npe == 4)
         pg::elem_moments_kernel<4><<<(hp.Ne + 127) / 128, 128, 0, c->stream>>>(
@@ -1756,7 +1804,6 @@ void run_moments(pg_ctx* c, Plan* pl, const double* x_dev, double* M_dev) {
     pg::node_moments_kernel<<<(hp.Nn + 127) / 128, 128, 0, c->stream>>>(hp.Nn, pl->inc_ptr.p, pl->inc_idx.p,
                                                                        em.p, M_dev);
     CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(c->stream));  // em is released on return
 }
 
 }  // namespace
@@ -1890,18 +1937,18 @@ int pg_set_stream(pg_ctx* c, void* stream) {
 int pg_solve(pg_ctx* c, const pg_problem* p, const pg_options* opt, double* x_out, pg_info* info) {
     zero_info(info);
     return guarded(c, info, [&] {
-        check_problem(p, true);
+        check_header(p, true);
         pg_options o;
         fill_options(opt, &o);
         const size_t n = 3 * (size_t)p->node_count;
         if (n && !x_out) throw Fail{PG_EINVAL, "x_out is NULL"};
-        for (size_t i = 0; i < n; i++)
-            if (!std::isfinite(p->F[i])) throw Fail{PG_ENONFINITE, "F contains NaN or Inf"};
         if (n == 0) {
+            check_problem(p, true);
             if (info) { info->converged = 1; info->stop_reason = PG_STOP_ZERO_RHS; }
             return;
         }
         const int G = o.ctas ? std::min(o.ctas, (int)p->node_count) : auto_ctas(c, (int)p->node_count);
+        if (!pg::finite_f(p->F, n)) throw Fail{PG_ENONFINITE, "F contains NaN or Inf"};
         bool cached = false;
         const auto tp = std::chrono::steady_clock::now();
         Plan* pl = get_plan(c, *p, G, halo_rings(o), &cached);
@@ -1923,7 +1970,7 @@ int pg_solve_load_cases(pg_ctx* c, const pg_problem* p, int count, const float* 
                         int cases_per_launch, double* x_out, pg_info* infos) {
     if (infos && count > 0) std::memset(infos, 0, (size_t)count * sizeof(pg_info));
     return guarded(c, nullptr, [&] {
-        check_problem(p, false);
+        check_header(p, false);
         if (count < 1 || !F) throw Fail{PG_EINVAL, "need count >= 1 load cases and F"};
         if (cases_per_launch != 0 && cases_per_launch != 1 && cases_per_launch != 2 && cases_per_launch != 4)
             throw Fail{PG_EINVAL, "cases_per_launch must be 0 (automatic), 1, 2 or 4"};
@@ -1931,9 +1978,9 @@ int pg_solve_load_cases(pg_ctx* c, const pg_problem* p, int count, const float* 
         fill_options(opt, &o);
         const size_t n = 3 * (size_t)p->node_count;
         if (n && !x_out) throw Fail{PG_EINVAL, "x_out is NULL"};
-        for (size_t i = 0; i < n * count; i++)
-            if (!std::isfinite(F[i])) throw Fail{PG_ENONFINITE, "F contains NaN or Inf"};
+        if (!pg::finite_f(F, n * count)) throw Fail{PG_ENONFINITE, "F contains NaN or Inf"};
         if (n == 0) {
+            check_problem(p, false);
             if (infos)
                 for (int k = 0; k < count; k++) { infos[k].converged = 1; infos[k].stop_reason = PG_STOP_ZERO_RHS; }
             return;
@@ -2282,21 +2329,26 @@ int pg_partition_nodes(const float* nodes, uint32_t node_count, int ctas, int32_
 int pg_moments(pg_ctx* c, const pg_problem* p, const double* x, double* Mx, double* My,
                           double* Mxy) {
     return guarded(c, nullptr, [&] {
-        check_problem(p, false);
+        check_header(p, false);
         const size_t Nn = p->node_count;
-        if (Nn == 0) return;
+        if (Nn == 0) return check_problem(p, false);
         if (!x || !Mx || !My || !Mxy) throw Fail{PG_EINVAL, "x / Mx / My / Mxy is NULL"};
         bool cached = false;
         Plan* pl = get_plan(c, *p, auto_ctas(c, (int)Nn), 1, &cached);
-        DevBuf<double> dx, dm;
-        dx.upload(x, 3 * Nn, c->stream);
-        dm.alloc(3 * Nn);
-        run_moments(c, pl, dx.p, dm.p);
-        std::vector<double> h(3 * Nn);
-        CK(cudaMemcpy(h.data(), dm.p, h.size() * sizeof(double), cudaMemcpyDeviceToHost));
-        std::memcpy(Mx, h.data(), Nn * sizeof(double));
-        std::memcpy(My, h.data() + Nn, Nn * sizeof(double));
-        std::memcpy(Mxy, h.data() + 2 * Nn, Nn * sizeof(double));
+        // x and the moments through pinned staging and the plan's own vectors
+        const size_t n = 3 * Nn;
+        if (pl->xw.n != n) pl->xw.alloc(n);
+        if (pl->kx.n != n) pl->kx.alloc(n);
+        ensure_staging(c, n);
+        std::memcpy(c->hx, x, n * sizeof(double));
+        CK(cudaMemcpyAsync(pl->xw.p, c->hx, n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+        if (p->element_count == 0) CK(cudaMemsetAsync(pl->kx.p, 0, n * sizeof(double), c->stream));
+        run_moments(c, pl, pl->xw.p, pl->kx.p);
+        CK(cudaMemcpyAsync(c->hx, pl->kx.p, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaStreamSynchronize(c->stream));
+        std::memcpy(Mx, c->hx, Nn * sizeof(double));
+        std::memcpy(My, c->hx + Nn, Nn * sizeof(double));
+        std::memcpy(Mxy, c->hx + 2 * Nn, Nn * sizeof(double));
     });
 }
 
@@ -2305,6 +2357,7 @@ int pg_plan_moments_device(pg_plan* h, const double* x_dev, double* M_dev) {
     return guarded(h->ctx, nullptr, [&] {
         if (!x_dev || !M_dev) throw Fail{PG_EINVAL, "x_dev / M_dev is NULL"};
         run_moments(h->ctx, h->plan.get(), x_dev, M_dev);
+        CK(cudaStreamSynchronize(h->ctx->stream));
     });
 }
 

@@ -309,27 +309,32 @@ def _ptr(a):
 
 
 class Problem:
-    """Owns contiguous copies of the arrays a PgProblem points at."""
+    """Owns contiguous copies of the arrays a PgProblem points at; copy=False
+    keeps arrays that are contiguous and of the right type as they are (for a
+    call that is over before its caller can change them)."""
 
-    def __init__(self, mesh, material, coloring, F=None, constrained=None):
-        self.nodes = np.array(mesh.nodes, np.float32, order="C")
-        self.elements = np.array(mesh.elements, np.uint32, order="C")
+    def __init__(self, mesh, material, coloring, F=None, constrained=None, copy=True):
+        def own(a, dtype):
+            return np.array(a, dtype, order="C") if copy else np.ascontiguousarray(a, dtype)
+
+        self.nodes = own(mesh.nodes, np.float32)
+        self.elements = own(mesh.elements, np.uint32)
         if coloring is not None:
-            offs, flat = coloring.flat()
-            self.color_offsets = np.array(offs, np.uint32, order="C")
-            self.elements_by_color = np.array(flat, np.uint32, order="C")
+            offs, flat = coloring.flat()  # arrays of this call
+            self.color_offsets = np.ascontiguousarray(offs, np.uint32)
+            self.elements_by_color = np.ascontiguousarray(flat, np.uint32)
             ncol = int(coloring.colorCount)
         else:
             self.color_offsets = self.elements_by_color = None
             ncol = 0
         self.elem_t = (None if getattr(material, "elem_t", None) is None
-                       else np.array(material.elem_t, np.float32, order="C"))
+                       else own(material.elem_t, np.float32))
         n = 3 * int(mesh.nodeCount)
-        self.F = np.zeros(n, np.float32) if F is None else np.array(F, np.float32, order="C")
+        self.F = np.zeros(n, np.float32) if F is None else own(F, np.float32)
         if self.F.size != n:
             raise ValueError(f"F has {self.F.size} entries, expected {n}")
         self.cons = (np.zeros(n, np.uint8) if constrained is None
-                     else np.array(constrained, np.uint8, order="C"))
+                     else own(constrained, np.uint8))
         if self.cons.size != n:
             raise ValueError(f"constrained mask has {self.cons.size} entries, expected {n}")
         s = PgProblem()
@@ -425,7 +430,7 @@ class Context:
             raise PlateGPUError(st, self.L.pg_last_error(self.h).decode())
 
     def solve(self, prob: Problem, opts: PgOptions):
-        x = np.zeros(prob.F.size, np.float64)
+        x = np.empty(prob.F.size, np.float64)
         info = PgInfo()
         st = self.L.pg_solve(self.h, C.byref(prob.struct), C.byref(opts), _ptr(x), C.byref(info))
         self._check(st)
@@ -438,7 +443,7 @@ class Context:
         if F.ndim != 2:
             raise ValueError("F must be [cases][3 * node_count]")
         k = F.shape[0]
-        x = np.zeros(F.shape, np.float64)
+        x = np.empty(F.shape, np.float64)
         infos = (PgInfo * k)()
         st = self.L.pg_solve_load_cases(self.h, C.byref(prob.struct), k, _ptr(F), C.byref(opts),
                                         int(cases_per_launch), _ptr(x), infos)
@@ -467,7 +472,7 @@ class Context:
         """pg_moments: nodal (Mx, My, Mxy) of displacements x (FP64)."""
         x = np.ascontiguousarray(x, np.float64)
         n = int(prob.struct.node_count)
-        out = [np.zeros(n, np.float64) for _ in range(3)]
+        out = [np.empty(n, np.float64) for _ in range(3)]
         self._check(self.L.pg_moments(self.h, C.byref(prob.struct), _ptr(x), *[_ptr(o) for o in out]))
         return tuple(out)
 

@@ -36,7 +36,13 @@ def constrained_mask(n_dof: int, constrainedDOFs) -> np.ndarray:
     """Set of DOF indices -> uint8 mask (the constrainedMask buffer of
     gpu/buffers.ts:262-266, one byte per DOF)."""
     m = np.zeros(n_dof, np.uint8)
-    idx = np.fromiter((int(d) for d in constrainedDOFs), dtype=np.int64)
+    if isinstance(constrainedDOFs, (set, frozenset, list, tuple)):
+        try:
+            idx = np.fromiter(constrainedDOFs, np.int64, len(constrainedDOFs))
+        except (TypeError, ValueError):  # numbers of another kind, one by one
+            idx = np.fromiter((int(d) for d in constrainedDOFs), dtype=np.int64)
+    else:
+        idx = np.fromiter((int(d) for d in constrainedDOFs), dtype=np.int64)
     if idx.size:
         if idx.min() < 0 or idx.max() >= n_dof:
             raise ValueError("constrained DOF index out of range")
