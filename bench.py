@@ -1035,7 +1035,7 @@ def batch_bench(args, ctx, check, world=1, rank=0, local=0):
     from plategpu import autotune
     part_nodes, tune = autotune.tune_batch(
         ctx, probs, batch_options("fp64_two_level"), torch.cuda.get_device_name(local),
-        candidates=(250, 400, 640), cache_path=os.path.join(tempfile.gettempdir(), "plategpu_autotune.json"))
+        candidates=(100, 160, 200, 400), cache_path=os.path.join(tempfile.gettempdir(), "plategpu_autotune.json"))
     for name in methods:
         opts = batch_options(name, part_nodes)
         steps = 1 if name == "fp64_block_jacobi" else max(1, args.batch_steps)

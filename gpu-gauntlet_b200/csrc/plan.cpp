@@ -473,13 +473,13 @@ std::string build_coarse_meta(const pg_problem& p, HostPlan& plan) {
     return "";
 }
 
-std::string schedule_batch(const std::vector<int>& nodes, const std::vector<int>& caps,
-                           const std::vector<int>& kinds, int sms, BatchSchedule& out, int part_nodes) {
+std::string schedule_batch(const std::vector<int>& nodes, const std::vector<int>& caps, int sms, BatchSchedule& out,
+                           int part_nodes) {
     const double target = part_nodes > 0 ? part_nodes : 400.0;
     out = BatchSchedule{};
     const int count = (int)nodes.size();
     if (count == 0) return "empty batch";
-    if (sms < 1 || (int)caps.size() != count || (int)kinds.size() != count) return "no blocks to schedule";
+    if (sms < 1 || (int)caps.size() != count) return "no blocks to schedule";
     int top = 1;  // largest power of two <= sms
     while (top * 2 <= sms) top *= 2;
     std::vector<int> d(count);
@@ -503,16 +503,11 @@ std::string schedule_batch(const std::vector<int>& nodes, const std::vector<int>
     std::vector<int> order(count);
     std::iota(order.begin(), order.end(), 0);
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return w[a] > w[b]; });
-    std::vector<int> ks;
-    for (int i = 0; i < count; i++)
-        if (std::find(ks.begin(), ks.end(), kinds[i]) == ks.end()) ks.push_back(kinds[i]);
-    std::sort(ks.rbegin(), ks.rend());
-    for (int kind : ks) {
-    // team sizes of this kind, largest first, first-fit into phases (one team
-    // of each size fits)
+    // team sizes, largest first, first-fit into phases (one team of each size
+    // fits)
     std::vector<int> cs;
     for (int i = 0; i < count; i++)
-        if (kinds[i] == kind && std::find(cs.begin(), cs.end(), d[i]) == cs.end()) cs.push_back(d[i]);
+        if (std::find(cs.begin(), cs.end(), d[i]) == cs.end()) cs.push_back(d[i]);
     std::sort(cs.rbegin(), cs.rend());
     std::vector<std::vector<int>> phase_sizes;
     std::vector<int> phase_sum;
@@ -533,7 +528,7 @@ std::string schedule_batch(const std::vector<int>& nodes, const std::vector<int>
         std::vector<int> teams(nc, 1), nplates(nc, 0);
         for (int i = 0; i < count; i++) {
             const auto it = std::find(pc.begin(), pc.end(), d[i]);
-            if (kinds[i] != kind || it == pc.end()) continue;
+            if (it == pc.end()) continue;
             W[it - pc.begin()] += w[i];
             nplates[it - pc.begin()]++;
         }
@@ -551,7 +546,6 @@ std::string schedule_batch(const std::vector<int>& nodes, const std::vector<int>
             used += pc[best];
         }
         BatchPhase P;
-        P.kind = kind;
         for (int k = 0; k < nc; k++)
             for (int t = 0; t < teams[k]; t++) {
                 P.team_base.push_back(P.grid);
@@ -562,7 +556,7 @@ std::string schedule_batch(const std::vector<int>& nodes, const std::vector<int>
         P.team_load.assign(T, 0.0);
         std::vector<std::vector<int>> q(T);
         for (int i : order) {
-            if (kinds[i] != kind || std::find(pc.begin(), pc.end(), d[i]) == pc.end()) continue;
+            if (std::find(pc.begin(), pc.end(), d[i]) == pc.end()) continue;
             int bt = -1;
             for (int t = 0; t < T; t++)
                 if (P.team_size[t] == d[i] && (bt < 0 || P.team_load[t] < P.team_load[bt])) bt = t;
@@ -579,7 +573,6 @@ std::string schedule_batch(const std::vector<int>& nodes, const std::vector<int>
         // the dynamic queues: one per class (team size), largest work first
         std::vector<std::vector<int>> cq(nc);
         for (int i : order) {
-            if (kinds[i] != kind) continue;
             const auto it = std::find(pc.begin(), pc.end(), d[i]);
             if (it != pc.end()) cq[it - pc.begin()].push_back(i);
         }
@@ -595,7 +588,6 @@ std::string schedule_batch(const std::vector<int>& nodes, const std::vector<int>
             P.log_off[t + 1] = P.log_off[t] + (int)cq[k].size();
         }
         out.phases.push_back(std::move(P));
-    }
     }
     return "";
 }

@@ -104,8 +104,7 @@ std::string build_coarse_meta(const pg_problem& p, HostPlan& plan);
 // among the team sizes in proportion to their estimated work (sqrt(n)
 // iterations of n + 300 d node-equivalents), one team per size at least,
 // and each size's plates go to its teams longest first to the least-loaded
-// team.  Plates of different kinds (element types: the launch's kernel is
-// specialised for one) never share a phase.
+// team.
 // Teams of one size form a class; a class's plates sit in one queue,
 // largest estimated work first, and each team takes the next plate of its
 // class's queue when it is free (a device-side counter per class), so the
@@ -113,7 +112,6 @@ std::string build_coarse_meta(const pg_problem& p, HostPlan& plan);
 // static assignment those estimates predict (each plate to the least
 // loaded team of its size), for reporting.
 struct BatchPhase {
-    int kind = 4;                         // nodes per element of all its plates
     int grid = 0;                         // blocks of the launch
     std::vector<int> team_base, team_size;
     std::vector<int> team_class;          // [teams] class of each team
@@ -126,7 +124,7 @@ struct BatchSchedule {
     std::vector<BatchPhase> phases;
     std::vector<int> plate_phase, plate_team, plate_size;  // [count]; team index within its phase
 };
-std::string schedule_batch(const std::vector<int>& nodes, const std::vector<int>& caps,
-                           const std::vector<int>& kinds, int sms, BatchSchedule& out, int part_nodes = 400);
+std::string schedule_batch(const std::vector<int>& nodes, const std::vector<int>& caps, int sms, BatchSchedule& out,
+                           int part_nodes = 400);
 
 }  // namespace pg

@@ -214,7 +214,7 @@ struct pg_plan {
 // size of the team of blocks that solves it, and the team schedule (one
 // launch per phase).
 struct BatchPhaseDev {
-    int grid = 0, kind = 4;
+    int grid = 0;
     DevBuf<int> block_team, team_base, team_class, class_off, class_queue, log_off;
     DevBuf<int> class_next;               // zeroed before each launch
     DevBuf<unsigned long long> claims;    // zeroed before each launch
@@ -1430,6 +1430,16 @@ bool smoother_halo_fits(const pg_ctx* c, const pg::HostPlan& hp, const pg_option
     return b <= (size_t)c->max_smem;
 }
 
+// Preferred nodes per block of a batch plate's team.  Smaller parts make an
+// iteration shorter (FP64 two-level: 4.5 us at 125 nodes a block, 6.5 at 250, 8.5
+// at 350) and the coarse space finer; larger ones leave more plates in flight,
+// which pays once a batch has many.  ms of whole batches at 100 / 160 / 200 / 400:
+// 12 plates 12.6 / 16.9 / 23.5 / 29.7, 24 plates 19.8 / 20.9 / 22.4 / 30.8, 128
+// plates 130 / 115 / 139 / 194, 256 plates 264 / 260 / 252 / 296.
+int batch_part_nodes(const pg_options& o, int count) {
+    return o.batch_part_nodes > 0 ? o.batch_part_nodes : count <= 32 ? 100 : 160;
+}
+
 std::unique_ptr<pg_batch> build_batch(pg_ctx* c, const pg_problem* probs, int count,
                                       const pg_options& o) {
     auto b = std::make_unique<pg_batch>();
@@ -1445,8 +1455,7 @@ std::unique_ptr<pg_batch> build_batch(pg_ctx* c, const pg_problem* probs, int co
     }
     // schedule, then check every plate's layout at its team size; lower the
     // capacity of the plates whose parts do not fit and reschedule
-    std::vector<int> caps(count), kinds(count), rings(count, b->rings);
-    for (int i = 0; i < count; i++) kinds[i] = (int)probs[i].nodes_per_element;
+    std::vector<int> caps(count), rings(count, b->rings);
     for (int i = 0; i < count; i++) {
         caps[i] = batch_capacity(o, rings[i], (int)probs[i].nodes_per_element);
         // a plate too large for the whole device at the first guess gets the
@@ -1455,7 +1464,7 @@ std::unique_ptr<pg_batch> build_batch(pg_ctx* c, const pg_problem* probs, int co
         caps[i] = std::max(caps[i], (nodes[i] + c->sms - 1) / c->sms);
     }
     for (int attempt = 0;; attempt++) {
-        std::string e = pg::schedule_batch(nodes, caps, kinds, c->sms, b->sched, o.batch_part_nodes);
+        std::string e = pg::schedule_batch(nodes, caps, c->sms, b->sched, batch_part_nodes(o, count));
         if (!e.empty() && attempt > 0)
             throw Fail{PG_EUNSUPPORTED, "a plate of the batch does not fit in shared memory even on the whole "
                                         "device with these options"};
@@ -1500,7 +1509,6 @@ std::unique_ptr<pg_batch> build_batch(pg_ctx* c, const pg_problem* probs, int co
         for (size_t t = 0; t < P.team_size.size(); t++)
             for (int k = 0; k < P.team_size[t]; k++) bt[P.team_base[t] + k] = (int)t;
         d->grid = P.grid;
-        d->kind = P.kind;
         d->block_team.upload(bt.data(), bt.size(), st);
         d->team_base.upload(P.team_base.data(), P.team_base.size(), st);
         d->team_class.upload(P.team_class.data(), P.team_class.size(), st);
@@ -2295,7 +2303,7 @@ int pg_batch_schedule(const uint32_t* node_counts, int count, int sms, int cap, 
     try {
         std::vector<int> nodes(node_counts, node_counts + count);
         pg::BatchSchedule S;
-        if (!pg::schedule_batch(nodes, std::vector<int>(count, cap), std::vector<int>(count, 4), sms, S).empty())
+        if (!pg::schedule_batch(nodes, std::vector<int>(count, cap), sms, S).empty())
             return PG_EUNSUPPORTED;
         for (int i = 0; i < count; i++) {
             plate_phase[i] = S.plate_phase[i];

@@ -18,7 +18,7 @@ import time
 
 from . import _lib
 
-CANDIDATES = (250, 320, 400, 500, 640)
+CANDIDATES = (100, 160, 200, 250, 400)
 
 
 def default_cache_path():

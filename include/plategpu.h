@@ -141,7 +141,7 @@ typedef struct pg_options {
                                      stopped by the same rule on x_m + d; 0 returns the
                                      stagnated result */
     int32_t batch_part_nodes;     /* batches: preferred nodes per block of a plate's team
-                                     (0 = automatic, 400); plategpu.autotune picks it per
+                                     (0 = automatic: 100 for up to 32 plates, else 160); plategpu.autotune picks it per
                                      GPU and batch */
 } pg_options;
 
