@@ -66,7 +66,7 @@ struct SmemLayout {
     int ctl;                        // int[4]: decision broadcast
     int dec;                        // Decision
     int clk;                        // long long[9]: phase timers
-    int nb, ainv;                   // T: per-node basis data, A_c^-1 rows
+    int nb, ainv, ct;               // T: per-node basis data, A_c^-1 rows, a round's P^T w
     int nslot;                      // int
     int gid;                       // int
     int gq, go;                    // int: the row groups' q-step offsets, staged offsets
@@ -753,7 +753,8 @@ constexpr int kResident = 1;
 constexpr int kBatchThreads = 512;
 constexpr int kMultiThreads = 512;  // the load-case kernel (128 registers)
 
-// Per-phase SM cycles of thread 0 of block 0, when timing is requested:
+// Per-phase SM cycles of thread 0 of the middle block (G / 2), when timing is
+// requested:
 // 0 K.u, dots and publishing w, 1 unused (0), 2 block reduction and
 // publishing the partials, 3 the Chebyshev smoother's K t, 4 exchange wait
 // and sum of the partials, 5 the barrier after the decision, 6 warp 0's
@@ -810,36 +811,44 @@ __device__ __forceinline__ void prolong3(const double* cvn, const unsigned char*
     if (!c[2]) u[2] -= (T)((double)bas[2] * cvn[2]);
 }
 
-// out[q] = sum_j Ai[q][j] y_j for the part's coarse rows q < rows, where
-// y_{3b+m} = (T) sp[b * stride + off + m] is the restriction of block b's
-// aggregate staged by the exchange (no contiguous copy needed).  Warps
-// w0.. take two rows each (16 lanes per row, lane l reading the 3 columns
-// of blocks l, l + 16, ...), then a 16-lane shuffle reduction: fixed order,
-// so every block computes the same bits for the same row.
+// out[q] = sum_j Ai[q][j] y_j for the part's coarse rows q < rows; y [C] in
+// shared memory, already in the rows' type (converting it here, once per row,
+// cost FP32 solves more than the product: a conversion issues at an eighth of
+// an FMA's rate).  Warps w0.. take two rows each, a lane columns lane,
+// lane + 32, ..., so one load of y serves both rows; then FP64 sums over the
+// lanes: fixed order, so every block computes the same bits for the same row.
+// Bound by reading the rows from shared memory (96 KB in FP64 on the 60k-DOF
+// plate, 750 cycles).
 template <typename T>
-__device__ __forceinline__ void coarse_apply(const T* __restrict__ Ai, int G, int rows,
-                                             const double* __restrict__ sp, int stride, int off,
+__device__ __forceinline__ void coarse_apply(const T* __restrict__ Ai, int C, int rows, const T* __restrict__ y,
                                              double* __restrict__ out, int w0) {
     const int lane = threadIdx.x & 31, warp = (int)(threadIdx.x >> 5) - w0;
     const int nw = (int)(blockDim.x >> 5) - w0;
     if (warp < 0) return;
-    const int half = lane >> 4, hl = lane & 15, C = 3 * G;
-    for (int q0 = 2 * warp; q0 < rows; q0 += 2 * nw) {
-        const int q = q0 + half;
-        T acc0 = T(0), acc1 = T(0), acc2 = T(0);
-        if (q < rows) {
-            const T* row = Ai + (size_t)q * C;
-            for (int b = hl; b < G; b += 16) {
-                const double* y = sp + b * stride + off;
-                acc0 += row[3 * b] * (T)y[0];
-                acc1 += row[3 * b + 1] * (T)y[1];
-                acc2 += row[3 * b + 2] * (T)y[2];
-            }
+    for (int q = 2 * warp; q < rows; q += 2 * nw) {
+        const T* r0 = Ai + (size_t)q * C;
+        const T* r1 = q + 1 < rows ? r0 + C : r0;
+        T a0 = T(0), a1 = T(0), b0 = T(0), b1 = T(0);
+        int j = lane;
+#pragma unroll 4
+        for (; j + 32 < C; j += 64) {
+            const T y0 = y[j], y1 = y[j + 32];
+            a0 = fma(r0[j], y0, a0);
+            b0 = fma(r1[j], y0, b0);
+            a1 = fma(r0[j + 32], y1, a1);
+            b1 = fma(r1[j + 32], y1, b1);
         }
-        double acc = (double)acc0 + (double)acc1 + (double)acc2;
+        if (j < C) {
+            a0 = fma(r0[j], y[j], a0);
+            b0 = fma(r1[j], y[j], b0);
+        }
+        const double sa = (double)a0 + (double)a1, sb = (double)b0 + (double)b1;
+        // lanes below 16 go on with the first row, the others with the second
+        const bool up = lane >= 16;
+        double v = (up ? sb : sa) + __shfl_xor_sync(0xffffffffu, up ? sa : sb, 16);
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (hl == 0 && q < rows) out[q] = acc;
+        for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if ((lane & 15) == 0 && q + (up ? 1 : 0) < rows) out[q + (up ? 1 : 0)] = v;
     }
 }
 
@@ -925,12 +934,12 @@ __device__ __forceinline__ void sum_publish(const double (&v)[K], double* red, u
 
 // This thread's share (items t, t + stride, ...) of the round's other
 // values: the 3 (nloc - no) ghost DOFs of vector buffer vb into dst, then
-// (KC = 3) partial sums 3..5 of every block into sp[3 b + m].  S items in
+// (KC = 3) partial sums 3..5 of every block into ct[3 b + m].  S items in
 // flight; a slot takes its next item as soon as its item has arrived.
 template <typename T, int S>
 __device__ bool poll_ghosts(const unsigned long long* __restrict__ pb, int G, int KC,
                             const unsigned long long* __restrict__ vb, T* dst, int no, int nloc,
-                            const int* __restrict__ gid, int g, unsigned f, double* sp, int t, int stride,
+                            const int* __restrict__ gid, int g, unsigned f, T* ct, int t, int stride,
                             Waiter& wt) {
     constexpr int TW = Tag<T>::W;
     const int ng = 3 * (nloc - no), n = ng + KC * G;
@@ -974,7 +983,7 @@ __device__ bool poll_ghosts(const unsigned long long* __restrict__ pb, int G, in
             if ((unsigned)(lo[s] >> 32) != f || (unsigned)(hi[s] >> 32) != f) continue;
             const int i = it[s];
             if (i >= ng) {
-                sp[i - ng] = __longlong_as_double((long long)((hi[s] << 32) | (lo[s] & 0xffffffffull)));
+                ct[i - ng] = (T)__longlong_as_double((long long)((hi[s] << 32) | (lo[s] & 0xffffffffull)));
             } else if constexpr (TW == 2) {
                 dst[3 * no + i] = (T)__longlong_as_double((long long)((hi[s] << 32) | (lo[s] & 0xffffffffull)));
             } else {
@@ -1089,7 +1098,7 @@ struct Dof {
 // and x updated behind the publication, while the block waits anyway.
 // Measured (us per iteration, before: element tasks in shared memory, 16
 // warps, five barriers): 60k-DOF Q4 plate on 148 blocks FP64 block Jacobi 5.13 ->
-// 3.32, FP64 two-level 6.94 -> 5.82, mixed two-level Chebyshev 7.96 -> 6.68;
+// 3.3, FP64 two-level 6.94 -> 5.82, mixed two-level Chebyshev 7.96 -> 6.68;
 // 3,267-DOF plate on 9 blocks 4.18 -> 3.0; 121k-DOF DKT plate 9.38 -> 6.2.
 // Two groups a warp in 8 warps (255 registers) was slower (5.7 on the 60k-DOF
 // plate): one warp's instructions then make up most of the iteration.
@@ -1147,6 +1156,7 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& a, const int g, unsigned
     const T* aig = COARSE ? (MIXED ? (const T*)a.ainv32 : (const T*)a.ainv64) + (size_t)a.ainv_off[g] * a.C
                             : nullptr;
     T* ais = (T*)(sm + L.ainv);
+    T* ct = (T*)(sm + L.ct);  // a round's restriction P^T w (or P^T r), every aggregate
     const T* Ai = a.ainv_smem ? (const T*)ais : aig;
     // FP64 x on every local node for the true residual, in the space of w
     // (and u): neither is live then
@@ -1364,7 +1374,7 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& a, const int g, unsigned
     };
 
     PhaseClock clk;
-    clk.start(a.timing && g == 0 && tid == 0, (long long*)(sm + L.clk));
+    clk.start(a.timing && g == a.G / 2 && tid == 0, (long long*)(sm + L.clk));
     Waiter wt;
     wt.start(a.timeout_ns, a.abort_flag, &a.res->wait_failures);
     unsigned e = a.tag0 + 1, xe = a.tag0 + 1;  // round tags
@@ -1388,7 +1398,9 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& a, const int g, unsigned
         block_publish<4>(v0, red, pb0, a.G, g, 3, e);
         const bool ok = exchange_round<T>(pb0, a.G, 3, nullptr, w, no, no, gid, g, e, sp, wt);
         if (__syncthreads_or(!ok)) status = ST_TIMEOUT;
-        else coarse_apply<T>(Ai, a.G, rows, sp, 3, 0, cvb, 0);
+        for (int i = tid; i < a.C; i += nt) ct[i] = (T)sp[i];
+        __syncthreads();
+        coarse_apply<T>(Ai, a.C, rows, ct, cvb, 0);
         __syncthreads();
         e++;
     }
@@ -1525,8 +1537,8 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& a, const int g, unsigned
             const int st = nt - 32 * wd, t0 = tid - 32 * wd;
             const int items = 3 * (nloc - no) + (COARSE ? 3 * a.G : 0);
             const bool ok = items <= 2 * st
-                ? poll_ghosts<T, 2>(pb, a.G, COARSE ? 3 : 0, vb, w, no, nloc, gid, g, e, sp, t0, st, wt)
-                : poll_ghosts<T, 4>(pb, a.G, COARSE ? 3 : 0, vb, w, no, nloc, gid, g, e, sp, t0, st, wt);
+                ? poll_ghosts<T, 2>(pb, a.G, COARSE ? 3 : 0, vb, w, no, nloc, gid, g, e, ct, t0, st, wt)
+                : poll_ghosts<T, 4>(pb, a.G, COARSE ? 3 : 0, vb, w, no, nloc, gid, g, e, ct, t0, st, wt);
             if (!ok) ctl[2] = 1;
         }
         double inv_g = 0.0, inv_a = 0.0, check = 0.0;
@@ -1554,7 +1566,7 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& a, const int g, unsigned
         }
         if (COARSE && (warp > 0 || nw == 1)) {
             asm volatile("bar.sync 1, %0;" ::"r"(nw == 1 ? 32 : nt - 32) : "memory");
-            coarse_apply<T>(Ai, a.G, rows, sp, 3, 0, qw, nw == 1 ? 0 : 1);
+            coarse_apply<T>(Ai, a.C, rows, ct, qw, nw == 1 ? 0 : 1);
         }
         clk.lap(4);
         if (warp == 0) {
@@ -1662,7 +1674,11 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& a, const int g, unsigned
             if (__syncthreads_or(!ok)) { status = ST_TIMEOUT; break; }
             sum_partials<1>(sp, a.G, KR, scal);
             // c = A_c^-1 P^T r from the true residual (cs is unchanged)
-            if (COARSE) coarse_apply<T>(Ai, a.G, rows, sp, 4, 1, cvb + cb * rows, 0);
+            if (COARSE) {
+                for (int i = tid; i < a.C; i += nt) ct[i] = (T)sp[i / 3 * 4 + 1 + i % 3];
+                __syncthreads();
+                coarse_apply<T>(Ai, a.C, rows, ct, cvb + cb * rows, 0);
+            }
             __syncthreads();
             e++;
             auto coarse_c = [&](const Prow& pr) { return cvb[cb * rows + pr.q + ld]; };
@@ -1830,6 +1846,8 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& a, const int g, unsigned
             }
         }
     }
+    if (clk.on)
+        for (int k = 0; k < 8; k++) a.res->phase_cycles[k] = clk.t[k];
     if (g == 0 && tid == 0) {
         a.res->status = status;
         a.res->iterations = dec->xupd;
@@ -1841,7 +1859,6 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& a, const int g, unsigned
         a.res->reliable_updates = dec->nru;
         a.res->reductions = (int)(e - 1 - a.tag0);
         a.res->last_tag = e > xe ? e : xe;
-        for (int k = 0; k < 8; k++) a.res->phase_cycles[k] = clk.on ? clk.t[k] : 0;
     }
 }
 

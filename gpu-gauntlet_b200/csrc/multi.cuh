@@ -436,7 +436,7 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
         __syncthreads();
     }
     PhaseClock clk;
-    clk.start(a.timing && g == 0 && tid == 0, (long long*)(sm + L.clk));
+    clk.start(a.timing && g == a.G / 2 && tid == 0, (long long*)(sm + L.clk));
     Waiter wt;
     wt.start(a.timeout_ns, a.abort_flag, &a.res->wait_failures);
     unsigned e = a.tag0 + 1, xe = a.tag0 + 1;
@@ -867,6 +867,8 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
             }
         }
     }
+    if (clk.on)
+        for (int k = 0; k < 8; k++) a.res[0].phase_cycles[k] = clk.t[k];
     if (g == 0 && tid < NR) {
         PcgResult& R = a.res[tid];
         R.status = status != ST_OK ? status : cs.status;
@@ -879,7 +881,6 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
         R.reliable_updates = cs.nru;
         R.reductions = (int)(e - 1 - a.tag0);
         R.last_tag = e > xe ? e : xe;
-        for (int k = 0; k < 8; k++) R.phase_cycles[k] = clk.on ? clk.t[k] : 0;
     }
 }
 

@@ -305,6 +305,8 @@ pg::SmemLayout make_layout(const pg::HostPlan& hp, int threads, bool mixed, bool
     const size_t xloc = nloc - std::min<size_t>(nloc, res);                            // not resident
     int groups = 0, steps = 0;
     largest_rows(hp, &groups, &steps);
+    // before the coarse space is built: every aggregate a block could touch, up to 25
+    const size_t C = 3 * (size_t)hp.G, kagg = hp.max_kagg ? hp.max_kagg : std::min(hp.G, 25);
     size_t off = 0;
     auto take = [&](size_t bytes) {
         const size_t o = off;
@@ -317,9 +319,9 @@ pg::SmemLayout make_layout(const pg::HostPlan& hp, int threads, bool mixed, bool
     L.red = take((size_t)(coarse ? 6 : 3) * threads * 8);  // [values][threads]
     L.scal = take(8 * 8);
     L.sp = take((size_t)4 * hp.G * 8);
-    L.qw = take(coarse ? (size_t)3 * hp.max_kagg * 8 : 0);
-    L.cs = take(coarse ? (size_t)2 * 3 * hp.max_kagg * 8 : 0);
-    L.cv = take(coarse ? (size_t)2 * 3 * hp.max_kagg * 8 : 0);
+    L.qw = take(coarse ? 3 * kagg * 8 : 0);
+    L.cs = take(coarse ? 2 * 3 * kagg * 8 : 0);
+    L.cv = take(coarse ? 2 * 3 * kagg * 8 : 0);
     L.ctl = take(4 * 4);
     L.dec = take(sizeof(pg::Decision));
     L.clk = take(9 * 8);
@@ -336,7 +338,8 @@ pg::SmemLayout make_layout(const pg::HostPlan& hp, int threads, bool mixed, bool
     L.kt = take((size_t)kq * 9 * pg::kRowLanes * T);
     L.kq = kq;
     L.nb = take(coarse ? 3 * nloc * T : 0);
-    L.ainv = take(coarse && ainv_smem ? (size_t)3 * hp.max_kagg * hp.C * T : 0);
+    L.ainv = take(coarse && ainv_smem ? 3 * kagg * C * T : 0);
+    L.ct = take(coarse ? C * T : 0);
     L.nslot = take(coarse ? nloc * 4 : 0);
     L.gid = take(nloc * 4);
     L.gq = take((size_t)(groups + 1) * 4);

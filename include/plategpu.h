@@ -170,7 +170,7 @@ typedef struct pg_info {
                                      correction (iterations, stop_reason and converged are
                                      then the correction's; the residuals refer to the final
                                      x and F; solve_ms covers both) */
-    double phase_us[8];           /* with phase_timing, block 0's time (SM cycles at
+    double phase_us[8];           /* with phase_timing, the middle block's time (SM cycles at
                                      the nominal clock) in: K.u, dots and publishing w
                                      (load cases: K.u); load cases: dots and publishing
                                      w; block reduction and publishing the
