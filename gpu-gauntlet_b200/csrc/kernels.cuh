@@ -860,22 +860,23 @@ __device__ __forceinline__ void coarse_apply(const T* __restrict__ Ai, int C, in
 // order (lane l blocks l, l + 32, ..., then an xor butterfly, so every lane
 // of every block holds the same bits).  Up to five blocks a lane are polled
 // at once, straight into registers.  False if a wait gave up.
+template <int SW = 16>  // words of a block's slot
 __device__ __forceinline__ bool poll_total(const unsigned long long* __restrict__ pb, int G, int g, int copies, int k,
                                            unsigned f, double& out, Waiter& wt) {
     constexpr int NB = 5;
     const int lane = threadIdx.x & 31;
-    pb += (size_t)(g % copies) * G * 16 + 2 * k + 16 * lane;
+    pb += (size_t)(g % copies) * G * SW + 2 * k + SW * lane;
     double acc = 0.0;
     bool ok = true;
     wt.spins = 0;
-    for (int base = lane; base < G && ok; base += 32 * NB, pb += 512 * NB) {
+    for (int base = lane; base < G && ok; base += 32 * NB, pb += 32 * SW * NB) {
         unsigned long long lo[NB], hi[NB];
         for (;;) {
             bool got = true;
 #pragma unroll
             for (int i = 0; i < NB; i++) {
                 lo[i] = hi[i] = (unsigned long long)f << 32;  // past the last block: 0
-                if (base + 32 * i < G) ld_relaxed2(pb + 512 * i, lo[i], hi[i]);
+                if (base + 32 * i < G) ld_relaxed2(pb + 32 * SW * i, lo[i], hi[i]);
             }
 #pragma unroll
             for (int i = 0; i < NB; i++) got = got && (unsigned)(lo[i] >> 32) == f && (unsigned)(hi[i] >> 32) == f;

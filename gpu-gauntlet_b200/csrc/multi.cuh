@@ -19,6 +19,11 @@
 // recurrences untouched and only use the true residual for an early
 // convergence test).
 //
+// The 3 NR dot products are polled and summed by warps of their own while the
+// others take the ghosts and the coarse restrictions, with the addresses'
+// divisions by constants: four cases of the 60k-DOF plate (mixed two-level
+// Chebyshev) went from 26.1 to 15.8 us per iteration, two from 11.4 to 10.8.
+//
 // Threads of the case-interleaved loops handle item q = (dof or node) * NR +
 // case with a block size that is a multiple of NR, so each thread works on
 // one case (threadIdx.x % NR) throughout.
@@ -29,9 +34,9 @@
 namespace pg {
 
 // Words of one block's partial-sum slot: up to 6 sums per case, 2 tagged
-// words per FP64 sum.
+// words per FP64 sum, in 128-byte lines of its own (see kRep).
 template <int NR>
-constexpr int multi_slot_words() { return 2 * 6 * NR; }
+constexpr int multi_slot_words() { return (2 * 6 * NR + 15) / 16 * 16; }
 
 // NR consecutive values (one per case) as one aligned access.
 template <typename T, int NR>
@@ -161,38 +166,37 @@ __device__ void block_publish_multi(double (&v)[KP], double* red, unsigned long 
     for (int r = 0; r < kRep; r++) Tag<double>::put(pb + ((size_t)r * G + g) * SW + 2 * lane, t, f);
 }
 
-// One exchange round for NR cases: the K = KP * NR partial sums of every
-// block (staged to sp[G][K]) and case k of each ghost DOF of vector buffer
-// vb (words ((dof * NR + k) * TW), written to dst[dof_local * NR + k] for
-// local DOFs [3 no, 3 nloc)).  Items: the ghost values first (their owners
-// publish them before their partial sums), then the partials; each thread
-// takes items tid, tid + nt, ... with S in flight, refilling a slot with
-// its next item as soon as the slot's item has arrived.  Returns false if a
-// wait gave up.
-template <typename T, int NR, int S = 4>
-__device__ bool exchange_round_multi(const unsigned long long* __restrict__ pb, int G, int K,
-                                     const unsigned long long* __restrict__ vb, T* dst, int no, int nloc,
-                                     const int* __restrict__ gid, int g, unsigned f, double* sp,
-                                     Waiter& wt) {
+// This thread's items t, t + stride, ... of an exchange round for NR cases: case k
+// of each ghost DOF of vector buffer vb (words ((dof * NR + k) * TW)), to
+// dst[dof_local * NR + k] for local DOFs [3 no, 3 nloc), then values K0 .. K0 +
+// K - 1 of every block's partial sums, to put(b * K + i, value).  The ghosts
+// come first (their owners publish them before their partial sums); S items in
+// flight, a slot takes its next item as soon as its item has arrived.  False
+// if a wait gave up.
+template <typename T, int NR, int K0, int K, int S, typename Put>
+__device__ __forceinline__ bool poll_multi(const unsigned long long* __restrict__ pb, int G,
+                                           const unsigned long long* __restrict__ vb, T* dst, int no, int nloc,
+                                           const int* __restrict__ gid, int g, unsigned f, int t, int stride,
+                                           Waiter& wt, Put put) {
     constexpr int TW = Tag<T>::W, SW = multi_slot_words<NR>();
-    const int ng = 3 * (nloc - no) * NR, n = ng + G * K, nt = blockDim.x;
-    pb += (size_t)(g % kRep) * G * SW;
+    const int ng = 3 * (nloc - no) * NR, n = ng + G * K;
+    pb += (size_t)(g % kRep) * G * SW + 2 * K0;
     auto addr = [&](int i) -> const unsigned long long* {
         if (i < ng) {
             const int k3 = 3 * no + i / NR;
             return vb + ((size_t)(3 * gid[k3 / 3] + k3 % 3) * NR + i % NR) * TW;
         }
         const int q = i - ng;
-        return pb + (size_t)(q / K) * SW + 2 * (q % K);
+        return pb + (size_t)(q / (K > 0 ? K : 1)) * SW + 2 * (q % (K > 0 ? K : 1));
     };
     int it[S];
     const unsigned long long* pp[S];
 #pragma unroll
     for (int s = 0; s < S; s++) {
-        it[s] = threadIdx.x + s * nt;
+        it[s] = t + s * stride;
         pp[s] = it[s] < n ? addr(it[s]) : nullptr;
     }
-    int next = threadIdx.x + S * nt;
+    int next = t + S * stride;
     wt.spins = 0;
     for (;;) {
         unsigned long long lo[S], hi[S];
@@ -209,69 +213,94 @@ __device__ bool exchange_round_multi(const unsigned long long* __restrict__ pb, 
                 hi[s] = lo[s];
             }
         }
-        if (!any) break;
+        if (!any) return true;
         bool moved = false;
 #pragma unroll
         for (int s = 0; s < S; s++) {
             if (it[s] >= n) continue;
             if ((unsigned)(lo[s] >> 32) != f || (unsigned)(hi[s] >> 32) != f) continue;
             const int i = it[s];
+            const double v = __longlong_as_double((long long)((hi[s] << 32) | (lo[s] & 0xffffffffull)));
             if (i >= ng) {
-                sp[i - ng] = __longlong_as_double((long long)((hi[s] << 32) | (lo[s] & 0xffffffffull)));
+                put(i - ng, v);
             } else if constexpr (TW == 2) {
-                dst[3 * no * NR + i] = (T)__longlong_as_double((long long)((hi[s] << 32) | (lo[s] & 0xffffffffull)));
+                dst[3 * no * NR + i] = (T)v;
             } else {
                 dst[3 * no * NR + i] = (T)__uint_as_float((unsigned)lo[s]);
             }
             it[s] = next;
-            next += nt;
+            next += stride;
             pp[s] = it[s] < n ? addr(it[s]) : nullptr;
             moved = true;
         }
         if (!moved && !wt.keep_going()) return false;
     }
-    return true;
 }
 
-// out[q * NR + k] = sum_j Ai[q][j] y_j^(k) for the part's coarse rows, with
-// y_{3b+m}^(k) = sp[b * stride + off + m * NR + k].  Warps w0.. take two
-// rows each (16 lanes per row), fixed order as in the single solve.  Only
-// the cases in `mask` are written.
+// One exchange round by all threads: the first K partial sums of every block
+// (staged to sp[G][K]) and the ghost values.
+template <typename T, int NR, int K>
+__device__ bool exchange_round_multi(const unsigned long long* __restrict__ pb, int G,
+                                     const unsigned long long* __restrict__ vb, T* dst, int no, int nloc,
+                                     const int* __restrict__ gid, int g, unsigned f, double* sp, Waiter& wt) {
+    return poll_multi<T, NR, 0, K, 4>(pb, G, vb, dst, no, nloc, gid, g, f, threadIdx.x, blockDim.x, wt,
+                                      [&](int i, double v) { sp[i] = v; });
+}
+
+// out[q * NR + k] = sum_j Ai[q][j] y_j^(k) for the part's coarse rows; y [C][NR]
+// in the rows' type.  Warps w0.. take two rows each, 16 lanes a row, fixed
+// order.  Only the cases in `mask` are written.
 template <typename T, int NR>
-__device__ __forceinline__ void coarse_apply_multi(const T* __restrict__ Ai, int G, int rows,
-                                                   const double* __restrict__ sp, int stride, int off,
-                                                   double* __restrict__ out, int w0,
-                                                   unsigned mask = 0xffffffffu) {
+__device__ __forceinline__ void coarse_apply_multi(const T* __restrict__ Ai, int C, int rows, const T* __restrict__ y,
+                                                   double* __restrict__ out, int w0, unsigned mask = 0xffffffffu) {
+    using V = CaseVec<T, NR>;
     const int lane = threadIdx.x & 31, warp = (int)(threadIdx.x >> 5) - w0;
     const int nw = (int)(blockDim.x >> 5) - w0;
     if (warp < 0) return;
-    const int half = lane >> 4, hl = lane & 15, C = 3 * G;
+    const int half = lane >> 4, hl = lane & 15;
     for (int q0 = 2 * warp; q0 < rows; q0 += 2 * nw) {
         const int q = q0 + half;
-        T acc[3][NR];
+        T acc[2][NR];
 #pragma unroll
-        for (int m = 0; m < 3; m++)
-#pragma unroll
-            for (int k = 0; k < NR; k++) acc[m][k] = T(0);
+        for (int k = 0; k < NR; k++) acc[0][k] = acc[1][k] = T(0);
         if (q < rows) {
             const T* row = Ai + (size_t)q * C;
-            for (int b = hl; b < G; b += 16) {
-                const double* y = sp + b * stride + off;
+            const V* yv = reinterpret_cast<const V*>(y);
+            int j = hl;
+#pragma unroll 4
+            for (; j + 16 < C; j += 32) {
+                const V y0 = yv[j], y1 = yv[j + 16];
+                const T m0 = row[j], m1 = row[j + 16];
 #pragma unroll
-                for (int m = 0; m < 3; m++) {
-                    const T am = row[3 * b + m];
-#pragma unroll
-                    for (int k = 0; k < NR; k++) acc[m][k] += am * (T)y[m * NR + k];
+                for (int k = 0; k < NR; k++) {
+                    acc[0][k] = fma(m0, y0.v[k], acc[0][k]);
+                    acc[1][k] = fma(m1, y1.v[k], acc[1][k]);
                 }
+            }
+            if (j < C) {
+                const V y0 = yv[j];
+#pragma unroll
+                for (int k = 0; k < NR; k++) acc[0][k] = fma(row[j], y0.v[k], acc[0][k]);
             }
         }
 #pragma unroll
         for (int k = 0; k < NR; k++) {
-            double s = (double)acc[0][k] + (double)acc[1][k] + (double)acc[2][k];
+            double s = (double)acc[0][k] + (double)acc[1][k];
 #pragma unroll
             for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
             if (hl == 0 && q < rows && ((mask >> k) & 1u)) out[q * NR + k] = s;
         }
+    }
+}
+
+// ct[(3 b + m) NR + k] = (T) sp[b stride + off + m NR + k]: a round's
+// restrictions in the type of the A_c^-1 rows (all threads; a barrier before
+// and after is the caller's).
+template <typename T, int NR>
+__device__ __forceinline__ void stage_coarse(const double* __restrict__ sp, int G, int stride, int off, T* __restrict__ ct) {
+    for (int i = threadIdx.x; i < 3 * NR * G; i += blockDim.x) {
+        const int b = i / (3 * NR);
+        ct[i] = (T)sp[b * stride + off + i - b * 3 * NR];
     }
 }
 
@@ -316,7 +345,7 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
     double* qw = (double*)(sm + L.qw);
     double* csb = (double*)(sm + L.cs);
     double* cvb = (double*)(sm + L.cv);
-    int* ctl = (int*)(sm + L.ctl);  // [0] action, [1] final residuals needed, [2] cases replacing r
+    int* ctl = (int*)(sm + L.ctl);  // [0] action, [1] final residuals needed, [2] cases replacing r, [3] a wait gave up
     T* nb = (T*)(sm + L.nb);
     int* nslot = (int*)(sm + L.nslot);
     const int rows = a.coarse ? 3 * (a.cagg_off[g + 1] - a.cagg_off[g]) : 0;
@@ -324,8 +353,8 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
     const T* aig = a.coarse ? (MIXED ? (const T*)a.ainv32 : (const T*)a.ainv64) + (size_t)a.ainv_off[g] * a.C
                             : nullptr;
     T* ais = (T*)(sm + L.ainv);
+    T* ct = (T*)(sm + L.ct);  // a round's restrictions [C][NR]
     const T* Ai = a.ainv_smem ? (const T*)ais : aig;
-    const int KP = a.coarse ? 6 : 3;
     // FP64 views for the true residual: own arrays in MIXED mode (ytd may
     // share the yt / w / u space), the (then dead) p / yt arrays in FP64
     double* xl = MIXED ? (double*)(sm + L.xl) : (double*)p;
@@ -339,6 +368,7 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
     for (int i = tid; i <= ng1; i += nt) gq[i] = a.grp_q[gb + i] - qb;
     __syncthreads();
     if (tid == 0) {
+        ctl[3] = 0;
         // the q-steps not in registers go to shared memory while they fit
         int used = 0;
         for (int k = 0; k < ng1; k++) {
@@ -454,11 +484,13 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
         }
         unsigned long long* pb0 = a.llp + (size_t)(e & 1) * kRep * a.G * SW;
         block_publish_multi<NR, 3>(v0, red, pb0, a.G, g, e);
-        const bool ok = exchange_round_multi<T, NR>(pb0, a.G, 3 * NR, nullptr, w, no, no, gid, g, e, sp, wt);
+        const bool ok = exchange_round_multi<T, NR, 3 * NR>(pb0, a.G, nullptr, w, no, no, gid, g, e, sp, wt);
         if (__syncthreads_or(!ok)) {
             status = ST_TIMEOUT;
         } else {
-            coarse_apply_multi<T, NR>(Ai, a.G, rows, sp, 3 * NR, 0, cvb, 0);
+            stage_coarse<T, NR>(sp, a.G, 3 * NR, 0, ct);
+            __syncthreads();
+            coarse_apply_multi<T, NR>(Ai, a.C, rows, ct, cvb, 0);
             __syncthreads();
             for (int q = tid; q < nloc * NR; q += nt) {
                 const int n = q / NR, sl = 3 * nslot[n];
@@ -523,8 +555,23 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
             block_publish_multi<NR, 3>(v3, red, pb, a.G, g, e);
         }
         clk.lap(2);
-        {
-            bool ok = exchange_round_multi<T, NR>(pb, a.G, KP * NR, vb, w, no, nloc, gid, g, e, sp, wt);
+        // ---- exchange: warps 0 .. ND - 1 the 3 NR dot products, the others the
+        //      ghosts and the coarse restrictions ----
+        constexpr int ND = NR == 2 ? 6 : 4;  // NR = 4: three dot products a warp
+        if (warp >= ND) {
+            const int t = tid - 32 * ND, st = nt - 32 * ND;
+            const bool ok = a.coarse
+                ? poll_multi<T, NR, 3 * NR, 3 * NR, 4>(pb, a.G, vb, w, no, nloc, gid, g, e, t, st, wt,
+                                                       [&](int i, double v) { ct[i] = (T)v; })
+                : poll_multi<T, NR, 0, 0, 3>(pb, a.G, vb, w, no, nloc, gid, g, e, t, st, wt, [](int, double) {});
+            if (!ok) ctl[3] = 1;
+        } else {
+            bool ok = true;
+            for (int k = warp; k < 3 * NR; k += ND) {
+                double d;
+                ok = poll_total<SW>(pb, a.G, g, kRep, k, e, d, wt) && ok;
+                if (lane == 0) scal[k] = d;
+            }
             if (a.test_stall && it == 0 && tid == 0) {
                 // the two spare words after the partial-sum buffers: a tag no
                 // block writes, so the wait must run out
@@ -532,8 +579,8 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
                 ok = ok && poll<double>(a.llp + (size_t)2 * kRep * a.G * multi_slot_words<4>(), 0xffffffffu,
                                         never, wt);
             }
-            if (__syncthreads_or(!ok)) { status = ST_TIMEOUT; break; }
-            sum_partials<3 * NR>(sp, a.G, KP * NR, scal);
+            if (!ok) ctl[3] = 1;
+            asm volatile("bar.sync 2, %0;" ::"r"(32 * ND) : "memory");
         }
         e++;
         clk.lap(4);
@@ -606,8 +653,12 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
             }
             clk.lap(6);
         }
-        if (a.coarse) coarse_apply_multi<T, NR>(Ai, a.G, rows, sp, KP * NR, 3 * NR, qw, 1);
+        if (a.coarse && warp > 0) {
+            asm volatile("bar.sync 1, %0;" ::"r"(nt - 32) : "memory");
+            coarse_apply_multi<T, NR>(Ai, a.C, rows, ct, qw, 1);
+        }
         __syncthreads();
+        if (ctl[3]) { status = ST_TIMEOUT; break; }
         const int act = ctl[0];
         if (act == ACT_STOP) break;
         clk.lap(5);
@@ -651,19 +702,21 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
                 }
                 if (a.coarse) restrict3(rtv, cm + 3 * n, nb + 3 * n, vt + 1);
             }
-            int KR = 1;
             if (a.coarse) {
                 block_publish_multi<NR, 4>(vt, red, qb, a.G, g, e);
-                KR = 4;
+                ok = exchange_round_multi<T, NR, 4 * NR>(qb, a.G, rb, r, no, nloc, gid, g, e, sp, wt);
             } else {
                 double v1[1] = {vt[0]};
                 block_publish_multi<NR, 1>(v1, red, qb, a.G, g, e);
+                ok = exchange_round_multi<T, NR, NR>(qb, a.G, rb, r, no, nloc, gid, g, e, sp, wt);
             }
-            ok = exchange_round_multi<T, NR>(qb, a.G, KR * NR, rb, r, no, nloc, gid, g, e, sp, wt);
             if (__syncthreads_or(!ok)) { status = ST_TIMEOUT; break; }
-            sum_partials<NR>(sp, a.G, KR * NR, scal);
-            if (a.coarse)
-                coarse_apply_multi<T, NR>(Ai, a.G, rows, sp, KR * NR, NR, cvb + cb * RN, 0, (unsigned)ctl[2]);
+            sum_partials<NR>(sp, a.G, a.coarse ? 4 * NR : NR, scal);
+            if (a.coarse) {
+                stage_coarse<T, NR>(sp, a.G, 4 * NR, NR, ct);
+                __syncthreads();
+                coarse_apply_multi<T, NR>(Ai, a.C, rows, ct, cvb + cb * RN, 0, (unsigned)ctl[2]);
+            }
             __syncthreads();
             e++;
             // u from r for every case: the FP64 products may have used u's
@@ -855,7 +908,7 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
             unsigned long long* pb = a.llp + (size_t)(e & 1) * kRep * a.G * SW;
             block_publish_multi<NR, 2>(v2, red, pb, a.G, g, e);
             if (g == 0) {
-                ok = exchange_round_multi<T, NR>(pb, a.G, 2 * NR, nullptr, w, no, no, gid, g, e, sp, wt);
+                ok = exchange_round_multi<T, NR, 2 * NR>(pb, a.G, nullptr, w, no, no, gid, g, e, sp, wt);
                 if (__syncthreads_or(!ok)) {
                     status = ST_TIMEOUT;
                 } else {

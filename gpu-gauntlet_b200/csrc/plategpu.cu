@@ -401,6 +401,7 @@ pg::SmemLayout make_layout_multi(const pg::HostPlan& hp, bool mixed, bool coarse
     L.kq = kq;
     L.nb = take(coarse ? 3 * nloc * T : 0);
     L.ainv = take(coarse && ainv_smem ? (size_t)3 * hp.max_kagg * hp.C * T : 0);
+    L.ct = take(coarse ? 3 * (size_t)hp.G * T * R : 0);
     L.nslot = take(coarse ? nloc * 4 : 0);
     L.gid = take(nloc * 4);
     L.gq = take((size_t)(groups + 1) * 4);
@@ -1209,10 +1210,10 @@ void solve_with_fallback(pg_ctx* c, Plan* pl, const pg_options& o, pg_info* info
 }
 
 // Layout of an NR-case launch, row blocks and A_c^-1 rows in shared memory as
-// in choose_layout (*all: every row block is on chip); false when none fits
-// (the plate's parts are then solved with fewer cases per launch).
-bool choose_layout_multi(pg_ctx* c, const pg::HostPlan& hp, const pg_options& o, int NR, bool* all,
-                         bool* ainv_smem, pg::SmemLayout* out) {
+// in choose_layout; false when none fits (the plate's parts are then solved
+// with fewer cases per launch).
+bool choose_layout_multi(pg_ctx* c, const pg::HostPlan& hp, const pg_options& o, int NR, bool* ainv_smem,
+                         pg::SmemLayout* out) {
     const bool mixed = o.precision == PG_PREC_MIXED, coarse = o.preconditioner == PG_PRECOND_TWO_LEVEL;
     const int need = steps_outside(hp, pg::kMultiThreads);
     const size_t step = 9 * pg::kRowLanes * (mixed ? 4 : 8);
@@ -1221,7 +1222,6 @@ bool choose_layout_multi(pg_ctx* c, const pg::HostPlan& hp, const pg_options& o,
         if (L.total > c->max_smem) continue;
         const int q = (int)std::min<size_t>(need, (size_t)(c->max_smem - L.total) / step);
         *ainv_smem = ainv != 0;
-        *all = q == need && (ainv || !coarse);
         *out = make_layout_multi(hp, mixed, coarse, ainv != 0, NR, q);
         return true;
     }
@@ -1244,9 +1244,9 @@ void run_solve_multi(pg_ctx* c, Plan* pl, const pg_options& o, int NR, int count
     const bool mixed = o.precision == PG_PREC_MIXED;
     const size_t n = 3 * (size_t)hp.Nn;
     prepare_plan_data(c, pl, o);
-    bool all = false, ainv_smem = false;
+    bool ainv_smem = false;
     pg::SmemLayout L{};
-    if (!choose_layout_multi(c, hp, o, NR, &all, &ainv_smem, &L))
+    if (!choose_layout_multi(c, hp, o, NR, &ainv_smem, &L))
         throw Fail{PG_EUNSUPPORTED, "load-case partition too large for shared memory"};
     cudaStream_t st = c->stream;
     if (pl->m_nr != NR) {
@@ -2000,28 +2000,19 @@ int pg_solve_load_cases(pg_ctx* c, const pg_problem* p, int count, const float* 
         bool cached = false;
         Plan* pl = get_plan(c, *p, G, halo_rings(o), &cached);
         prepare_plan_data(c, pl, o);
-        // group width: automatic = with the two-level preconditioner two cases,
-        // else the widest of 4 and 2 whose layout keeps the row blocks on
-        // chip, else the widest that fits.  A case adds 3 partial sums per block
-        // to what every block reads each round (block Jacobi) or 6 (two-level),
-        // and four cases' 3,552 values cost more than they share: 60k-DOF
-        // plate, ms per case with 1 / 2 / 4 cases a launch: FP64 block Jacobi
-        // 5.17 / 4.20 / 3.86, FP64 two-level 1.95 / 1.66 / 2.05, mixed two-level
-        // Chebyshev 1.37 / 1.26 / 1.58
-        auto fits = [&](int NR, bool* on_chip = nullptr) {
-            bool all = false, ai = false;
+        // group width: automatic = the widest of 4 and 2 that fits: a wider group
+        // pays even where it leaves row blocks or A_c^-1 rows in L2.  ms per case
+        // with 1 / 2 / 4 cases a launch, 60k-DOF plate: FP64 block Jacobi 5.17 / 4.18 /
+        // 3.88, FP64 two-level 1.86 / 1.48 / 1.20, mixed two-level Chebyshev 1.21 /
+        // 1.19 / 0.96; 73k-DOF plate, partly in L2: 7.35 / 5.63 / 5.14, 2.49 / 1.82 /
+        // 1.49, 1.81 / 1.45 / 1.19
+        auto fits = [&](int NR) {
+            bool ai = false;
             pg::SmemLayout L{};
-            const bool ok = choose_layout_multi(c, pl->hp, o, NR, &all, &ai, &L);
-            if (on_chip) *on_chip = ok && all;
-            return ok;
+            return choose_layout_multi(c, pl->hp, o, NR, &ai, &L);
         };
         int W = cases_per_launch;
-        if (W == 0) {
-            bool all4 = false, all2 = false;
-            const bool f4 = fits(4, &all4), f2 = fits(2, &all2);
-            const bool two = o.preconditioner == PG_PRECOND_TWO_LEVEL && f2;
-            W = two ? 2 : all4 ? 4 : all2 ? 2 : f4 ? 4 : f2 ? 2 : 1;
-        }
+        if (W == 0) W = fits(4) ? 4 : fits(2) ? 2 : 1;
         else if (W > 1 && !fits(W)) throw Fail{PG_EUNSUPPORTED, "load-case partition too large for shared memory"};
         for (int k0 = 0; k0 < count;) {
             const int m = std::min(W, count - k0);
