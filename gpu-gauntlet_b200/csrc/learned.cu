@@ -30,10 +30,12 @@
 // iterations, and before the solve may stop, the residual is recomputed as
 // r = F - K x in FP64 and the stop test is made on that true residual.
 //
-// Execution: the whole solve is one CUDA graph launch: a conditional WHILE
-// node whose body is one iteration (about 30 kernels), ended from the
-// device by cudaGraphSetConditional once the true residual meets the
-// tolerance (or the iteration limit, a breakdown or a non-finite value).
+// Execution: with the network on a grid of up to about 272 x 272 pixels the
+// whole solve is one persistent cooperative kernel (fp_persist_kernel).  Else,
+// and without the network, it is one CUDA graph launch: a conditional WHILE
+// node whose body is one iteration, ended from the device by
+// cudaGraphSetConditional once the true residual meets the tolerance (or the
+// iteration limit, a breakdown or a non-finite value).
 // Training is a second graph whose WHILE body is one Adam step (batch
 // gather, forward, energy-norm loss through the library's own K.p,
 // backward, Adam), so an epoch is one launch.
@@ -345,6 +347,7 @@ void net_forward(pg_net* n, Workspace* w, cudaStream_t st, const int* skip, bool
     const pgn::LayerTable& T = n->T;
     auto wf = [&](int k) { return n->wf.p + T.l[k].off_f; };
     const bool fuse = !w->grads;
+    // (forward_layers gives the same layers to the persistent kernel)
     auto dec = [&](pgn::ConvArgs a, const bf16* up, int cs, int from) { return fuse ? upsampled(a, up, cs, from) : a; };
     using namespace pgn;
     conv(OUT_BF16_RELU, 16, 16, cargs(B, H0, W0, w->in.p, 16, wf(E0A), 16, w->e0a.p, 16, 0, 16, skip), st, pdl);
@@ -366,6 +369,31 @@ void net_forward(pg_net* n, Workspace* w, cudaStream_t st, const int* skip, bool
     conv(OUT_BF16_RELU, 16, 16, cargs(B, H0, W0, w->d0a.p, 16, wf(D0B), 16, w->d0.p, 16, 0, 16, skip), st, pdl);
     conv(OUT_F32, 16, 16, cargs(B, H0, W0, w->d0.p, 16, wf(OUTL), 16, w->out.p, 4, 0, 3, skip), st, pdl);
     LCK(cudaGetLastError());
+}
+
+// The layers of the batch-1 forward pass as net_forward launches them, the
+// decoder upsampling in its own loads.
+void forward_layers(pg_net* n, Workspace* w, pgn::ConvArgs (&L)[pgn::kLayers]) {
+    const int H0 = n->H, W0 = n->W, H1 = H0 / 2, W1 = W0 / 2, H2 = H1 / 2, W2 = W1 / 2, H3 = H2 / 2, W3 = W2 / 2;
+    auto wf = [&](int k) { return n->wf.p + n->T.l[k].off_f; };
+    auto l = [&](int H, int W, const bf16* in, int cs, int k, int rows, void* out, int out_cs, int real) {
+        return cargs(1, H, W, in, cs, wf(k), rows, out, out_cs, 0, real, nullptr);
+    };
+    L[E0A] = l(H0, W0, w->in.p, 16, E0A, 16, w->e0a.p, 16, 16);
+    L[E0B] = pooled(l(H0, W0, w->e0a.p, 16, E0B, 16, w->cat0.p, 48, 16), w->p1.p, 16);
+    L[E1A] = l(H1, W1, w->p1.p, 16, E1A, 32, w->e1a.p, 32, 32);
+    L[E1B] = pooled(l(H1, W1, w->e1a.p, 32, E1B, 32, w->cat1.p, 96, 32), w->p2.p, 32);
+    L[E2A] = l(H2, W2, w->p2.p, 32, E2A, 64, w->e2a.p, 64, 64);
+    L[E2B] = pooled(l(H2, W2, w->e2a.p, 64, E2B, 64, w->cat2.p, 192, 64), w->p3.p, 64);
+    L[E3A] = l(H3, W3, w->p3.p, 64, E3A, 128, w->e3a.p, 128, 128);
+    L[E3B] = l(H3, W3, w->e3a.p, 128, E3B, 128, w->e3.p, 128, 128);
+    L[D2A] = upsampled(l(H2, W2, w->cat2.p, 192, D2A, 64, w->d2a.p, 64, 64), w->e3.p, 128, 64);
+    L[D2B] = l(H2, W2, w->d2a.p, 64, D2B, 64, w->d2.p, 64, 64);
+    L[D1A] = upsampled(l(H1, W1, w->cat1.p, 96, D1A, 32, w->d1a.p, 32, 32), w->d2.p, 64, 32);
+    L[D1B] = l(H1, W1, w->d1a.p, 32, D1B, 32, w->d1.p, 32, 32);
+    L[D0A] = upsampled(l(H0, W0, w->cat0.p, 48, D0A, 16, w->d0a.p, 16, 16), w->d1.p, 32, 16);
+    L[D0B] = l(H0, W0, w->d0a.p, 16, D0B, 16, w->d0.p, 16, 16);
+    L[OUTL] = l(H0, W0, w->d0.p, 16, OUTL, 16, w->out.p, 4, 3);
 }
 
 void wgrad(pg_net* n, int k, int B, int H, int W, const bf16* x, int x_cs, const bf16* g, int g_cs,
@@ -589,14 +617,24 @@ __device__ __forceinline__ void kv_block_sum(const Op& op, int n, int h, int ste
                                              float& s1, float& s2) {
     const int s = n >> 5, lane = n & 31;
     const int j1 = op.nm_off[s + 1];
-#pragma unroll 3
-    for (int j = op.nm_off[s] + h; j < j1; j += step) {
-        const int m = op.nm_col[32 * j + lane];
-        const float* B = op.nm_val + (size_t)288 * j + lane;
-        const float v0 = getv(m, 0), v1 = getv(m, 1), v2 = getv(m, 2);
-        s0 += B[0] * v0 + B[32] * v1 + B[64] * v2;
-        s1 += B[96] * v0 + B[128] * v1 + B[160] * v2;
-        s2 += B[192] * v0 + B[224] * v1 + B[256] * v2;
+    // five slots' loads in flight (an inner Q4 node's share of nine when two
+    // threads split them), the ones past the end repeating the last
+    for (int j0 = op.nm_off[s] + h; j0 < j1; j0 += 5 * step) {
+#pragma unroll
+        for (int i = 0; i < 5; i++) {
+            const int j = min(j0 + i * step, j1 - 1);
+            const int m = op.nm_col[32 * j + lane];
+            const float* B = op.nm_val + (size_t)288 * j + lane;
+            const float v0 = getv(m, 0), v1 = getv(m, 1), v2 = getv(m, 2);
+            const float a0 = B[0] * v0 + B[32] * v1 + B[64] * v2;
+            const float a1 = B[96] * v0 + B[128] * v1 + B[160] * v2;
+            const float a2 = B[192] * v0 + B[224] * v1 + B[256] * v2;
+            if (j0 + i * step < j1) {
+                s0 += a0;
+                s1 += a1;
+                s2 += a2;
+            }
+        }
     }
 }
 
@@ -1142,6 +1180,22 @@ __global__ void fp_update_kernel(FArgs a) {
     }
 }
 
+// This thread's share of (K x)_n in FP64 (every op.tpn-th incident element).
+template <int NPE>
+__device__ __forceinline__ void true_product(const FArgs& a, int n, int h, double (&kx)[3]) {
+    constexpr int ND = 3 * NPE;
+    for (int q = a.op.inc_ptr[n] + h; q < a.op.inc_ptr[n + 1]; q += a.op.tpn) {
+        const int e = a.op.inc_idx[q] >> 2, k = a.op.inc_idx[q] & 3;
+        const double* Ke = a.op.ke64 + (size_t)e * ND * ND + 3 * k * ND;
+        for (int b = 0; b < NPE; b++) {
+            const int m = (int)a.op.el[(size_t)e * NPE + b];
+            const double x0 = a.x[3 * m], x1 = a.x[3 * m + 1], x2 = a.x[3 * m + 2];
+            for (int d = 0; d < 3; d++) kx[d] += Ke[d * ND + 3 * b] * x0 + Ke[d * ND + 3 * b + 1] * x1 +
+                                                 Ke[d * ND + 3 * b + 2] * x2;
+        }
+    }
+}
+
 // TR: when the recursive residual meets the tolerance, every replace_every
 // iterations and at the iteration limit: r = F - K x in FP64 (then rounded),
 // and |F - K x|^2 for the stop test.
@@ -1149,7 +1203,6 @@ template <int NPE>
 __global__ void fp_true_res_kernel(FArgs a) {
     pgn::pdl_trigger();
     pgn::pdl_wait();
-    constexpr int ND = 3 * NPE;
     FState* st = a.st;
     if (st->done) return;
     const int it = st->it;
@@ -1169,17 +1222,7 @@ __global__ void fp_true_res_kernel(FArgs a) {
     // the node's FP64 product split between the two threads (every other
     // incident element), then exchanged
     double kx[3] = {0, 0, 0};
-    if (n < a.op.Nn)
-        for (int q = a.op.inc_ptr[n] + h; q < a.op.inc_ptr[n + 1]; q += a.op.tpn) {
-            const int e = a.op.inc_idx[q] >> 2, k = a.op.inc_idx[q] & 3;
-            const double* Ke = a.op.ke64 + (size_t)e * ND * ND + 3 * k * ND;
-            for (int b = 0; b < NPE; b++) {
-                const int m = (int)a.op.el[(size_t)e * NPE + b];
-                const double x0 = a.x[3 * m], x1 = a.x[3 * m + 1], x2 = a.x[3 * m + 2];
-                for (int d = 0; d < 3; d++) kx[d] += Ke[d * ND + 3 * b] * x0 + Ke[d * ND + 3 * b + 1] * x1 +
-                                                     Ke[d * ND + 3 * b + 2] * x2;
-            }
-        }
+    if (n < a.op.Nn) true_product<NPE>(a, n, h, kx);
     if (a.op.tpn == 2)
         for (int d = 0; d < 3; d++) kx[d] += __shfl_xor_sync(0xffffffffu, kx[d], 1);
     if (n < a.op.Nn && h == 0) {
@@ -1426,6 +1469,389 @@ __global__ void fp_dir_kernel(FArgs a) {
     }
 }
 
+// ----- the learned solve in one persistent kernel ------------------------------
+//
+// As a graph an iteration was 24 kernels of 3 to 9 us, most of it launch, ramp
+// and drain around little work.  Here one cooperative launch (a block per SM,
+// 512 threads) runs the whole solve: the same steps with a barrier of all
+// blocks between them, the scalars in every block's registers (each block sums
+// the same partials in the same order), a layer's weights and tile addresses
+// fetched while the block waits at the barrier before it.  A layer's tiles go
+// to groups of 128 threads, at most one each on the 144 x 144 grid.  142 x 142
+// nodes: 127 -> 102 us an iteration (42 in the layers' tiles, 2 to 5 each, about
+// as much in 21 barriers, the rest in the five products with K); bound by the
+// latency of that chain, not by memory or the tensor cores.
+
+constexpr int kPersistThreads = 512;
+
+struct PersistArgs {
+    FArgs f;
+    pgn::ConvArgs conv[pgn::kLayers];
+    int smem;                       // dynamic shared memory, bytes
+    unsigned* bar;                  // blocks arrived, over all barriers of the launch (zero at launch)
+    int* abort_flag;                // a wait gave up (zero at launch)
+    unsigned long long timeout_ns;  // limit of one wait
+};
+
+// Barrier of all blocks; `ahead` runs in every thread once the block has
+// arrived. False when a wait gave up (its limit, or another block's).
+template <typename F>
+__device__ __forceinline__ bool grid_barrier(const PersistArgs& a, unsigned& round, F&& ahead) {
+    __syncthreads();
+    round++;
+    if (threadIdx.x == blockDim.x - 1) {
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(a.bar) : "memory");
+    }
+    ahead();
+    int bad = 0;
+    if (threadIdx.x == blockDim.x - 1) {
+        const unsigned want = round * gridDim.x;
+        unsigned long long t0 = 0;
+        for (unsigned spin = 1;; spin++) {
+            unsigned v;
+            asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
+            if (v >= want) break;
+            if ((spin & 63u) != 0) continue;
+            unsigned long long now;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+            if (t0 == 0) t0 = now;
+            if (*(volatile int*)a.abort_flag || now - t0 >= a.timeout_ns) {
+                atomicExch(a.abort_flag, 1);
+                bad = 1;
+                break;
+            }
+        }
+        __threadfence();  // acquire, once, instead of with every look
+    }
+    return !__syncthreads_or(bad);
+}
+
+// A group's tiles of a layer: the first (blocks first, then groups), the step
+// to the next, and where in shared memory.  Found, with its weights queued,
+// while the block waits for the layer's input: the divisions and the weights'
+// round trip cost nothing there.
+struct LayerTiles {
+    int i, n, step;   // tile, tiles of the layer, tiles in flight
+    int shift;        // log2 of the channel groups (16 channels) of a pixel tile
+    int y, x, co;     // of tile i
+    bf16* s;
+};
+
+__device__ __forceinline__ void tile_at(const pgn::ConvArgs& c, LayerTiles& t) {
+    const int tx = (c.W + 7) >> 3, px = t.i >> t.shift;
+    t.y = px / tx * 8;
+    t.x = (px - t.y / 8 * tx) * 8;
+    t.co = (t.i - (px << t.shift)) * 16;
+}
+
+template <int CIN>
+__device__ __forceinline__ void tiles_ahead(const PersistArgs& a, const pgn::ConvArgs& c, unsigned char* sm, LayerTiles& t) {
+    constexpr int bytes = pgn::conv_smem_bytes(CIN, 16);
+    const int grp = threadIdx.x / pgn::kConvThreads, ng = min((int)(blockDim.x / pgn::kConvThreads), a.smem / bytes);
+    t.shift = 31 - __clz(c.w_rows >> 4);
+    t.n = ((c.W + 7) >> 3) * ((c.H + 7) >> 3) << t.shift;
+    t.i = grp < ng ? grp * gridDim.x + blockIdx.x : t.n;
+    t.step = ng * gridDim.x;
+    t.s = reinterpret_cast<bf16*>(sm + grp * bytes);
+    if (t.i < t.n) {
+        tile_at(c, t);
+        pgn::conv_weights<CIN, 16>(c, t.co, t.s, threadIdx.x % pgn::kConvThreads);
+    }
+}
+
+template <int CIN, int MODE>
+__device__ __forceinline__ void tiles_run(const pgn::ConvArgs& c, LayerTiles& t) {
+    const int tid = threadIdx.x % pgn::kConvThreads;
+    auto join = [] {
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + threadIdx.x / pgn::kConvThreads), "n"(pgn::kConvThreads) : "memory");
+    };
+    while (t.i < t.n) {
+        pgn::conv_tile<CIN, 16, MODE>(c, 0, t.y, t.x, t.co, t.s, tid, join);
+        t.i += t.step;
+        if (t.i >= t.n) break;
+        tile_at(c, t);
+        join();  // the last tile's shared memory has been read
+        pgn::conv_weights<CIN, 16>(c, t.co, t.s, tid);
+    }
+}
+
+template <int NPE>
+__global__ void __launch_bounds__(kPersistThreads, 1) fp_persist_kernel(const __grid_constant__ PersistArgs pa) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const FArgs& a = pa.f;
+    const Op& op = a.op;
+    const int G = gridDim.x, tpn = op.tpn;
+    // warps are dealt to the blocks in turn, so a small plate uses every SM
+    const int stride = G * blockDim.x;
+    const int tid0 = ((threadIdx.x >> 5) * G + blockIdx.x) * 32 + (threadIdx.x & 31);
+    const int span = (tpn * op.Nn + 31) / 32 * 32;  // whole warps, for the products' shuffles
+    unsigned round = 0;
+    auto none = [] {};
+    // f(node, thread of the node, first thread of a live node)
+    auto nodes = [&](auto&& f) {
+        for (int t = tid0; t < span; t += stride) {
+            const int h = tpn == 2 ? (t & 1) : 0, n = tpn == 2 ? (t >> 1) : t;
+            f(n, h, n < op.Nn && h == 0);
+        }
+    };
+    // the loop's scalars, the same in every thread of every block
+    int it = 0, net_off = 0, net_off_at = 0, bad_count = 0, stall = 0, net_iters = 0, replacements = 0;
+    int converged = 0, reason = PG_STOP_MAX_ITER, error = 0;
+    double bn2 = 0.0, true_rr = 0.0, tr_prev = 0.0, gamma_prev = 1.0;
+    bool ok = true;
+    {
+        double acc[1] = {0.0};
+        nodes([&](int n, int, bool own) {
+            if (!own) return;
+            for (int d = 0; d < 3; d++) {
+                const int i = 3 * n + d;
+                const float f = a.F[i];
+                a.x[i] = 0.0;
+                a.r[i] = f;
+                a.r_prev[i] = f;
+                a.p0[i] = a.p1[i] = a.q[i] = 0.f;
+                acc[0] += (double)f * f;
+            }
+        });
+        block_partials<1>(acc, a.pI);
+        ok = grid_barrier(pa, round, none);
+    }
+    for (; ok && it <= a.maxit + 1; it++) {
+        // ---- x += alpha p, r -= alpha q, alpha = p.r / p.Kp of the last direction ----
+        double alpha = 0.0;
+        if (it == 0) {
+            double s[1];
+            reduce_parts<1>(a.pI, G, s);
+            bn2 = s[0];
+            if (!isfinite(bn2)) { error = 1; reason = PG_STOP_BREAKDOWN; break; }
+            if (bn2 < 1e-60) { converged = 1; reason = PG_STOP_ZERO_RHS; break; }
+        } else {
+            double s[2];
+            reduce_parts<2>(a.pD, G, s);
+            if (!isfinite(s[0]) || !isfinite(s[1])) { error = 1; reason = PG_STOP_BREAKDOWN; break; }
+            if (fabs(s[0]) < 1e-30) { reason = PG_STOP_BREAKDOWN; break; }
+            alpha = s[1] / s[0];
+        }
+        {
+            const float* p = (it & 1) ? a.p1 : a.p0;
+            double acc[1] = {0.0};
+            nodes([&](int n, int, bool own) {
+                if (!own) return;
+                float rv[3];
+                for (int d = 0; d < 3; d++) {
+                    const int i = 3 * n + d;
+                    const float ri = a.r[i];
+                    a.x[i] += alpha * (double)p[i];
+                    a.r_prev[i] = ri;
+                    const float rn = (float)((double)ri - alpha * (double)a.q[i]);
+                    a.r[i] = rn;
+                    rv[d] = rn;
+                    acc[0] += (double)rn * rn;
+                }
+                write_t(a, n, rv);
+            });
+            block_partials<1>(acc, a.pU);
+        }
+        if (!(ok = grid_barrier(pa, round, none))) break;
+        // ---- FP64 true residual when the recursive one meets the tolerance,
+        //      every replace_every iterations and at the iteration limit ----
+        double rr[1];
+        reduce_parts<1>(a.pU, G, rr);
+        if (stop_test(a, rr[0], bn2) || (it > 0 && it % a.replace_every == 0) || it >= a.maxit || !isfinite(rr[0])) {
+            replacements++;
+            double acc[1] = {0.0};
+            nodes([&](int n, int h, bool own) {
+                double kx[3] = {0, 0, 0};
+                if (n < op.Nn) true_product<NPE>(a, n, h, kx);
+                if (tpn == 2)
+                    for (int d = 0; d < 3; d++) kx[d] += __shfl_xor_sync(0xffffffffu, kx[d], 1);
+                if (!own) return;
+                float rv[3];
+                for (int d = 0; d < 3; d++) {
+                    const int i = 3 * n + d;
+                    const double rt = (double)a.F[i] - (op.cons[i] ? a.x[i] : kx[d]);
+                    rv[d] = (float)rt;
+                    a.r[i] = rv[d];
+                    acc[0] += rt * rt;
+                }
+                write_t(a, n, rv);
+            });
+            block_partials<1>(acc, a.pTR);
+            if (!(ok = grid_barrier(pa, round, none))) break;
+            double s[1];
+            reduce_parts<1>(a.pTR, G, s);
+            true_rr = s[0];
+            const bool fin = isfinite(s[0]), conv = fin && stop_test(a, s[0], bn2);
+            if (conv || it >= a.maxit || !fin) {
+                converged = conv;
+                reason = conv ? PG_STOP_CONVERGED : PG_STOP_MAX_ITER;
+                error = !fin;
+                break;
+            }
+            // stall guard: with the network on, a replacement interval that did
+            // not cut the true residual norm by 20% switches it off; the first
+            // interval compares with |F|
+            const double prev = tr_prev > 0 ? tr_prev : bn2;
+            if (it % a.replace_every == 0) {
+                if (!net_off && s[0] > 0.64 * prev) stall = 1;
+                tr_prev = s[0];
+            }
+        }
+        bool use = false;
+        float c = 0.f;
+        if (!net_off) {
+            // ---- r1 = r - K t and the network's input ----
+            nodes([&](int n, int h, bool own) {
+                auto tv = [&](int m, int d) { return a.t[3 * m + d]; };
+                float u[3];
+                kv2<NPE>(op, n, h, tv, u);
+                if (!own) return;
+                const float sc[3] = {a.si0, a.si1, a.si2};
+                bf16* px = a.img_in + (size_t)a.node_pixel[n] * 16;
+                for (int d = 0; d < 3; d++) {
+                    const float r1 = a.r[3 * n + d] - u[d];
+                    a.r1[3 * n + d] = r1;
+                    px[d] = __float2bfloat16_rn(sc[d] * r1);
+                }
+            });
+            // ---- the network ----
+            LayerTiles t;
+#define PG_LAYER(K, CIN, MODE)                                                                              \
+    if (!(ok = grid_barrier(pa, round, [&] { tiles_ahead<CIN>(pa, pa.conv[K], smem_raw, t); }))) break;      \
+    tiles_run<CIN, pgn::MODE>(pa.conv[K], t);
+            PG_LAYER(E0A, 16, OUT_BF16_RELU)
+            PG_LAYER(E0B, 16, OUT_BF16_RELU)
+            PG_LAYER(E1A, 16, OUT_BF16_RELU)
+            PG_LAYER(E1B, 32, OUT_BF16_RELU)
+            PG_LAYER(E2A, 32, OUT_BF16_RELU)
+            PG_LAYER(E2B, 64, OUT_BF16_RELU)
+            PG_LAYER(E3A, 64, OUT_BF16_RELU)
+            PG_LAYER(E3B, 128, OUT_BF16_RELU)
+            PG_LAYER(D2A, 192, OUT_BF16_RELU)
+            PG_LAYER(D2B, 64, OUT_BF16_RELU)
+            PG_LAYER(D1A, 96, OUT_BF16_RELU)
+            PG_LAYER(D1B, 32, OUT_BF16_RELU)
+            PG_LAYER(D0A, 48, OUT_BF16_RELU)
+            PG_LAYER(D0B, 16, OUT_BF16_RELU)
+            PG_LAYER(OUTL, 16, OUT_F32)
+#undef PG_LAYER
+            if (!(ok = grid_barrier(pa, round, none))) break;
+            // ---- y = s_out N(r1), then the smoothing sweeps w <- w + S (r1 - K w);
+            //      w.r1 and w.K w of the last for the correction's step ----
+            float* w_in = a.y;
+            for (int k = 0; k <= kCorrectionSweeps; k++) {
+                float* v_out = k & 1 ? a.v2 : a.r2;
+                float* w_next = k < kCorrectionSweeps ? (w_in == a.y ? a.y2 : a.y) : nullptr;
+                const float so[3] = {a.so0, a.so1, a.so2};
+                auto wv = [&](int m, int d) -> float {
+                    if (k > 0) return w_in[3 * m + d];
+                    return op.cons[3 * m + d] ? 0.f : so[d] * a.img_out[(size_t)a.node_pixel[m] * 4 + d];
+                };
+                double acc[2] = {0.0, 0.0};
+                nodes([&](int n, int h, bool own) {
+                    float v[3], w[3];
+                    kv2<NPE>(op, n, h, wv, v);
+                    if (!own) return;
+                    for (int d = 0; d < 3; d++) {
+                        const int i = 3 * n + d;
+                        w[d] = wv(n, d);
+                        if (k == 0) a.y[i] = w[d];
+                        v_out[i] = v[d];
+                        acc[0] += (double)w[d] * a.r1[i];
+                        acc[1] += (double)w[d] * v[d];
+                    }
+                    if (w_next) write_sweep(a, n, w, v, w_next);
+                });
+                block_partials<2>(acc, a.pB);
+                if (w_next) w_in = w_next;
+                if (!(ok = grid_barrier(pa, round, none))) break;
+            }
+            if (!ok) break;
+            double s[2];
+            reduce_parts<2>(a.pB, G, s);
+            const double cd = s[0] / s[1];
+            use = s[0] > 0.0 && s[1] > 0.0 && isfinite(cd);
+            c = use ? (float)cd : 0.f;
+        }
+        // ---- z = t + c w + S (r1 - c K w), or D^-1 r without the correction ----
+        {
+            const float* y = kCorrectionSweeps & 1 ? a.y2 : a.y;
+            const float* ky = kCorrectionSweeps & 1 ? a.v2 : a.r2;
+            double acc[2] = {0.0, 0.0};
+            nodes([&](int n, int, bool own) {
+                if (!own) return;
+                const float* B9 = op.binv32 + 9 * n;
+                const int i = 3 * n;
+                const float r0 = a.r[i], r1_ = a.r[i + 1], r2_ = a.r[i + 2];
+                const float om = a.omega;
+                float z[3];
+                for (int d = 0; d < 3; d++) z[d] = binv_row(B9, d, r0, r1_, r2_);
+                if (use) {
+                    const float q0 = a.r1[i] - c * ky[i], q1 = a.r1[i + 1] - c * ky[i + 1], q2 = a.r1[i + 2] - c * ky[i + 2];
+                    for (int d = 0; d < 3; d++) z[d] = om * z[d] + c * y[i + d] + om * binv_row(B9, d, q0, q1, q2);
+                }
+                for (int d = 0; d < 3; d++) {
+                    a.z[i + d] = z[d];
+                    acc[0] += (double)z[d] * a.r[i + d];
+                    acc[1] += (double)z[d] * a.r_prev[i + d];
+                }
+            });
+            block_partials<2>(acc, a.pC);
+        }
+        if (!(ok = grid_barrier(pa, round, none))) break;
+        // ---- p = z + beta p (Polak-Ribiere), q = K p ----
+        double s[2];
+        reduce_parts<2>(a.pC, G, s);
+        double beta = it == 0 ? 0.0 : (s[0] - s[1]) / gamma_prev;
+        if (!isfinite(beta)) beta = 0.0;
+        {
+            const float* po = (it & 1) ? a.p1 : a.p0;
+            float* pn = (it & 1) ? a.p0 : a.p1;
+            const float bf = (float)beta;
+            auto pv = [&](int m, int d) { return a.z[3 * m + d] + bf * po[3 * m + d]; };
+            double acc[2] = {0.0, 0.0};
+            nodes([&](int n, int h, bool own) {
+                float qv[3];
+                kv2<NPE>(op, n, h, pv, qv);
+                if (!own) return;
+                for (int d = 0; d < 3; d++) {
+                    const int i = 3 * n + d;
+                    const float pi = pv(n, d);
+                    pn[i] = pi;
+                    a.q[i] = qv[d];
+                    acc[0] += (double)pi * qv[d];
+                    acc[1] += (double)pi * a.r[i];
+                }
+            });
+            block_partials<2>(acc, a.pD);
+        }
+        if (!(ok = grid_barrier(pa, round, none))) break;
+        gamma_prev = s[0];
+        if (!net_off) {
+            bad_count = use ? 0 : bad_count + 1;
+            net_iters += use;
+            if (bad_count >= a.fallback_after || stall) {
+                net_off = 1;
+                net_off_at = it;
+            }
+        }
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        FState st{};
+        st.iterations = it;
+        st.converged = converged;
+        st.stop_reason = reason;
+        st.error = error;
+        st.net_iters = net_iters;
+        st.net_off = net_off;
+        st.net_off_at = net_off_at;
+        st.replacements = replacements;
+        st.bnorm2 = bn2;
+        st.true_rr = true_rr;
+        *a.st = st;
+    }
+}
+
 // y = K x by the flexible PCG's operator (pg_learned_apply_k)
 template <int NPE>
 __global__ void apply_op_kernel(Op op, const float* __restrict__ x, float* __restrict__ y) {
@@ -1487,6 +1913,7 @@ struct FpcgSolver {
     Buf<int> nm_off, nm_col;  // node-block form of the operator (op.nm_*)
     Buf<float> nm_val;
     Buf<FState> st;
+    Buf<unsigned> bar;  // the persistent kernel's barrier count and abort flag
     cudaStream_t cap = nullptr;  // capture stream
     cudaGraphExec_t exec = nullptr;
     bool pdl = false, pdl_refused = false;  // graph built with programmatic dependent launch
@@ -1844,6 +2271,43 @@ void fpcg_build(FpcgSolver* S, const pg_options& o, int mode, pg_net* n, const i
     S->tol = o.tolerance;
 }
 
+// Whether the persistent kernel takes the network's grid (the rule stands
+// where it is used).
+bool persist_fits(const FpcgSolver* S, const pg_net* n) {
+    int sms = 0;
+    LCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, pgi::ctx_device(S->ctx)));
+    return (long)((n->H + 7) / 8) * ((n->W + 7) / 8) <= 2L * (kPersistThreads / pgn::kConvThreads) * sms;
+}
+
+// The learned solve (mode 1) as one cooperative launch on st.
+void persist_launch(FpcgSolver* S, const pg_options& o, pg_net* n, const int* node_pixel, int HW, cudaStream_t st) {
+    Workspace* w = workspace(n, 1, false);
+    PersistArgs pa{};
+    pa.f = make_fargs(S, o, 1, n, w, node_pixel, HW, 3, 50);
+    forward_layers(n, w, pa.conv);
+    const void* fn = S->npe == 4 ? (const void*)fp_persist_kernel<4> : (const void*)fp_persist_kernel<3>;
+    int dev = 0, sms = 0, nb = 0;
+    LCK(cudaGetDevice(&dev));
+    LCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    // four groups of the widest layers' tiles (shared memory for four of the
+    // deep ones measured the same at 400 x 400 and 105 to 102 us at 141 x 141)
+    pa.smem = std::max(4 * pgn::conv_smem_bytes(48, 16), pgn::conv_smem_bytes(192, 16));
+    LCK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, pa.smem));
+    LCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, kPersistThreads, pa.smem));
+    if (nb < 1) throw LFail{PG_EUNSUPPORTED, "the learned solve's grid does not fit on the device"};
+    // the partials' arrays hold grid_nodes blocks' sums each; no more blocks than that
+    const int grid = std::min(sms, pa.f.G);
+    if (S->bar.n != 2) S->bar.alloc(2);
+    S->bar.zero(st);
+    pa.bar = S->bar.p;
+    pa.abort_flag = reinterpret_cast<int*>(S->bar.p + 1);
+    // at least a second: the graph this replaces had no waits to limit, so a
+    // caller's short limit stays accepted
+    pa.timeout_ns = (unsigned long long)(std::max(o.wait_timeout_ms, 1000.0) * 1e6);
+    void* args[] = {&pa};
+    LCK(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kPersistThreads), args, pa.smem, st));
+}
+
 // One solve with S (graph rebuilt when the options, the mode or the
 // network's scales changed).  F and x on the host or the device.
 void fpcg_run(FpcgSolver* S, const pg_options& o, int mode, pg_net* n, const int* node_pixel, int HW,
@@ -1853,8 +2317,16 @@ void fpcg_run(FpcgSolver* S, const pg_options& o, int mode, pg_net* n, const int
     cudaStream_t st = pgi::ctx_stream(S->ctx);
     const size_t n3 = 3 * (size_t)S->op.Nn;
     auto t0 = std::chrono::steady_clock::now();
-    if (!S->exec || S->mode != mode || S->maxit != o.max_iterations || S->rule != o.stop_rule ||
-        S->tol != o.tolerance || S->version != (n ? n->version : 0)) {
+    // The persistent kernel up to two rounds of its tile groups in the widest
+    // layers (272 x 272 pixels on 148 SMs), the graph above: us per iteration
+    // with the network, kernel / graph, 65 x 65 nodes 100 / 114, 142 x 142
+    // 102 / 127, 201 x 201 151 / 153, 281 x 281 216 / 217, 401 x 401 377 / 359
+    // (there a block's tiles run three or four after another, while the
+    // graph's smaller blocks leave an SM to one another).
+    const bool persist = mode == 1 && !o.phase_timing && persist_fits(S, n);
+    if (!persist && !o.phase_timing &&
+        (!S->exec || S->mode != mode || S->maxit != o.max_iterations || S->rule != o.stop_rule ||
+         S->tol != o.tolerance || S->version != (n ? n->version : 0))) {
         // with programmatic dependent launch where the driver takes it in a
         // captured conditional body, else without
         try {
@@ -1877,7 +2349,9 @@ void fpcg_run(FpcgSolver* S, const pg_options& o, int mode, pg_net* n, const int
     double phase[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     int timed_its = 0;
     LCK(cudaEventRecord(e0, st));
-    if (!o.phase_timing) {
+    if (persist) {
+        persist_launch(S, o, n, node_pixel, HW, st);
+    } else if (!o.phase_timing) {
         LCK(cudaGraphLaunch(S->exec, st));
     } else {
         // the same kernels without the graph (profilers cannot look inside a
@@ -1910,11 +2384,14 @@ void fpcg_run(FpcgSolver* S, const pg_options& o, int mode, pg_net* n, const int
                         host_x ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice, st));
     FState s{};
     LCK(cudaMemcpyAsync(&s, S->st.p, sizeof s, cudaMemcpyDeviceToHost, st));
+    unsigned waits[2] = {0, 0};
+    if (persist) LCK(cudaMemcpyAsync(waits, S->bar.p, sizeof waits, cudaMemcpyDeviceToHost, st));
     LCK(cudaStreamSynchronize(st));
     float ms = 0;
     LCK(cudaEventElapsedTime(&ms, e0, e1));
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    if (waits[1]) throw LFail{PG_ETIMEOUT, "a wait for another block exceeded wait_timeout_ms"};
     if (s.error) throw LFail{PG_ENONFINITE, "non-finite value in the flexible PCG iteration"};
     if (info) {
         info->iterations = s.iterations;
@@ -1935,7 +2412,7 @@ void fpcg_run(FpcgSolver* S, const pg_options& o, int mode, pg_net* n, const int
         ls->network_off_at = s.net_off ? s.net_off_at : -1;
         ls->replacements = s.replacements;
         ls->mode = mode;
-        ls->pdl = S->pdl;
+        ls->pdl = mode == 1 ? 0 : S->pdl;
     }
 }
 

@@ -108,38 +108,33 @@ __host__ __device__ constexpr int conv_smem_bytes(int cin, int cot) {
     return (100 + 9 * cot) * (cin + 8) * 2;
 }
 
-// 3 x 3 convolution, zero padding, no bias.  A block computes an 8 x 8
-// pixel tile (four warps, each a 2-row x 8-column m16 tile) for COT output
-// channels.  All nine taps' COT x CIN weights are staged in shared memory
-// before the block waits for the kernel before it, the 10 x 10 input halo (CIN
-// channels) behind that wait, so the block pays one L2 round trip before its
-// MMAs (streaming the taps one by one left each small layer waiting nine
-// times); COT is chosen so the weights fit (conv_smem_bytes).
-// Grid: (ceil(W/8), ceil(H/8) * B, w_rows / COT).
-template <int CIN, int COT, int MODE>
-__global__ void __launch_bounds__(kConvThreads) conv3x3_kernel(ConvArgs a) {
-    static_assert(CIN % 16 == 0 && COT % 16 == 0, "channels in multiples of 16");
-    pdl_trigger();
-    constexpr int SP = CIN + 8;  // padded pixel / weight-row stride in shared memory
-    constexpr int C8 = CIN / 8;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    bf16* sIn = reinterpret_cast<bf16*>(smem_raw);
+// One tile of a 3 x 3 convolution (zero padding, no bias) by a group of
+// kConvThreads threads: 8 x 8 pixels (four warps, each a 2-row x 8-column m16
+// tile) for COT output channels.  conv_weights queues all nine taps' COT x CIN
+// weights into shared memory, which no kernel of the chain writes, so it runs
+// ahead of the wait for the input; conv_tile then queues the 10 x 10 input halo
+// and pays one L2 round trip before its MMAs (streaming the taps one by one
+// left each small layer waiting nine times).  COT is chosen so the weights fit
+// (conv_smem_bytes).  t: thread of the group; `join` a barrier of the group.
+template <int CIN, int COT>
+__device__ __forceinline__ void conv_weights(const ConvArgs& a, int co0, bf16* sIn, int tid) {
+    constexpr int SP = CIN + 8, C8 = CIN / 8;
     bf16* sW = sIn + 100 * SP;  // [9][COT][SP]
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int tiles_y = (a.H + 7) >> 3;
-    const int b = blockIdx.y / tiles_y;
-    const int ty0 = (blockIdx.y - b * tiles_y) * 8, tx0 = blockIdx.x * 8;
-    const int co0 = blockIdx.z * COT;
     for (int q = tid; q < 9 * COT * C8; q += kConvThreads) {
         const int row = q / C8, c8 = q - row * C8;  // row = tap * COT + co
         const int tap = row / COT, co = row - tap * COT;
         cp_async16(sW + row * SP + c8 * 8, a.w + ((size_t)tap * a.w_rows + co0 + co) * CIN + c8 * 8, true);
     }
-    pdl_wait();
-    if (a.skip && *a.skip) {
-        cp_async_wait<0>();
-        return;
-    }
+}
+
+template <int CIN, int COT, int MODE, typename Join>
+__device__ __forceinline__ void conv_tile(const ConvArgs& a, int b, int ty0, int tx0, int co0, bf16* sIn, int tid,
+                                          Join join) {
+    static_assert(CIN % 16 == 0 && COT % 16 == 0, "channels in multiples of 16");
+    constexpr int SP = CIN + 8;  // padded pixel / weight-row stride in shared memory
+    constexpr int C8 = CIN / 8;
+    bf16* sW = sIn + 100 * SP;  // [9][COT][SP]
+    const int warp = tid >> 5, lane = tid & 31;
     for (int q = tid; q < 100 * C8; q += kConvThreads) {
         const int pix = q / C8, c8 = q - pix * C8;
         const int gy = ty0 - 1 + pix / 10, gx = tx0 - 1 + pix % 10;
@@ -158,8 +153,9 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_kernel(ConvArgs a) {
     for (int i = 0; i < COT / 8; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
     const int j = lane >> 3, i8 = lane & 7;
     cp_async_wait<0>();
-    __syncthreads();
-#pragma unroll 1
+    join();
+    constexpr int kTaps = CIN * COT <= 256 ? 9 : CIN * COT <= 1024 ? 3 : 1;  // about nine 16 x 16 steps at a time
+#pragma unroll kTaps
     for (int tap = 0; tap < 9; tap++) {
         const int dy = tap / 3, dx = tap - 3 * (tap / 3);
         const bf16* sWt = sW + tap * COT * SP;
@@ -233,6 +229,23 @@ __global__ void __launch_bounds__(kConvThreads) conv3x3_kernel(ConvArgs a) {
             }
         }
     }
+}
+
+// One tile per block.  Grid: (ceil(W/8), ceil(H/8) * B, w_rows / COT).
+template <int CIN, int COT, int MODE>
+__global__ void __launch_bounds__(kConvThreads) conv3x3_kernel(ConvArgs a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    bf16* sIn = reinterpret_cast<bf16*>(smem_raw);
+    const int tiles_y = (a.H + 7) >> 3, b = blockIdx.y / tiles_y, co0 = blockIdx.z * COT;
+    pdl_trigger();
+    conv_weights<CIN, COT>(a, co0, sIn, threadIdx.x);
+    pdl_wait();
+    if (a.skip && *a.skip) {
+        cp_async_wait<0>();
+        return;
+    }
+    conv_tile<CIN, COT, MODE>(a, b, (blockIdx.y - b * tiles_y) * 8, blockIdx.x * 8, co0, sIn, threadIdx.x,
+                              [] { __syncthreads(); });
 }
 
 struct WgradArgs {

@@ -504,7 +504,9 @@ typedef struct pg_learned_stats {
     int32_t network_off_at;      /* iteration after which the network was switched off, or -1 */
     int32_t replacements;        /* FP64 true-residual recomputations */
     int32_t pdl;                 /* 1 when the solve graph's kernels use programmatic dependent
-                                    launch (each starts while its predecessor finishes) */
+                                    launch (each starts while its predecessor finishes); 0 without,
+                                    and where the solve is one persistent kernel (the network's
+                                    mode up to about 272 x 272 pixels) */
 } pg_learned_stats;
 
 /* Flexible PCG (Polak-Ribiere) with the two-level preconditioner
