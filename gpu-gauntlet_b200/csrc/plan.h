@@ -4,16 +4,15 @@
 // launch: nodes sorted by y are cut into R strips (R ~ sqrt(G * height /
 // width)), and each strip, sorted by x, into its share of the G blocks, so
 // parts are near-square for any G and any node cloud.  A part owns its
-// nodes.  Its work items ("tasks") are the (element, owned node) incidences:
-// a task computes the node's 3 rows of Ke u_e.  Tasks are ordered node by
-// node, so a node's K u is the sum of a contiguous run of task results (an
-// owner-computes gather: no scatter, no atomics, fixed summation order).
+// nodes and the rows of K that belong to them, stored as assembled 3x3 node
+// blocks in groups of rows (rows.cuh): no scatter, no atomics, fixed summation
+// order.  The (element, owned node) incidences of the rows ("tasks") are
+// listed for the plan inspection only.
 // Nodes of a part's elements that it does not own are its ghosts (ring 1);
 // with rings = 2 the nodes of the elements around ring-1 nodes that are in
-// neither set form ring 2, and ring-1 nodes get tasks too (the polynomial
+// neither set form ring 2, and ring-1 nodes get rows too (the polynomial
 // smoother needs K t on owned and ring-1 rows).  Local numbering: owned
-// nodes, then ring 1, then ring 2; tasks: owned nodes' tasks, then ring-1
-// nodes' tasks.
+// nodes, then ring 1, then ring 2; rows and tasks in the same order.
 #pragma once
 
 #include <cstdint>
@@ -97,9 +96,7 @@ std::string build_coarse_meta(const pg_problem& p, HostPlan& plan);
 // Team schedule of a batch of independent plates.  A plate of n nodes gets
 // a team of d blocks: a power of two, or every block of the device for the
 // largest plates, with at most caps[i] nodes per block (so its parts fit in
-// shared memory) and about part_nodes (default 400) nodes per block otherwise (fewer blocks
-// per plate cost less block time, since an iteration's latency hardly
-// depends on the part size).  Team sizes that fit side by side form a
+// shared memory) and about part_nodes nodes per block otherwise (the caller's preference).  Team sizes that fit side by side form a
 // phase, one persistent launch; inside a phase the blocks are shared out
 // among the team sizes in proportion to their estimated work (sqrt(n)
 // iterations of n + 300 d node-equivalents), one team per size at least,

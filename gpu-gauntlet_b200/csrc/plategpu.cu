@@ -153,7 +153,7 @@ struct Plan {
     bool has_elem_t = false;
     DevBuf<int> node_off, nown, nodes, inc_ptr, inc_idx, n1;
     double lambda_max = 0;  // of D^-1 K, for the polynomial smoother (0 = not estimated)
-    bool setup_done = false;  // element matrices, block inverses and task blocks queued
+    bool setup_done = false;  // element matrices, block inverses and row blocks queued
     // exchange buffers: tags up to tag0 may sit in them (valid when ll_ready)
     unsigned tag0 = 0;
     bool ll_ready = false;
@@ -364,7 +364,7 @@ int steps_outside(const pg::HostPlan& hp, int threads) {
 }
 
 // Shared-memory layout of a launch of NR load cases: every per-DOF vector
-// and the task results hold NR values per entry; the partial sums 6 per case.
+// and the row products hold NR values per entry; the partial sums 6 per case.
 pg::SmemLayout make_layout_multi(const pg::HostPlan& hp, bool mixed, bool coarse, bool ainv_smem, int NR, int kq) {
     const size_t T = mixed ? 4 : 8, R = NR;
     const size_t nloc = hp.max_nloc, nown = hp.max_nown, n1 = std::max(hp.max_n1, hp.max_nown);
@@ -1139,7 +1139,7 @@ pgi::OperatorView operator_view(Plan* pl) {
     return v;
 }
 
-// Whether the smallest layout of the persistent kernel (element blocks and
+// Whether the smallest layout of the persistent kernel (row blocks and
 // coarse rows in L2) fits one block's shared memory for this plan's parts.
 bool persistent_fits(const pg_ctx* c, const Plan* pl, const pg_options& o) {
     const pg::SmemLayout L = make_layout(pl->hp, solve_threads(o), o.precision == PG_PREC_MIXED, o.smoother == PG_SMOOTHER_CHEBYSHEV,
@@ -1399,9 +1399,8 @@ void zero_info(pg_info* info) {
 namespace {
 
 // Owned nodes per block that the shared-memory layout holds (vectors, block
-// inverses, task results; the Ke blocks then stay in L2): a first guess,
-// checked against each plate's actual layout by build_batch.  DKT nodes
-// carry about 6 element tasks instead of 4.
+// inverses; the row blocks then stay in L2): a first guess, checked against
+// each plate's actual layout by build_batch.
 int batch_capacity(const pg_options& o, int rings, int npe) {
     const bool mixed = o.precision == PG_PREC_MIXED;
     // about 85% of what the layout holds for a 257 x 257-node plate's parts
@@ -1462,7 +1461,7 @@ std::unique_ptr<pg_batch> build_batch(pg_ctx* c, const pg_problem* probs, int co
     for (int i = 0; i < count; i++) {
         caps[i] = batch_capacity(o, rings[i], (int)probs[i].nodes_per_element);
         // a plate too large for the whole device at the first guess gets the
-        // whole device anyway; its layout (element blocks and A_c^-1 rows then
+        // whole device anyway; its layout (row blocks and A_c^-1 rows then
         // possibly in L2, as in a one-plate solve) is checked below
         caps[i] = std::max(caps[i], (nodes[i] + c->sms - 1) / c->sms);
     }

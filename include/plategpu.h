@@ -234,7 +234,7 @@ int pg_solve(pg_ctx* ctx, const pg_problem* prob, const pg_options* opt, double*
  * FP64, infos (optional): [count].  Up to cases_per_launch cases (0 =
  * automatic: the widest of 4 and 2 that fits, else 1; or 1, 2, 4) run in
  * lockstep in one persistent launch: one
- * exchange round per iteration for all of them, each element block read
+ * exchange round per iteration for all of them, each row of K read
  * once for all of them, each case with its own PCG scalars and stop.  The
  * launch runs until its last case stops; each case's info carries that
  * launch's solve_ms.  In mixed precision a residual replacement asked for
@@ -249,7 +249,7 @@ int pg_solve_load_cases(pg_ctx* ctx, const pg_problem* prob, int count, const fl
 /* Device-resident solves.  A plan holds the partition of one mesh and its
  * device copies (nodes, elements, colouring, constraints, material).  The
  * first solve on a plan computes the element stiffness, block-Jacobi and
- * task set-up on the device (they depend only on the plan's own copies, so
+ * row-block set-up on the device (they depend only on the plan's own copies, so
  * later solves reuse them); every pg_plan_solve_device runs the persistent
  * PCG for a new load.  F_dev is
  * a device float [3*node_count], x_dev a device double [3*node_count]; work
