@@ -94,13 +94,14 @@ struct PcgArgs {
     const int* node_off;
     const int* nown;
     const int* nodes;
-    // row blocks (see row_matvec): group offsets of each part, q-step
+    // row blocks (rows.cuh): group offsets of each part, q-step
     // offsets of each group, columns and blocks of each q-step
     const int* grp_off;          // [G+1]
     const int* grp_q;            // [groups+1]
     const uint16_t* rcol;        // [q-steps][30]
     const double* rk64;          // [q-steps][9][30]
     const float* rk32;
+    int w_rigid;                 // 1 (Q4): a translation in w has no stiffness; see rows.cuh
     const double* binv64;        // [Nn][9]
     const float* binv32;         // [Nn][9]
     const uint8_t* cons;         // [3Nn]
@@ -1017,41 +1018,43 @@ struct RowMem {
     const T* kg;          // global: the part's q-steps
 };
 
-// s += q-steps [done, w) of group grp times v (lanes < 30).
+// s += q-steps [done, w) of group grp times v (lanes < 30); w0: see row_steps.
 template <typename T>
-__device__ __forceinline__ void rows_rest(const RowMem<T>& A, const T* __restrict__ v, int grp, int done, T (&s)[3]) {
+__device__ __forceinline__ void rows_rest(const RowMem<T>& A, const T* __restrict__ v, int grp, int done, T w0,
+                                          T (&s)[3]) {
     const int lane = threadIdx.x & 31;
     const int q0 = A.gq[grp], w = A.gq[grp + 1] - q0;
     if (done >= w || lane >= kRowLanes) return;
     const int g0 = A.go[grp];
     const uint16_t* cq = A.col + (q0 + done) * kRowLanes + lane;
     if (g0 >= 0)
-        row_steps<T, T>(v, cq, A.ks + g0 * 9 * kRowLanes + lane, w - done, s);
+        row_steps<T>(v, cq, A.ks + g0 * 9 * kRowLanes + lane, w - done, w0, s);
     else
-        row_steps<T, T>(v, cq, A.kg + (size_t)(q0 + done) * 9 * kRowLanes + lane, w - done, s);
+        row_steps<T>(v, cq, A.kg + (size_t)(q0 + done) * 9 * kRowLanes + lane, w - done, w0, s);
 }
 
-// Component of K v of this lane's DOF in a group whose rows are in registers.
+// Component of K v of this lane's DOF in a group whose rows are in registers
+// (w0: see row_steps).
 template <typename T>
 __device__ __forceinline__ T rows_reg(const RegRows<T>& R, const RowMem<T>& A, const T* __restrict__ v, int grp,
-                                      bool more) {
+                                      bool more, T w0) {
     T s[3] = {T(0), T(0), T(0)};
 #pragma unroll
     for (int q = 0; q < kRegSteps; q++) {
-        const T v0 = v[R.c[q]], v1 = v[R.c[q] + 1], v2 = v[R.c[q] + 2];
+        const T v0 = sizeof(T) == 4 ? v[R.c[q]] - w0 : v[R.c[q]], v1 = v[R.c[q] + 1], v2 = v[R.c[q] + 2];
 #pragma unroll
         for (int r = 0; r < 3; r++)
             s[r] = fma(R.k[9 * q + 3 * r + 2], v2, fma(R.k[9 * q + 3 * r + 1], v1, fma(R.k[9 * q + 3 * r], v0, s[r])));
     }
-    if (more) rows_rest(A, v, grp, kRegSteps, s);
+    if (more) rows_rest(A, v, grp, kRegSteps, w0, s);
     return row_join(s);
 }
 
 // ... in any other group.
 template <typename T>
-__device__ __forceinline__ T rows_mem(const RowMem<T>& A, const T* __restrict__ v, int grp) {
+__device__ __forceinline__ T rows_mem(const RowMem<T>& A, const T* __restrict__ v, int grp, T w0) {
     T s[3] = {T(0), T(0), T(0)};
-    rows_rest(A, v, grp, 0, s);
+    rows_rest(A, v, grp, 0, w0, s);
     return row_join(s);
 }
 
@@ -1314,6 +1317,8 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& a, const int g, unsigned
     }
     __syncthreads();
 
+    // what an FP32 row subtracts from w
+    auto own_w = [&](const T* v, int n) -> T { return MIXED && a.w_rigid && lact && n < nn1 ? v[3 * n] : T(0); };
     // runs f(n, dof, constrained, row of P, component of K v) over this warp's
     // groups below `groups`; resident ones straight from registers
     auto each_row = [&](const T* v, int groups, auto&& f) {
@@ -1321,7 +1326,7 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& a, const int g, unsigned
 #pragma unroll
             for (int j = 0; j < NG; j++) {
                 const int grp = warp + j * nw, n = grp * kRowGroup + li;
-                if (grp < groups) f(n, D[j], ((cbits >> j) & 1u) != 0, Pr[j], rows_reg(R[j], A, v, grp, (more >> j) & 1u));
+                if (grp < groups) f(n, D[j], ((cbits >> j) & 1u) != 0, Pr[j], rows_reg(R[j], A, v, grp, (more >> j) & 1u, own_w(v, n)));
             }
         }
         for (int grp = warp + NG * nw; grp < groups; grp += nw) {
@@ -1331,7 +1336,7 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& a, const int g, unsigned
             const bool c = get_dof(n, live, o);
             Prow pr{0.0, 0.0, false, 0};
             if (COARSE) pr = prow(n, live, c);
-            f(n, o, c, pr, rows_mem(A, v, grp));
+            f(n, o, c, pr, rows_mem(A, v, grp, own_w(v, n)));
         }
     };
     // (P c) at this lane's DOF, lane 3 i + m of a node holding value m of its
@@ -1366,11 +1371,11 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& a, const int g, unsigned
             double sd[3] = {0.0, 0.0, 0.0};
             const int q0 = gq[grp];
             if (lact)
-                row_steps<double, double>(xl, rcol + q0 * kRowLanes + lane,
-                                          a.rk64 + (size_t)(qb + q0) * 9 * kRowLanes + lane, gq[grp + 1] - q0, sd);
+                row_steps<double>(xl, rcol + q0 * kRowLanes + lane, a.rk64 + (size_t)(qb + q0) * 9 * kRowLanes + lane,
+                                  gq[grp + 1] - q0, 0.0, sd);
             return row_join(sd);
         } else {
-            return rows_mem(A, (const T*)xl, grp);
+            return rows_mem(A, (const T*)xl, grp, T(0));
         }
     };
 
@@ -1483,7 +1488,7 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& a, const int g, unsigned
                 if (grp < ngo) {
                     double kx;
                     if constexpr (MIXED) kx = true_row(grp);
-                    else kx = rows_reg(R[j], A, (const T*)xl, grp, (more >> j) & 1u);
+                    else kx = rows_reg(R[j], A, (const T*)xl, grp, (more >> j) & 1u, T(0));
                     const T v = f(n, ((cbits >> j) & 1u) != 0, Pr[j], kx);
                     if (set && lact && n < no) D[j].r = v;
                 }

@@ -44,20 +44,31 @@ struct alignas(sizeof(T) * NR <= 16 ? sizeof(T) * NR : 16) CaseVec {
     T v[NR];
 };
 
+// v -= o, case by case
+template <typename T, int NR>
+__device__ __forceinline__ void case_sub(CaseVec<T, NR>& v, const CaseVec<T, NR>& o) {
+#pragma unroll
+    for (int i = 0; i < NR; i++) v.v[i] -= o.v[i];
+}
+
 // s[r][k] += the blocks of q-steps [0, steps) at b (lane offset included) times
-// case k of u at the columns c.
-template <typename T, typename KT, int NR>
+// case k of u at the columns c, its w less w0 (0, or the row's own w; FP32
+// only).
+template <typename T, int NR>
 __device__ __forceinline__ void row_steps_multi(const T* __restrict__ u, const uint16_t* __restrict__ c,
-                                                const KT* __restrict__ k, int steps, T (&s)[3][NR]) {
+                                                const T* __restrict__ k, int steps, const CaseVec<T, NR>& w0,
+                                                T (&s)[3][NR]) {
     using V = CaseVec<T, NR>;
 #pragma unroll 1
     for (int q = 0; q < steps; q++) {
         const V* v = reinterpret_cast<const V*>(u) + 3 * (int)c[q * kRowLanes];
-        const V v0 = v[0], v1 = v[1], v2 = v[2];
-        const KT* b = k + q * 9 * kRowLanes;
+        V v0 = v[0];
+        const V v1 = v[1], v2 = v[2];
+        if constexpr (sizeof(T) == 4) case_sub(v0, w0);
+        const T* b = k + q * 9 * kRowLanes;
 #pragma unroll
         for (int r = 0; r < 3; r++) {
-            const T k0 = (T)b[3 * r * kRowLanes], k1 = (T)b[(3 * r + 1) * kRowLanes], k2 = (T)b[(3 * r + 2) * kRowLanes];
+            const T k0 = b[3 * r * kRowLanes], k1 = b[(3 * r + 1) * kRowLanes], k2 = b[(3 * r + 2) * kRowLanes];
 #pragma unroll
             for (int i = 0; i < NR; i++) s[r][i] = fma(k2, v2.v[i], fma(k1, v1.v[i], fma(k0, v0.v[i], s[r][i])));
         }
@@ -83,7 +94,7 @@ __device__ __forceinline__ void join_store(const T (&s)[3][NR], T* __restrict__ 
 // first group from registers.
 template <typename T, int NR>
 __device__ __forceinline__ void rows_multi(const RegRows<T>& R, const RowMem<T>& A, const T* __restrict__ u,
-                                           T* __restrict__ y, int nrows) {
+                                           T* __restrict__ y, int nrows, int w_rigid) {
     using V = CaseVec<T, NR>;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int grp = warp; grp * kRowGroup < nrows; grp += nw) {
@@ -92,6 +103,9 @@ __device__ __forceinline__ void rows_multi(const RegRows<T>& R, const RowMem<T>&
         for (int r = 0; r < 3; r++)
 #pragma unroll
             for (int i = 0; i < NR; i++) s[r][i] = T(0);
+        V w0{};
+        const int own = grp * kRowGroup + lane / 3;
+        if (sizeof(T) == 4 && w_rigid && lane < kRowLanes && own < nrows) w0 = reinterpret_cast<const V*>(u)[3 * own];
         const int q0 = A.gq[grp], w = A.gq[grp + 1] - q0;
         int done = 0;
         if (grp == warp) {
@@ -99,7 +113,9 @@ __device__ __forceinline__ void rows_multi(const RegRows<T>& R, const RowMem<T>&
 #pragma unroll
             for (int q = 0; q < kRegSteps; q++) {
                 const V* v = reinterpret_cast<const V*>(u) + R.c[q];
-                const V v0 = v[0], v1 = v[1], v2 = v[2];
+                V v0 = v[0];
+                const V v1 = v[1], v2 = v[2];
+                if constexpr (sizeof(T) == 4) case_sub(v0, w0);
 #pragma unroll
                 for (int r = 0; r < 3; r++)
 #pragma unroll
@@ -112,9 +128,9 @@ __device__ __forceinline__ void rows_multi(const RegRows<T>& R, const RowMem<T>&
             const int g0 = A.go[grp];
             const uint16_t* cq = A.col + (q0 + done) * kRowLanes + lane;
             if (g0 >= 0)
-                row_steps_multi<T, T, NR>(u, cq, A.ks + g0 * 9 * kRowLanes + lane, w - done, s);
+                row_steps_multi<T, NR>(u, cq, A.ks + g0 * 9 * kRowLanes + lane, w - done, w0, s);
             else
-                row_steps_multi<T, T, NR>(u, cq, A.kg + (size_t)(q0 + done) * 9 * kRowLanes + lane, w - done, s);
+                row_steps_multi<T, NR>(u, cq, A.kg + (size_t)(q0 + done) * 9 * kRowLanes + lane, w - done, w0, s);
         }
         join_store<T, NR>(s, y, grp, nrows);
     }
@@ -134,8 +150,8 @@ __device__ __forceinline__ void rows_multi64(const int* __restrict__ gq, const u
             for (int i = 0; i < NR; i++) s[r][i] = 0.0;
         const int q0 = gq[grp];
         if (lane < kRowLanes)
-            row_steps_multi<double, double, NR>(u, col + q0 * kRowLanes + lane, kg + (size_t)q0 * 9 * kRowLanes + lane,
-                                                gq[grp + 1] - q0, s);
+            row_steps_multi<double, NR>(u, col + q0 * kRowLanes + lane, kg + (size_t)q0 * 9 * kRowLanes + lane,
+                                        gq[grp + 1] - q0, CaseVec<double, NR>{}, s);
         join_store<double, NR>(s, y, grp, nrows);
     }
 }
@@ -460,7 +476,7 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
         for (int d = 0; d < 3; d++) u[(3 * n + d) * NR + kc] = uv[d];
     };
     if (cheb) {
-        rows_multi<T, NR>(R, A, u, yt, nn1);
+        rows_multi<T, NR>(R, A, u, yt, nn1, a.w_rigid);
         __syncthreads();
         for (int q = tid; q < nn1 * NR; q += nt) smooth(q / NR);
         __syncthreads();
@@ -515,7 +531,7 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
 
     for (int it = 0; status == ST_OK; it++) {
         // ---- w = A u on owned rows, every case ----
-        rows_multi<T, NR>(R, A, u, yt, no);
+        rows_multi<T, NR>(R, A, u, yt, no, a.w_rigid);
         __syncthreads();
         clk.lap(0);
         // ---- BC rows, dot products, publish w ----
@@ -738,7 +754,7 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
             }
             if (cheb) {
                 __syncthreads();
-                rows_multi<T, NR>(R, A, u, yt, nn1);
+                rows_multi<T, NR>(R, A, u, yt, nn1, a.w_rigid);
                 __syncthreads();
                 for (int q = tid; q < nn1 * NR; q += nt) {
                     const int n = q / NR;
@@ -841,7 +857,7 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
         __syncthreads();
         clk.lap(7);
         if (cheb) {
-            rows_multi<T, NR>(R, A, u, yt, nn1);
+            rows_multi<T, NR>(R, A, u, yt, nn1, a.w_rigid);
             __syncthreads();
             clk.lap(3);
             for (int q = tid; q < nn1 * NR; q += nt) {
@@ -888,7 +904,7 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
             if constexpr (MIXED)
                 rows_multi64<NR>(gq, rcol, kg64, xl, ytd, no);
             else
-                rows_multi<T, NR>(R, A, xl, ytd, no);
+                rows_multi<T, NR>(R, A, xl, ytd, no, a.w_rigid);
             __syncthreads();
             double v2[2] = {0.0, 0.0};
             for (int q = tid; q < no * NR; q += nt) {

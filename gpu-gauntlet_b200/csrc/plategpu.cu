@@ -856,6 +856,7 @@ pg::PcgArgs fill_args(Plan* pl, const pg_options& o, const pg::SmemLayout& L, bo
     a.rcol = pl->rcol.p;
     a.rk64 = pl->rk64.p;
     a.rk32 = pl->rk32.p;
+    a.w_rigid = hp.npe == 4 ? 1 : 0;
     a.binv64 = pl->binv64.p;
     a.binv32 = pl->binv32.p;
     a.cons = pl->cons.p;

@@ -24,6 +24,19 @@
 // 60k-DOF plate read no coefficients at all; a lane reads u of a slot's node
 // once for three components (9 loads a lane where a thread per component
 // needs 27).
+//
+// FP32 rows of Q4 plates multiply w's difference to the row's own node.  A
+// translation in w has no stiffness there (sum_m K_nm e_w = 0: the shape
+// functions' gradients sum to zero), so for a smooth u the products with w are
+// large and cancel: rounded to FP32 their sum had 1.6 times the error of the
+// element form (lowest mode of a clamped 141 x 141 plate: 7.4e-2 of |K u|), and
+// mixed solves that converged with the element form stagnated.
+// sum_m K_nm (w_m - w_n, thx_m, thy_m) is the same sum, its differences are
+// almost exact, and its error there is 1.0e-3.  Cost, a load and three
+// subtractions a lane: not measurable (mixed two-level Chebyshev on the 60k-DOF
+// plate 1.53 -> 1.50 ms a solve).  FP64 rows keep the plain form, FP64 has the
+// digits; so do DKT rows: the reference's element, which this one restates, does
+// have stiffness in a translation (and few iterations).
 #pragma once
 
 #include <cstdint>
@@ -127,19 +140,19 @@ __global__ void mark_ghosts_kernel(const int* __restrict__ node_off, const int* 
 }
 
 // s += the blocks k[9 (q - qa) ..][lane] of q-steps [qa, qb) times u at the
-// columns c[q - qa][lane].
-template <typename T, typename KT>
+// columns c[q - qa][lane], its w less w0 (0, or the row's own w; FP32 only).
+template <typename T>
 __device__ __forceinline__ void row_steps(const T* __restrict__ u, const uint16_t* __restrict__ c,
-                                          const KT* __restrict__ k, int steps, T (&s)[3]) {
+                                          const T* __restrict__ k, int steps, T w0, T (&s)[3]) {
 #pragma unroll 3
     for (int q = 0; q < steps; q++) {
         const T* v = u + 3 * (int)c[q * kRowLanes];
-        const T v0 = v[0], v1 = v[1], v2 = v[2];
-        const KT* b = k + q * 9 * kRowLanes;
+        const T v0 = sizeof(T) == 4 ? v[0] - w0 : v[0], v1 = v[1], v2 = v[2];
+        const T* b = k + q * 9 * kRowLanes;
 #pragma unroll
         for (int r = 0; r < 3; r++)
-            s[r] = fma((T)b[(3 * r + 2) * kRowLanes], v2,
-                       fma((T)b[(3 * r + 1) * kRowLanes], v1, fma((T)b[3 * r * kRowLanes], v0, s[r])));
+            s[r] = fma(b[(3 * r + 2) * kRowLanes], v2,
+                       fma(b[(3 * r + 1) * kRowLanes], v1, fma(b[3 * r * kRowLanes], v0, s[r])));
     }
 }
 
