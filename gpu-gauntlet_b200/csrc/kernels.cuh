@@ -133,7 +133,10 @@ struct PcgArgs {
     const float* ainv32;        // [rows][C]
     int ainv_smem;
     int reliable_interval;
-    int stall_limit;            // replacements without halving the FP64 residual: stagnated
+    // stagnated: replacements without halving the FP64 residual, one that the
+    // interval brought counted once and one that the residual asked for
+    // stall_step times, reach stall_limit
+    int stall_limit, stall_step;
     double reliable_delta;
     // polynomial smoother (smoother = 1; needs a plan with a 2-ring halo):
     // u = a D^-1 r - b D^-1 K D^-1 r (the degree-2 Chebyshev step for
@@ -1068,7 +1071,7 @@ struct Decision {
     double thr_check;         // rho at or below it needs the full tests
     double thr_abs, thr_rel, thr_ru, bnorm, best_trn, final_res, true_rel;
     int xupd, xupd_ref, nru;  // updates, at the last replacement, replacements
-    int stall;                // replacements since the FP64 residual last halved
+    int stall;                // replacements since the FP64 residual last halved (stall_step)
     int stop, first;
 };
 
@@ -1721,6 +1724,7 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& a, const int g, unsigned
                 dec->nru++;
                 dec->thr_ru = a.reliable_delta * trn * (a.reliable_delta * trn);
                 dec->thr_check = fmax(fmax(dec->thr_abs, dec->thr_rel), dec->thr_ru);
+                const int stalled = dec->xupd - dec->xupd_ref >= a.reliable_interval ? 1 : a.stall_step;
                 dec->xupd_ref = dec->xupd;
                 if (!isfinite(trn)) {
                     ctl[0] = ACT_NONFINITE;
@@ -1731,7 +1735,7 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& a, const int g, unsigned
                 } else if (trn < 0.5 * dec->best_trn) {
                     dec->best_trn = trn;
                     dec->stall = 0;
-                } else if (++dec->stall >= a.stall_limit) {
+                } else if ((dec->stall += stalled) >= a.stall_limit) {
                     // that many replacements in a row without halving the FP64
                     // residual: the FP32 inner iterations no longer reduce
                     // the error (condition number near 1 / FP32 epsilon)

@@ -772,6 +772,7 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
                 const bool me = lane < NR;
                 if (me && !cs.done) {
                     const double trn = sqrt(scal[lane]);
+                    const int stalled = cs.xupd - cs.xupd_ref >= a.reliable_interval ? 1 : a.stall_step;
                     if (cs.asked) {
                         cs.nru++;
                         cs.rn_ref = trn;
@@ -789,9 +790,9 @@ __device__ __forceinline__ void pcg_multi_body(const PcgArgs& a, const int g, un
                     } else if (trn < 0.5 * cs.best_trn) {
                         cs.best_trn = trn;
                         cs.stall = 0;
-                    } else if (++cs.stall >= 3) {
-                        // three of its own replacements without halving the FP64
-                        // residual: the FP32 inner iterations stopped helping
+                    } else if ((cs.stall += stalled) >= a.stall_limit) {
+                        // its own replacements without halving the FP64 residual:
+                        // the FP32 inner iterations stopped helping
                         cs.stop = STOP_STAGNATED; cs.final_res = trn; cs.true_rel = trn / cs.bnorm; cs.done = true;
                     }
                 }

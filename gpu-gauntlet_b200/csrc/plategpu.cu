@@ -892,12 +892,15 @@ pg::PcgArgs fill_args(Plan* pl, const pg_options& o, const pg::SmemLayout& L, bo
     // automatic: a replacement at least every 200 updates, so a mixed solve
     // whose FP32 residual stalls along with the true one is still checked
     // (with the coarse space after 50: its FP32 recurrence drifts sooner, and with
-    // reliable_delta = 0.01 the 60k-DOF plate stagnated at 200, 1.2 -> 6.2 ms)
-    a.reliable_interval = o.reliable_interval > 0                      ? o.reliable_interval
-                          : o.preconditioner == PG_PRECOND_TWO_LEVEL ? 50
-                                                                     : 200;
+    // reliable_delta = 0.01 the 60k-DOF plate stagnated at 200, 1.2 -> 6.2 ms).
+    // Either gives up after 600 updates without halving the true residual, or
+    // three replacements that the FP32 residual asked for: a thin clamped plate's
+    // residual may stay flat for some hundred updates and then fall.
+    const bool often = o.reliable_interval <= 0 && o.preconditioner == PG_PRECOND_TWO_LEVEL;
+    a.reliable_interval = o.reliable_interval > 0 ? o.reliable_interval : often ? 50 : 200;
     a.reliable_delta = o.reliable_delta > 0 ? o.reliable_delta : 0.1;
-    a.stall_limit = 3;
+    a.stall_step = often ? 4 : 1;
+    a.stall_limit = 3 * a.stall_step;
     a.L = L;
     return a;
 }
@@ -977,10 +980,10 @@ const void* batch_kernel_of(bool coarse, bool cheb) {
 // Queues set-up (first solve of the plan) and the persistent PCG launch on
 // the context stream, then waits for the result record (one readback).
 // x_dst (optional) receives the solution by a copy of `kind` queued right
-// behind the kernel, so the call waits for the device once.  stall_limit:
-// residual replacements without halving that end a mixed solve.
+// behind the kernel, so the call waits for the device once.  stall_limit (0 =
+// fill_args'): residual replacements without halving that end a mixed solve.
 void run_solve(pg_ctx* c, Plan* pl, const pg_options& o, pg_info* info, void* x_dst = nullptr,
-               cudaMemcpyKind kind = cudaMemcpyDeviceToDevice, int stall_limit = 3) {
+               cudaMemcpyKind kind = cudaMemcpyDeviceToDevice, int stall_limit = 0) {
     const pg::HostPlan& hp = pl->hp;
     const int threads = solve_threads(o);
     const bool lean = threads <= pg::kLeanThreads;
@@ -994,7 +997,10 @@ void run_solve(pg_ctx* c, Plan* pl, const pg_options& o, pg_info* info, void* x_
     reset_for_launch(c, pl, pl->res.p);
     CK(cudaMemsetAsync(pl->abort_flag.p, 0, sizeof(int), c->stream));
     pg::PcgArgs a = fill_args(pl, o, L, ainv_smem, pl->abort_flag.p, pl->res.p);
-    a.stall_limit = stall_limit;
+    if (stall_limit > 0) {
+        a.stall_limit = stall_limit;
+        a.stall_step = 1;
+    }
     if (a.trace_it > 0)
         CK(cudaMemsetAsync(pl->trace.p, 0, pl->trace.n * sizeof(unsigned long long), c->stream));
 

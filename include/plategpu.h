@@ -123,7 +123,8 @@ typedef struct pg_options {
     int32_t threads;              /* threads per CTA; 0 = automatic */
     double wait_timeout_ms;       /* limit on each wait for another block's data; default 1000 */
     int32_t reliable_interval;    /* mixed: max inner iterations between FP64
-                                     residual replacements; 0 = automatic (200) */
+                                     residual replacements; 0 = automatic (200, with the
+                                     two-level preconditioner 50) */
     double reliable_delta;        /* mixed: replace when the FP32 residual fell
                                      by this factor; 0 = automatic (0.1) */
     int32_t phase_timing;         /* 1: record per-phase device time (pg_info.phase_us) */
