@@ -180,8 +180,8 @@ struct Plan {
     // for the coarse-space arrays
     DevBuf<unsigned char> arena, coarse_arena;
     // load cases solved together (NR cases per launch): their loads,
-    // solutions, exchange buffers and result records
-    int m_nr = 0;
+    // solutions, exchange buffers and result records, for the widest launch so far
+    int m_cap = 0;
     unsigned m_tag0 = 0;
     bool m_ready = false;
     const void* m_ok_fn = nullptr;
@@ -1260,15 +1260,20 @@ void run_solve_multi(pg_ctx* c, Plan* pl, const pg_options& o, int NR, int count
     if (!choose_layout_multi(c, hp, o, NR, &ainv_smem, &L))
         throw Fail{PG_EUNSUPPORTED, "load-case partition too large for shared memory"};
     cudaStream_t st = c->stream;
-    if (pl->m_nr != NR) {
+    // grown and kept: a call of 4 + 2 cases would else free and allocate twice,
+    // 2.9 ms of its 9.4.  A narrower launch uses the front; each exchange word
+    // carries its tag, and the tags go on over all widths, so words of another
+    // layout never match
+    if (pl->m_cap < NR) {
+        pl->m_cap = 0;  // until every array is there
+        pl->m_ready = false;
         pl->mF.alloc(n * NR);
         pl->mx.alloc(n * NR);
         pl->mllv.alloc(2 * n * NR * 2);
         pl->mllx.alloc(n * NR * 2);
         pl->mllp.alloc(2 * (size_t)pg::kRep * pl->G * pg::multi_slot_words<4>() + 2);
         pl->mres.alloc(NR);
-        pl->m_nr = NR;
-        pl->m_ready = false;
+        pl->m_cap = NR;
     }
     ensure_staging(c, n * NR);
     for (int k = 0; k < NR; k++) {
