@@ -1081,7 +1081,7 @@ double correction_tolerance(const pg_options& o, double bnorm, double r0) {
 }
 
 bool persistent_fits(const pg_ctx* c, const Plan* pl, const pg_options& o);
-void global_solve(pg_ctx* c, Plan* pl, const pg_options& o, pg_info* info, void* x_dst, cudaMemcpyKind kind);
+void global_solve_after(pg_ctx* c, Plan* pl, const pg_options& o, pg_info* fi, void* x_dst, cudaMemcpyKind kind);
 
 // After a mixed solve of pl stagnated (pl->x holds its x_m, pl->F the
 // load): solves K d = F - K x_m in FP64, its load the FP32-rounded residual
@@ -1101,10 +1101,8 @@ void fp64_correction(pg_ctx* c, Plan* pl, const pg_options& o, pg_info* mi, void
     if (!persistent_fits(c, pl, o64)) {
         // FP64 state does not fit shared memory: the whole solve again on the
         // global-memory path
-        const double mixed_ms = mi->setup_ms + mi->solve_ms;
-        global_solve(c, pl, o, mi, x_dst, kind);
+        global_solve_after(c, pl, o, mi, x_dst, kind);
         mi->fallback = 1;
-        mi->solve_ms += mixed_ms;
         return;
     }
     if (pl->xw.n != n) pl->xw.alloc(n);
@@ -1186,6 +1184,17 @@ void global_solve(pg_ctx* c, Plan* pl, const pg_options& o, pg_info* info, void*
     fi->global_path = 1;
 }
 
+// global_solve after an attempt that gave up, whose record is in fi: the
+// attempt's time and the plan's set-up times stay, the rest of it goes.
+void global_solve_after(pg_ctx* c, Plan* pl, const pg_options& o, pg_info* fi, void* x_dst, cudaMemcpyKind kind) {
+    const double ms = fi->setup_ms + fi->solve_ms, coarse_ms = fi->coarse_ms, eigen_ms = fi->eigen_ms;
+    *fi = pg_info{};
+    global_solve(c, pl, o, fi, x_dst, kind);
+    fi->solve_ms += ms;
+    fi->coarse_ms = coarse_ms;
+    fi->eigen_ms = eigen_ms;
+}
+
 void solve_with_fallback(pg_ctx* c, Plan* pl, const pg_options& o, pg_info* info, void* x_dst = nullptr,
                          cudaMemcpyKind kind = cudaMemcpyDeviceToDevice) {
     pg_info local{};
@@ -1195,22 +1204,29 @@ void solve_with_fallback(pg_ctx* c, Plan* pl, const pg_options& o, pg_info* info
         // FP32 vectors in the persistent kernel, where those fit (FP64 x, dot
         // products and true-residual stop, as on the global-memory path that
         // takes what is left: larger plates, the 2-ring halo, and solves that
-        // FP32 stalls).  The two-level solve replaces its residual as often as
-        // that path, every 50 updates: with 200 the FP32 residual of a plate this
-        // large drifts and the solve stalls, with 50 none did (plates of 380 to
-        // 420 elements a side, two seeds each).  Block Jacobi, whose residual stays
-        // flat for hundreds of updates, keeps 200; either gives up after 800
-        // updates without halving the true residual.  482k-DOF plate, 1e-8:
+        // FP32 stalls, breaks down or overflows).  The two-level solve replaces its
+        // residual every 50 updates, block Jacobi, whose residual stays flat for
+        // hundreds of updates, every 200; either gives up after 800 updates
+        // without halving the true residual.  The request is for FP64, so the
+        // caller's reliable_* of mixed solves have no say.  482k-DOF plate, 1e-8:
         // two-level 144 -> 25 ms (1,230 iterations instead of 2,949 of two
         // smoothing steps), block Jacobi 194 -> 58 ms
-        pg_options om = o;
-        om.precision = PG_PREC_MIXED;
-        const int ri = o.preconditioner == PG_PRECOND_TWO_LEVEL ? 50 : 200;
-        if (om.reliable_interval <= 0) om.reliable_interval = ri;
-        if (pl->G >= c->sms && o.precision == PG_PREC_FP64 && persistent_fits(c, pl, om)) {
-            run_solve(c, pl, om, fi, x_dst, kind, std::max(3, 800 / ri));
-            fi->global_path = 1;
-            if (fi->stop_reason != PG_STOP_STAGNATED) return;
+        if (pl->G >= c->sms && o.precision == PG_PREC_FP64) {
+            pg_options om = o;
+            om.precision = PG_PREC_MIXED;
+            om.reliable_interval = o.preconditioner == PG_PRECOND_TWO_LEVEL ? 50 : 200;
+            om.reliable_delta = 0.0;
+            if (persistent_fits(c, pl, om)) {
+                try {
+                    run_solve(c, pl, om, fi, x_dst, kind, 800 / om.reliable_interval);
+                    fi->global_path = 1;
+                    if (fi->stop_reason != PG_STOP_STAGNATED && fi->stop_reason != PG_STOP_BREAKDOWN) return;
+                } catch (const Fail& f) {
+                    if (f.status != PG_ENONFINITE) throw;
+                }
+                global_solve_after(c, pl, o, fi, x_dst, kind);
+                return;
+            }
         }
         global_solve(c, pl, o, fi, x_dst, kind);
         return;
