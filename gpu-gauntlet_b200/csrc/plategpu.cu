@@ -297,16 +297,16 @@ void largest_rows(const pg::HostPlan& hp, int* groups, int* steps) {
 
 // Shared memory of one block of the one-plate and batch kernels: the part's
 // vectors (u, w and t of every local node, the rest of the nodes that are not
-// resident), its row columns and kq staged q-steps of row blocks.
+// resident), its row columns and kq staged q-steps of row blocks.  kagg: the
+// most aggregates a part touches (0: the coarse space's own).
 pg::SmemLayout make_layout(const pg::HostPlan& hp, int threads, bool mixed, bool cheb, bool coarse, bool ainv_smem,
-                           int kq) {
+                           int kq, int kagg_guess = 0) {
     const size_t T = mixed ? 4 : 8, res = (size_t)pg::kRowGroup * resident_groups(threads);
     const size_t nloc = hp.max_nloc;
     const size_t xloc = nloc - std::min<size_t>(nloc, res);                            // not resident
     int groups = 0, steps = 0;
     largest_rows(hp, &groups, &steps);
-    // before the coarse space is built: every aggregate a block could touch, up to 25
-    const size_t C = 3 * (size_t)hp.G, kagg = hp.max_kagg ? hp.max_kagg : std::min(hp.G, 25);
+    const size_t C = 3 * (size_t)hp.G, kagg = kagg_guess ? kagg_guess : hp.max_kagg;
     size_t off = 0;
     auto take = [&](size_t bytes) {
         const size_t o = off;
@@ -660,6 +660,13 @@ void fill_options(const pg_options* in, pg_options* o) {
 // polynomial smoother, else 1.
 int halo_rings(const pg_options& o) { return o.smoother == PG_SMOOTHER_CHEBYSHEV ? 2 : 1; }
 
+// The host part of the coarse space, once per plan.
+void build_meta(Plan* pl) {
+    if (pl->hp.max_kagg) return;
+    const std::string e = pg::build_coarse_meta(pl->prob_view, pl->hp);
+    if (!e.empty()) throw Fail{PG_EINVAL, e};
+}
+
 // Coarse data of the two-level preconditioner, built once per plan: the
 // aggregate lists and basis data on the host (build_coarse_meta), A_c = P^T K P,
 // its inverse and each part's A_c^-1 rows on the device (coarse.cuh), from the
@@ -668,8 +675,7 @@ int halo_rings(const pg_options& o) { return o.smoother == PG_SMOOTHER_CHEBYSHEV
 void queue_coarse(pg_ctx* c, Plan* pl) {
     pg::HostPlan& hp = pl->hp;
     run_setup(c, pl);
-    std::string e = pg::build_coarse_meta(pl->prob_view, hp);
-    if (!e.empty()) throw Fail{PG_EINVAL, e};
+    build_meta(pl);
     cudaStream_t st = c->stream;
     const int C = hp.C;
     const size_t CC = (size_t)C * C;
@@ -1080,7 +1086,7 @@ double correction_tolerance(const pg_options& o, double bnorm, double r0) {
     return r0 > 0 ? std::min(0.5, target / r0) : o.tolerance;
 }
 
-bool persistent_fits(const pg_ctx* c, const Plan* pl, const pg_options& o);
+bool persistent_fits(const pg_ctx* c, Plan* pl, const pg_options& o);
 void global_solve_after(pg_ctx* c, Plan* pl, const pg_options& o, pg_info* fi, void* x_dst, cudaMemcpyKind kind);
 
 // After a mixed solve of pl stagnated (pl->x holds its x_m, pl->F the
@@ -1149,12 +1155,24 @@ pgi::OperatorView operator_view(Plan* pl) {
 }
 
 // Whether the smallest layout of the persistent kernel (row blocks and
-// coarse rows in L2) fits one block's shared memory for this plan's parts.
-bool persistent_fits(const pg_ctx* c, const Plan* pl, const pg_options& o) {
-    const pg::SmemLayout L = make_layout(pl->hp, solve_threads(o), o.precision == PG_PREC_MIXED, o.smoother == PG_SMOOTHER_CHEBYSHEV,
-                                          o.preconditioner == PG_PRECOND_TWO_LEVEL, false, 0);
-    return L.total <= c->max_smem;
+// coarse rows in L2) fits one block's shared memory for this plan's parts, with
+// `threads` threads.  The answer is the same before and after the coarse space is
+// built: how many aggregates a part touches (9 on a regular grid, any number up
+// to G) is counted where it decides.
+bool persistent_fits(const pg_ctx* c, Plan* pl, const pg_options& o, int threads) {
+    const bool coarse = o.preconditioner == PG_PRECOND_TWO_LEVEL;
+    auto fits = [&](int kagg) {
+        return make_layout(pl->hp, threads, o.precision == PG_PREC_MIXED, o.smoother == PG_SMOOTHER_CHEBYSHEV, coarse,
+                           false, 0, kagg).total <= c->max_smem;
+    };
+    if (coarse && !pl->hp.max_kagg) {
+        if (fits(pl->G)) return true;
+        if (!fits(1)) return false;
+        build_meta(pl);
+    }
+    return fits(0);
 }
+bool persistent_fits(const pg_ctx* c, Plan* pl, const pg_options& o) { return persistent_fits(c, pl, o, solve_threads(o)); }
 
 // A plate whose parts do not fit shared memory even with one part per SM:
 // flexible PCG over global memory (FP32 vectors in L2/HBM, FP64 x, dot
@@ -1508,12 +1526,9 @@ std::unique_ptr<pg_batch> build_batch(pg_ctx* c, const pg_problem* probs, int co
         for (int i = 0; i < count; i++) {
             const int G = b->sched.plate_size[i];
             b->plans.push_back(build_plan(c, probs[i], G, rings[i]));
-            bool ainv = false;
-            try {
-                const pg::HostPlan& hp = b->plans.back()->hp;
-                choose_layout(c, hp, plate_options(o, b->plans.back().get()), pg::kBatchThreads, &ainv);
-                if (rings[i] == 2 && !smoother_halo_fits(c, hp, o)) throw Fail{PG_EUNSUPPORTED, "halo"};
-            } catch (const Fail&) {
+            Plan* pl = b->plans.back().get();
+            if (!persistent_fits(c, pl, plate_options(o, pl), pg::kBatchThreads) ||
+                (rings[i] == 2 && !smoother_halo_fits(c, pl->hp, o))) {
                 fits = false;
                 if (rings[i] == 2 && G == c->sms) {
                     // the 2-ring halo does not fit even on the whole device:
