@@ -1910,6 +1910,7 @@ struct FpcgSolver {
     float omega = 1.f;
     Buf<float> F, r, r_prev, r1, y, r2, z, p0, p1, q, y2, v2, t;
     Buf<double> x, parts;
+    int part_blocks = 0;
     Buf<int> nm_off, nm_col;  // node-block form of the operator (op.nm_*)
     Buf<float> nm_val;
     Buf<FState> st;
@@ -2095,7 +2096,10 @@ void fpcg_init(FpcgSolver* S, pg_ctx* c, const Op& op, int npe, float omega) {
     }
     S->x.alloc(n3);
     S->op.tpn = op.Nn < kTwoThreadNodes ? 2 : 1;
-    S->parts.alloc(14 * (size_t)grid_nodes(op.Nn, S->op.tpn));
+    // the blocks whose partial sums the arrays hold: the graph's kernels', or the
+    // persistent kernel's (at most one a SM)
+    S->part_blocks = std::max(grid_nodes(op.Nn, S->op.tpn), pgi::ctx_sms(c));
+    S->parts.alloc(14 * (size_t)S->part_blocks);
     S->st.alloc(1);
     LCK(cudaStreamCreateWithFlags(&S->cap, cudaStreamNonBlocking));
     build_node_blocks(S, st);
@@ -2190,13 +2194,14 @@ FArgs make_fargs(FpcgSolver* S, const pg_options& o, int mode, pg_net* n, Worksp
     a.p1 = S->p1.p;
     a.q = S->q.p;
     double* P = S->parts.p;
+    const int B = S->part_blocks;
     a.pU = P;
-    a.pTR = P + 2 * G;
-    a.pA = P + 4 * G;
-    a.pB = P + 6 * G;
-    a.pC = P + 8 * G;
-    a.pD = P + 10 * G;
-    a.pI = P + 12 * G;
+    a.pTR = P + 2 * B;
+    a.pA = P + 4 * B;
+    a.pB = P + 6 * B;
+    a.pC = P + 8 * B;
+    a.pD = P + 10 * B;
+    a.pI = P + 12 * B;
     a.st = S->st.p;
     a.G = G;
     a.tol2 = o.tolerance * o.tolerance;
@@ -2295,8 +2300,18 @@ void persist_launch(FpcgSolver* S, const pg_options& o, pg_net* n, const int* no
     LCK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, pa.smem));
     LCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, kPersistThreads, pa.smem));
     if (nb < 1) throw LFail{PG_EUNSUPPORTED, "the learned solve's grid does not fit on the device"};
-    // the partials' arrays hold grid_nodes blocks' sums each; no more blocks than that
-    const int grid = std::min(sms, pa.f.G);
+    // as many blocks as the nodes or the widest layer's tiles fill: a plate of few
+    // nodes may sit in a large image (33 x 33 nodes in 144 x 144 pixels, us per
+    // iteration: blocks for the nodes alone 387, with the tiles' 103; in
+    // 272 x 272 1,122 and 168; 8 x 8 nodes in 16 x 16 120 and 71)
+    int grid = pa.f.G;
+    for (int k = 0; k < pgn::kLayers; k++) {
+        const pgn::ConvArgs& a = pa.conv[k];
+        const int tiles = ((a.W + 7) / 8) * ((a.H + 7) / 8) * (a.w_rows / 16);
+        const int groups = std::min(kPersistThreads / pgn::kConvThreads, pa.smem / pgn::conv_smem_bytes(n->T.l[k].cin, 16));
+        grid = std::max(grid, (tiles + groups - 1) / groups);
+    }
+    grid = std::min(grid, sms);
     if (S->bar.n != 2) S->bar.alloc(2);
     S->bar.zero(st);
     pa.bar = S->bar.p;
