@@ -2427,7 +2427,7 @@ void fpcg_run(FpcgSolver* S, const pg_options& o, int mode, pg_net* n, const int
         ls->network_off_at = s.net_off ? s.net_off_at : -1;
         ls->replacements = s.replacements;
         ls->mode = mode;
-        ls->pdl = mode == 1 ? 0 : S->pdl;
+        ls->pdl = persist ? 0 : S->pdl;
     }
 }
 
