@@ -1484,11 +1484,17 @@ __global__ void fp_dir_kernel(FArgs a) {
 
 constexpr int kPersistThreads = 512;
 
+// The arrivals wrap around in a long solve (after 29M barriers of 148 blocks, 1.4M
+// iterations with the network), so they are compared by their difference; blocks
+// are at most one barrier apart.  The count starts just below the wrap, so that
+// every solve passes it.
+constexpr unsigned kBarStart = 0xffffffffu;
+
 struct PersistArgs {
     FArgs f;
     pgn::ConvArgs conv[pgn::kLayers];
     int smem;                       // dynamic shared memory, bytes
-    unsigned* bar;                  // blocks arrived, over all barriers of the launch (zero at launch)
+    unsigned* bar;                  // kBarStart + blocks arrived, over all barriers of the launch
     int* abort_flag;                // a wait gave up (zero at launch)
     unsigned long long timeout_ns;  // limit of one wait
 };
@@ -1505,12 +1511,12 @@ __device__ __forceinline__ bool grid_barrier(const PersistArgs& a, unsigned& rou
     ahead();
     int bad = 0;
     if (threadIdx.x == blockDim.x - 1) {
-        const unsigned want = round * gridDim.x;
+        const unsigned want = kBarStart + round * gridDim.x;
         unsigned long long t0 = 0;
         for (unsigned spin = 1;; spin++) {
             unsigned v;
             asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(a.bar) : "memory");
-            if (v >= want) break;
+            if ((int)(v - want) >= 0) break;
             if ((spin & 63u) != 0) continue;
             unsigned long long now;
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
@@ -2314,6 +2320,7 @@ void persist_launch(FpcgSolver* S, const pg_options& o, pg_net* n, const int* no
     grid = std::min(grid, sms);
     if (S->bar.n != 2) S->bar.alloc(2);
     S->bar.zero(st);
+    LCK(cudaMemsetAsync(S->bar.p, 0xff, sizeof kBarStart, st));
     pa.bar = S->bar.p;
     pa.abort_flag = reinterpret_cast<int*>(S->bar.p + 1);
     // at least a second: the graph this replaces had no waits to limit, so a
