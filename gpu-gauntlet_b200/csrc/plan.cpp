@@ -35,6 +35,8 @@ std::string validate_header(const pg_problem& p, bool need_rhs) {
     if (!std::isfinite(p.E) || !std::isfinite(p.nu) || !std::isfinite(p.t))
         return "material E, nu, t must be finite";
     if (p.color_count > 0 && (!p.color_offsets || !p.elements_by_color)) return "colouring arrays are NULL";
+    if (p.color_count > 0 && (p.color_offsets[0] != 0 || p.color_offsets[p.color_count] != p.element_count))
+        return "color_offsets must start at 0 and end at element_count";
     return "";
 }
 
@@ -50,8 +52,6 @@ std::string validate_problem(const pg_problem& p, bool need_rhs) {
     for (size_t i = 0; i < ne; i++) top = std::max(top, p.elements[i]);
     if (ne && top >= p.node_count) return "element node index out of range";
     if (p.color_count > 0) {
-        if (p.color_offsets[0] != 0 || p.color_offsets[p.color_count] != p.element_count)
-            return "color_offsets must start at 0 and end at element_count";
         for (uint32_t c = 0; c < p.color_count; c++)
             if (p.color_offsets[c + 1] < p.color_offsets[c]) return "color_offsets must not decrease";
         std::vector<uint8_t> seen(p.element_count, 0);

@@ -412,30 +412,38 @@ pg::SmemLayout make_layout_multi(const pg::HostPlan& hp, bool mixed, bool coarse
     return L;
 }
 
-std::unique_ptr<Plan> build_plan(pg_ctx* c, const pg_problem& p, int G, int rings) {
+// The plan of a problem whose header is checked, made from the plan's own
+// copies of its arrays alone: the caller's are read once.  validate: the copies
+// are checked first (what another thread wrote meanwhile included).
+std::unique_ptr<Plan> build_plan(pg_ctx* c, const pg_problem& theirs, int G, int rings, bool validate = false) {
     auto pl = std::make_unique<Plan>();
-    std::string e = pg::build_structure(p, pl->hp);
+    const size_t tn = theirs.node_count, te = theirs.element_count;
+    pl->h_nodes.assign(theirs.nodes, theirs.nodes + 2 * tn);
+    pl->h_elements.assign(theirs.elements, theirs.elements + theirs.nodes_per_element * te);
+    pl->h_cons.assign(theirs.constrained, theirs.constrained + 3 * tn);
+    if (theirs.elem_t) pl->h_elem_t.assign(theirs.elem_t, theirs.elem_t + te);
+    pl->h_color_count = theirs.color_count;
+    if (theirs.color_count) {
+        pl->h_color_off.assign(theirs.color_offsets, theirs.color_offsets + theirs.color_count + 1);
+        pl->h_by_color.assign(theirs.elements_by_color, theirs.elements_by_color + te);
+    }
+    pg_problem p = theirs;
+    p.nodes = pl->h_nodes.data();
+    p.elements = pl->h_elements.data();
+    p.constrained = pl->h_cons.data();
+    p.elem_t = theirs.elem_t ? pl->h_elem_t.data() : nullptr;
+    p.F = nullptr;
+    p.color_offsets = pl->h_color_off.data();
+    p.elements_by_color = pl->h_by_color.data();
+    std::string e = validate ? pg::validate_problem(p, false) : std::string();
+    if (e.empty()) e = pg::build_structure(p, pl->hp);
     if (e.empty()) e = pg::build_partition(p, G, rings, pl->hp);
     if (!e.empty()) throw Fail{PG_EINVAL, e};
     pl->G = pl->hp.G;
-    pl->h_nodes.assign(p.nodes, p.nodes + 2 * (size_t)p.node_count);
-    pl->h_elements.assign(p.elements, p.elements + (size_t)p.nodes_per_element * p.element_count);
-    pl->h_cons.assign(p.constrained, p.constrained + 3 * (size_t)p.node_count);
     pl->prob_view = p;
-    pl->prob_view.nodes = pl->h_nodes.data();
-    pl->prob_view.elements = pl->h_elements.data();
-    pl->prob_view.constrained = pl->h_cons.data();
-    pl->prob_view.F = nullptr;
     pl->prob_view.color_count = 0;  // a plan rebuilt from the view recolours greedily
     pl->prob_view.color_offsets = nullptr;
     pl->prob_view.elements_by_color = nullptr;
-    if (p.elem_t) pl->h_elem_t.assign(p.elem_t, p.elem_t + (size_t)p.element_count);
-    pl->prob_view.elem_t = p.elem_t ? pl->h_elem_t.data() : nullptr;
-    pl->h_color_count = p.color_count;
-    if (p.color_count) {
-        pl->h_color_off.assign(p.color_offsets, p.color_offsets + p.color_count + 1);
-        pl->h_by_color.assign(p.elements_by_color, p.elements_by_color + p.element_count);
-    }
     pl->E = p.E;
     pl->nu = p.nu;
     pl->t = p.t;
@@ -519,9 +527,7 @@ Plan* get_plan(pg_ctx* c, const pg_problem& p, int G, int rings, bool* cached) {
         }
     }
     *cached = false;
-    std::string e = pg::validate_problem(p, false);
-    if (!e.empty()) throw Fail{PG_EINVAL, e};
-    auto pl = build_plan(c, p, G, rings);
+    auto pl = build_plan(c, p, G, rings, true);
     c->plans.push_front(std::move(pl));
     while (c->plans.size() > kMaxPlans) c->plans.pop_back();
     return c->plans.front().get();

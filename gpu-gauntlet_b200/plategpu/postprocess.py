@@ -19,7 +19,7 @@ from .types import PlateMaterial, PlateMesh
 def computeMoments(mesh: PlateMesh, displacements, material: PlateMaterial, device: int = 0):
     """Nodal bending moments {Mx, My, Mxy} of a displacement vector."""
     from .solver import get_context
-    prob = _lib.Problem(mesh, material, None, copy=False)
+    prob = _lib.Problem(mesh, material, None, copy=not _lib.may_borrow())
     Mx, My, Mxy = get_context(device).moments(prob, np.asarray(displacements, np.float64))
     return {"Mx": Mx.astype(np.float32), "My": My.astype(np.float32), "Mxy": Mxy.astype(np.float32)}
 

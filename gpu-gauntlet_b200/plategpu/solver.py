@@ -92,7 +92,7 @@ def solveGPU(mesh: PlateMesh, material: PlateMaterial, coloring: Optional[Elemen
                                  f"F has {F.size} entries, expected {3 * mesh.nodeCount}")
     opts = _make_options(options)
     ctx = get_context(device)
-    prob = _lib.Problem(mesh, material, coloring, F, _mask(mesh, constrainedDOFs), copy=False)
+    prob = _lib.Problem(mesh, material, coloring, F, _mask(mesh, constrainedDOFs), copy=not _lib.may_borrow())
     x, info = ctx.solve(prob, opts)
     sol = x if options.returnFloat64 else x.astype(np.float32)
     return GPUSolveResult(solution=sol, iterations=int(info.iterations),
@@ -117,7 +117,7 @@ def solveGPULoadCases(mesh: PlateMesh, material: PlateMaterial, coloring: Option
         raise _lib.PlateGPUError(_lib.PG_EINVAL, f"each load needs {3 * mesh.nodeCount} entries")
     opts = _make_options(options)
     ctx = get_context(device)
-    prob = _lib.Problem(mesh, material, coloring, F[0], _mask(mesh, constrainedDOFs), copy=False)
+    prob = _lib.Problem(mesh, material, coloring, F[0], _mask(mesh, constrainedDOFs), copy=not _lib.may_borrow())
     t0 = time.perf_counter()
     X, infos = ctx.solve_load_cases(prob, F, opts, casesPerLaunch)
     ms = (time.perf_counter() - t0) * 1e3
