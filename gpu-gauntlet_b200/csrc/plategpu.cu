@@ -1445,6 +1445,13 @@ void check_header(const pg_problem* p, bool need_rhs) {
     if (!e.empty()) throw Fail{PG_EINVAL, e};
 }
 
+// A problem that is invalid itself is PG_EINVAL, whatever its load.
+void check_load(const pg_problem* p, const float* F, size_t n) {
+    if (pg::finite_f(F, n)) return;
+    check_problem(p, false);
+    throw Fail{PG_ENONFINITE, "F contains NaN or Inf"};
+}
+
 void zero_info(pg_info* info) {
     if (!info) return;
     std::memset(info, 0, sizeof(*info));
@@ -2011,7 +2018,7 @@ int pg_solve(pg_ctx* c, const pg_problem* p, const pg_options* opt, double* x_ou
             return;
         }
         const int G = o.ctas ? std::min(o.ctas, (int)p->node_count) : auto_ctas(c, (int)p->node_count);
-        if (!pg::finite_f(p->F, n)) throw Fail{PG_ENONFINITE, "F contains NaN or Inf"};
+        check_load(p, p->F, n);
         bool cached = false;
         const auto tp = std::chrono::steady_clock::now();
         Plan* pl = get_plan(c, *p, G, halo_rings(o), &cached);
@@ -2041,7 +2048,7 @@ int pg_solve_load_cases(pg_ctx* c, const pg_problem* p, int count, const float* 
         fill_options(opt, &o);
         const size_t n = 3 * (size_t)p->node_count;
         if (n && !x_out) throw Fail{PG_EINVAL, "x_out is NULL"};
-        if (!pg::finite_f(F, n * count)) throw Fail{PG_ENONFINITE, "F contains NaN or Inf"};
+        check_load(p, F, n * count);
         if (n == 0) {
             check_problem(p, false);
             if (infos)
