@@ -22,7 +22,9 @@
 #include "coarse.cuh"
 #include "internal.h"
 #include "kernels.cuh"
+#include "launch.h"
 #include "multi.cuh"
+#include "setup.cuh"
 #include "plan.h"
 #include "plategpu.h"
 
@@ -970,30 +972,11 @@ void opt_in_smem(pg_ctx* c, const void* fn) {
     }
 }
 
-template <typename T, bool MIXED, int MAXT>
-const void* solve_kernel_of(bool coarse, bool cheb) {
-    if (coarse)
-        return cheb ? (const void*)pg::pcg_kernel<T, MIXED, MAXT, true, true>
-                    : (const void*)pg::pcg_kernel<T, MIXED, MAXT, true, false>;
-    return cheb ? (const void*)pg::pcg_kernel<T, MIXED, MAXT, false, true>
-                : (const void*)pg::pcg_kernel<T, MIXED, MAXT, false, false>;
-}
-
 const void* solve_kernel(const pg_options& o, bool lean) {
     const bool coarse = o.preconditioner == PG_PRECOND_TWO_LEVEL, cheb = o.smoother == PG_SMOOTHER_CHEBYSHEV;
-    constexpr int LT = pg::kLeanThreads, MT = pg::kMaxThreads;
-    if (o.precision == PG_PREC_MIXED)
-        return lean ? solve_kernel_of<float, true, LT>(coarse, cheb) : solve_kernel_of<float, true, MT>(coarse, cheb);
-    return lean ? solve_kernel_of<double, false, LT>(coarse, cheb) : solve_kernel_of<double, false, MT>(coarse, cheb);
-}
-
-template <typename T, bool MIXED>
-const void* batch_kernel_of(bool coarse, bool cheb) {
-    if (coarse)
-        return cheb ? (const void*)pg::pcg_batch_kernel<T, MIXED, true, true>
-                    : (const void*)pg::pcg_batch_kernel<T, MIXED, true, false>;
-    return cheb ? (const void*)pg::pcg_batch_kernel<T, MIXED, false, true>
-                : (const void*)pg::pcg_batch_kernel<T, MIXED, false, false>;
+    const bool mixed = o.precision == PG_PREC_MIXED;
+    if (!lean) return pgi::pcg_wide_kernel(mixed, coarse, cheb);
+    return mixed ? pgi::pcg32_kernel(coarse, cheb) : pgi::pcg64_kernel(coarse, cheb);
 }
 
 // Queues set-up (first solve of the plan) and the persistent PCG launch on
@@ -1286,12 +1269,6 @@ bool choose_layout_multi(pg_ctx* c, const pg::HostPlan& hp, const pg_options& o,
     return false;
 }
 
-const void* multi_kernel(bool mixed, int NR) {
-    if (NR == 2)
-        return mixed ? (const void*)pg::pcg_multi_kernel<float, true, 2> : (const void*)pg::pcg_multi_kernel<double, false, 2>;
-    return mixed ? (const void*)pg::pcg_multi_kernel<float, true, 4> : (const void*)pg::pcg_multi_kernel<double, false, 4>;
-}
-
 // count <= NR load cases of plan pl in one launch of the NR-case kernel
 // (cases count..NR-1 get a zero load and stop at once).  F[k] / x[k] are
 // host vectors of 3 Nn; infos (optional) gets one record per case.  Cases
@@ -1350,7 +1327,7 @@ void run_solve_multi(pg_ctx* c, Plan* pl, const pg_options& o, int NR, int count
     a.llp = pl->mllp.p;
     a.tag0 = pl->m_tag0;
     a.trace_it = -1;
-    const void* fn = multi_kernel(mixed, NR);
+    const void* fn = mixed ? pgi::multi32_kernel(NR) : pgi::multi64_kernel(NR);
     opt_in_smem(c, fn);
     if (pl->m_ok_fn != fn || pl->m_ok_smem != L.total) {
         int nb = 0;
@@ -1663,7 +1640,7 @@ void run_batch(pg_batch* b, const pg_options& o, const float* const* F, double* 
     const unsigned long long claim_timeout_ns = (unsigned long long)(o.wait_timeout_ms * 1e6);
     const bool mixed = o.precision == PG_PREC_MIXED;
     const bool coarse = o.preconditioner == PG_PRECOND_TWO_LEVEL, cheb = o.smoother == PG_SMOOTHER_CHEBYSHEV;
-    const void* const fn = mixed ? batch_kernel_of<float, true>(coarse, cheb) : batch_kernel_of<double, false>(coarse, cheb);
+    const void* const fn = mixed ? pgi::batch32_kernel(coarse, cheb) : pgi::batch64_kernel(coarse, cheb);
     const int prec_key = (mixed ? 1 : 2) + (coarse ? 4 : 0) + (cheb ? 8 : 0);
     int grid_max = 0;
     for (auto& ph : b->phases) grid_max = std::max(grid_max, ph->grid);

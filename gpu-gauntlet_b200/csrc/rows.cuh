@@ -47,98 +47,6 @@ constexpr int kRowGroup = 10;   // rows per group (3 lanes each: 30 of a warp's 
 constexpr int kRowLanes = 30;
 constexpr int kRegSteps = 3;    // q-steps of a resident group kept in registers
 
-// Local index of global node m in a part: three runs of ascending node ids,
-// the owned nodes [0, no), ring 1 [no, n1) and the rest [n1, nloc) (one halo
-// ring: n1 = no).
-__device__ __forceinline__ int local_index(const int* __restrict__ nodes, int no, int n1, int nloc, int m) {
-    const int seg[4] = {0, no, n1, nloc};
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        int lo = seg[k], hi = seg[k + 1];
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (nodes[mid] < m) lo = mid + 1;
-            else hi = mid;
-        }
-        if (lo < seg[k + 1] && nodes[lo] == m) return lo;
-    }
-    return 0;
-}
-
-// Columns and blocks of every part's rows from the element matrices: one
-// thread per (row, slot residue), blockIdx.x the part, blockIdx.y a share of
-// its groups.
-template <int NPE>
-__global__ void row_fill_kernel(const int* __restrict__ node_off, const int* __restrict__ nown,
-                                const int* __restrict__ n1, const int* __restrict__ nodes,
-                                const int* __restrict__ grp_off, const int* __restrict__ grp_q,
-                                const int* __restrict__ inc_ptr, const int* __restrict__ inc_idx,
-                                const uint32_t* __restrict__ elements, const double* __restrict__ ke64,
-                                uint16_t* __restrict__ rcol, double* __restrict__ rk64,
-                                float* __restrict__ rk32) {
-    constexpr int ND = 3 * NPE;
-    const int g = blockIdx.x, n0 = node_off[g], nloc = node_off[g + 1] - n0, no = nown[g], nn1 = n1[g];
-    const int gb = grp_off[g], ng = grp_off[g + 1] - gb;
-    const int* pn = nodes + n0;
-    for (int t = blockIdx.y * blockDim.x + threadIdx.x; t < ng * kRowLanes; t += gridDim.y * blockDim.x) {
-        const int grp = t / kRowLanes, lane = t - grp * kRowLanes, i = grp * kRowGroup + lane / 3, d = lane % 3;
-        const int q0 = grp_q[gb + grp], q1 = grp_q[gb + grp + 1];
-        int q = q0;
-        if (i < nn1) {
-            const int n = pn[i], a = inc_ptr[n], b = inc_ptr[n + 1];
-            int prev = -1;
-            for (int j = 0;; j++) {
-                // the next node id of the row: the smallest above the last
-                int m = 0x7fffffff;
-                for (int k = a; k < b; k++) {
-                    const uint32_t* en = elements + (size_t)(inc_idx[k] >> 2) * NPE;
-#pragma unroll
-                    for (int p = 0; p < NPE; p++) {
-                        const int v = (int)en[p];
-                        if (v > prev && v < m) m = v;
-                    }
-                }
-                if (m == 0x7fffffff) break;
-                prev = m;
-                if (j % 3 != d) continue;
-                double blk[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-                for (int k = a; k < b; k++) {
-                    const int e = inc_idx[k] >> 2;
-                    const double* K = ke64 + (size_t)e * ND * ND + 3 * (inc_idx[k] & 3) * ND;
-#pragma unroll
-                    for (int p = 0; p < NPE; p++)
-                        if ((int)elements[(size_t)e * NPE + p] == m)
-#pragma unroll
-                            for (int r = 0; r < 9; r++) blk[r] += K[(r / 3) * ND + 3 * p + r % 3];
-                }
-                rcol[(size_t)q * kRowLanes + lane] = (uint16_t)local_index(pn, no, nn1, nloc, m);
-#pragma unroll
-                for (int r = 0; r < 9; r++) {
-                    const size_t o = ((size_t)q * 9 + r) * kRowLanes + lane;
-                    rk64[o] = blk[r];
-                    rk32[o] = (float)blk[r];
-                }
-                q++;
-            }
-        }
-        for (; q < q1; q++) {  // padding: a zero block on the row itself
-            rcol[(size_t)q * kRowLanes + lane] = (uint16_t)(i < nn1 ? i : 0);
-            for (int r = 0; r < 9; r++) {
-                const size_t o = ((size_t)q * 9 + r) * kRowLanes + lane;
-                rk64[o] = 0.0;
-                rk32[o] = 0.0f;
-            }
-        }
-    }
-}
-
-// shared[n] = 1 for every node that is a ghost of some part.
-__global__ void mark_ghosts_kernel(const int* __restrict__ node_off, const int* __restrict__ nown,
-                                   const int* __restrict__ nodes, uint8_t* __restrict__ shared) {
-    const int g = blockIdx.x;
-    for (int i = node_off[g] + nown[g] + threadIdx.x; i < node_off[g + 1]; i += blockDim.x) shared[nodes[i]] = 1;
-}
-
 // s += the blocks k[9 (q - qa) ..][lane] of q-steps [qa, qb) times u at the
 // columns c[q - qa][lane], its w less w0 (0, or the row's own w; FP32 only).
 template <typename T>
