@@ -475,7 +475,7 @@ std::string build_coarse_meta(const pg_problem& p, HostPlan& plan) {
 
 std::string schedule_batch(const std::vector<int>& nodes, const std::vector<int>& caps, int sms, BatchSchedule& out,
                            int part_nodes) {
-    const double target = part_nodes > 0 ? part_nodes : 400.0;
+    const double target = part_nodes;
     out = BatchSchedule{};
     const int count = (int)nodes.size();
     if (count == 0) return "empty batch";

@@ -96,8 +96,8 @@ std::string build_coarse_meta(const pg_problem& p, HostPlan& plan);
 // Team schedule of a batch of independent plates.  A plate of n nodes gets
 // a team of d blocks: a power of two, or every block of the device for the
 // largest plates, with at most caps[i] nodes per block (so its parts fit in
-// shared memory) and about part_nodes nodes per block otherwise (the caller's preference).  Team sizes that fit side by side form a
-// phase, one persistent launch; inside a phase the blocks are shared out
+// shared memory) and about part_nodes nodes per block otherwise (the caller's
+// preference).  Team sizes that fit side by side form a phase, one persistent launch; inside a phase the blocks are shared out
 // among the team sizes in proportion to their estimated work (sqrt(n)
 // iterations of n + 300 d node-equivalents), one team per size at least,
 // and each size's plates go to its teams longest first to the least-loaded
@@ -122,6 +122,6 @@ struct BatchSchedule {
     std::vector<int> plate_phase, plate_team, plate_size;  // [count]; team index within its phase
 };
 std::string schedule_batch(const std::vector<int>& nodes, const std::vector<int>& caps, int sms, BatchSchedule& out,
-                           int part_nodes = 400);
+                           int part_nodes);
 
 }  // namespace pg

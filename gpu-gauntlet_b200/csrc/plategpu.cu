@@ -2340,8 +2340,7 @@ int pg_batch_schedule(const uint32_t* node_counts, int count, int sms, int cap, 
     try {
         std::vector<int> nodes(node_counts, node_counts + count);
         pg::BatchSchedule S;
-        if (!pg::schedule_batch(nodes, std::vector<int>(count, cap), sms, S).empty())
-            return PG_EUNSUPPORTED;
+        if (!pg::schedule_batch(nodes, std::vector<int>(count, cap), sms, S, 400).empty()) return PG_EUNSUPPORTED;
         for (int i = 0; i < count; i++) {
             plate_phase[i] = S.plate_phase[i];
             plate_size[i] = S.plate_size[i];

@@ -310,10 +310,11 @@ void pg_batch_destroy(pg_batch* batch);
 /* pg_batch_create + pg_batch_solve + pg_batch_destroy in one call. */
 int pg_solve_batch(pg_ctx* ctx, const pg_problem* probs, int count, const pg_options* opt,
                    double* const* x_out, pg_info* infos, pg_batch_info* info);
-/* Host-only: the schedule pg_batch_create uses for plates of these node
- * counts on `sms` blocks with at most `cap` nodes per block: per plate its
- * phase, team size and predicted team (index within the phase) [count
- * each]; per phase its grid [count, the first *phases_out entries used].
+/* Host-only: the schedule pg_batch_create makes with batch_part_nodes = 400
+ * (its own default prefers smaller parts) for plates of these node counts on
+ * `sms` blocks with at most `cap` nodes per block: per plate its phase,
+ * team size and predicted team (index within the phase) [count each]; per
+ * phase its grid [count, the first *phases_out entries used].
  * At run time the teams of one size share one queue of their plates
  * (largest estimated work first) and a free team takes the next one, so
  * the team that solves a plate can differ from the prediction. */
