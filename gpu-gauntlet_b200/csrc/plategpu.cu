@@ -1466,10 +1466,14 @@ pg_options plate_options(const pg_options& o, const Plan* pl) {
     return oi;
 }
 
-// Whether a batch plate on a 2-ring halo keeps the Chebyshev smoother: its
-// vectors (24 words a local node), 3 words and npe column ids per element
-// incidence of its rows, and x must fit shared memory.  A larger part would
-// read most of its row blocks from L2 twice an iteration (K u and K t).
+// Whether a batch plate on a 2-ring halo keeps the Chebyshev smoother: up to
+// the size at which the element-task layout (24 words a local node, 3 words and
+// npe column ids per element incidence of its rows, x) filled shared memory.  The
+// row blocks need less, but which plates of a batch run with which smoother is
+// part of what callers see (pg_info.smoother_lambda_max) and stays.  It costs a
+// little between the two limits: one FP64 two-level plate of 272 and 280
+// elements a side 7.47 and 6.98 ms without the smoother, 6.55 and 6.68 with it;
+// mixed, 340 to 370 a side, 10.7 to 13.5 against 10.3 to 12.7.
 bool smoother_halo_fits(const pg_ctx* c, const pg::HostPlan& hp, const pg_options& o) {
     const size_t T = o.precision == PG_PREC_MIXED ? 4 : 8;
     const size_t nloc = hp.max_nloc, inc = hp.max_ntask;
