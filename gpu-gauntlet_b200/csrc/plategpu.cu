@@ -914,13 +914,17 @@ pg::PcgArgs fill_args(Plan* pl, const pg_options& o, const pg::SmemLayout& L, bo
     // whose FP32 residual stalls along with the true one is still checked
     // (with the coarse space after 50: its FP32 recurrence drifts sooner, and with
     // reliable_delta = 0.01 the 60k-DOF plate stagnated at 200, 1.2 -> 6.2 ms).
-    // Either gives up after 600 updates without halving the true residual, or
-    // three replacements that the FP32 residual asked for: a thin clamped plate's
-    // residual may stay flat for some hundred updates and then fall.
+    // Given up after three replacements without halving the true residual, with
+    // the interval of 50 six that the interval brought (300 updates): a thin
+    // plate's residual may stay flat for some hundred updates and then fall.  Of
+    // 316 solves of random plates (thickness 0.01 to 0.3 on 10 m) 172 converged at
+    // interval 200 with three; at 50 with 3, 5, 6, 8, 12 of them 162, 172, 172, 172,
+    // 172 and 247, 275, 276, 277, 282 in all, the rest stalling after 37, 40, 47,
+    // 64, 58 thousand updates together.
     const bool often = o.reliable_interval <= 0 && o.preconditioner == PG_PRECOND_TWO_LEVEL;
     a.reliable_interval = o.reliable_interval > 0 ? o.reliable_interval : often ? 50 : 200;
     a.reliable_delta = o.reliable_delta > 0 ? o.reliable_delta : 0.1;
-    a.stall_step = often ? 4 : 1;
+    a.stall_step = often ? 2 : 1;
     a.stall_limit = 3 * a.stall_step;
     a.L = L;
     return a;

@@ -92,7 +92,8 @@ typedef enum pg_stop_reason {
     PG_STOP_BREAKDOWN = 2, /* |p.Ap| < 1e-30 (pcg.ts:154, gpu/solver.ts:496) */
     PG_STOP_ZERO_RHS = 3,  /* ||b|| < 1e-30: x = 0, 0 iterations */
     PG_STOP_STAGNATED = 4  /* mixed precision: the FP64 residual did not halve over three
-                              residual replacements (FP32 cannot resolve the problem);
+                              residual replacements, six where the automatic interval
+                              of 50 brought them (FP32 cannot resolve the problem);
                               with pg_options.fallback the call re-solves in FP64 */
 } pg_stop_reason;
 
@@ -142,8 +143,8 @@ typedef struct pg_options {
                                      stopped by the same rule on x_m + d; 0 returns the
                                      stagnated result */
     int32_t batch_part_nodes;     /* batches: preferred nodes per block of a plate's team
-                                     (0 = automatic: 100 for up to 32 plates, else 160); plategpu.autotune picks it per
-                                     GPU and batch */
+                                     (0 = automatic: 100 for up to 32 plates, else 160);
+                                     plategpu.autotune picks it per GPU and batch */
 } pg_options;
 
 /* Per-solve result (GPUSolveResult plus extended statistics). */
@@ -523,10 +524,13 @@ typedef struct pg_learned_stats {
  * and alpha/beta; the stop test (opt: tolerance, max_iterations,
  * stop_rule) is made on the FP64 true residual F - K x, which also
  * replaces the recursive residual every 50 iterations.  The whole solve is
- * one CUDA graph launch (a conditional WHILE node).
+ * one launch: with the network on a grid of up to about 272 x 272 pixels a
+ * persistent kernel, whose blocks wait for one another (opt->wait_timeout_ms
+ * limits each wait, values below 1000 counting as 1000: PG_ETIMEOUT), else a
+ * CUDA graph (a conditional WHILE node).
  * _device: F_dev / x_dev device [3n] float / double; otherwise host buffers
- * (copies included).  info->solve_ms is the graph's device time.  With
- * opt->phase_timing the iterations run without the graph, one launch at a
+ * (copies included).  info->solve_ms is the launch's device time.  With
+ * opt->phase_timing the iterations run as separate kernels, one launch at a
  * time with the host checking the stop flag after each, and
  * info->phase_us[0..7] receives the average device time per iteration of:
  * update; true residual; smoothing and network input; network; K y and the

@@ -1,7 +1,7 @@
 """How long a mixed two-level solve keeps going while its FP64 residual is flat: with the automatic interval of 50
-updates, as long as with the 200 of block Jacobi (600 updates).  These thin plates' residuals stay flat for more than
-150 updates and then fall below the tolerance; each must converge without the FP64 correction, by one load and by load
-cases in lockstep.  Three replacements at a caller's own interval of 50 still end the solve."""
+updates, for 300.  These thin plates' residuals stay flat for more than 150 updates and then fall below the tolerance;
+each must converge without the FP64 correction, by one load and by load cases in lockstep.  Three replacements at a
+caller's own interval of 50 still end the solve."""
 import numpy as np
 import pytest
 
