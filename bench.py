@@ -23,6 +23,8 @@ Every variant's FP64 error is checked on the plate's own load and 16
 seeded random-field loads; only a variant whose largest error is <= 1e-6
 can be the headline.
 
+The whole line goes to stderr; stdout gets it with its sections cut to
+their main numbers (summary), so that it survives in the tail of a log.
 Further sections of the line: ``learned`` (the learned two-level
 preconditioner: flexible PCG with the trained U-Net, one CUDA graph per
 solve; timed like the variants, checked on the same loads, evaluated on
@@ -665,7 +667,8 @@ def run_plategpu(args, world, rank, local):
                        "of solvePCG/applyGlobalK, single thread")}
     else:
         line["cpu_baseline"] = None
-    print(json.dumps(line), flush=True)
+    print(json.dumps(line), file=sys.stderr, flush=True)
+    print(json.dumps(summary(line)), flush=True)
     ctx.close()
 
 
@@ -673,6 +676,43 @@ def run_plategpu(args, world, rank, local):
 # loop without the network: at 1e-6 one of the 512 held-out loads ended at
 # 1.02e-6 FP64 error; 5e-7 keeps every load under the 1e-6 bar
 LEARNED_TOL = 5e-7
+
+
+SECTIONS = ("variants", "load_cases", "learned", "other_configs", "batch", "first_solve_new_mesh_split",
+            "first_solve_new_mesh_phases", "roofline", "method", "accuracy", "cpu_baseline")
+
+
+def scalars(d, depth=0):
+    """d's numbers (five digits) and short texts; `depth` levels of nested dicts likewise, lists left out."""
+    out = {}
+    for k, v in d.items():
+        if isinstance(v, float):
+            out[k] = float(f"{v:.5g}")
+        elif isinstance(v, dict) and depth:
+            out[k] = scalars(v, depth - 1)
+        elif v is None or isinstance(v, (bool, int)) or (isinstance(v, str) and len(v) <= 60):
+            out[k] = v
+    return out
+
+
+def summary(line):
+    """The line with its sections cut to what fits a log's tail (about 4 KB); the whole of it goes to stderr."""
+    out = {k: v for k, v in line.items() if k not in SECTIONS}
+    out["variants"] = {v: scalars({"ms": r["value"], "iterations": r["iterations"],
+                                   "rel_l2_max": ((r.get("accuracy") or {}).get("loads") or {}).get("rel_l2_max")})
+                       for v, r in line.get("variants", {}).items()}
+    for k in ("roofline", "method", "load_cases", "batch"):
+        if line.get(k):
+            out[k] = scalars(line[k])
+    if line.get("learned"):
+        out["learned"] = scalars(line["learned"])
+        out["learned"]["held_out"] = scalars(line["learned"].get("held_out") or {})
+    out["other_configs"] = {n: scalars({k: r[k] for k in ("best", "best_ms") if k in r})
+                            for n, r in (line.get("other_configs") or {}).items()}
+    out["first_solve_new_mesh_phases"] = scalars(line.get("first_solve_new_mesh_phases") or {})
+    out["accuracy"] = scalars(line.get("accuracy") or {}, 1) or None
+    out["cpu_baseline"] = scalars(line["cpu_baseline"]) if line.get("cpu_baseline") else None
+    return out
 
 
 def learned_bench(args, ctx, stream, flush, local, wl, chk, extra_F):
