@@ -668,7 +668,7 @@ def run_plategpu(args, world, rank, local):
     else:
         line["cpu_baseline"] = None
     print(json.dumps(line), file=sys.stderr, flush=True)
-    print(json.dumps(summary(line)), flush=True)
+    print(json.dumps(summary(line), separators=(",", ":")), flush=True)
     ctx.close()
 
 
@@ -678,40 +678,30 @@ def run_plategpu(args, world, rank, local):
 LEARNED_TOL = 5e-7
 
 
-SECTIONS = ("variants", "load_cases", "learned", "other_configs", "batch", "first_solve_new_mesh_split",
+SECTIONS = ("config", "variants", "load_cases", "learned", "other_configs", "batch", "first_solve_new_mesh_split",
             "first_solve_new_mesh_phases", "roofline", "method", "accuracy", "cpu_baseline")
 
 
-def scalars(d, depth=0):
-    """d's numbers (five digits) and short texts; `depth` levels of nested dicts likewise, lists left out."""
-    out = {}
-    for k, v in d.items():
-        if isinstance(v, float):
-            out[k] = float(f"{v:.5g}")
-        elif isinstance(v, dict) and depth:
-            out[k] = scalars(v, depth - 1)
-        elif v is None or isinstance(v, (bool, int)) or (isinstance(v, str) and len(v) <= 60):
-            out[k] = v
-    return out
+def pick(d, *keys):
+    """Those of `keys` that d has (d may be None), floats to five digits."""
+    return {k: float(f"{d[k]:.5g}") if isinstance(d[k], float) else d[k] for k in keys if d and k in d}
 
 
 def summary(line):
-    """The line with its sections cut to what fits a log's tail (about 4 KB); the whole of it goes to stderr."""
+    """The line with its sections cut to their main numbers, under 2.5 KB, which survives in the tail of a log; the
+    whole of it goes to stderr."""
     out = {k: v for k, v in line.items() if k not in SECTIONS}
-    out["variants"] = {v: scalars({"ms": r["value"], "iterations": r["iterations"],
-                                   "rel_l2_max": ((r.get("accuracy") or {}).get("loads") or {}).get("rel_l2_max")})
-                       for v, r in line.get("variants", {}).items()}
-    for k in ("roofline", "method", "load_cases", "batch"):
-        if line.get(k):
-            out[k] = scalars(line[k])
-    if line.get("learned"):
-        out["learned"] = scalars(line["learned"])
-        out["learned"]["held_out"] = scalars(line["learned"].get("held_out") or {})
-    out["other_configs"] = {n: scalars({k: r[k] for k in ("best", "best_ms") if k in r})
-                            for n, r in (line.get("other_configs") or {}).items()}
-    out["first_solve_new_mesh_phases"] = scalars(line.get("first_solve_new_mesh_phases") or {})
-    out["accuracy"] = scalars(line.get("accuracy") or {}, 1) or None
-    out["cpu_baseline"] = scalars(line["cpu_baseline"]) if line.get("cpu_baseline") else None
+    out["config"] = {k: v for k, v in line["config"].items() if not (isinstance(v, str) and len(v) > 60)}
+    out["variants_ms"] = {v: float(f"{r['value']:.5g}") for v, r in line.get("variants", {}).items()}
+    out["method"] = line["method"]["name"]
+    out["rel_l2_max"] = ((line.get("accuracy") or {}).get("loads") or {}).get("rel_l2_max")
+    out["roofline"] = pick(line.get("roofline"), "bound", "achieved", "peak", "unit", "frac")
+    for name, keys in (("load_cases", ("cases", "device_ms_per_case", "e2e_ms_per_case", "speedup_e2e")),
+                       ("learned", ("value", "iterations", "us_per_iteration")),
+                       ("batch", ("method", "batch_ms", "solves_per_s", "plate_ms_p99", "max_rel_l2_vs_fp64_truth")),
+                       ("cpu_baseline", ("value", "unit", "cores", "kind"))):
+        out[name] = pick(line.get(name), *keys) or None
+    out["other_configs_ms"] = {n: pick(r, "best_ms").get("best_ms") for n, r in (line.get("other_configs") or {}).items()}
     return out
 
 

@@ -15,7 +15,7 @@ def full_line():
            "reliable_updates": 3, "tolerance": 5e-6, "true_rel_residual": 4.9e-6, "coarse_dim": 444, "accuracy": acc}
     return {"metric": bench.METRIC, "value": 1.2, "unit": "ms", "n_gpus": 1, "steps": 20, "warmup": 5,
             "ms_per_step": 1.2, "higher_is_better": False, "scaling": "weak", "vs_baseline": None,
-            "dtype": "f32 inner / f64 refinement", "data": "synthetic", "config": {"model": "plate", "l2": "y" * 150},
+            "dtype": "f32 inner / f64 refinement", "data": "synthetic", "config": {"workload": "plate", "dof": 60492, "l2": "flushed between steps", "note": "y" * 150},
             "method": {"name": "mixed_two_level_cheb", "preconditioner": "z" * 90, "ctas": 148},
             "variants": {f"variant_{i}": dict(row) for i in range(7)},
             "roofline": {"achieved": 1.0, "frac": 0.1, "l2": {"peak": 2.0, "peak_source": "w" * 150}},
@@ -33,16 +33,17 @@ def test_summary_keeps_the_contract_and_fits():
     line = full_line()
     short = json.loads(json.dumps(bench.summary(line)))
     for k in ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
-              "vs_baseline", "dtype", "data", "config", "e2e", "gpu_launches", "clocks"):
+              "vs_baseline", "dtype", "data", "e2e", "gpu_launches", "clocks"):
         assert short[k] == line[k], k
-    assert len(json.dumps(short)) < 4000
-    assert short["variants"]["variant_3"] == {"ms": 1.2346, "iterations": 187, "rel_l2_max": 9.8765e-7}
-    assert short["batch"]["batch_ms"] == 260.0 and short["learned"]["held_out"]["loads"] == 512
-    assert short["accuracy"]["loads"]["count"] == 17
+    assert short["config"] == {"workload": "plate", "dof": 60492, "l2": "flushed between steps"}
+    assert len(json.dumps(short)) < 2500
+    assert short["variants_ms"]["variant_3"] == 1.2346 and short["method"] == "mixed_two_level_cheb"
+    assert short["batch"]["batch_ms"] == 260.0 and short["learned"]["value"] == 40.0
+    assert short["rel_l2_max"] == 9.87654321e-7 and short["other_configs_ms"]["c2"] == 1.0
 
 
 def test_summary_without_sections():
     line = {k: v for k, v in full_line().items()
             if k not in ("load_cases", "learned", "other_configs", "batch", "accuracy", "cpu_baseline")}
     short = bench.summary(line)
-    assert short["accuracy"] is None and short["cpu_baseline"] is None and short["other_configs"] == {}
+    assert short["rel_l2_max"] is None and short["cpu_baseline"] is None and short["other_configs_ms"] == {}
