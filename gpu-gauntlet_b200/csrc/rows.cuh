@@ -35,8 +35,8 @@
 // almost exact, and its error there is 1.0e-3.  Cost, a load and three
 // subtractions a lane, at equal iterations on the 60k-DOF plate (ms on the
 // device): block Jacobi 4.64 -> 4.73, with the smoother 3.28 -> 3.43, two-level
-// Chebyshev 1.26 -> 1.30; the 256-plate batch in mixed precision stagnates on 5
-// plates instead of 71.  FP64 rows keep the plain form, FP64 has the
+// Chebyshev 1.26 -> 1.30.  It returns elsewhere: of the 256-plate batch in mixed
+// precision 44 plates stagnated (element form 71), now 3 to 5.  FP64 rows keep the plain form, FP64 has the
 // digits; so do DKT rows: the reference's element, which this one restates, does
 // have stiffness in a translation (and few iterations).
 #pragma once
