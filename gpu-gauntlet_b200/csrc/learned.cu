@@ -2641,6 +2641,15 @@ void pg_learned_destroy(pg_learned* L) {
     delete L;
 }
 
+namespace {
+
+// The context's own stream does not wait for the legacy default stream, on which a
+// host program's tensors are usually written; these calls wait for the device
+// themselves, so they let its earlier work finish first.
+void wait_default_stream() { LCK(cudaStreamSynchronize(cudaStreamLegacy)); }
+
+}  // namespace
+
 int pg_learned_make_pairs(pg_learned* L, int count, const float* F_dev, const double* xstar_dev,
                           const double* xk_dev, float* R_out, float* E_out) {
     if (!L) return PG_EINVAL;
@@ -2648,6 +2657,7 @@ int pg_learned_make_pairs(pg_learned* L, int count, const float* F_dev, const do
         if (count < 0 || (count > 0 && (!F_dev || !xstar_dev || !R_out || !E_out)))
             throw LFail{PG_EINVAL, "NULL buffer"};
         if (count == 0) return;
+        wait_default_stream();
         cudaStream_t st = pgi::ctx_stream(L->ctx);
         dim3 grid(grid_nodes1(L->op.Nn), count);
         if (L->ov.npe == 4)
@@ -2665,6 +2675,7 @@ namespace {
 // set_scales, the network's input / output scales become 1 / rms(r1_c)
 // and rms(e1_c) over the pairs.
 void load_pairs(pg_learned* L, int count, const float* R, const float* E, bool set_scales) {
+    wait_default_stream();
     pg_net* n = L->net;
     cudaStream_t st = pgi::ctx_stream(L->ctx);
     dim3 grid(grid_nodes1(L->op.Nn), count);

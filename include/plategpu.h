@@ -448,7 +448,9 @@ void pg_learned_destroy(pg_learned* learned);
 /* Residual/error pairs from solver output, on the device: for each of
  * `count` loads, r = F - K x_k (FP64 K) and e = x* - x_k, with x_k = 0 when
  * xk_dev is NULL.  F_dev [count][3n] float, xstar_dev / xk_dev [count][3n]
- * double, R_out / E_out [count][3n] float. */
+ * double, R_out / E_out [count][3n] float.  Here and in pg_learned_train and
+ * pg_learned_loss, earlier work on the legacy default stream is waited for
+ * (device arrays written on another stream are the caller's to order). */
 int pg_learned_make_pairs(pg_learned* learned, int count, const float* F_dev, const double* xstar_dev,
                           const double* xk_dev, float* R_out, float* E_out);
 
